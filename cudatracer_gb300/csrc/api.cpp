@@ -298,6 +298,7 @@ ct_status finish_bvh(ct_ctx* ctx, const ct_scene* scene, ct_bvh* b) {
   b->dev.prim_count = (uint32_t)b->host.prims.size();
   b->dev.node_count = (uint32_t)b->host.quad.size();
   b->dev.stack_entries = b->layout.stack_entries;
+  b->dev.odd = b->layout.odd ? 1 : 0;
   b->nt = scene->nt;
   const auto t1 = std::chrono::high_resolution_clock::now();
   ct_bvh_info& i = b->info;
@@ -652,7 +653,7 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   void* prims = nullptr;
   if ((s = dev_alloc(ctx, b->allocs, &quad, (size_t)r.quad_nodes * sizeof(QuadNode))) != CT_OK) return cleanup(s);
   if ((s = dev_alloc(ctx, b->allocs, &nodes, (size_t)r.quad_nodes * sizeof(QNodeDev))) != CT_OK) return cleanup(s);
-  if ((s = dev_alloc(ctx, b->allocs, &tris, (size_t)n * 3 * sizeof(float4))) != CT_OK) return cleanup(s);
+  if ((s = dev_alloc(ctx, b->allocs, &tris, tri_array_bytes(n))) != CT_OK) return cleanup(s);
   if ((s = dev_alloc(ctx, b->allocs, &prims, (size_t)n * 4)) != CT_OK) return cleanup(s);
   e = fast ? gpu_fbvh_emit(scene->dev, scratch, r, shift, quad, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st)
            : gpu_bvh_emit(scene->dev, scratch, r, shift, quad, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st);

@@ -512,18 +512,20 @@ std::string to_device_layout(const HostBVH& h, const float* verts, const uint32_
       }
     }
     d.child = make_int4(ref[0], ref[1], ref[2], ref[3]);
+    for (const float* p : {s.bminx, s.bmaxx, s.bminy, s.bmaxy, s.bminz, s.bmaxz})
+      for (int c = 0; c < 4; c++) out.odd = out.odd || !std::isfinite(p[c]);
     std::memcpy(out.nodes.data() + i * sizeof(QNodeDev), &d, sizeof(d));
   }
   out.depth = depth;
   // every inner level can leave three siblings on the stack
   out.stack_entries = (int32_t)std::min<uint32_t>(3 * depth + 1, 256);
-  out.tris.assign(12 * (size_t)np, 0.0f);
+  out.tris.assign(tri_array_bytes(np) / sizeof(float), 0.0f);
   for (uint32_t j = 0; j < np; j++) {
     const uint32_t p = h.prims[j];
     const float* p0 = verts + 3 * (size_t)idx[3 * (size_t)p];
     const float* p1 = verts + 3 * (size_t)idx[3 * (size_t)p + 1];
     const float* p2 = verts + 3 * (size_t)idx[3 * (size_t)p + 2];
-    float* o = out.tris.data() + 12 * (size_t)j;
+    float* o = out.tris.data() + 4 * kTriFloat4 * (size_t)j;
     o[0] = p0[0], o[1] = p0[1], o[2] = p0[2];
     std::memcpy(&o[3], &p, 4);
     o[4] = p1[0] - p0[0], o[5] = p1[1] - p0[1], o[6] = p1[2] - p0[2], o[7] = 0.0f;

@@ -49,7 +49,8 @@ std::string validate_binary(const std::vector<BinNode>& b, uint32_t prim_count);
 
 struct DeviceLayout {
   std::vector<uint8_t> nodes;  // QNodeDev records
-  std::vector<float> tris;     // 12 floats per leaf slot
+  std::vector<float> tris;     // 4 * kTriFloat4 floats per leaf slot, and one slot more
+  bool odd = false;            // a plane of the tree is not finite
   uint32_t leaf_shift = 0, first_mask = 0, count_mask = 0;
   uint32_t depth = 0, max_leaf = 0;
   int32_t stack_entries = 0;

@@ -12,7 +12,7 @@ namespace ct {
 // Device data layout (all arrays in HBM, 16-byte vector loads)
 // ---------------------------------------------------------------------------
 
-// Quad-BVH node: 128 bytes, 128-byte aligned, read as eight LDG.128. Bounds are
+// Quad-BVH node: 128 bytes, 128-byte aligned, read with four 32-byte loads. Bounds are
 // the reference MBVHNode planes bit for bit (src/BVH/MBVHNode.cuh:35-60) so the
 // slab test and its child order reproduce the reference; children are packed
 // 32-bit references:
@@ -27,9 +27,14 @@ struct __align__(128) QNodeDev {
 static_assert(sizeof(QNodeDev) == 128, "QNodeDev is 128 bytes");
 constexpr int32_t kEmptyChild = -1;
 
-// Triangle in leaf order, 48 bytes: {p0.xyz, prim id}, {p1-p0, 0}, {p2-p0, 0}.
-// The edges are the exact float differences the reference forms per test
-// (src/Core/Triangle.cuh:15-16), precomputed once.
+// Triangle in leaf order, 64 bytes: {p0.xyz, prim id}, {p1-p0, 0}, {p2-p0, 0},
+// unused. The edges are the exact float differences the reference forms per test
+// (src/Core/Triangle.cuh:15-16), precomputed once. 64 bytes rather than 48 keep
+// every record on a 32-byte boundary and two records within 128 bytes, so a leaf
+// step reads two with the loads of a node step (trace.cuh); the array holds one
+// record more than there are primitives, which such a step may read and ignores.
+constexpr size_t kTriFloat4 = 4;
+inline size_t tri_array_bytes(size_t prims) { return (prims + 1) * kTriFloat4 * sizeof(float4); }
 
 // 8-wide node with 8-bit child bounds, 80 bytes (five LDG.128). A child box
 // is lo = fma(2^(e - 127), qlo, p), hi = fma(2^(e - 127), qhi, p) per axis,
@@ -62,13 +67,14 @@ struct DevWBVH {
 
 struct DevBVH {
   const QNodeDev* nodes;
-  const float4* tris;  // 3 float4 per leaf slot
+  const float4* tris;  // kTriFloat4 float4 per leaf slot
   uint32_t leaf_shift;
   uint32_t first_mask;
   uint32_t count_mask;
   uint32_t prim_count;
   uint32_t node_count;
   int32_t stack_entries;
+  int32_t odd;  // a plane is not finite (imported trees): the exact slab takes compare-select min/max
 };
 
 // 64-byte material (reference Material fields, padded to 4 x float4).
@@ -233,7 +239,7 @@ cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& 
 
 struct QuadNode;  // bvh_build.h
 // QuadNode -> traversal node conversion, and the leaf-ordered triangle records
-// (3 x float4 per primitive: v0 + id, e1, e2), for trees built on the device.
+// (kTriFloat4 float4 per primitive: v0 + id, e1, e2, unused), for trees built on the device.
 cudaError_t launch_quad_to_dev(const QuadNode* quad, uint32_t nq, uint32_t leaf_shift, QNodeDev* nodes, cudaStream_t s);
 cudaError_t launch_leaf_tris(const DevScene& sc, const uint32_t* prims, uint32_t n, float4* tris, cudaStream_t s);
 

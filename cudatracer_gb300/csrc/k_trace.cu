@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kBlock) k_connect(DevBVH b, DevQueues q, float
   for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
     const float4 o = __ldg(q.sorg + i), d = __ldg(q.sdir + i);
     RayState r;
-    ray_begin(r, o, d, d.w);
+    ray_begin(b, r, o, d, d.w);
     if (!traverse<true, FASTMM>(b, r, eps, stack, kBlock)) {
       atomicOr(q.error, kErrStackOverflow);
       continue;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(BLOCK) k_batch_connect(DevBatch bt, DevQueues 
     const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, pix)];
     const DevBVH b = J.bvh;
     RayState r;
-    ray_begin(r, o, d, d.w);
+    ray_begin(b, r, o, d, d.w);
     if (!traverse<true, FASTMM>(b, r, J.f.tri_eps, stack, BLOCK)) {
       atomicOr(q.error, kErrStackOverflow);
       continue;

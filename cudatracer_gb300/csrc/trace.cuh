@@ -8,15 +8,29 @@
 // makes closest-hit primitive ids and t bit-exact against it.
 //
 // Min/max: glm::min(x,y) = y < x ? y : x and glm::max(x,y) = x < y ? y : x.
-// With FASTMM the hardware min/max is used instead; the two agree except when
-// a slab term is NaN (a zero direction component with the origin exactly on a
-// bounding plane) or when two zeros of opposite sign meet (an origin on two
-// planes). The fast-math render path uses FASTMM; exact paths never do.
+// Hardware min/max agree with them except on NaN (a zero direction component
+// with the origin exactly on a bounding plane) and when two zeros of opposite
+// sign meet (an origin on two planes). The fast path (FASTMM) uses hardware
+// min/max throughout; the exact path uses it where the two agree (inner_step).
 // FASTMM traversal also computes each slab plane with one fused multiply-add
 // and, for closest hit, visits hit children in true distance order
 // (inner_step_sorted) instead of the reference's partial order network: the
 // same nearest hit up to exact ties and the rounding of box distances, fewer
 // instructions per node.
+//
+// What bounds it, and the shape that follows. A divergent load takes one pass
+// through the L1 data pipe per distinct 128-byte line and lane whatever its
+// width, and a missed 32-byte sector about 1.5 passes (measured with random
+// lines on GB300), so a ray step reads its 128-byte node, or the next two
+// triangles of its leaf, with four 32-byte loads instead of up to eight 16-byte
+// ones. Both kinds of step start from the same four loads (Fetch), so a warp
+// whose lanes are at nodes and at leaves waits for memory once per round. The
+// plane distances of two children are one packed f32x2 instruction, and the
+// exact path takes hardware min/max wherever they give the reference's bits
+// (inner_step). Against 16-byte loads, separate leaf loads and compare-select
+// min/max: closest hit on an 81,920-triangle sphere, 4.2 M rays, 1,553 -> 1,204
+// us, 65,536 rays 218 -> 145 us; 641x360 exact frames 303 -> 241 us each;
+// 1920x1080 frames on 3.1 M triangles 1.80 -> 1.68 ms each.
 #pragma once
 
 #include "ct_internal.h"
@@ -28,49 +42,83 @@ __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b)
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 
-template <bool FASTMM>
-__device__ __forceinline__ float mn(float x, float y) {
-  return FASTMM ? fminf(x, y) : gmin(x, y);
-}
-template <bool FASTMM>
-__device__ __forceinline__ float mx(float x, float y) {
-  return FASTMM ? fmaxf(x, y) : gmax(x, y);
-}
-
-template <typename T>
-__device__ __forceinline__ T sel4(T a, T b, T c, T d, int i) {
-  return i == 0 ? a : (i == 1 ? b : (i == 2 ? c : d));
-}
-
 // One child's slab interval, reference order: x, then y, then z.
-template <bool FASTMM>
 __device__ __forceinline__ void slab(float bminx, float bmaxx, float bminy, float bmaxy, float bminz, float bmaxz,
                                      float ox, float oy, float oz, float ix, float iy, float iz, float& tmin,
                                      float& tmax) {
   float t1 = fmul(fsub(bminx, ox), ix), t2 = fmul(fsub(bmaxx, ox), ix);
-  tmin = mn<FASTMM>(t1, t2);
-  tmax = mx<FASTMM>(t1, t2);
+  tmin = gmin(t1, t2);
+  tmax = gmax(t1, t2);
   t1 = fmul(fsub(bminy, oy), iy);
   t2 = fmul(fsub(bmaxy, oy), iy);
-  tmin = mx<FASTMM>(tmin, mn<FASTMM>(t1, t2));
-  tmax = mn<FASTMM>(tmax, mx<FASTMM>(t1, t2));
+  tmin = gmax(tmin, gmin(t1, t2));
+  tmax = gmin(tmax, gmax(t1, t2));
   t1 = fmul(fsub(bminz, oz), iz);
   t2 = fmul(fsub(bmaxz, oz), iz);
-  tmin = mx<FASTMM>(tmin, mn<FASTMM>(t1, t2));
-  tmax = mn<FASTMM>(tmax, mx<FASTMM>(t1, t2));
+  tmin = gmax(tmin, gmin(t1, t2));
+  tmax = gmin(tmax, gmax(t1, t2));
 }
 
-// Fast-math slab: one fused multiply-add per plane, b * inv + (-o * inv). A
-// zero direction component makes that axis NaN, which the hardware min/max
-// drop: the axis then culls nothing (more boxes visited, never a hit lost).
-__device__ __forceinline__ void slab_fma(float bminx, float bmaxx, float bminy, float bmaxy, float bminz,
-                                         float bmaxz, float nox, float noy, float noz, float ix, float iy, float iz,
-                                         float& tmin, float& tmax) {
-  const float x1 = fmaf(bminx, ix, nox), x2 = fmaf(bmaxx, ix, nox);
-  const float y1 = fmaf(bminy, iy, noy), y2 = fmaf(bmaxy, iy, noy);
-  const float z1 = fmaf(bminz, iz, noz), z2 = fmaf(bmaxz, iz, noz);
-  tmin = fmaxf(fmaxf(fminf(x1, x2), fminf(y1, y2)), fminf(z1, z2));
-  tmax = fminf(fminf(fmaxf(x1, x2), fmaxf(y1, y2)), fmaxf(z1, z2));
+// Two floats in one 64-bit register pair and the packed operations on them:
+// each half is the scalar operation, rounded to nearest.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// 32 bytes of read-only memory in one load; p is 32-byte aligned. Volatile so
+// that the loads of a step are issued together, before the branch on its kind.
+__device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
+}
+
+// The 128 bytes of one ray step. Inner node: x planes (min, max of the four
+// children), y planes, z planes, child references. Leaf: the records of the
+// leaf's next two triangles, {p0, id}, {e1}, {e2} each (a leaf with one left
+// reads past it: the array has room for one record beyond its last).
+struct Fetch {
+  float4 v0, v1, v2, v3, v4, v5, v6;
+};
+__device__ __forceinline__ void fetch(const DevBVH& b, int ref, Fetch& f) {
+  const float4* p = ref >= 0 ? reinterpret_cast<const float4*>(b.nodes + ref)
+                             : b.tris + kTriFloat4 * (size_t)((uint32_t)ref & b.first_mask);
+  float4 unused;
+  ldg256(p, f.v0, f.v1);
+  ldg256(p + 2, f.v2, f.v3);
+  ldg256(p + 4, f.v4, f.v5);
+  ldg256(p + 6, f.v6, unused);
 }
 
 // Moller-Trumbore with the reference's absolute epsilon. Returns the new t
@@ -108,12 +156,18 @@ struct RayState {
   float ox, oy, oz, dx, dy, dz, ix, iy, iz, t;
   float nox, noy, noz;  // -o * inv, read by the fast-math slab only
   int hit, sp, ref;
+  bool odd;  // the exact slab may meet a NaN (inner_step); read by the exact path only
 };
 
-__device__ __forceinline__ void ray_begin(RayState& r, float4 o, float4 d, float t0) {
+// A slab term is NaN only as 0 * inf, inf - inf or from a NaN input: never for a
+// finite origin and finite reciprocals on finite planes.
+__device__ __forceinline__ void ray_begin(const DevBVH& b, RayState& r, float4 o, float4 d, float t0) {
   r.ox = o.x, r.oy = o.y, r.oz = o.z, r.dx = d.x, r.dy = d.y, r.dz = d.z;
   r.ix = __frcp_rn(d.x), r.iy = __frcp_rn(d.y), r.iz = __frcp_rn(d.z);
   r.nox = -o.x * r.ix, r.noy = -o.y * r.iy, r.noz = -o.z * r.iz;
+  const float big = 3.4028235e38f;  // the largest float
+  r.odd = b.odd || !(fabsf(r.ix) <= big && fabsf(r.iy) <= big && fabsf(r.iz) <= big && fabsf(o.x) <= big &&
+                     fabsf(o.y) <= big && fabsf(o.z) <= big);
   r.t = t0;
   r.hit = -1;
   r.sp = 0;
@@ -122,15 +176,48 @@ __device__ __forceinline__ void ray_begin(RayState& r, float4 o, float4 d, float
 
 enum StepResult { kContinue = 0, kDone = 1, kOverflow = 2 };
 
-// The four child intervals of a node in fast math.
-__device__ __forceinline__ void fast_slab4(const float4& nx0, const float4& nx1, const float4& ny0, const float4& ny1,
-                                           const float4& nz0, const float4& nz1, const RayState& r, float& tn0,
-                                           float& tn1, float& tn2, float& tn3, float& tf0, float& tf1, float& tf2,
-                                           float& tf3) {
-  slab_fma(nx0.x, nx1.x, ny0.x, ny1.x, nz0.x, nz1.x, r.nox, r.noy, r.noz, r.ix, r.iy, r.iz, tn0, tf0);
-  slab_fma(nx0.y, nx1.y, ny0.y, ny1.y, nz0.y, nz1.y, r.nox, r.noy, r.noz, r.ix, r.iy, r.iz, tn1, tf1);
-  slab_fma(nx0.z, nx1.z, ny0.z, ny1.z, nz0.z, nz1.z, r.nox, r.noy, r.noz, r.ix, r.iy, r.iz, tn2, tf2);
-  slab_fma(nx0.w, nx1.w, ny0.w, ny1.w, nz0.w, nz1.w, r.nox, r.noy, r.noz, r.ix, r.iy, r.iz, tn3, tf3);
+// Plane distances of the four children on one axis. FMA (fast math): one fused
+// multiply-add, b * inv + (-o * inv); a zero direction component makes the axis
+// NaN, which the hardware min/max drop: the axis then culls nothing (more boxes
+// visited, never a hit lost). Otherwise (b - o) * inv as the reference rounds it.
+template <bool FMA>
+__device__ __forceinline__ void axis_planes(float4& lo, float4& hi, float inv, float off) {
+  const f32x2 ii = pack2(inv, inv), oo = pack2(off, off);
+  auto t = [&](f32x2 b) { return FMA ? fma2(b, ii, oo) : mul2(add2(b, oo), ii); };
+  unpack2(t(pack2(lo.x, lo.y)), lo.x, lo.y);
+  unpack2(t(pack2(lo.z, lo.w)), lo.z, lo.w);
+  unpack2(t(pack2(hi.x, hi.y)), hi.x, hi.y);
+  unpack2(t(pack2(hi.z, hi.w)), hi.z, hi.w);
+}
+__device__ __forceinline__ void interval(float x1, float x2, float y1, float y2, float z1, float z2, float& tn,
+                                         float& tf) {
+  tn = max3(fminf(x1, x2), fminf(y1, y2), fminf(z1, z2));
+  tf = min3(fmaxf(x1, x2), fmaxf(y1, y2), fmaxf(z1, z2));
+}
+// The four child intervals of a node with hardware min/max.
+template <bool FMA>
+__device__ __forceinline__ void slab4(Fetch f, const RayState& r, float& tn0, float& tn1, float& tn2, float& tn3,
+                                      float& tf0, float& tf1, float& tf2, float& tf3) {
+  axis_planes<FMA>(f.v0, f.v1, r.ix, FMA ? r.nox : -r.ox);
+  axis_planes<FMA>(f.v2, f.v3, r.iy, FMA ? r.noy : -r.oy);
+  axis_planes<FMA>(f.v4, f.v5, r.iz, FMA ? r.noz : -r.oz);
+  interval(f.v0.x, f.v1.x, f.v2.x, f.v3.x, f.v4.x, f.v5.x, tn0, tf0);
+  interval(f.v0.y, f.v1.y, f.v2.y, f.v3.y, f.v4.y, f.v5.y, tn1, tf1);
+  interval(f.v0.z, f.v1.z, f.v2.z, f.v3.z, f.v4.z, f.v5.z, tn2, tf2);
+  interval(f.v0.w, f.v1.w, f.v2.w, f.v3.w, f.v4.w, f.v5.w, tn3, tf3);
+}
+// The same intervals with the reference's compare-select min/max, the planes
+// read again (rare: see inner_step).
+__device__ __forceinline__ void slab4_ref(const DevBVH& b, const RayState& r, float& tn0, float& tn1, float& tn2,
+                                          float& tn3, float& tf0, float& tf1, float& tf2, float& tf3) {
+  const QNodeDev* n = b.nodes + r.ref;
+  const float4 x0 = __ldg(&n->bminx), x1 = __ldg(&n->bmaxx);
+  const float4 y0 = __ldg(&n->bminy), y1 = __ldg(&n->bmaxy);
+  const float4 z0 = __ldg(&n->bminz), z1 = __ldg(&n->bmaxz);
+  slab(x0.x, x1.x, y0.x, y1.x, z0.x, z1.x, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn0, tf0);
+  slab(x0.y, x1.y, y0.y, y1.y, z0.y, z1.y, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn1, tf1);
+  slab(x0.z, x1.z, y0.z, y1.z, z0.z, z1.z, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn2, tf2);
+  slab(x0.w, x1.w, y0.w, y1.w, z0.w, z1.w, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn3, tf3);
 }
 
 // Compare-and-swap of (distance, child) pairs: the nearer pair goes first.
@@ -149,109 +236,95 @@ __device__ __forceinline__ void cas_pair(float& ka, int& ca, float& kb, int& cb)
 // next and the others pushed far to near with predicated stores. Frames in
 // fast math do not reproduce the reference's visiting order, only its nearest
 // hit, which no order changes beyond exact ties.
-__device__ __forceinline__ StepResult inner_step_sorted(const DevBVH& b, RayState& r, int* stack, int stride,
+__device__ __forceinline__ StepResult inner_step_sorted(const Fetch& f, RayState& r, int* stack, int stride,
                                                         int limit) {
-  const QNodeDev* n = b.nodes + r.ref;
-  const float4 nx0 = __ldg(&n->bminx), nx1 = __ldg(&n->bmaxx);
-  const float4 ny0 = __ldg(&n->bminy), ny1 = __ldg(&n->bmaxy);
-  const float4 nz0 = __ldg(&n->bminz), nz1 = __ldg(&n->bmaxz);
-  const int4 ch = __ldg(&n->child);
   float tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3;
-  fast_slab4(nx0, nx1, ny0, ny1, nz0, nz1, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  slab4<true>(f, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  int c0 = __float_as_int(f.v6.x), c1 = __float_as_int(f.v6.y), c2 = __float_as_int(f.v6.z),
+      c3 = __float_as_int(f.v6.w);
   const float t = r.t, inf = __int_as_float(0x7f800000);
-  const bool h0 = tf0 > 0.0f && tn0 <= tf0 && tn0 < t && ch.x != kEmptyChild;
-  const bool h1 = tf1 > 0.0f && tn1 <= tf1 && tn1 < t && ch.y != kEmptyChild;
-  const bool h2 = tf2 > 0.0f && tn2 <= tf2 && tn2 < t && ch.z != kEmptyChild;
-  const bool h3 = tf3 > 0.0f && tn3 <= tf3 && tn3 < t && ch.w != kEmptyChild;
-  const int cnt = (int)h0 + (int)h1 + (int)h2 + (int)h3;
-  if (cnt == 0) {
+  // a hit child's entry distance is below t, so finite or -inf; misses sort last
+  float k0 = (tf0 > 0.0f && tn0 <= tf0 && tn0 < t && c0 != kEmptyChild) ? tn0 : inf;
+  float k1 = (tf1 > 0.0f && tn1 <= tf1 && tn1 < t && c1 != kEmptyChild) ? tn1 : inf;
+  float k2 = (tf2 > 0.0f && tn2 <= tf2 && tn2 < t && c2 != kEmptyChild) ? tn2 : inf;
+  float k3 = (tf3 > 0.0f && tn3 <= tf3 && tn3 < t && c3 != kEmptyChild) ? tn3 : inf;
+  cas_pair(k0, c0, k1, c1);
+  cas_pair(k2, c2, k3, c3);
+  cas_pair(k0, c0, k2, c2);
+  cas_pair(k1, c1, k3, c3);
+  cas_pair(k1, c1, k2, c2);
+  if (!(k0 < inf)) {
     if (r.sp == 0) return kDone;
     r.ref = stack[--r.sp * stride];
     return kContinue;
   }
-  float k0 = h0 ? tn0 : inf, k1 = h1 ? tn1 : inf, k2 = h2 ? tn2 : inf, k3 = h3 ? tn3 : inf;
-  int c0 = ch.x, c1 = ch.y, c2 = ch.z, c3 = ch.w;
-  if (cnt > 1) {
-    cas_pair(k0, c0, k1, c1);
-    cas_pair(k2, c2, k3, c3);
-    cas_pair(k0, c0, k2, c2);
-    cas_pair(k1, c1, k3, c3);
-    cas_pair(k1, c1, k2, c2);
-    if (r.sp + cnt - 1 > limit) return kOverflow;
-    if (cnt > 3) stack[r.sp++ * stride] = c3;
-    if (cnt > 2) stack[r.sp++ * stride] = c2;
+  if (k1 < inf) {
+    if (r.sp + 1 + (int)(k2 < inf) + (int)(k3 < inf) > limit) return kOverflow;
+    if (k3 < inf) stack[r.sp++ * stride] = c3;
+    if (k2 < inf) stack[r.sp++ * stride] = c2;
     stack[r.sp++ * stride] = c1;
-  } else {
-    c0 = h0 ? ch.x : (h1 ? ch.y : (h2 ? ch.z : ch.w));
   }
   r.ref = c0;
   return kContinue;
 }
 
+// Compare-and-swap of (packed distance, child) pairs as the reference's network
+// swaps them: on a > b, so a NaN stays where it is.
+__device__ __forceinline__ void cas_packed(float& pa, int& ca, float& pb, int& cb) {
+  const bool sw = pa > pb;
+  const float p = sw ? pb : pa;
+  const int c = sw ? cb : ca;
+  pb = sw ? pa : pb;
+  cb = sw ? ca : cb;
+  pa = p;
+  ca = c;
+}
+
+// The child id in the low two bits of tmin (MBVHNode.cuh:91-94).
+__device__ __forceinline__ float with_id(float tn, int id) { return __int_as_float((__float_as_int(tn) & ~3) | id); }
+
 // Visit the inner node r.ref: slab-test the four children (MBVHNode.cuh:69-110),
 // then continue with the nearest hit child and push the others far to near
-// (:153-161). With zero or one child hit the order network cannot matter, so
-// it is skipped; with two or more it runs over all four packed tmin values,
-// exactly as the reference's does.
-template <bool FASTMM>
-__device__ __forceinline__ StepResult inner_step(const DevBVH& b, RayState& r, int* stack, int stride, int limit) {
-  const QNodeDev* n = b.nodes + r.ref;
-  const float4 nx0 = __ldg(&n->bminx), nx1 = __ldg(&n->bmaxx);
-  const float4 ny0 = __ldg(&n->bminy), ny1 = __ldg(&n->bmaxy);
-  const float4 nz0 = __ldg(&n->bminz), nz1 = __ldg(&n->bmaxz);
-  const int4 ch = __ldg(&n->child);
+// (:153-161), in the order the reference's network leaves the four packed tmin
+// values in; a missed child's reference is replaced by kEmptyChild and swapped
+// along, so what is left at a position says whether it is pushed. The hardware
+// min/max equal the reference's compare-select except on NaN (rays marked odd)
+// and for the sign of a zero, which shows in a packed tmin of magnitude below 4
+// denormal steps only (an origin exactly on a box plane): those nodes take the
+// compare-select slabs.
+__device__ __forceinline__ StepResult inner_step(const DevBVH& b, const Fetch& f, RayState& r, int* stack, int stride,
+                                                 int limit) {
   float tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3;
-  slab<FASTMM>(nx0.x, nx1.x, ny0.x, ny1.x, nz0.x, nz1.x, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn0, tf0);
-  slab<FASTMM>(nx0.y, nx1.y, ny0.y, ny1.y, nz0.y, nz1.y, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn1, tf1);
-  slab<FASTMM>(nx0.z, nx1.z, ny0.z, ny1.z, nz0.z, nz1.z, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn2, tf2);
-  slab<FASTMM>(nx0.w, nx1.w, ny0.w, ny1.w, nz0.w, nz1.w, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn3, tf3);
-  // child id in the low two bits of tmin (MBVHNode.cuh:91-94)
-  float p0 = __int_as_float((__float_as_int(tn0) & ~3) | 0);
-  float p1 = __int_as_float((__float_as_int(tn1) & ~3) | 1);
-  float p2 = __int_as_float((__float_as_int(tn2) & ~3) | 2);
-  float p3 = __int_as_float((__float_as_int(tn3) & ~3) | 3);
+  slab4<false>(f, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  const float tiny = __int_as_float(4);
+  if (r.odd || fminf(min3(fabsf(tn0), fabsf(tn1), fabsf(tn2)), fabsf(tn3)) < tiny)
+    slab4_ref(b, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  float p0 = with_id(tn0, 0), p1 = with_id(tn1, 1), p2 = with_id(tn2, 2), p3 = with_id(tn3, 3);
   const float t = r.t;
-  // hit mask by child slot (MBVHNode.cuh:96); empty slots are never pushed
-  const unsigned vm = ((tf0 > 0.0f && p0 <= tf0 && p0 < t && ch.x != kEmptyChild) ? 1u : 0u) |
-                      ((tf1 > 0.0f && p1 <= tf1 && p1 < t && ch.y != kEmptyChild) ? 2u : 0u) |
-                      ((tf2 > 0.0f && p2 <= tf2 && p2 < t && ch.z != kEmptyChild) ? 4u : 0u) |
-                      ((tf3 > 0.0f && p3 <= tf3 && p3 < t && ch.w != kEmptyChild) ? 8u : 0u);
-  if (vm == 0) {
+  // hit test by child slot (MBVHNode.cuh:96); empty slots are never pushed
+  int c0 = (tf0 > 0.0f && p0 <= tf0 && p0 < t) ? __float_as_int(f.v6.x) : kEmptyChild;
+  int c1 = (tf1 > 0.0f && p1 <= tf1 && p1 < t) ? __float_as_int(f.v6.y) : kEmptyChild;
+  int c2 = (tf2 > 0.0f && p2 <= tf2 && p2 < t) ? __float_as_int(f.v6.z) : kEmptyChild;
+  int c3 = (tf3 > 0.0f && p3 <= tf3 && p3 < t) ? __float_as_int(f.v6.w) : kEmptyChild;
+  // the reference's 5-exchange network, last pair (2,3) (MBVHNode.cuh:98-107)
+  cas_packed(p0, c0, p1, c1);
+  cas_packed(p2, c2, p3, c3);
+  cas_packed(p0, c0, p2, c2);
+  cas_packed(p1, c1, p3, c3);
+  cas_packed(p2, c2, p3, c3);
+  const bool h0 = c0 != kEmptyChild, h1 = c1 != kEmptyChild, h2 = c2 != kEmptyChild, h3 = c3 != kEmptyChild;
+  if (!(h0 || h1 || h2 || h3)) {
     if (r.sp == 0) return kDone;
     r.ref = stack[--r.sp * stride];
     return kContinue;
   }
-  if ((vm & (vm - 1)) == 0) {
-    r.ref = vm == 1 ? ch.x : (vm == 2 ? ch.y : (vm == 4 ? ch.z : ch.w));
-    return kContinue;
-  }
-  // the reference's 5-exchange network, last pair (2,3) (MBVHNode.cuh:98-107)
-  float s;
-  if (p0 > p1) s = p0, p0 = p1, p1 = s;
-  if (p2 > p3) s = p2, p2 = p3, p3 = s;
-  if (p0 > p2) s = p0, p0 = p2, p2 = s;
-  if (p1 > p3) s = p1, p1 = p3, p3 = s;
-  if (p2 > p3) s = p2, p2 = p3, p3 = s;
-  int held = kEmptyChild;
-  bool have = false;
-#pragma unroll
-  for (int i = 3; i >= 0; i--) {
-    const int c = __float_as_int(sel4(p0, p1, p2, p3, i)) & 3;
-    if ((vm >> c) & 1u) {
-      const int cr = sel4(ch.x, ch.y, ch.z, ch.w, c);
-      if (have) {
-        if (r.sp >= limit) return kOverflow;
-        stack[r.sp * stride] = held;
-        r.sp++;
-      }
-      held = cr;
-      have = true;
-    }
-  }
-  r.ref = held;
+  if (r.sp + (int)h0 + (int)h1 + (int)h2 + (int)h3 - 1 > limit) return kOverflow;
+  if (h3 && (h0 || h1 || h2)) stack[r.sp++ * stride] = c3;
+  if (h2 && (h0 || h1)) stack[r.sp++ * stride] = c2;
+  if (h1 && h0) stack[r.sp++ * stride] = c1;
+  r.ref = h0 ? c0 : (h1 ? c1 : (h2 ? c2 : c3));
   return kContinue;
 }
-
 
 // Any-hit variant of inner_step: whether the ray is occluded does not depend
 // on the order in which hit children are visited (every node whose packed
@@ -259,90 +332,68 @@ __device__ __forceinline__ StepResult inner_step(const DevBVH& b, RayState& r, i
 // the order network is skipped: the lowest hit slot continues, the others are
 // pushed.
 template <bool FASTMM>
-__device__ __forceinline__ StepResult inner_step_any(const DevBVH& b, RayState& r, int* stack, int stride, int limit) {
-  const QNodeDev* n = b.nodes + r.ref;
-  const float4 nx0 = __ldg(&n->bminx), nx1 = __ldg(&n->bmaxx);
-  const float4 ny0 = __ldg(&n->bminy), ny1 = __ldg(&n->bmaxy);
-  const float4 nz0 = __ldg(&n->bminz), nz1 = __ldg(&n->bmaxz);
-  const int4 ch = __ldg(&n->child);
+__device__ __forceinline__ StepResult inner_step_any(const DevBVH& b, const Fetch& f, RayState& r, int* stack,
+                                                     int stride, int limit) {
   float tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3;
-  if (FASTMM) {
-    fast_slab4(nx0, nx1, ny0, ny1, nz0, nz1, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
-  } else {
-    slab<false>(nx0.x, nx1.x, ny0.x, ny1.x, nz0.x, nz1.x, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn0, tf0);
-    slab<false>(nx0.y, nx1.y, ny0.y, ny1.y, nz0.y, nz1.y, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn1, tf1);
-    slab<false>(nx0.z, nx1.z, ny0.z, ny1.z, nz0.z, nz1.z, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn2, tf2);
-    slab<false>(nx0.w, nx1.w, ny0.w, ny1.w, nz0.w, nz1.w, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, tn3, tf3);
-  }
-  const float p0 = __int_as_float((__float_as_int(tn0) & ~3) | 0);
-  const float p1 = __int_as_float((__float_as_int(tn1) & ~3) | 1);
-  const float p2 = __int_as_float((__float_as_int(tn2) & ~3) | 2);
-  const float p3 = __int_as_float((__float_as_int(tn3) & ~3) | 3);
+  slab4<FASTMM>(f, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  // the sign of a zero tmin changes no hit test, so only NaN needs the compare-select slabs
+  if (!FASTMM && r.odd) slab4_ref(b, r, tn0, tn1, tn2, tn3, tf0, tf1, tf2, tf3);
+  const int c0 = __float_as_int(f.v6.x), c1 = __float_as_int(f.v6.y), c2 = __float_as_int(f.v6.z),
+            c3 = __float_as_int(f.v6.w);
+  const float p0 = with_id(tn0, 0), p1 = with_id(tn1, 1), p2 = with_id(tn2, 2), p3 = with_id(tn3, 3);
   const float t = r.t;
-  unsigned vm = ((tf0 > 0.0f && p0 <= tf0 && p0 < t && ch.x != kEmptyChild) ? 1u : 0u) |
-                ((tf1 > 0.0f && p1 <= tf1 && p1 < t && ch.y != kEmptyChild) ? 2u : 0u) |
-                ((tf2 > 0.0f && p2 <= tf2 && p2 < t && ch.z != kEmptyChild) ? 4u : 0u) |
-                ((tf3 > 0.0f && p3 <= tf3 && p3 < t && ch.w != kEmptyChild) ? 8u : 0u);
-  if (vm == 0) {
+  const bool h0 = tf0 > 0.0f && p0 <= tf0 && p0 < t && c0 != kEmptyChild;
+  const bool h1 = tf1 > 0.0f && p1 <= tf1 && p1 < t && c1 != kEmptyChild;
+  const bool h2 = tf2 > 0.0f && p2 <= tf2 && p2 < t && c2 != kEmptyChild;
+  const bool h3 = tf3 > 0.0f && p3 <= tf3 && p3 < t && c3 != kEmptyChild;
+  if (!(h0 || h1 || h2 || h3)) {
     if (r.sp == 0) return kDone;
     r.ref = stack[--r.sp * stride];
     return kContinue;
   }
   // the lowest hit slot continues; the others (never slot 0) are pushed in slot order
-  const unsigned rest = vm & (vm - 1);
-  if (r.sp + __popc(rest) > limit) return kOverflow;
-  if (rest & 2u) stack[r.sp++ * stride] = ch.y;
-  if (rest & 4u) stack[r.sp++ * stride] = ch.z;
-  if (rest & 8u) stack[r.sp++ * stride] = ch.w;
-  r.ref = (vm & 1u) ? ch.x : ((vm & 2u) ? ch.y : ((vm & 4u) ? ch.z : ch.w));
+  if (r.sp + (int)h0 + (int)h1 + (int)h2 + (int)h3 - 1 > limit) return kOverflow;
+  if (h1 && h0) stack[r.sp++ * stride] = c1;
+  if (h2 && (h0 || h1)) stack[r.sp++ * stride] = c2;
+  if (h3 && (h0 || h1 || h2)) stack[r.sp++ * stride] = c3;
+  r.ref = h0 ? c0 : (h1 ? c1 : (h2 ? c2 : c3));
   return kContinue;
 }
 
-// Test the leaf r.ref's triangles in primitive order, then pop.
+// Test the leaf r.ref's next two triangles (in primitive order, already
+// fetched), then pop; the rest of the leaf stays in r.ref (first + 2, count - 2),
+// so a round is not held up by the warp's largest leaf.
 template <bool ANY>
-__device__ __forceinline__ StepResult leaf_step(const DevBVH& b, RayState& r, float eps, int* stack, int stride) {
+__device__ __forceinline__ StepResult leaf_step(const DevBVH& b, const Fetch& f, RayState& r, float eps, int* stack,
+                                                int stride) {
   const uint32_t u = (uint32_t)r.ref;
-  const uint32_t first = u & b.first_mask;
   const uint32_t cnt = (u >> b.leaf_shift) & b.count_mask;
-  const float4* tp = b.tris + 3 * (size_t)first;
-  for (uint32_t k = 0; k < cnt; k++) {
-    const float4 a = __ldg(tp + 3 * k), e1 = __ldg(tp + 3 * k + 1), e2 = __ldg(tp + 3 * k + 2);
-    if (tri_test(a, e1, e2, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, eps, r.t)) {
-      r.hit = __float_as_int(a.w);
-      if (ANY) return kDone;
-    }
+  if (cnt > 0 && tri_test(f.v0, f.v1, f.v2, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, eps, r.t)) {
+    r.hit = __float_as_int(f.v0.w);
+    if (ANY) return kDone;
   }
-  if (r.sp == 0) return kDone;
-  r.ref = stack[--r.sp * stride];
-  return kContinue;
-}
-
-// leaf_step that tests at most P triangles per call: the rest of the leaf stays
-// in r.ref (first + k, count - k), so a round of the persistent loop is not
-// held up by the warp's largest leaf (P = 2 measured best; 1, 3 and 4 close).
-// Each ray still tests its triangles in the same order, so results are those
-// of leaf_step.
-template <bool ANY, int P>
-__device__ __forceinline__ StepResult leaf_step_part(const DevBVH& b, RayState& r, float eps, int* stack, int stride) {
-  const uint32_t u = (uint32_t)r.ref;
-  const uint32_t first = u & b.first_mask;
-  const uint32_t cnt = (u >> b.leaf_shift) & b.count_mask;
-  const uint32_t m = cnt < (uint32_t)P ? cnt : (uint32_t)P;
-  const float4* tp = b.tris + 3 * (size_t)first;
-  for (uint32_t k = 0; k < m; k++) {
-    const float4 a = __ldg(tp + 3 * k), e1 = __ldg(tp + 3 * k + 1), e2 = __ldg(tp + 3 * k + 2);
-    if (tri_test(a, e1, e2, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, eps, r.t)) {
-      r.hit = __float_as_int(a.w);
-      if (ANY) return kDone;
-    }
+  if (cnt > 1 && tri_test(f.v4, f.v5, f.v6, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, eps, r.t)) {
+    r.hit = __float_as_int(f.v4.w);
+    if (ANY) return kDone;
   }
-  if (cnt > m) {
-    r.ref = (int)(u + m - (m << b.leaf_shift));
+  if (cnt > 2) {
+    r.ref = (int)(u + 2u - (2u << b.leaf_shift));
     return kContinue;
   }
   if (r.sp == 0) return kDone;
   r.ref = stack[--r.sp * stride];
   return kContinue;
+}
+
+// One step of a ray: an inner node or up to two triangles of a leaf.
+template <bool ANY, bool FASTMM>
+__device__ __forceinline__ StepResult ray_step(const DevBVH& b, RayState& r, float eps, int* stack, int stride,
+                                               int limit) {
+  Fetch f;
+  fetch(b, r.ref, f);
+  if (r.ref < 0) return leaf_step<ANY>(b, f, r, eps, stack, stride);
+  if (ANY) return inner_step_any<FASTMM>(b, f, r, stack, stride, limit);
+  return FASTMM ? inner_step_sorted(f, r, stack, stride, limit) : inner_step(b, f, r, stack, stride, limit);
 }
 
 // Whole traversal of one ray by one thread. ANY = stop at the first hit
@@ -353,10 +404,7 @@ template <bool ANY, bool FASTMM>
 __device__ __forceinline__ bool traverse(const DevBVH& b, RayState& r, float eps, int* stack, int stride) {
   const int limit = b.stack_entries;
   while (true) {
-    const StepResult s = r.ref >= 0 ? (ANY ? inner_step_any<FASTMM>(b, r, stack, stride, limit)
-                                           : (FASTMM ? inner_step_sorted(b, r, stack, stride, limit)
-                                                     : inner_step<false>(b, r, stack, stride, limit)))
-                                    : leaf_step<ANY>(b, r, eps, stack, stride);
+    const StepResult s = ray_step<ANY, FASTMM>(b, r, eps, stack, stride, limit);
     if (s == kDone) return true;
     if (s == kOverflow) return false;
   }
@@ -401,7 +449,7 @@ __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cu
             float4 o, d;
             float t0;
             io.load(my, o, d, t0);
-            ray_begin(r, o, d, t0);
+            ray_begin(b, r, o, d, t0);
             rid = my;
           }
         }
@@ -409,10 +457,7 @@ __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cu
     }
     if (__ballot_sync(FULL, rid >= 0) == 0) break;
     if (rid < 0) continue;
-    const StepResult s = r.ref >= 0 ? (ANY ? inner_step_any<FASTMM>(b, r, stack, stride, limit)
-                                           : (FASTMM ? inner_step_sorted(b, r, stack, stride, limit)
-                                                     : inner_step<false>(b, r, stack, stride, limit)))
-                                    : leaf_step_part<ANY, 2>(b, r, eps, stack, stride);
+    const StepResult s = ray_step<ANY, FASTMM>(b, r, eps, stack, stride, limit);
     if (s != kContinue) {
       io.store(rid, r, s == kOverflow);
       rid = -1;
@@ -448,7 +493,7 @@ __device__ __forceinline__ void trace_persistent_batch(int n, int* cursor, IO& i
             float4 o, d;
             float t0;
             io.load(my, o, d, t0, b, eps);
-            ray_begin(r, o, d, t0);
+            ray_begin(b, r, o, d, t0);
             rid = my;
           }
         }
@@ -456,11 +501,7 @@ __device__ __forceinline__ void trace_persistent_batch(int n, int* cursor, IO& i
     }
     if (__ballot_sync(FULL, rid >= 0) == 0) break;
     if (rid < 0) continue;
-    const StepResult s =
-        r.ref >= 0 ? (ANY ? inner_step_any<FASTMM>(b, r, stack, stride, b.stack_entries)
-                          : (FASTMM ? inner_step_sorted(b, r, stack, stride, b.stack_entries)
-                                    : inner_step<false>(b, r, stack, stride, b.stack_entries)))
-                   : leaf_step_part<ANY, 2>(b, r, eps, stack, stride);
+    const StepResult s = ray_step<ANY, FASTMM>(b, r, eps, stack, stride, b.stack_entries);
     if (s != kContinue) {
       io.store(rid, r, s == kOverflow);
       rid = -1;
