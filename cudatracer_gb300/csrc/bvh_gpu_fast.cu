@@ -206,21 +206,60 @@ __device__ __forceinline__ void bin_frame(const uint32_t* k, float lo[3], float 
   }
 }
 
-__device__ __forceinline__ void bin_prim(uint32_t* bins, const float lo[3], const float scale[3], const float4& c,
-                                         const float4& l, const float4& h) {
-  const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)};
-  const uint32_t kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
+// Adds the warp's primitives (one per lane, those with `in`) to bins bin[0..2] of
+// the three axes (-1: the axis has none). Consecutive primitives mostly lie close
+// together, so an axis often has few bins in a warp, and one atomic per lane and
+// field would serialise on them: a bin that holds kBinGroup lanes or more takes
+// their seven values reduced over the warp, in one atomic each; the lanes left
+// over add their own.
+constexpr int kBinGroup = 6;
+__device__ __forceinline__ void bin_warp(uint32_t* bins, const int bin[3], const float4& l, const float4& h, bool in) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t key[6] = {fkey(l.x), fkey(l.y), fkey(l.z), fkey(h.x), fkey(h.y), fkey(h.z)};
+  unsigned have = 0;  // the lanes whose union `mine` holds
+  uint32_t mine = 0;  // lane f < 7: field f of that union
 #pragma unroll
   for (int a = 0; a < 3; a++) {
-    if (!(scale[a] > 0.0f)) continue;
-    uint32_t* b = bins + (a * kBins + bin_of(comp(c, a), lo[a], scale[a])) * kBinFields;
-    atomicAdd(b, 1u);
+    unsigned rem = __ballot_sync(FULL, in && bin[a] >= 0);
+    while (rem) {
+      const int b0 = __shfl_sync(FULL, bin[a], __ffs(rem) - 1);
+      const unsigned same = __ballot_sync(FULL, in && bin[a] == b0);
+      if (__popc(same) < kBinGroup) break;
+      if (same != have) {
+        have = same;
+        mine = (uint32_t)__popc(same);
+        const bool member = (same >> lane) & 1u;
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      atomicMin(b + 1 + k, kl[k]);
-      atomicMax(b + 4 + k, kh[k]);
+        for (int k = 0; k < 3; k++) {
+          const uint32_t mn = __reduce_min_sync(FULL, member ? key[k] : 0xffffffffu);
+          const uint32_t mx = __reduce_max_sync(FULL, member ? key[3 + k] : 0u);
+          if (lane == 1 + k) mine = mn;
+          if (lane == 4 + k) mine = mx;
+        }
+      }
+      uint32_t* e = bins + (a * kBins + b0) * kBinFields + lane;
+      if (lane == 0) atomicAdd(e, mine);
+      else if (lane < 4) atomicMin(e, mine);
+      else if (lane < 7) atomicMax(e, mine);
+      rem &= ~same;
+    }
+    if ((rem >> lane) & 1u) {
+      uint32_t* e = bins + (a * kBins + bin[a]) * kBinFields;
+      atomicAdd(e, 1u);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        atomicMin(e + 1 + k, key[k]);
+        atomicMax(e + 4 + k, key[3 + k]);
+      }
     }
   }
+}
+
+// The bins of one primitive per axis (-1 where all centroids coincide).
+__device__ __forceinline__ void bins_of(const float lo[3], const float scale[3], const float4& c, int bin[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; a++) bin[a] = scale[a] > 0.0f ? bin_of(comp(c, a), lo[a], scale[a]) : -1;
 }
 
 struct Cand {
@@ -347,6 +386,24 @@ __global__ void k_finit(uint32_t* counters) {
                                                               : 0u;
 }
 
+// Root bounds: reduced over the block before the six counters every block shares
+// are touched. With one atomic per warp the 2.0 M-triangle prep spent 290 of its
+// us on them.
+__device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn[3], uint32_t kmx[3]) {
+  __shared__ uint32_t red[6];
+  if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+  __syncthreads();
+  for (int k = 0; k < 3; k++) {
+    kmn[k] = __reduce_min_sync(0xffffffffu, kmn[k]);
+    kmx[k] = __reduce_max_sync(0xffffffffu, kmx[k]);
+  }
+  if ((threadIdx.x & 31) == 0)
+    for (int k = 0; k < 3; k++) atomicMin(&red[k], kmn[k]), atomicMax(&red[3 + k], kmx[k]);
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
+}
+
 __global__ void __launch_bounds__(256) k_fmag(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
                                               uint32_t* counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -357,8 +414,13 @@ __global__ void __launch_bounds__(256) k_fmag(const float4* __restrict__ v, cons
     for (int k = 0; k < 3; k++) m = gmax(m, gmax(fabsf(p[k].x), gmax(fabsf(p[k].y), fabsf(p[k].z))));
   }
   // non-negative floats order as their bit patterns
+  __shared__ uint32_t red;
+  if (threadIdx.x == 0) red = 0;
+  __syncthreads();
   const uint32_t r = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  if ((threadIdx.x & 31) == 0) atomicMax(&counters[kMag], r);
+  if ((threadIdx.x & 31) == 0) atomicMax(&red, r);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(&counters[kMag], red);
 }
 
 // rel_pad: kPad for the traversal-speed quad tree, 0 (exact bounds) for the wide tree
@@ -391,15 +453,7 @@ __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, con
     prims[i] = i;
     for (int k = 0; k < 3; k++) kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
   }
-  for (int k = 0; k < 3; k++) {
-    kmn[k] = __reduce_min_sync(0xffffffffu, kmn[k]);
-    kmx[k] = __reduce_max_sync(0xffffffffu, kmx[k]);
-  }
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; k++) {
-      atomicMin(&counters[kRootKeys + k], kmn[k]);
-      atomicMax(&counters[kRootKeys + 3 + k], kmx[k]);
-    }
+  block_root_keys(counters, kmn, kmx);
 }
 
 __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t n, uint32_t* counters) {
@@ -419,28 +473,34 @@ __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t 
 }
 
 // ---------------------------------------------------------------- large nodes, one level
-__global__ void k_fchunks(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large, uint32_t nl,
-                          uint32_t max_chunks, Chunk* chunks, FSplit* split, uint32_t* bins, uint32_t* cbk,
-                          uint32_t* counters) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nl) return;
+// One warp per node: its lanes write the chunks and the empty bins (one thread
+// took up to 31 us a level over the 336 bin words of its node).
+__global__ void __launch_bounds__(256) k_fchunks(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
+                                                 uint32_t nl, uint32_t max_chunks, Chunk* chunks, FSplit* split,
+                                                 uint32_t* bins, uint32_t* cbk, uint32_t* counters) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (s >= nl) return;  // whole warp
   const FNodeD& nd = arena[large[s]];
   const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + kChunk - 1) / kChunk;
-  const uint32_t base = atomicAdd(&counters[kChunkCursor], nc);
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
+  base = __shfl_sync(0xffffffffu, base, 0);
   if (base + nc > max_chunks) {
-    atomicOr(&counters[kError], kErrArena);
-    split[s] = FSplit{-2, 0, 0.0f, 0.0f, 0, 0u, 0u, 0u};
+    if (lane == 0) {
+      atomicOr(&counters[kError], kErrArena);
+      split[s] = FSplit{-2, 0, 0.0f, 0.0f, 0, 0u, 0u, 0u};
+    }
     return;
   }
-  for (uint32_t c = 0; c < nc; c++) {
+  for (uint32_t c = lane; c < nc; c += 32) {
     const uint32_t b = (uint32_t)nd.first + c * kChunk;
     chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * kChunk)};
   }
-  split[s] = FSplit{-1, 0, 0.0f, 0.0f, 0, 0u, base, 0u};
+  if (lane == 0) split[s] = FSplit{-1, 0, 0.0f, 0.0f, 0, 0u, base, 0u};
   uint32_t* b = bins + (size_t)s * kBinWords;
-  for (int w = 0; w < kBinWords; w++) b[w] = bin_init(w);
-  uint32_t* k = cbk + 6 * (size_t)s;
-  for (int a = 0; a < 3; a++) k[a] = fkey(1e34f), k[3 + a] = fkey(-1e34f);
+  for (int w = lane; w < kBinWords; w += 32) b[w] = bin_init(w);
+  if (lane < 6) cbk[6 * (size_t)s + lane] = lane < 3 ? fkey(1e34f) : fkey(-1e34f);
 }
 
 __device__ __forceinline__ uint32_t nchunks_used(const uint32_t* counters, uint32_t max_chunks) {
@@ -487,9 +547,12 @@ __global__ void __launch_bounds__(256) k_fbin(const Chunk* __restrict__ chunks, 
   bin_frame(cbk + 6 * (size_t)ch.slot, blo, bscale);
   for (int w = threadIdx.x; w < kBinWords; w += blockDim.x) bins[w] = bin_init(w);
   __syncthreads();
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
-    const uint32_t p = prims[k];
-    bin_prim(bins, blo, bscale, cent[p], lo[p], hi[p]);
+  for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
+    const bool in = k0 + threadIdx.x < ch.end;
+    const uint32_t p = in ? prims[k0 + threadIdx.x] : 0u;
+    int bin[3];
+    bins_of(blo, bscale, cent[p], bin);
+    bin_warp(bins, bin, lo[p], hi[p], in);
   }
   __syncthreads();
   uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
@@ -548,8 +611,13 @@ __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, const uint32_t* __r
   const FNodeD nd = A.arena[ni];
   float blo[3], bscale[3];
   bin_frame(cbk + 6 * (size_t)s, blo, bscale);
+  // the candidates walk the bins word by word: from shared memory
+  __shared__ uint32_t sbins[8][kBinWords];
+  uint32_t* bins = sbins[threadIdx.x >> 5];
+  for (int w = lane; w < kBinWords; w += 32) bins[w] = gbins[(size_t)s * kBinWords + w];
+  __syncwarp();
   Cand c;
-  choose_bin_split(gbins + (size_t)s * kBinWords, bscale, A.ascale, lane, c);
+  choose_bin_split(bins, bscale, A.ascale, lane, c);
   const uint32_t count = (uint32_t)nd.count;
   if (c.j < kCands) {
     if (lane == 0) {
@@ -806,9 +874,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
         bin_frame(keys, blo, bscale);
         for (int w = lane; w < kBinWords; w += 32) bins[w] = bin_init(w);
         __syncwarp();
-        for (uint32_t k = lane; k < count; k += 32) {
-          const uint32_t p = prims[first + k];
-          bin_prim(bins, blo, bscale, cent[p], lo[p], hi[p]);
+        for (uint32_t k0 = 0; k0 < count; k0 += 32) {
+          const bool in = k0 + lane < count;
+          const uint32_t p = in ? prims[first + k0 + lane] : 0u;
+          int bin[3];
+          bins_of(blo, bscale, cent[p], bin);
+          bin_warp(bins, bin, lo[p], hi[p], in);
         }
         __syncwarp();
         Cand c;
@@ -1234,7 +1305,8 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* __restrict__ aren
     if (j >= ns) continue;
     if (lf[j]) {
       r.leafmask |= 1u << j;
-      atomicMax(&counters[kMaxLeaf], (uint32_t)arena[sl[j]].count);
+      const uint32_t cnt = (uint32_t)arena[sl[j]].count;
+      if (cnt > __ldcg(&counters[kMaxLeaf])) atomicMax(&counters[kMaxLeaf], cnt);  // few raise it
     } else {
       const uint32_t at_ = next_base + atomicAdd(&counters[kQNext], 1u);
       if (at_ >= qcap) {
@@ -1459,7 +1531,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     A.large = large[cur];
     A.nl = nl;
     A.next_large = large[cur ^ 1];
-    k_fchunks<<<blocks(nl, 128), 128, 0, s>>>(arena, large[cur], nl, Lo.max_chunks, chunks, split, bins, cbk,
+    k_fchunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.max_chunks, chunks, split, bins, cbk,
                                               counters);
     const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / kChunk + nl + 1, Lo.max_chunks);
     k_fcb<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cent, prims, cbk);
