@@ -18,8 +18,9 @@
 //             chunks of kChunk primitives bin into shared memory and flush to
 //             the node's global bins; one warp per node picks the split; a
 //             chunk-ordered scan gives a stable partition through a scratch copy
-//   small     one warp builds the whole subtree of each node of <= kWarpMax
-//             primitives, bins and partition in shared memory
+//   small     one warp splits the subtree of each node of <= kWarpMax primitives
+//             down to ranges of <= kLeafTask, bins and partition in shared memory
+//   leaf      one thread builds the whole subtree of each such range
 //   collapse  quad nodes are the inner binary nodes at even depth; subtree
 //             quad counts bottom-up (arrival counters), each quad node's
 //             pre-order index from its ancestors' left-sibling counts, then
@@ -40,6 +41,7 @@ constexpr int kIntervals = kPlanes + 1;
 constexpr int kBinFields = 7;  // count, min key x/y/z, max key x/y/z
 constexpr int kBinWords = 3 * kIntervals * kBinFields;
 constexpr uint32_t kWarpMax = 128;  // nodes up to this size are built by one warp
+constexpr uint32_t kLeafTask = 16;  // subtrees up to this size are built by one thread
 constexpr uint32_t kChunk = 2048;   // primitives binned by one block
 constexpr int32_t kMaxSplitDepth = 61;
 constexpr int kSmallStack = 64;
@@ -51,6 +53,7 @@ enum Counter : int {
   kSmallCount = 1,
   kLargeNext = 2,
   kChunkCursor = 3,
+  kTasks = kChunkCursor,  // ranges for k_leaf, once the levels are done
   kError = 4,
   kMaxLeaf = 5,
   kQuadDepth = 6,
@@ -151,23 +154,64 @@ __device__ __forceinline__ float plane_at(float mn, float mx, int i) {
 __device__ __forceinline__ float centroid(float lo, float hi) { return __fmul_rn(__fadd_rn(lo, hi), 0.5f); }
 __device__ __forceinline__ float comp(const float4& v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
 
-// Bin one primitive into 3 x 11 intervals (counts + box keys) with atomics.
-__device__ __forceinline__ void bin_prim(uint32_t* bins, const float* planes, const float4& l, const float4& h) {
-  const float c[3] = {centroid(l.x, h.x), centroid(l.y, h.y), centroid(l.z, h.z)};
-  const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)};
-  const uint32_t kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
+// Adds the warp's primitives (one per lane, those with `in`) to bins bin[0..2] of
+// the three axes (-1: the axis has none). Consecutive primitives mostly lie close
+// together, so an axis often has few bins in a warp, and one atomic per lane and
+// field would serialise on them: a bin that holds kBinGroup lanes or more takes
+// their seven values reduced over the warp, in one atomic each; the lanes left
+// over add their own.
+constexpr int kBinGroup = 6;
+__device__ __forceinline__ void bin_warp(uint32_t* bins, const int bin[3], const float4& l, const float4& h, bool in) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t key[6] = {fkey(l.x), fkey(l.y), fkey(l.z), fkey(h.x), fkey(h.y), fkey(h.z)};
+  unsigned have = 0;  // the lanes whose union `mine` holds
+  uint32_t mine = 0;  // lane f < 7: field f of that union
 #pragma unroll
   for (int a = 0; a < 3; a++) {
-    int iv = 0;
+    unsigned rem = __ballot_sync(FULL, in && bin[a] >= 0);
+    while (rem) {
+      const int b0 = __shfl_sync(FULL, bin[a], __ffs(rem) - 1);
+      const unsigned same = __ballot_sync(FULL, in && bin[a] == b0);
+      if (__popc(same) < kBinGroup) break;
+      if (same != have) {
+        have = same;
+        mine = (uint32_t)__popc(same);
+        const bool member = (same >> lane) & 1u;
 #pragma unroll
-    for (int j = 0; j < kPlanes; j++) iv += !(c[a] <= planes[a * kPlanes + j]);
-    uint32_t* b = bins + (a * kIntervals + iv) * kBinFields;
-    atomicAdd(b, 1u);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      atomicMin(b + 1 + k, kl[k]);
-      atomicMax(b + 4 + k, kh[k]);
+        for (int k = 0; k < 3; k++) {
+          const uint32_t mn = __reduce_min_sync(FULL, member ? key[k] : 0xffffffffu);
+          const uint32_t mx = __reduce_max_sync(FULL, member ? key[3 + k] : 0u);
+          if (lane == 1 + k) mine = mn;
+          if (lane == 4 + k) mine = mx;
+        }
+      }
+      uint32_t* e = bins + (a * kIntervals + b0) * kBinFields + lane;
+      if (lane == 0) atomicAdd(e, mine);
+      else if (lane < 4) atomicMin(e, mine);
+      else if (lane < 7) atomicMax(e, mine);
+      rem &= ~same;
     }
+    if ((rem >> lane) & 1u) {
+      uint32_t* e = bins + (a * kIntervals + bin[a]) * kBinFields;
+      atomicAdd(e, 1u);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        atomicMin(e + 1 + k, key[k]);
+        atomicMax(e + 4 + k, key[3 + k]);
+      }
+    }
+  }
+}
+
+// The interval of one primitive per axis.
+__device__ __forceinline__ void intervals_of(const float* planes, const float4& l, const float4& h, int iv[3]) {
+  const float c[3] = {centroid(l.x, h.x), centroid(l.y, h.y), centroid(l.z, h.z)};
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    iv[a] = 0;
+#pragma unroll
+    for (int j = 0; j < kPlanes; j++) iv[a] += !(c[a] <= planes[a * kPlanes + j]);
   }
 }
 
@@ -246,6 +290,24 @@ __global__ void k_init(uint32_t* counters) {
                                                               : 0u;
 }
 
+// Root bounds: reduced over the block before the six counters every block shares
+// are touched. With one atomic per warp the 2.0 M-triangle prep spent 290 of its
+// us on them.
+__device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn[3], uint32_t kmx[3]) {
+  __shared__ uint32_t red[6];
+  if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+  __syncthreads();
+  for (int k = 0; k < 3; k++) {
+    kmn[k] = __reduce_min_sync(0xffffffffu, kmn[k]);
+    kmx[k] = __reduce_max_sync(0xffffffffu, kmx[k]);
+  }
+  if ((threadIdx.x & 31) == 0)
+    for (int k = 0; k < 3; k++) atomicMin(&red[k], kmn[k]), atomicMax(&red[3 + k], kmx[k]);
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
+}
+
 __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
                                               float4* __restrict__ lo, float4* __restrict__ hi,
                                               uint32_t* __restrict__ prims, uint32_t* counters) {
@@ -265,15 +327,7 @@ __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, cons
     prims[i] = i;
     for (int k = 0; k < 3; k++) kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
   }
-  for (int k = 0; k < 3; k++) {
-    kmn[k] = __reduce_min_sync(0xffffffffu, kmn[k]);
-    kmx[k] = __reduce_max_sync(0xffffffffu, kmx[k]);
-  }
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; k++) {
-      atomicMin(&counters[kRootKeys + k], kmn[k]);
-      atomicMax(&counters[kRootKeys + 3 + k], kmx[k]);
-    }
+  block_root_keys(counters, kmn, kmx);
 }
 
 __global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n, uint32_t* counters) {
@@ -293,20 +347,25 @@ __global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n,
 }
 
 // ---------------------------------------------------------------- large nodes, one level
-__global__ void k_chunks(const BNode* __restrict__ arena, const int32_t* __restrict__ large, uint32_t nl,
-                         Chunk* chunks, Split* split, uint32_t* bins, uint32_t* counters) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nl) return;
+// One warp per node: its lanes write the chunks and the empty bins.
+__global__ void __launch_bounds__(256) k_chunks(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
+                                                uint32_t nl, Chunk* chunks, Split* split, uint32_t* bins,
+                                                uint32_t* counters) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (s >= nl) return;  // whole warp
   const BNode& nd = arena[large[s]];
   const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + kChunk - 1) / kChunk;
-  const uint32_t base = atomicAdd(&counters[kChunkCursor], nc);
-  for (uint32_t c = 0; c < nc; c++) {
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
+  base = __shfl_sync(0xffffffffu, base, 0);
+  for (uint32_t c = lane; c < nc; c += 32) {
     const uint32_t b = (uint32_t)nd.first + c * kChunk;
     chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * kChunk)};
   }
-  split[s] = Split{-1, 0.0f, 0u, base};
+  if (lane == 0) split[s] = Split{-1, 0.0f, 0u, base};
   uint32_t* b = bins + (size_t)s * kBinWords;
-  for (int w = 0; w < kBinWords; w++) b[w] = bin_init(w);
+  for (int w = lane; w < kBinWords; w += 32) b[w] = bin_init(w);
 }
 
 __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
@@ -324,9 +383,12 @@ __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, co
   }
   for (int w = threadIdx.x; w < kBinWords; w += blockDim.x) bins[w] = bin_init(w);
   __syncthreads();
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
-    const uint32_t p = prims[k];
-    bin_prim(bins, planes, lo[p], hi[p]);
+  for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
+    const bool in = k0 + threadIdx.x < ch.end;
+    const uint32_t p = in ? prims[k0 + threadIdx.x] : 0u;
+    int iv[3];
+    intervals_of(planes, lo[p], hi[p], iv);
+    bin_warp(bins, iv, lo[p], hi[p], in);
   }
   __syncthreads();
   uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
@@ -361,8 +423,13 @@ __global__ void __launch_bounds__(256) k_split(BNode* arena, const int32_t* __re
   if (s >= nl) return;  // whole warp
   const int32_t ni = large[s];
   const BNode nd = arena[ni];
+  // the candidates walk the bins word by word: from shared memory
+  __shared__ uint32_t sbins[8][kBinWords];
+  uint32_t* bins = sbins[threadIdx.x >> 5];
+  for (int w = lane; w < kBinWords; w += 32) bins[w] = gbins[(size_t)s * kBinWords + w];
+  __syncwarp();
   Cand c;
-  const int best = choose_split(gbins + (size_t)s * kBinWords, lane, c);
+  const int best = choose_split(bins, lane, c);
   const float parent_cost = __fmul_rn(area3(nd.mn, nd.mx), __uint2float_rn((uint32_t)nd.count));
   if (best == 32) {
     // no candidate below 1e34: a leaf unless the parent's cost is not below it either
@@ -489,10 +556,12 @@ __global__ void __launch_bounds__(256) k_part_copy(const Chunk* __restrict__ chu
 }
 
 // ---------------------------------------------------------------- small subtrees, one warp each
+// tasks: ranges of 4..kLeafTask primitives for k_leaf, counted in counters[kTasks]
+// (disjoint, so at most n / 4).
 __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const int32_t* __restrict__ small,
                                                             const uint32_t* counters_ro, const float4* __restrict__ lo,
                                                             const float4* __restrict__ hi, uint32_t* prims,
-                                                            uint32_t* counters, uint32_t cap) {
+                                                            uint32_t* counters, uint32_t cap, uint32_t* tasks) {
   __shared__ uint32_t sbins[kSmallWarps][kBinWords];
   __shared__ float splanes[kSmallWarps][3 * kPlanes];
   __shared__ int32_t sstack[kSmallWarps][kSmallStack];
@@ -505,9 +574,13 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
   uint32_t* tmp = stmp[warp];
   const uint32_t nsmall = counters_ro[kSmallCount];
   for (uint32_t s = blockIdx.x * kSmallWarps + warp; s < nsmall; s += gridDim.x * kSmallWarps) {
-    int sp = 0;
-    if (lane == 0) stack[0] = small[s];
-    sp = 1;
+    const int32_t root = small[s];
+    if ((uint32_t)arena[root].count <= kLeafTask) {
+      if (lane == 0) tasks[atomicAdd(&counters[kTasks], 1u)] = (uint32_t)root;
+      continue;
+    }
+    if (lane == 0) stack[0] = root;
+    int sp = 1;
     __syncwarp();
     while (sp > 0) {
       const int32_t ni = stack[--sp];
@@ -517,9 +590,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
       if (lane < 3 * kPlanes) planes[lane] = plane_at(nd.mn[lane / kPlanes], nd.mx[lane / kPlanes], lane % kPlanes + 1);
       for (int w = lane; w < kBinWords; w += 32) bins[w] = bin_init(w);
       __syncwarp();
-      for (uint32_t k = lane; k < count; k += 32) {
-        const uint32_t p = prims[first + k];
-        bin_prim(bins, planes, lo[p], hi[p]);
+      for (uint32_t k0 = 0; k0 < count; k0 += 32) {
+        const bool in = k0 + lane < count;
+        const uint32_t p = in ? prims[first + k0 + lane] : 0u;
+        int iv[3];
+        intervals_of(planes, lo[p], hi[p], iv);
+        bin_warp(bins, iv, lo[p], hi[p], in);
       }
       __syncwarp();
       Cand c;
@@ -563,8 +639,15 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
         arena[cid + 1] = make_node(c.rmn, c.rmx, first + c.lc, c.rc, ni, nd.depth + 1);
         arena[ni].left = (int32_t)cid;
       }
-      const bool push_r = c.rc >= 4 && nd.depth + 1 <= kMaxSplitDepth;
-      const bool push_l = c.lc >= 4 && nd.depth + 1 <= kMaxSplitDepth;
+      const bool more_r = c.rc >= 4 && nd.depth + 1 <= kMaxSplitDepth;
+      const bool more_l = c.lc >= 4 && nd.depth + 1 <= kMaxSplitDepth;
+      const bool task_r = more_r && c.rc <= kLeafTask, task_l = more_l && c.lc <= kLeafTask;
+      const bool push_r = more_r && !task_r, push_l = more_l && !task_l;
+      if (lane == 0 && (task_l || task_r)) {
+        uint32_t at_ = atomicAdd(&counters[kTasks], (uint32_t)task_l + (uint32_t)task_r);
+        if (task_l) tasks[at_++] = cid;
+        if (task_r) tasks[at_] = cid + 1;
+      }
       if (sp + (int)push_r + (int)push_l > kSmallStack) {
         if (lane == 0) atomicOr(&counters[kError], kErrStack);
         continue;
@@ -579,14 +662,192 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
   }
 }
 
+// ---------------------------------------------------------------- subtrees of at most kLeafTask primitives, one thread each
+// The SAH of k_small by one thread for a whole subtree, 32 of them per warp. The
+// range is sorted once per axis by centroid; an order is 16 nibbles of a 64-bit
+// word, and a split partitions every order stably. A plane's left primitives
+// are then a prefix of its axis' order, so the ten planes of an axis cost one
+// suffix pass (areas) and one prefix walk. `cur` is the range's own order, which
+// the stable partition of k_small would leave. Boxes lie in shared memory
+// [value][thread], free of bank conflicts whatever primitive a thread reads.
+// Splits are found first, so the arena is asked for the nodes that exist.
+//
+// One warp per node spent its shuffles and 231 bin words on four primitives as
+// on 128: k_small took 2.69 ms of a 2.0 M-triangle build; with the leaves here it
+// takes 0.55 and this kernel 0.57 ms.
+constexpr int kLeafThreads = 64;
+// boxes, centroids or right areas, ids, nodes: a node of 4 or more splits, so 16
+// primitives make at most 13 splits and 27 nodes
+constexpr int kLeafWords = 16 * 6 + 16 + 16 + 27;
+constexpr size_t kLeafShared = sizeof(float) * kLeafWords * kLeafThreads;
+
+__device__ __forceinline__ uint32_t nib(unsigned long long o, uint32_t i) { return (uint32_t)(o >> (4 * i)) & 15u; }
+// Positions b..b+n-1 of order o, those of `left` first, each part in its order.
+__device__ __forceinline__ unsigned long long part_order(unsigned long long o, uint32_t b, uint32_t n, uint32_t nl,
+                                                         uint32_t left) {
+  const unsigned long long src = o;
+  uint32_t pl = b, pr = b + nl;
+  for (uint32_t i = 0; i < n; i++) {
+    const uint32_t j = nib(src, b + i);
+    const uint32_t to = (left >> j) & 1u ? pl++ : pr++;
+    o = (o & ~(15ull << (4 * to))) | ((unsigned long long)j << (4 * to));
+  }
+  return o;
+}
+
+__global__ void __launch_bounds__(kLeafThreads) k_leaf(BNode* arena, const uint32_t* __restrict__ tasks,
+                                                       const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                       uint32_t* prims, uint32_t* counters, uint32_t cap) {
+  extern __shared__ float sh[];
+  constexpr int T = kLeafThreads;
+  float* box = sh + threadIdx.x;                           // box[(6 j + c) T]: min x/y/z, max x/y/z of primitive j
+  float* val = box + 96 * T;                               // val[i T]: centroids while sorting, then right areas
+  uint32_t* id = reinterpret_cast<uint32_t*>(val + 16 * T);  // id[j T]
+  uint32_t* node = id + 16 * T;  // node k (k-th made): b | n << 4 | left count << 9 | depth << 14
+  const uint32_t ntask = counters[kTasks];
+  const int lane = threadIdx.x & 31;
+  for (uint32_t t0 = blockIdx.x * T + (threadIdx.x & ~31u); t0 < ntask; t0 += gridDim.x * T) {
+    const bool in = t0 + lane < ntask;
+    const int32_t root = in ? (int32_t)tasks[t0 + lane] : 0;
+    uint32_t first = 0, count = 0, splits = 0;
+    int32_t depth0 = 0;
+    unsigned long long ord[3] = {0, 0, 0}, cur = 0xfedcba9876543210ull;
+    if (in) {
+      const BNode nd = arena[root];
+      first = (uint32_t)nd.first, count = (uint32_t)nd.count, depth0 = nd.depth;
+      for (uint32_t j = 0; j < count; j++) {
+        const uint32_t p = prims[first + j];
+        const float4 l = lo[p], h = hi[p];
+        float* b = box + 6 * j * T;
+        b[0] = l.x, b[T] = l.y, b[2 * T] = l.z, b[3 * T] = h.x, b[4 * T] = h.y, b[5 * T] = h.z;
+        id[j * T] = p;
+      }
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        unsigned long long o = 0;
+        for (uint32_t j = 0; j < count; j++) {  // insertion: o's nibbles 0..j-1 are sorted
+          const float c = centroid(box[(6 * j + a) * T], box[(6 * j + 3 + a) * T]);
+          val[j * T] = c;
+          uint32_t k = j;
+          while (k > 0 && !(val[nib(o, k - 1) * T] <= c)) k--;
+          const unsigned long long low = o & ((1ull << (4 * k)) - 1ull);
+          o = low | ((unsigned long long)j << (4 * k)) | ((o - low) << 4);
+        }
+        ord[a] = o;
+      }
+      node[0] = count << 4;
+      // nodes in the order they are made; the two children of the k-th split are nodes 2 k + 1 and 2 k + 2
+      for (uint32_t k = 0; k <= 2 * splits; k++) {
+        const uint32_t w = node[k * T], b = w & 15u, n = (w >> 4) & 31u, dep = w >> 14;
+        if (n < 4 || depth0 + (int32_t)dep > kMaxSplitDepth) continue;
+        float nmn[3] = {1e34f, 1e34f, 1e34f}, nmx[3] = {-1e34f, -1e34f, -1e34f};
+        for (uint32_t i = 0; i < n; i++) {
+          const float* q = box + 6 * nib(cur, b + i) * T;
+          for (int c = 0; c < 3; c++) nmn[c] = fminf(nmn[c], q[c * T]), nmx[c] = fmaxf(nmx[c], q[(3 + c) * T]);
+        }
+        const float parent_cost = __fmul_rn(area3(nmn, nmx), __uint2float_rn(n));
+        float best = 1e34f, coord = 0.0f;
+        int bax = -1;
+        uint32_t blc = 0;
+        for (int a = 0; a < 3; a++) {
+          const unsigned long long o = (a == 0 ? ord[0] : a == 1 ? ord[1] : ord[2]) >> (4 * b);
+          float mn[3] = {1e34f, 1e34f, 1e34f}, mx[3] = {-1e34f, -1e34f, -1e34f};
+          for (uint32_t i = n - 1; i > 0; i--) {
+            const float* q = box + 6 * nib(o, i) * T;
+            for (int c = 0; c < 3; c++) mn[c] = fminf(mn[c], q[c * T]), mx[c] = fmaxf(mx[c], q[(3 + c) * T]);
+            val[i * T] = area3(mn, mx);
+          }
+          for (int c = 0; c < 3; c++) mn[c] = 1e34f, mx[c] = -1e34f;
+          const float pmn = a == 0 ? nmn[0] : a == 1 ? nmn[1] : nmn[2], pmx = a == 0 ? nmx[0] : a == 1 ? nmx[1] : nmx[2];
+          uint32_t lc = 0;
+          for (int i = 1; i <= kPlanes; i++) {
+            const float plane = plane_at(pmn, pmx, i);
+            while (lc < n) {
+              const float* q = box + 6 * nib(o, lc) * T;
+              if (!(centroid(q[a * T], q[(3 + a) * T]) <= plane)) break;
+              for (int c = 0; c < 3; c++) mn[c] = fminf(mn[c], q[c * T]), mx[c] = fmaxf(mx[c], q[(3 + c) * T]);
+              lc++;
+            }
+            // an empty side has no area: its cost is not a number, and no candidate
+            if (lc == 0 || lc == n) continue;
+            const float cost = __fadd_rn(__fmul_rn(area3(mn, mx), __uint2float_rn(lc)),
+                                         __fmul_rn(val[lc * T], __uint2float_rn(n - lc)));
+            if (cost < best) best = cost, bax = a, blc = lc, coord = plane;
+          }
+        }
+        if (bax < 0) {
+          if (!(parent_cost < 1e34f)) atomicOr(&counters[kError], kErrDegenerate);
+          continue;
+        }
+        if (parent_cost < best) continue;
+        uint32_t left = 0;
+        for (uint32_t i = 0; i < n; i++) {
+          const uint32_t j = nib(cur, b + i);
+          const float* q = box + 6 * j * T;
+          if (centroid(q[bax * T], q[(3 + bax) * T]) <= coord) left |= 1u << j;
+        }
+        if (__popc(left) != (int)blc) {
+          atomicOr(&counters[kError], kErrPartition);
+          continue;
+        }
+        cur = part_order(cur, b, n, blc, left);
+#pragma unroll
+        for (int a = 0; a < 3; a++) ord[a] = part_order(ord[a], b, n, blc, left);
+        node[k * T] = w | (blc << 9);
+        node[(2 * splits + 1) * T] = b | (blc << 4) | ((dep + 1) << 14);
+        node[(2 * splits + 2) * T] = (b + blc) | ((n - blc) << 4) | ((dep + 1) << 14);
+        splits++;
+      }
+    }
+    // the warp's nodes from the arena with one atomic
+    const uint32_t need = 2u * splits;
+    uint32_t inc = need;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += y;
+    }
+    uint32_t base = 0;
+    if (lane == 31) base = atomicAdd(&counters[kArenaCount], inc);
+    base = __shfl_sync(0xffffffffu, base, 31) + inc - need;
+    if (base + need > cap) {
+      if (need) atomicOr(&counters[kError], kErrArena);
+      continue;
+    }
+    uint32_t made = 0;
+    for (uint32_t k = 0; in && k <= 2 * splits; k++) {
+      const uint32_t w = node[k * T], b = w & 15u, n = (w >> 4) & 31u, lc = (w >> 9) & 31u, dep = w >> 14;
+      if (lc == 0) continue;
+      const int32_t ni = k == 0 ? root : (int32_t)(base + k - 1);
+      const uint32_t cid = base + 2 * made++;
+      for (uint32_t side = 0; side < 2; side++) {
+        const uint32_t cb = side ? b + lc : b, cn = side ? n - lc : lc;
+        float mn[3] = {1e34f, 1e34f, 1e34f}, mx[3] = {-1e34f, -1e34f, -1e34f};
+        for (uint32_t i = 0; i < cn; i++) {
+          const float* q = box + 6 * nib(cur, cb + i) * T;
+          for (int c = 0; c < 3; c++) mn[c] = fminf(mn[c], q[c * T]), mx[c] = fmaxf(mx[c], q[(3 + c) * T]);
+        }
+        arena[cid + side] = make_node(mn, mx, first + cb, cn, ni, depth0 + (int32_t)dep + 1);
+      }
+    }
+    // after every child record (each written with left = -1)
+    made = 0;
+    for (uint32_t k = 0; in && k <= 2 * splits; k++)
+      if ((node[k * T] >> 9) & 31u) arena[k == 0 ? root : (int32_t)(base + k - 1)].left = (int32_t)(base + 2 * made++);
+    if (splits)
+      for (uint32_t i = 0; i < count; i++) prims[first + i] = id[nib(cur, i) * T];
+  }
+}
+
 // ---------------------------------------------------------------- collapse
 __device__ __forceinline__ bool is_quad(const BNode& b) { return b.left >= 0 && (b.depth & 1) == 0; }
 
 __global__ void k_qcount(BNode* arena, uint32_t* arrive, const uint32_t* counters_ro, uint32_t* counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= counters_ro[kArenaCount]) return;
-  if (arena[i].left >= 0) return;
-  atomicMax(&counters[kMaxLeaf], (uint32_t)arena[i].count);
+  const bool leaf = i < counters_ro[kArenaCount] && arena[i].left < 0;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, leaf ? (uint32_t)arena[i].count : 0u);
+  if ((threadIdx.x & 31) == 0 && most > __ldcg(&counters[kMaxLeaf])) atomicMax(&counters[kMaxLeaf], most);
+  if (!leaf) return;
   int32_t cur = (int32_t)i;
   while (true) {
     const int32_t p = arena[cur].parent;
@@ -604,9 +865,10 @@ __global__ void k_qcount(BNode* arena, uint32_t* arrive, const uint32_t* counter
 __global__ void k_qindex(const BNode* __restrict__ arena, const uint32_t* counters_ro, uint32_t* qidx,
                          uint32_t* counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= counters_ro[kArenaCount]) return;
-  const BNode b = arena[i];
-  if (!is_quad(b)) return;
+  const bool quad = i < counters_ro[kArenaCount] && is_quad(arena[i]);
+  const uint32_t deep = __reduce_max_sync(0xffffffffu, quad ? (uint32_t)(arena[i].depth / 2 + 1) : 0u);
+  if ((threadIdx.x & 31) == 0 && deep > __ldcg(&counters[kQuadDepth])) atomicMax(&counters[kQuadDepth], deep);
+  if (!quad) return;
   // pre-order position: one for each quad ancestor step, plus the quad nodes of
   // every earlier slot (MergeNodes visits slots left to right, depth first)
   uint32_t idx = 0;
@@ -620,7 +882,6 @@ __global__ void k_qindex(const BNode* __restrict__ arena, const uint32_t* counte
     cur = p;
   }
   qidx[i] = idx;
-  atomicMax(&counters[kQuadDepth], (uint32_t)(b.depth / 2 + 1));
 }
 
 __device__ __forceinline__ void set_slot(QuadNode& q, int s, const float mn[3], const float mx[3], int32_t child,
@@ -744,7 +1005,7 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   while (nl > 0) {
     if (nl > L.max_large) return cudaErrorInvalidValue;
     GB_TRY(cudaMemsetAsync(counters + kLargeNext, 0, 8, s));  // kLargeNext, kChunkCursor
-    k_chunks<<<blocks(nl, 128), 128, 0, s>>>(arena, large[cur], nl, chunks, split, bins, counters);
+    k_chunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, chunks, split, bins, counters);
     const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / kChunk + nl + 1, L.max_chunks);
     k_bin<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, counters, lo, hi, prims, bins);
     k_split<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, bins, split, large[cur ^ 1], small,
@@ -766,7 +1027,16 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   if (nsmall > 0 && !host_counters[kError]) {
     const int sms = sm_count();
     const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sms * 8);
-    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, small, counters, lo, hi, prims, counters, L.cap);
+    GB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
+    // the partition's scratch (4 bytes per primitive) is free now: it takes the tasks
+    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, small, counters, lo, hi, prims, counters, L.cap, tmp);
+    GB_TRY(cudaGetLastError());
+    GB_TRY(cudaFuncSetAttribute(k_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
+    int per_sm = 0;
+    GB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_leaf, kLeafThreads, kLeafShared));
+    const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 4 + 1, kLeafThreads),
+                                                     (uint64_t)sms * std::max(1, per_sm));
+    k_leaf<<<gl, kLeafThreads, kLeafShared, s>>>(arena, tmp, lo, hi, prims, counters, L.cap);
     GB_TRY(cudaGetLastError());
   }
   GB_TRY(cudaMemsetAsync(arrive, 0, 4 * (size_t)L.cap, s));

@@ -1,8 +1,9 @@
-"""The device builder's subtrees of at most 16 primitives (built by one thread
-each) at the edges of that range: the device tree equals the host's byte for
-byte around 16 and 128 primitives (the sizes at which a range changes hands),
-with centroid ties on one axis or all, and along chains whose subtrees may and
-may not reach the depth limit."""
+"""The device builders' subtrees of at most 16 primitives (built by one thread
+each) at the edges of that range: the traversal-speed tree equals the host's
+byte for byte, and the reference's tree its quad nodes and every leaf's
+primitives, around 16 and 128 primitives (the sizes at which a range changes
+hands), with centroid ties on one axis or all, and along chains whose subtrees
+may and may not reach the depth limit."""
 import numpy as np
 import pytest
 
@@ -18,7 +19,14 @@ def _compare(ctx, v, ix):
     qd, pd = d.export()
     assert np.array_equal(ph, pd)
     assert np.array_equal(qh.view(np.int32), qd.view(np.int32))
-    for x in (h, d, sc):
+    hr, dr = sc.build_bvh(), sc.build_bvh_device()
+    qh, ph = hr.export()
+    qd, pd = dr.export()
+    assert np.array_equal(qh.view(np.int32), qd.view(np.int32))
+    counts, childs = qh[:, 28:32], qh[:, 24:28]
+    for first, cnt in zip(childs[counts > 0], counts[counts > 0]):
+        assert np.array_equal(np.sort(ph[first:first + cnt]), np.sort(pd[first:first + cnt]))
+    for x in (h, d, hr, dr, sc):
         x.close()
 
 
