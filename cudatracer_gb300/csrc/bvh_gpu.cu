@@ -15,7 +15,7 @@
 // Phases:
 //   prep      per-primitive padded bounds (triangle::getBounds) and the root box
 //   levels    nodes with more than kWarpMax primitives, one level per round:
-//             chunks of kChunk primitives bin into shared memory and flush to
+//             chunks of primitives bin into shared memory and flush to
 //             the node's global bins; one warp per node picks the split; a
 //             chunk-ordered scan gives a stable partition through a scratch copy
 //   small     one warp splits the subtree of each node of <= kWarpMax primitives
@@ -42,7 +42,16 @@ constexpr int kBinFields = 7;  // count, min key x/y/z, max key x/y/z
 constexpr int kBinWords = 3 * kIntervals * kBinFields;
 constexpr uint32_t kWarpMax = 128;  // nodes up to this size are built by one warp
 constexpr uint32_t kLeafTask = 16;  // subtrees up to this size are built by one thread
-constexpr uint32_t kChunk = 2048;   // primitives binned by one block
+// Primitives per block of the level kernels: the fewest, as a power of two from
+// 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
+// of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
+// their threads rather than 10 of eight (k_bin 18 -> 8 us a level); above 1.2 M
+// triangles the 2,048 of one wave stay (fewer bin flushes).
+inline uint32_t chunk_size(uint32_t n) {
+  uint32_t c = 256;
+  while (c < 2048 && n / c > 152 * 8) c *= 2;
+  return c;
+}
 constexpr int32_t kMaxSplitDepth = 61;
 constexpr int kSmallStack = 64;
 constexpr int kSmallWarps = 8;
@@ -88,11 +97,12 @@ struct Split {
 struct Layout {
   size_t lo, hi, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, chunk_loff, split, bins,
       counters, total;
-  uint32_t cap, max_large, max_chunks, max_small;
+  uint32_t chunk, cap, max_large, max_chunks, max_small;
   explicit Layout(uint32_t n) {
     cap = 2 * n + 2;
     max_large = n / (kWarpMax + 1) + 2;
-    max_chunks = n / kChunk + max_large + 2;
+    chunk = chunk_size(n);
+    max_chunks = n / chunk + max_large + 2;
     max_small = n / 4 + 2;
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -349,19 +359,19 @@ __global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n,
 // ---------------------------------------------------------------- large nodes, one level
 // One warp per node: its lanes write the chunks and the empty bins.
 __global__ void __launch_bounds__(256) k_chunks(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                                uint32_t nl, Chunk* chunks, Split* split, uint32_t* bins,
+                                                uint32_t nl, uint32_t chunk, Chunk* chunks, Split* split, uint32_t* bins,
                                                 uint32_t* counters) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= nl) return;  // whole warp
   const BNode& nd = arena[large[s]];
-  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + kChunk - 1) / kChunk;
+  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + chunk - 1) / chunk;
   uint32_t base = 0;
   if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
   base = __shfl_sync(0xffffffffu, base, 0);
   for (uint32_t c = lane; c < nc; c += 32) {
-    const uint32_t b = (uint32_t)nd.first + c * kChunk;
-    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * kChunk)};
+    const uint32_t b = (uint32_t)nd.first + c * chunk;
+    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * chunk)};
   }
   if (lane == 0) split[s] = Split{-1, 0.0f, 0u, base};
   uint32_t* b = bins + (size_t)s * kBinWords;
@@ -481,7 +491,7 @@ __global__ void __launch_bounds__(256) k_part_count(const Chunk* __restrict__ ch
 }
 
 __global__ void __launch_bounds__(256) k_part_offsets(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                                      uint32_t nl, Split* split,
+                                                      uint32_t nl, uint32_t chunk, Split* split,
                                                       const uint32_t* __restrict__ chunk_left, uint32_t* chunk_loff,
                                                       uint32_t* counters) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -489,7 +499,7 @@ __global__ void __launch_bounds__(256) k_part_offsets(const BNode* __restrict__ 
   if (s >= nl) return;
   const Split sp = split[s];
   if (sp.axis < 0) return;
-  const uint32_t nc = ((uint32_t)arena[large[s]].count + kChunk - 1) / kChunk;
+  const uint32_t nc = ((uint32_t)arena[large[s]].count + chunk - 1) / chunk;
   uint32_t run = 0;
   for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
     const uint32_t c = c0 + lane;
@@ -1005,13 +1015,13 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   while (nl > 0) {
     if (nl > L.max_large) return cudaErrorInvalidValue;
     GB_TRY(cudaMemsetAsync(counters + kLargeNext, 0, 8, s));  // kLargeNext, kChunkCursor
-    k_chunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, chunks, split, bins, counters);
-    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / kChunk + nl + 1, L.max_chunks);
+    k_chunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, chunks, split, bins, counters);
+    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / L.chunk + nl + 1, L.max_chunks);
     k_bin<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, counters, lo, hi, prims, bins);
     k_split<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, bins, split, large[cur ^ 1], small,
                                                           counters, L.cap);
     k_part_count<<<nchunk, 256, 0, s>>>(chunks, split, counters, lo, hi, prims, chunk_left);
-    k_part_offsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, split, chunk_left, chunk_loff,
+    k_part_offsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, split, chunk_left, chunk_loff,
                                                                  counters);
     k_part_scatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, chunk_loff, lo, hi, prims, tmp);
     k_part_copy<<<nchunk, 256, 0, s>>>(chunks, split, counters, tmp, prims);

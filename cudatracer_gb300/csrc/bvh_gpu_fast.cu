@@ -14,7 +14,7 @@
 //   prep      the largest coordinate magnitude M, padded boxes and centroids,
 //             the root box
 //   levels    nodes of more than kWarpMax primitives, one level per round:
-//             per chunk of kChunk primitives the centroid bounds, then the bins
+//             per chunk of primitives the centroid bounds, then the bins
 //             (shared memory, flushed into the node's global bins); one warp per
 //             node evaluates the 45 bin splits; a chunk-ordered scan gives the
 //             stable partition through a scratch copy
@@ -51,7 +51,16 @@ constexpr int32_t kDepthLimit = 60;
 constexpr float kPad = 1e-5f;
 constexpr uint32_t kSweepMax = 16;
 constexpr uint32_t kWarpMax = 128;  // subtrees up to this size: one warp
-constexpr uint32_t kChunk = 2048;
+// Primitives per block of the level kernels: the fewest, as a power of two from
+// 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
+// of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
+// their threads rather than 10 of eight (k_fbin 18 -> 8 us a level); above 1.2 M
+// triangles the 2,048 of one wave stay (fewer bin flushes).
+inline uint32_t chunk_size(uint32_t n) {
+  uint32_t c = 256;
+  while (c < 2048 && n / c > 152 * 8) c *= 2;
+  return c;
+}
 constexpr int kSmallWarps = 4;
 constexpr int kSmallStack = 64;  // depth limit 60: at most 61 pending nodes
 constexpr int kScanBlock = 1024;
@@ -119,12 +128,13 @@ static_assert(sizeof(QRec) == 64, "QRec");
 struct Layout {
   size_t lo, hi, cent, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, chunk_loff, split,
       bins, cbk, qlist, qrec, scan, sums, counters, total;
-  uint32_t cap, qcap, max_large, max_chunks, max_small, max_sums;
+  uint32_t chunk, cap, qcap, max_large, max_chunks, max_small, max_sums;
   explicit Layout(uint32_t n, int wide = 0) {
     cap = 2 * n + 2;
     qcap = n + 2;
     max_large = n / (kWarpMax + 1) + 2;
-    max_chunks = n / kChunk + max_large + 2;
+    chunk = chunk_size(n);
+    max_chunks = n / chunk + max_large + 2;
     max_small = n / 2 + 2;
     max_sums = qcap / kScanBlock + 2;
     size_t o = 0;
@@ -476,13 +486,13 @@ __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t 
 // One warp per node: its lanes write the chunks and the empty bins (one thread
 // took up to 31 us a level over the 336 bin words of its node).
 __global__ void __launch_bounds__(256) k_fchunks(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
-                                                 uint32_t nl, uint32_t max_chunks, Chunk* chunks, FSplit* split,
+                                                 uint32_t nl, uint32_t chunk, uint32_t max_chunks, Chunk* chunks, FSplit* split,
                                                  uint32_t* bins, uint32_t* cbk, uint32_t* counters) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= nl) return;  // whole warp
   const FNodeD& nd = arena[large[s]];
-  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + kChunk - 1) / kChunk;
+  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + chunk - 1) / chunk;
   uint32_t base = 0;
   if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
   base = __shfl_sync(0xffffffffu, base, 0);
@@ -494,8 +504,8 @@ __global__ void __launch_bounds__(256) k_fchunks(const FNodeD* __restrict__ aren
     return;
   }
   for (uint32_t c = lane; c < nc; c += 32) {
-    const uint32_t b = (uint32_t)nd.first + c * kChunk;
-    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * kChunk)};
+    const uint32_t b = (uint32_t)nd.first + c * chunk;
+    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * chunk)};
   }
   if (lane == 0) split[s] = FSplit{-1, 0, 0.0f, 0.0f, 0, 0u, base, 0u};
   uint32_t* b = bins + (size_t)s * kBinWords;
@@ -669,14 +679,14 @@ __global__ void __launch_bounds__(256) k_fpcount(const Chunk* __restrict__ chunk
 }
 
 __global__ void __launch_bounds__(256) k_fpoffsets(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
-                                                   uint32_t nl, FSplit* split, const uint32_t* __restrict__ chunk_left,
+                                                   uint32_t nl, uint32_t chunk, FSplit* split, const uint32_t* __restrict__ chunk_left,
                                                    uint32_t* chunk_loff, uint32_t* counters) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= nl) return;
   const FSplit sp = split[s];
   if (sp.mode != 0) return;
-  const uint32_t nc = ((uint32_t)arena[large[s]].count + kChunk - 1) / kChunk;
+  const uint32_t nc = ((uint32_t)arena[large[s]].count + chunk - 1) / chunk;
   uint32_t run = 0;
   for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
     const uint32_t c = c0 + lane;
@@ -1531,14 +1541,14 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     A.large = large[cur];
     A.nl = nl;
     A.next_large = large[cur ^ 1];
-    k_fchunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.max_chunks, chunks, split, bins, cbk,
+    k_fchunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, Lo.max_chunks, chunks, split, bins, cbk,
                                               counters);
-    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / kChunk + nl + 1, Lo.max_chunks);
+    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / Lo.chunk + nl + 1, Lo.max_chunks);
     k_fcb<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cent, prims, cbk);
     k_fbin<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cbk, lo, hi, cent, prims, bins);
     k_fsplit<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(A, bins, cbk, split, lo, hi, prims);
     k_fpcount<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, cent, prims, chunk_left);
-    k_fpoffsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, split, chunk_left, chunk_loff,
+    k_fpoffsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, split, chunk_left, chunk_loff,
                                                               counters);
     k_fpscatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, Lo.max_chunks, chunk_loff, cent,
                                        prims, tmp);
