@@ -1300,11 +1300,23 @@ static ct_status ensure_logs(ct_ctx* ctx, ct_render* r, int max_depth, bool* ok)
   return CT_OK;
 }
 
+// Frames of at most this many pixels run as one kernel (launch_path) unless their
+// stages are profiled. Sixteen frames in a row on a 571,000-triangle terrain, depth
+// 8, one kernel against the stages: 256x192 0.79 and 2.31 ms (on 256,000
+// triangles), 362x362 2.79 and 3.44 ms, 400x400 3.37 and 3.27 ms, 512x384 3.97 and
+// 3.73 ms: beyond about 160,000 pixels the stages' compaction and refills pay (a
+// frame waited for alone is faster in one kernel up to 640x360).
+constexpr int kPathPixels = 131072;
+
 // Issue one frame's stages on stream st into queues q.
 static ct_status emit_frame(ct_ctx* ctx, ct_render* r, const DevQueues& q, const ct_scene* scene, const ct_bvh* bvh,
                             const FrameConst& f, const ct_render_params* p, cudaStream_t st) {
   const bool fast = math_fast_traversal(p->exact_math);
   const int exact_shade = math_exact_shading(p->exact_math);
+  if (!r->profile && !bvh->wide && r->w * r->h <= kPathPixels) {
+    CT_CUDA(ctx, launch_path(scene->dev, bvh->dev, q, f, p->max_depth, exact_shade, fast, st));
+    return CT_OK;
+  }
   CT_CUDA(ctx, staged(r, 0, st, [&] { return launch_raygen(q, f, exact_shade, st); }));
   for (int pass = 0; pass < p->max_depth; pass++) {
     const int cur = pass & 1;

@@ -219,6 +219,10 @@ cudaError_t launch_connect(const DevBVH& b, const DevQueues& q, float eps, bool 
 cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact, cudaStream_t s);
 cudaError_t launch_shade(const DevScene& sc, const DevQueues& q, const FrameConst& f, int queue, int path_length,
                          int exact, cudaStream_t s);
+// A whole frame in one kernel on a quad tree (frames of few pixels): as raygen and
+// max_depth x (extend, shade, connect if f.shadow) into the same q.accum or q.log.
+cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
+                        int exact_math, bool fast_traversal, cudaStream_t s);
 cudaError_t launch_present(const float4* accum, float4* out, int n, float samples, cudaStream_t s);
 // Device SAH build (bvh_gpu.cu). gpu_bvh_build runs the binary build and the
 // collapse bookkeeping in `scratch` (gpu_bvh_scratch_bytes) and returns the

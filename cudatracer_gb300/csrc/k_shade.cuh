@@ -17,6 +17,7 @@
 #include "bsdf_full.cuh"
 #include "ct_internal.h"
 #include "portable_math.h"
+#include "trace.cuh"
 #include "vmath.cuh"
 
 #ifndef CT_MODE_FULL
@@ -35,6 +36,7 @@ constexpr float kMaxDistance = 1e34f;
 constexpr float kOneOverPi = 0.318309886183790671537767526745028724f;
 constexpr float kTwoPi = 6.28318530717958647692528676655900576f;
 constexpr int kBlock = 128;
+constexpr int kPathBlock = 32;  // k_path: a block's threads share nothing, and few pixels spread over all SMs
 
 #if CT_EXACT
 // reproducible binary32 functions (portable_math.h): the oracle evaluates the
@@ -170,11 +172,9 @@ __device__ __forceinline__ TriRec load_tri(const DevScene& sc, int prim) {
   return t;
 }
 
-__device__ __forceinline__ void shade_compat(const DevScene& sc, const DevQueues& q, const FrameConst& f, int cur,
-                                             int i, uint32_t path_length, Emit& e, int pix_base = 0,
-                                             float4* acc = nullptr) {
-  const float4 o4 = q.org_q(cur)[i], d4 = q.dir_q(cur)[i], t4 = q.thr_q(cur)[i];
-  const int2 h = q.hit[i];
+__device__ __forceinline__ void shade_compat(const DevScene& sc, const DevQueues& q, const FrameConst& f,
+                                             const float4 o4, const float4 d4, const float4 t4, const int2 h,
+                                             uint32_t path_length, Emit& e, int pix_base = 0, float4* acc = nullptr) {
   const int pix = __float_as_int(o4.w);
   V3 org = v3(o4), dir = v3(d4), T = v3(t4);
   const float last_pdf = t4.w;
@@ -347,11 +347,9 @@ __device__ __forceinline__ void onb(V3 n, V3& t, V3& b) {
   b = v3(bb, sign + n.y * n.y * a, -n.y);
 }
 
-__device__ __forceinline__ void shade_full(const DevScene& sc, const DevQueues& q, const FrameConst& f, int cur, int i,
-                                           uint32_t path_length, Emit& e, int pix_base = 0,
-                                           float4* acc = nullptr) {
-  const float4 o4 = q.org_q(cur)[i], d4 = q.dir_q(cur)[i], t4 = q.thr_q(cur)[i];
-  const int2 h = q.hit[i];
+__device__ __forceinline__ void shade_full(const DevScene& sc, const DevQueues& q, const FrameConst& f,
+                                           const float4 o4, const float4 d4, const float4 t4, const int2 h,
+                                           uint32_t path_length, Emit& e, int pix_base = 0, float4* acc = nullptr) {
   const int pix = __float_as_int(o4.w);
   const V3 dir = v3(d4);
   V3 T = v3(t4);
@@ -490,10 +488,12 @@ __global__ void __launch_bounds__(kBlock) k_shade(DevScene sc, DevQueues q, Fram
     e.cont = false;
     e.shadow = false;
     if (i < n) {
+      const float4 o = q.org_q(cur)[i], d = q.dir_q(cur)[i], t = q.thr_q(cur)[i];
+      const int2 h = q.hit[i];
       if (f.shading_mode == CT_MODE_FULL)
-        shade_full(sc, q, f, cur, i, path_length, e);
+        shade_full(sc, q, f, o, d, t, h, path_length, e);
       else
-        shade_compat(sc, q, f, cur, i, path_length, e);
+        shade_compat(sc, q, f, o, d, t, h, path_length, e);
     }
     const int si = warp_append(e.shadow, &q.counts[2]);
     if (si >= 0) {
@@ -532,6 +532,22 @@ __device__ __forceinline__ int tile_pixel(int j, int w, int h) {
   return (h4 + j / w) * w + j % w;
 }
 
+// The jittered pinhole ray of pixel i (origin.w = pixel, direction.w = 0: last bounce specular).
+__device__ __forceinline__ void primary_ray(const FrameConst& f, int i, float4& o, float4& d) {
+  const float invw = 1.0f / (float)f.width, invh = 1.0f / (float)f.height;
+  const V3 w = v3(f.cam_w.x, f.cam_w.y, f.cam_w.z), hor = v3(f.hor.x, f.hor.y, f.hor.z),
+           ver = v3(f.ver.x, f.ver.y, f.ver.z);
+  uint32_t seed = ((uint32_t)i + f.frame * 147565741u) * 720898027u;
+  const int x = i % f.width, y = (i / f.width) % f.height;
+  const float px = ((float)x + rnd_float(seed)) - 0.5f;
+  const float py = ((float)y + rnd_float(seed)) - 0.5f;
+  const float sx = 2.0f * (px * invw) - 1.0f;
+  const float sy = 1.0f - 2.0f * (py * invh);
+  const V3 p = (w + hor * sx) + ver * sy;
+  o = make_float4(f.cam_pos.x, f.cam_pos.y, f.cam_pos.z, __int_as_float(i));
+  d = f4(normalize(p), __int_as_float(0));
+}
+
 __global__ void __launch_bounds__(kBlock) k_raygen(DevQueues q, FrameConst f) {
   const int npix = f.width * f.height;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -540,23 +556,111 @@ __global__ void __launch_bounds__(kBlock) k_raygen(DevQueues q, FrameConst f) {
     atomicAdd(&q.stats[2], (unsigned long long)npix);
     atomicAdd(&q.stats[3], 1ull);
   }
-  const float invw = 1.0f / (float)f.width, invh = 1.0f / (float)f.height;
-  const V3 w = v3(f.cam_w.x, f.cam_w.y, f.cam_w.z), hor = v3(f.hor.x, f.hor.y, f.hor.z),
-           ver = v3(f.ver.x, f.ver.y, f.ver.z);
   for (int j = blockIdx.x * kBlock + threadIdx.x; j < npix; j += gridDim.x * kBlock) {
-    const int i = tile_pixel(j, f.width, f.height);
-    uint32_t seed = ((uint32_t)i + f.frame * 147565741u) * 720898027u;
-    const int x = i % f.width, y = (i / f.width) % f.height;
-    const float px = ((float)x + rnd_float(seed)) - 0.5f;
-    const float py = ((float)y + rnd_float(seed)) - 0.5f;
-    const float sx = 2.0f * (px * invw) - 1.0f;
-    const float sy = 1.0f - 2.0f * (py * invh);
-    const V3 p = (w + hor * sx) + ver * sy;
-    q.org_q(0)[j] = make_float4(f.cam_pos.x, f.cam_pos.y, f.cam_pos.z, __int_as_float(i));
-    q.dir_q(0)[j] = f4(normalize(p), __int_as_float(0));  // lastBounceType = SPECULAR
+    float4 o, d;
+    primary_ray(f, tile_pixel(j, f.width, f.height), o, d);
+    q.org_q(0)[j] = o;
+    q.dir_q(0)[j] = d;
     q.thr_q(0)[j] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);  // throughput 1, lastBsdfPDF 1
   }
 }
+
+// A value the wavefront would store to a queue and load again: no operation is
+// fused across this point, so both ways round alike in every build.
+__device__ __forceinline__ void stored(float4& v) { asm volatile("" : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)); }
+
+// A whole frame in one kernel, one path per thread: ray generation, then up to
+// max_depth x (closest hit, shade, shadow any hit). For frames of few pixels,
+// whose wavefront stages (1 + 3 max_depth launches) are a few warps each: what
+// counts there is the launches and the wait for the longest ray of every stage,
+// and the compaction between stages has nothing to fill. Each path does what
+// the stages do with the same operations in the same order, so the frame's
+// contributions are the same bits, added to q.accum (or logged) per pixel in
+// the same order. A 64x48, depth-5 frame takes 126 us when waited for and 50 us
+// among others (the host calls), with the stages 343 and 98 us.
+// shade_full as a function of its own: k_path then holds 93 registers instead of
+// 124 (362x362 frames 191 -> 174 us), and in the build with FMA contraction it is
+// contracted as k_shade's copy is (inlined beside the traversal it was not).
+__device__ __noinline__ void shade_full_call(const DevScene* sc, const DevQueues* q, const FrameConst* f, float4 o4,
+                                             float4 d4, float4 t4, int2 h, uint32_t path_length, Emit* e) {
+  shade_full(*sc, *q, *f, o4, d4, t4, h, path_length, *e);
+}
+
+template <bool FASTMM>
+__device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b, DevQueues& q, const FrameConst& f,
+                                            int max_depth) {
+  extern __shared__ int s_stack[];
+  int* stack = s_stack + threadIdx.x;
+  const int npix = f.width * f.height;
+  unsigned long long n_ext = 0, n_shadow = 0;
+  const int j = blockIdx.x * kPathBlock + threadIdx.x;
+  bool alive = j < npix;
+  float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o, t = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+  if (alive) primary_ray(f, tile_pixel(j, f.width, f.height), o, d);
+  stored(o), stored(d);
+  for (int pass = 0; pass < max_depth; pass++) {
+    if (!__any_sync(0xffffffffu, alive)) break;
+    Emit e;
+    e.cont = false;
+    e.shadow = false;
+    if (alive) {
+      n_ext++;
+      RayState r;
+      ray_begin(b, r, o, d, kMaxDistance);
+      int2 h;
+      if (traverse<false, FASTMM>(b, r, f.tri_eps, stack, kPathBlock)) {
+        h = make_int2(r.hit, __float_as_int(r.t));
+      } else {
+        atomicOr(q.error, kErrStackOverflow);
+        h = make_int2(-1, __float_as_int(kMaxDistance));
+      }
+      q.log_entry = 2u * (uint32_t)pass;
+      const uint32_t path_length = pass == 0 ? 0u : (uint32_t)pass + 1u;  // Kernel.cu:306, 330
+      if (f.shading_mode == CT_MODE_FULL)
+        shade_full_call(&sc, &q, &f, o, d, t, h, path_length, &e);
+      else
+        shade_compat(sc, q, f, o, d, t, h, path_length, e);
+    }
+    if (e.shadow) {
+      n_shadow++;
+      stored(e.so), stored(e.sd), stored(e.sc);
+      RayState r;
+      ray_begin(b, r, e.so, e.sd, e.sd.w);
+      if (!traverse<true, FASTMM>(b, r, f.tri_eps, stack, kPathBlock)) {
+        atomicOr(q.error, kErrStackOverflow);
+      } else if (r.hit < 0) {
+        const int pix = __float_as_int(e.so.w);
+        q.log_entry = 2u * (uint32_t)pass + 1u;
+        add_contribution(q, nullptr, pix, 0, v3(e.sc));
+      }
+    }
+    alive = e.cont;
+    if (alive) o = e.no, d = e.nd, t = e.nt;
+    stored(o), stored(d), stored(t);
+  }
+  for (int off = 16; off; off >>= 1) {
+    n_ext += __shfl_xor_sync(0xffffffffu, n_ext, off);
+    n_shadow += __shfl_xor_sync(0xffffffffu, n_shadow, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (n_ext) atomicAdd(&q.stats[0], n_ext);
+    if (n_shadow) atomicAdd(&q.stats[1], n_shadow);
+    if (j == 0) {
+      atomicAdd(&q.stats[2], (unsigned long long)npix);
+      atomicAdd(&q.stats[3], 1ull);
+    }
+  }
+}
+__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth) {
+  trace_paths<true>(sc, b, q, f, max_depth);
+}
+#if CT_EXACT
+// with the reference's traversal (CT_MATH_EXACT)
+__global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
+                                                         int max_depth) {
+  trace_paths<false>(sc, b, q, f, max_depth);
+}
+#endif
 
 // ---- batches: one launch per stage for every job (see DevBatch)
 
@@ -570,20 +674,9 @@ __global__ void __launch_bounds__(kBlock) k_batch_raygen(DevBatch bt, DevQueues 
     if (g < bt.total_pix) {
       const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, g)];
       if (J.spp_left > 0) {
-        const FrameConst& f = J.f;
-        const int i = tile_pixel(g - J.pix_base, f.width, f.height);  // the job's pixels in 8x4 tiles
-        uint32_t seed = ((uint32_t)i + f.frame * 147565741u) * 720898027u;
-        const int x = i % f.width, y = (i / f.width) % f.height;
-        const float invw = 1.0f / (float)f.width, invh = 1.0f / (float)f.height;
-        const float px = ((float)x + rnd_float(seed)) - 0.5f;
-        const float py = ((float)y + rnd_float(seed)) - 0.5f;
-        const float sx = 2.0f * (px * invw) - 1.0f;
-        const float sy = 1.0f - 2.0f * (py * invh);
-        const V3 w = v3(f.cam_w.x, f.cam_w.y, f.cam_w.z), hor = v3(f.hor.x, f.hor.y, f.hor.z),
-                 ver = v3(f.ver.x, f.ver.y, f.ver.z);
-        const V3 p = (w + hor * sx) + ver * sy;
-        o = make_float4(f.cam_pos.x, f.cam_pos.y, f.cam_pos.z, __int_as_float(J.pix_base + i));
-        d = f4(normalize(p), __int_as_float(0));
+        const int i = tile_pixel(g - J.pix_base, J.f.width, J.f.height);  // the job's pixels in 8x4 tiles
+        primary_ray(J.f, i, o, d);
+        o.w = __int_as_float(J.pix_base + i);
         want = true;
       }
     }
@@ -611,12 +704,13 @@ __global__ void __launch_bounds__(kBlock) k_batch_shade(DevBatch bt, DevQueues q
     e.cont = false;
     e.shadow = false;
     if (i < n) {
-      const int pix = __float_as_int(q.org_q(cur)[i].w);
-      const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, pix)];
+      const float4 o = q.org_q(cur)[i], d = q.dir_q(cur)[i], t = q.thr_q(cur)[i];
+      const int2 h = q.hit[i];
+      const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, __float_as_int(o.w))];
       if (J.f.shading_mode == CT_MODE_FULL)
-        shade_full(J.sc, q, J.f, cur, i, path_length, e, J.pix_base, J.accum);
+        shade_full(J.sc, q, J.f, o, d, t, h, path_length, e, J.pix_base, J.accum);
       else
-        shade_compat(J.sc, q, J.f, cur, i, path_length, e, J.pix_base, J.accum);
+        shade_compat(J.sc, q, J.f, o, d, t, h, path_length, e, J.pix_base, J.accum);
       if (pass + 1 >= J.max_depth) e.cont = false;
     }
     const int si = warp_append(e.shadow, &q.counts[2]);

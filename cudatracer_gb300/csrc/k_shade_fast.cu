@@ -6,11 +6,15 @@
 
 namespace ct {
 namespace exact {
+constexpr int kPathBlock = fast::kPathBlock;
 __global__ void __launch_bounds__(128) k_shade(DevScene sc, DevQueues q, FrameConst f, int cur, uint32_t path_length);
 __global__ void __launch_bounds__(128) k_raygen(DevQueues q, FrameConst f);
 __global__ void __launch_bounds__(128) k_batch_raygen(DevBatch bt, DevQueues q);
 __global__ void __launch_bounds__(128) k_batch_shade(DevBatch bt, DevQueues q, int cur, uint32_t path_length, int pass);
 __global__ void k_batch_advance(DevBatch bt, DevQueues q);
+__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth);
+__global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
+                                                         int max_depth);
 }  // namespace exact
 
 namespace {
@@ -84,6 +88,15 @@ cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact_mat
   } else {
     fast::k_raygen<<<fill_grid(fast::k_raygen, npix), kBlock, 0, s>>>(q, f);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
+                        int exact_math, bool fast_traversal, cudaStream_t s) {
+  auto kernel = !exact_math ? fast::k_path : (fast_traversal ? exact::k_path : exact::k_path_ref);
+  const size_t smem = (size_t)b.stack_entries * fast::kPathBlock * sizeof(int);  // at most 256 entries: 32 KB
+  const int grid = (f.width * f.height + fast::kPathBlock - 1) / fast::kPathBlock;
+  kernel<<<grid, fast::kPathBlock, smem, s>>>(sc, b, q, f, max_depth);
   return cudaGetLastError();
 }
 
