@@ -874,8 +874,8 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   if (werr) return cleanup(fail(ctx, CT_ERR_UNSUPPORTED, "wide BVH collapse failed (code " + std::to_string(werr) +
                                                               "): a leaf needs more than 8 slots or a box did not quantise"));
   void* nodes = nullptr;
-  if ((s = pool_alloc(ctx, b->allocs, &nodes, (size_t)nw * sizeof(WNode8), st)) != CT_OK) return cleanup(s);
-  e = gpu_wbvh_copy_nodes(scratch2, r.binary_nodes, (WNode8*)nodes, nw, st);
+  if ((s = pool_alloc(ctx, b->allocs, &nodes, (size_t)nw * sizeof(WNodeDev), st)) != CT_OK) return cleanup(s);
+  e = gpu_wbvh_copy_nodes(scratch2, r.binary_nodes, (WNodeDev*)nodes, nw, st);
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "wide BVH copy"));
   e = st ? cudaStreamSynchronize(st) : cudaDeviceSynchronize();
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "wide BVH build"));
@@ -883,7 +883,7 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   b->wide = true;
   b->device_built = true;
   b->device = ctx->device;
-  b->wdev.nodes = (const WNode8*)nodes;
+  b->wdev.nodes = (const WNodeDev*)nodes;
   b->wdev.tris = (const float4*)tris;
   b->wdev.node_count = nw;
   b->wdev.prim_count = n;
@@ -987,9 +987,15 @@ ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, ui
   if (bvh->wide) {
     if (layout != CT_BVH_WIDE8_Q8) return nodes ? CT_ERR_UNSUPPORTED : CT_OK;
     if (cudaSetDevice(bvh->device) != cudaSuccess) return CT_ERR_CUDA;
-    if (nodes && cudaMemcpy(nodes, bvh->wdev.nodes, (size_t)bvh->wdev.node_count * sizeof(WNode8),
-                            cudaMemcpyDeviceToHost) != cudaSuccess)
-      return CT_ERR_CUDA;
+    if (nodes) {
+      std::vector<WNodeDev> dev(bvh->wdev.node_count);
+      if (cudaMemcpy(dev.data(), bvh->wdev.nodes, dev.size() * sizeof(WNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return CT_ERR_CUDA;
+      for (size_t i = 0; i < dev.size(); i++) {
+        const WNode8 w = wide_node8(dev[i]);
+        std::memcpy((char*)nodes + i * sizeof(w), &w, sizeof(w));
+      }
+    }
     if (prim_indices) {
       std::vector<float4> tri((size_t)bvh->nt * 3);
       if (cudaMemcpy(tri.data(), bvh->wdev.tris, tri.size() * sizeof(float4), cudaMemcpyDeviceToHost) != cudaSuccess)

@@ -1324,10 +1324,57 @@ cudaError_t gpu_wbvh_collapse(const DevScene& sc, const void* arena_v, const uin
   return cudaSuccess;
 }
 
-cudaError_t gpu_wbvh_copy_nodes(void* scratch2, uint32_t binary_nodes, WNode8* out, uint32_t count, cudaStream_t s) {
+namespace {
+__global__ void __launch_bounds__(256) k_wdev(const WNode8* __restrict__ in, uint32_t n, WNodeDev* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const WNode8 w = in[i];
+  WNodeDev d;
+  d.p[0] = w.px, d.p[1] = w.py, d.p[2] = w.pz;
+  d.imask = w.imask;
+  for (int a = 0; a < 3; a++) {
+    d.e[a] = w.e[a];
+    for (int k = 0; k < 8; k++) d.q[a][0][k] = w.qlo[a][k], d.q[a][1][k] = w.qhi[a][k];
+  }
+  for (int k = 0; k < 8; k++) {
+    const uint32_t m = w.meta[k];
+    d.ent[k] = m == 0 ? 0u
+               : (m & 0x80u) ? w.child_base + (m & 7u)
+                             : (0x80000000u | ((m >> 5) << 29) | (w.prim_base + (m & 31u)));
+  }
+  out[i] = d;
+}
+}  // namespace
+
+cudaError_t gpu_wbvh_copy_nodes(void* scratch2, uint32_t binary_nodes, WNodeDev* out, uint32_t count, cudaStream_t s) {
   const WLayout W(binary_nodes);
-  GB_TRY(cudaMemcpyAsync(out, at<WNode8>(scratch2, W.nodes), sizeof(WNode8) * (size_t)count, cudaMemcpyDeviceToDevice, s));
-  return cudaSuccess;
+  if (count) k_wdev<<<blocks(count, 256), 256, 0, s>>>(at<WNode8>(scratch2, W.nodes), count, out);
+  return cudaGetLastError();
 }
 
+WNode8 wide_node8(const WNodeDev& d) {
+  WNode8 w;
+  std::memset(&w, 0, sizeof(w));
+  w.px = d.p[0], w.py = d.p[1], w.pz = d.p[2];
+  w.imask = d.imask;
+  for (int a = 0; a < 3; a++) {
+    w.e[a] = d.e[a];
+    for (int k = 0; k < 8; k++) w.qlo[a][k] = d.q[a][0][k], w.qhi[a][k] = d.q[a][1][k];
+  }
+  // children and triangles are numbered in slot order from the node's first ones
+  bool child = false, prim = false;
+  for (int k = 0; k < 8; k++) {
+    const uint32_t ent = d.ent[k];
+    if (ent == 0) continue;
+    if (ent & 0x80000000u) {
+      const uint32_t first = ent & 0x1fffffffu;
+      if (!prim) w.prim_base = first, prim = true;
+      w.meta[k] = (uint8_t)((((ent >> 29) & 3u) << 5) | (first - w.prim_base));
+    } else {
+      if (!child) w.child_base = ent, child = true;
+      w.meta[k] = (uint8_t)(0x80u | (ent - w.child_base));
+    }
+  }
+  return w;
+}
 }  // namespace ct

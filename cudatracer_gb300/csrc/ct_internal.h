@@ -54,10 +54,23 @@ struct __align__(16) WNode8 {
 };
 static_assert(sizeof(WNode8) == 80, "WNode8 is 80 bytes");
 
+// The same node as the kernels read it: 96 bytes, three 32-byte loads, the slot
+// codes resolved.
+//   ent[i]: 0 empty; bit 31 leaf, bits 29-30 triangles, bits 0-28 first triangle;
+//           otherwise the child node
+struct __align__(32) WNodeDev {
+  float p[3];
+  uint8_t e[3];
+  uint8_t imask;
+  uint8_t q[3][2][8];  // axis, lo / hi, slot
+  uint32_t ent[8];
+};
+static_assert(sizeof(WNodeDev) == 96, "WNodeDev is 96 bytes");
+
 // Triangles of the wide tree in leaf order, 48 bytes: {p0, prim id}, {p1, 0}, {p2, 0}
 // (raw vertices: the watertight test shears them per ray).
 struct DevWBVH {
-  const WNode8* nodes;
+  const WNodeDev* nodes;
   const float4* tris;
   uint32_t node_count;
   uint32_t prim_count;
@@ -290,7 +303,9 @@ size_t gpu_wbvh_scratch_bytes(uint32_t binary_nodes);
 cudaError_t gpu_wbvh_collapse(const DevScene& sc, const void* arena, const uint32_t* prims, const WideCost* cost,
                               void* scratch2, uint32_t binary_nodes, float4* tris, uint32_t* host_counters,
                               cudaStream_t s, uint32_t* wide_nodes, uint32_t* depth, uint32_t* error);
-cudaError_t gpu_wbvh_copy_nodes(void* scratch2, uint32_t binary_nodes, WNode8* out, uint32_t count, cudaStream_t s);
+cudaError_t gpu_wbvh_copy_nodes(void* scratch2, uint32_t binary_nodes, WNodeDev* out, uint32_t count, cudaStream_t s);
+// The 80-byte node a WNodeDev was made from (host).
+WNode8 wide_node8(const WNodeDev& d);
 
 // Wide-tree queries: FP32 watertight tests; hits within the FP32 error bound
 // of an edge or of another hit's t are settled by FP64 tests in a second

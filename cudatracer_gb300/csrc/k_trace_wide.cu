@@ -188,72 +188,79 @@ __device__ __forceinline__ bool tri64(const Ray64& q, const float4* tris, uint32
 // Slab distances of a node's eight slots, set up once per node and ray.
 // Per axis a, with s = 2^(e - 127) the quantisation step and inv = 1/d:
 //   A = s * inv (exact: a power of two times a float),  B = (p - o) * inv,
-// so a plane q (0..255) lies at t = q * A + B, one fused multiply-add. Only the
-// ray's near plane (lo for inv >= 0, hi otherwise) and far plane of each axis
-// are evaluated, so no min/max per axis is needed. Every computed t differs
-// from the exact distance (L - o) / d of the builder's outward-rounded plane
+// so a plane q (0..255) lies at t = q * A + B. The byte goes into the middle of
+// the bits of 2^15, where it counts in ones (m = 2^15 + q, one byte permute and no
+// conversion), and t = m * A + (B - 2^15 A) is half of one packed fused
+// multiply-add, near and far plane together. Only the ray's near plane (lo for
+// inv >= 0, hi otherwise) and far plane of each axis are evaluated, so no min/max
+// per axis is needed. Without the offset every computed t would differ from the
+// exact distance (L - o) / d of the builder's outward-rounded plane
 // L = fl(p + s q) by at most
 //   E = 5u (255 |A| + |B| + |p inv|) + 1e-30      (u = 2^-24)
 // (the rounding of inv, of p - o, of the product and of the FMA, and the
 // half-ulp by which p + s q may lie inside L; the last term covers underflow).
-// E is folded into the offsets: near planes use Bn = B - E, far planes
-// Bf = B + E (E is raised by the rounding of those two sums), so a slot's
-// [max near, min far] interval contains the exact one and no box the ray
-// touches is rejected.
+// B - 2^15 A and the two sums below round once each, by at most u of
+// 2^15 |A| + |B| + E, and E is raised by three of those (6e-3 steps). E is folded
+// into the offsets: near planes use B - E, far planes B + E, so a slot's
+// [max near, min far] interval contains the exact one and no box the ray touches
+// is rejected.
 struct SlabSetup {
   uint32_t nq[3][2], fq[3][2];  // near / far plane bytes of slots 0-3 and 4-7, per axis
-  float A[3], Bn[3], Bf[3];
+  float A[3], Bn[3], Bf[3];     // Bn, Bf less 2^15 A
+  uint32_t ent[8];              // WNodeDev::ent
 };
 
-__device__ __forceinline__ void slab_axis(float p, float e_scale, float o, float inv, uint2 lo, uint2 hi,
-                                          uint32_t* nq, uint32_t* fq, float& A, float& Bn, float& Bf) {
-  A = __fmul_rn(e_scale, inv);
+__device__ __forceinline__ void slab_axis(float p, uint32_t e, float o, float inv, uint32_t lo0, uint32_t lo1,
+                                          uint32_t hi0, uint32_t hi1, uint32_t* nq, uint32_t* fq, float& A, float& Bn,
+                                          float& Bf) {
+  A = __fmul_rn(__uint_as_float(e << 23), inv);
   const float B = __fmul_rn(__fsub_rn(p, o), inv);
   const float u = 5.9604645e-08f;
   float E = (5.0f * u) * (255.0f * fabsf(A) + fabsf(B) + fabsf(__fmul_rn(p, inv))) + 1e-30f;
-  E = E + (2.0f * u) * (fabsf(B) + E);  // the rounding of B -/+ E below
-  Bn = __fsub_rn(B, E);
-  Bf = __fadd_rn(B, E);
+  E = E + (3.0f * u) * (32768.0f * fabsf(A) + fabsf(B) + E);
+  const float off = __fmaf_rn(-32768.0f, A, B);
+  Bn = __fsub_rn(off, E);
+  Bf = __fadd_rn(off, E);
   const bool pos = inv >= 0.0f;
-  nq[0] = pos ? lo.x : hi.x, nq[1] = pos ? lo.y : hi.y;
-  fq[0] = pos ? hi.x : lo.x, fq[1] = pos ? hi.y : lo.y;
+  nq[0] = pos ? lo0 : hi0, nq[1] = pos ? lo1 : hi1;
+  fq[0] = pos ? hi0 : lo0, fq[1] = pos ? hi1 : lo1;
 }
 
-__device__ __forceinline__ void slab_setup(const WNode8& n, float ox, float oy, float oz, float ix, float iy, float iz,
-                                           SlabSetup& S) {
-  const uint2* qlo = reinterpret_cast<const uint2*>(&n.qlo[0][0]);
-  const uint2* qhi = reinterpret_cast<const uint2*>(&n.qhi[0][0]);
-  slab_axis(n.px, __int_as_float((int)n.e[0] << 23), ox, ix, qlo[0], qhi[0], S.nq[0], S.fq[0], S.A[0], S.Bn[0],
-            S.Bf[0]);
-  slab_axis(n.py, __int_as_float((int)n.e[1] << 23), oy, iy, qlo[1], qhi[1], S.nq[1], S.fq[1], S.A[1], S.Bn[1],
+__device__ __forceinline__ void load_slabs(const WNodeDev* nodes, uint32_t i, float ox, float oy, float oz, float ix,
+                                           float iy, float iz, SlabSetup& S) {
+  const float4* n = reinterpret_cast<const float4*>(nodes + i);
+  float4 p, qx, qy, qz, e0, e1;
+  ldg256(n, p, qx);
+  ldg256(n + 2, qy, qz);
+  ldg256(n + 4, e0, e1);
+  const uint32_t e = __float_as_uint(p.w);
+  auto w = [](float f) { return __float_as_uint(f); };
+  slab_axis(p.x, e & 0xffu, ox, ix, w(qx.x), w(qx.y), w(qx.z), w(qx.w), S.nq[0], S.fq[0], S.A[0], S.Bn[0], S.Bf[0]);
+  slab_axis(p.y, (e >> 8) & 0xffu, oy, iy, w(qy.x), w(qy.y), w(qy.z), w(qy.w), S.nq[1], S.fq[1], S.A[1], S.Bn[1],
             S.Bf[1]);
-  slab_axis(n.pz, __int_as_float((int)n.e[2] << 23), oz, iz, qlo[2], qhi[2], S.nq[2], S.fq[2], S.A[2], S.Bn[2],
+  slab_axis(p.z, (e >> 16) & 0xffu, oz, iz, w(qz.x), w(qz.y), w(qz.z), w(qz.w), S.nq[2], S.fq[2], S.A[2], S.Bn[2],
             S.Bf[2]);
+  S.ent[0] = w(e0.x), S.ent[1] = w(e0.y), S.ent[2] = w(e0.z), S.ent[3] = w(e0.w);
+  S.ent[4] = w(e1.x), S.ent[5] = w(e1.y), S.ent[6] = w(e1.z), S.ent[7] = w(e1.w);
 }
 
-__device__ __forceinline__ float qbyte(const uint32_t* w, int i) { return (float)((w[i >> 2] >> (8 * (i & 3))) & 0xffu); }
+// 2^15 + byte i of w as a float
+__device__ __forceinline__ float qbyte(const uint32_t* w, int i) {
+  return __uint_as_float(__byte_perm(i < 4 ? w[0] : w[1], 0x47000000u, 0x7404u | ((uint32_t)(i & 3) << 4)));
+}
+__device__ __forceinline__ void slot_axis(const SlabSetup& S, int a, int i, float& tn, float& tf) {
+  unpack2(fma2(pack2(qbyte(S.nq[a], i), qbyte(S.fq[a], i)), pack2(S.A[a], S.A[a]), pack2(S.Bn[a], S.Bf[a])), tn, tf);
+}
 
-// Entry distance of slot i (clamped at 0), or +inf when the slot's box is
-// missed or begins beyond tfar.
+// Entry distance of slot i (clamped at 0), or +inf when the slot is empty, its
+// box is missed or begins beyond tfar.
 __device__ __forceinline__ float slot_test(const SlabSetup& S, int i, float tfar) {
-  const float nx = __fmaf_rn(qbyte(S.nq[0], i), S.A[0], S.Bn[0]), fx = __fmaf_rn(qbyte(S.fq[0], i), S.A[0], S.Bf[0]);
-  const float ny = __fmaf_rn(qbyte(S.nq[1], i), S.A[1], S.Bn[1]), fy = __fmaf_rn(qbyte(S.fq[1], i), S.A[1], S.Bf[1]);
-  const float nz = __fmaf_rn(qbyte(S.nq[2], i), S.A[2], S.Bn[2]), fz = __fmaf_rn(qbyte(S.fq[2], i), S.A[2], S.Bf[2]);
-  const float tn = fmaxf(fmaxf(nx, ny), fmaxf(nz, 0.0f));
-  const float tf = fminf(fminf(fx, fy), fminf(fz, tfar));
-  return tn <= tf ? tn : __int_as_float(0x7f800000);
-}
-
-__device__ __forceinline__ void load_node(const WNode8* nodes, uint32_t i, WNode8& n) {
-  const float4* s = reinterpret_cast<const float4*>(nodes + i);
-  float4* d = reinterpret_cast<float4*>(&n);
-#pragma unroll
-  for (int k = 0; k < 5; k++) d[k] = __ldg(s + k);
-}
-
-__device__ __forceinline__ uint32_t meta_at(const WNode8& n, int i) {
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(n.meta);
-  return ((i < 4 ? w[0] : w[1]) >> (8 * (i & 3))) & 0xffu;
+  float nx, ny, nz, fx, fy, fz;
+  slot_axis(S, 0, i, nx, fx);
+  slot_axis(S, 1, i, ny, fy);
+  slot_axis(S, 2, i, nz, fz);
+  const float tn = fmaxf(max3(nx, ny, nz), 0.0f), tf = fminf(min3(fx, fy, fz), tfar);
+  return tn <= tf && S.ent[i] != 0u ? tn : __int_as_float(0x7f800000);
 }
 
 // A warp refills its idle lanes from the cursor once this many are idle (or
@@ -262,6 +269,8 @@ __device__ __forceinline__ uint32_t meta_at(const WNode8& n, int i) {
 // and 16; frames on the wide tree: 8.
 constexpr int kWideRefill = 4;
 constexpr int kWideFrameRefill = 8;
+
+constexpr uint32_t kLeafEntry = 0x80000000u;  // WNodeDev::ent, stack entries
 
 // Whole traversal in FP64 triangle tests (boxes as above, culled with the FP64
 // best distance rounded up): the fallback for rays with too many candidates.
@@ -278,27 +287,27 @@ __device__ bool trace_fp64(const DevWBVH& b, const WRay& r, uint32_t* st_node, f
     const uint32_t ni = st_node[sp];
     const float far = __double2float_ru(tb) * kFarScale;
     if (st_t[sp] > far) continue;
-    WNode8 n;
     SlabSetup S;
-    load_node(b.nodes, ni, n);
-    slab_setup(n, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
+    load_slabs(b.nodes, ni, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
+    float tns[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) tns[i] = slot_test(S, i, far);
     for (int i = 0; i < 8; i++) {
-      const uint32_t m = meta_at(n, i);
-      if (!m) continue;
-      const float tn = slot_test(S, i, far);
-      if (!(tn <= far)) continue;
-      if (m & 0x80u) {
+      const float tn = tns[i];
+      if (!(tn <= far) || S.ent[i] == 0u) continue;
+      const uint32_t ent = S.ent[i];
+      if (!(ent & kLeafEntry)) {
         if (sp >= kWStack) {
           atomicOr(err, kErrStackOverflow);
           continue;
         }
-        st_node[sp] = n.child_base + (m & 7u), st_t[sp] = tn, sp++;
+        st_node[sp] = ent, st_t[sp] = tn, sp++;
         continue;
       }
-      const uint32_t cnt = m >> 5, off = m & 31u;
+      const uint32_t cnt = (ent >> 29) & 3u;
       for (uint32_t k = 0; k < cnt; k++) {
         double t;
-        const uint32_t slot = n.prim_base + off + k;
+        const uint32_t slot = (ent & 0x1fffffffu) + k;
         if (!tri64(q, b.tris, slot, t)) continue;
         const int prim = __float_as_int(__ldg(b.tris + 3 * (size_t)slot).w);
         if (ANY) {
@@ -313,8 +322,6 @@ __device__ bool trace_fp64(const DevWBVH& b, const WRay& r, uint32_t* st_node, f
   return best >= 0;
 }
 
-constexpr uint32_t kLeafEntry = 0x80000000u;  // stack entry: bit 31 leaf, bits 29-30 count, 0-28 first triangle
-
 // Settlement records: a ray whose closest hit (or occlusion) FP32 could not
 // decide is not settled in the traversal kernel, where the few lanes doing
 // FP64 work would hold their warp's other lanes idle (binary64 runs at a small
@@ -328,13 +335,36 @@ constexpr uint32_t kLeafEntry = 0x80000000u;  // stack entry: bit 31 leaf, bits 
 constexpr int kRecCand = 5;
 constexpr uint32_t kRecFull = 0x80000000u;
 
+// A traversal stack of {entry, entry distance}: the first kWShared entries in
+// shared memory, the rest, which few rays reach, in local memory. Entries in local
+// memory went through the L1 lines that nodes and triangles need: 4 M incoherent
+// rays against 4 M triangles 4.98 -> 4.48 ms with the first 16 in shared memory
+// (8 or 12: 4.52, 20: 4.47; 16 leaves room for the 8 blocks).
+constexpr int kWShared = 16;
+struct WStack {
+  uint2* sm;  // stride 128
+  uint2 far[kWStack + 7 - kWShared];  // a node pushes at most seven before the check
+  __device__ __forceinline__ void set(int i, uint2 v) {
+    if (i < kWShared) sm[i * 128] = v;
+    else far[i - kWShared] = v;
+  }
+  __device__ __forceinline__ uint2 at(int i) const { return i < kWShared ? sm[i * 128] : far[i - kWShared]; }
+};
+
 // Persistent traversal: each lane owns a ray and takes one step per round —
 // an inner node (eight slab tests; inner children and leaf groups pushed,
-// the nearest on top) or one leaf group (up to three triangle tests) — so
-// the warp's lanes do similar work each round; a lane whose ray is done takes
-// the next ray from the device cursor (one atomicAdd per warp). A ray that
-// would overflow the stack or keep more than kRecCand candidates is recorded
-// for a traversal entirely in FP64.
+// the nearest on top) or one triangle of a leaf group — so the warp's lanes do
+// similar work each round; a lane whose ray is done takes the next ray from the
+// device cursor (one atomicAdd per warp). A ray that would overflow the stack or
+// keep more than kRecCand candidates is recorded for a traversal entirely in FP64.
+//
+// Bound by instruction issue (62 %) with half of a warp's lanes at work, and by the
+// 32-byte sectors of nodes and triangles from L2. Hence three 32-byte loads for a
+// node (L1 serves one line of one lane per load, at any width), slot codes resolved
+// when the tree is built, eight slots tested without a branch, and one triangle per
+// round. 4 M incoherent rays, 4 M triangles: 6.07 -> 4.62 ms; 1 M rays, 100 k
+// triangles: 1.04 -> 0.80 ms. Lanes that wait until eight are at a leaf gain 3 %
+// there and lose 10 % on small calls; they don't wait.
 //   counters[0]  ray fetch cursor;  counters[1]  records written
 template <bool ANY>
 // 8 resident blocks of 128 threads per SM (64 registers): measured ahead of 6 (80 registers)
@@ -343,8 +373,8 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const fl
                                                     float* __restrict__ t_out, uint8_t* __restrict__ occ_out,
                                                     uint32_t n, int* counters, uint4* recs,
                                                     unsigned long long* stats) {
-  uint32_t st_node[kWStack];
-  float st_t[kWStack];
+  __shared__ uint2 s_stack[kWShared][128];
+  WStack st{&s_stack[0][threadIdx.x]};
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -382,33 +412,33 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const fl
     }
     if (__ballot_sync(FULL, rid >= 0) == 0) break;
     bool record = false;
+    const float far = (tb + tberr) * kFarScale;
+    if (rid >= 0 && !have_cur) {
+      while (sp > 0 && !have_cur) {
+        const uint2 e = st.at(--sp);
+        if (!(__uint_as_float(e.y) > far)) cur = e.x, have_cur = true;  // else culled
+      }
+    }
     if (rid >= 0) {
-      // ---- one step
-      const float far = (tb + tberr) * kFarScale;
-      if (!have_cur)
-        while (sp > 0 && st_t[sp - 1] > far) sp--;  // culled entries
-      bool finished = (!have_cur && sp == 0) || overflow || (ANY && occluded);
+      // ---- one step: a node, or one triangle of a leaf group
+      bool finished = !have_cur || overflow || (ANY && occluded);
       if (!finished) {
-        const uint32_t ent = have_cur ? cur : st_node[--sp];
         have_cur = false;
-        if (ent & kLeafEntry) {
-          const uint32_t cnt = (ent >> 29) & 3u, first = ent & 0x1fffffffu;
-          for (uint32_t k = 0; k < cnt; k++) {
-            const uint32_t slot = first + k;
+        if (cur & kLeafEntry) {
+          const uint32_t cnt = (cur >> 29) & 3u, slot = cur & 0x1fffffffu;
+          if (cnt > 1) cur = (cur - (1u << 29)) + 1u, have_cur = true;  // the rest of the group
+          do {
             const float4* tr = b.tris + 3 * (size_t)slot;
             float t, terr;
             const int res = tri32(r, __ldg(tr), __ldg(tr + 1), __ldg(tr + 2), t, terr);
-            if (res == 0) continue;
+            if (res == 0) break;
             if (res == 1 && t - terr > 0.0f && t + terr < tb - tberr) {
               // certainly in range and certainly nearer than the best so far
               best = (int)slot, tb = t, tberr = terr;
-              if (ANY) {
-                occluded = true;
-                break;
-              }
-              continue;
+              if (ANY) occluded = true;
+              break;
             }
-            if (!(t - terr < tb + tberr)) continue;  // certainly beyond the best (or the ray's end)
+            if (!(t - terr < tb + tberr)) break;  // certainly beyond the best (or the ray's end)
             if (res == 1 && t - terr > 0.0f && t < tb && t + terr < tb + tberr) {
               // a certain hit nearer than the best within their errors: FP64 orders them
               if (best >= 0) {
@@ -416,64 +446,41 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const fl
                 else overflow = true;
               }
               best = (int)slot, tb = t, tberr = terr;
-              continue;
+              break;
             }
             if (nc < kRecCand) cand[nc] = slot, cand_lo[nc] = t - terr, nc++;
             else overflow = true;
-          }
+          } while (false);
         } else {
-          WNode8 nd;
           SlabSetup S;
-          load_node(b.nodes, ent, nd);
-          slab_setup(nd, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
-          // the nearest hit slot is visited next without a stack round trip; the
-          // others are pushed (a slot displaced as nearest is pushed when replaced).
-          // Closest hit also keeps the second nearest in a register and pushes it
-          // last, so it is the next entry popped (closer hits found sooner cull
-          // more; any hit stops at its first hit, where the order only costs)
-          float tcur = __int_as_float(0x7f800000), tsec = __int_as_float(0x7f800000);
-          uint32_t sec = 0;
-          bool have_sec = false;
+          load_slabs(b.nodes, cur, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
+          // All slots first, without a branch. The nearest hit slot is visited next
+          // without a stack round trip; closest hit pushes the second nearest last, so
+          // that it is the next entry popped (closer hits found sooner cull more; any
+          // hit stops at its first hit, where the order only costs), and a third in
+          // order costs more than it culls (4.66 against 4.48 ms).
+          constexpr int kOrdered = ANY ? 1 : 2;
+          const float inf = __int_as_float(0x7f800000);
+          float tn[8];
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const uint32_t m = meta_at(nd, i);
-            if (!m) continue;
-            const float tn = slot_test(S, i, far);
-            if (!(tn <= far)) continue;
-            const uint32_t ce = (m & 0x80u) ? nd.child_base + (m & 7u)
-                                            : (kLeafEntry | ((m >> 5) << 29) | (nd.prim_base + (m & 31u)));
-            uint32_t pe = ce;
-            float pt = tn;
-            if (tn < tcur) {
-              pe = cur, pt = tcur;
-              cur = ce, tcur = tn;
-              if (!have_cur) {
-                have_cur = true;
-                continue;
-              }
-            }
-            if (!ANY) {
-              if (!have_sec) {
-                sec = pe, tsec = pt, have_sec = true;
-                continue;
-              }
-              if (pt < tsec) {
-                const uint32_t e2 = sec;
-                const float t2 = tsec;
-                sec = pe, tsec = pt;
-                pe = e2, pt = t2;
-              }
-            }
-            if (sp >= kWStack) {
-              overflow = true;  // settled by the full FP64 traversal
-              continue;
-            }
-            st_node[sp] = pe, st_t[sp] = pt, sp++;
+          for (int i = 0; i < 8; i++) tn[i] = slot_test(S, i, far);
+          uint32_t near_e[kOrdered];
+          float near_t[kOrdered];
+#pragma unroll
+          for (int k = 0; k < kOrdered; k++) {
+            near_t[k] = fminf(min3(tn[0], tn[1], tn[2]), fminf(min3(tn[3], tn[4], tn[5]), fminf(tn[6], tn[7])));
+            near_e[k] = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              if (near_e[k] == 0 && tn[i] == near_t[k] && near_t[k] < inf) near_e[k] = S.ent[i], tn[i] = inf;
           }
-          if (!ANY && have_sec) {
-            if (sp >= kWStack) overflow = true;
-            else st_node[sp] = sec, st_t[sp] = tsec, sp++;
-          }
+          if (near_t[0] < inf) cur = near_e[0], have_cur = true;
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            if (tn[i] < inf) st.set(sp++, make_uint2(S.ent[i], __float_as_uint(tn[i])));
+          if (!ANY && near_t[kOrdered - 1] < inf)
+            st.set(sp++, make_uint2(near_e[kOrdered - 1], __float_as_uint(near_t[kOrdered - 1])));
+          if (sp > kWStack) overflow = true;  // settled by the full FP64 traversal
         }
         finished = (!have_cur && sp == 0) || overflow || (ANY && occluded);
       }
@@ -649,23 +656,18 @@ __device__ __forceinline__ void trace_wide_mt(int n, int* cursor, IO& io, uint32
         }
         finished = ANY && hit >= 0;
       } else {
-        WNode8 nd;
         SlabSetup S;
-        load_node(b.nodes, ent, nd);
-        slab_setup(nd, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
+        load_slabs(b.nodes, ent, r.ox, r.oy, r.oz, r.ix, r.iy, r.iz, S);
         const int sp0 = sp;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          const uint32_t m = meta_at(nd, i);
-          if (!m) continue;
           const float tn = slot_test(S, i, far);
-          if (!(tn <= far)) continue;
+          if (!(tn < __int_as_float(0x7f800000))) continue;
           if (sp >= kWStack) {
             overflow = true;
             continue;
           }
-          st_node[sp] = (m & 0x80u) ? nd.child_base + (m & 7u)
-                                    : (kLeafEntry | ((m >> 5) << 29) | (nd.prim_base + (m & 31u)));
+          st_node[sp] = S.ent[i];
           st_t[sp] = tn;
           sp++;
         }
