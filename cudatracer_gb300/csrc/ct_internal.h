@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstddef>
 
 namespace ct {
@@ -234,6 +235,16 @@ cudaError_t launch_shade(const DevScene& sc, const DevQueues& q, const FrameCons
                          int exact, cudaStream_t s);
 // A whole frame in one kernel on a quad tree (frames of few pixels): as raygen and
 // max_depth x (extend, shade, connect if f.shadow) into the same q.accum or q.log.
+// How many lanes of a warp take rays (or paths) when a call has n of them: a
+// small call is as long as its longest ray, and a warp's round is shorter the
+// fewer rays share it (fewer lines to fetch, seldom a node and a leaf in one round),
+// so up to 24,576 rays are spread over 768 warps, about 5 an SM. More warps cost
+// more than they give: 65,536 incoherent rays 121 us with 32 lanes, 147 with 16 and
+// 222 with 8; 16,384: 91 with 32, 90 with 16, 102 with 8; 4,096 rays on an
+// 81,920-triangle sphere 161 us with 32, 143 with 6, 135 with 4; a 64x48 frame 129
+// with 32, 99 with 4; a 16x16 frame 161 with 32, 100 with 1.
+inline int lanes_for(uint32_t n) { return (int)std::min<uint32_t>(32, (n - 1) / 768 + 1); }
+
 cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
                         int exact_math, bool fast_traversal, cudaStream_t s);
 cudaError_t launch_present(const float4* accum, float4* out, int n, float samples, cudaStream_t s);

@@ -576,7 +576,7 @@ __device__ __forceinline__ void stored(float4& v) { asm volatile("" : "+f"(v.x),
 // and the compaction between stages has nothing to fill. Each path does what
 // the stages do with the same operations in the same order, so the frame's
 // contributions are the same bits, added to q.accum (or logged) per pixel in
-// the same order. A 64x48, depth-5 frame takes 126 us when waited for and 50 us
+// the same order. A 64x48, depth-5 frame takes 99 us when waited for and 50 us
 // among others (the host calls), with the stages 343 and 98 us.
 // shade_full as a function of its own: k_path then holds 93 registers instead of
 // 124 (362x362 frames 191 -> 174 us), and in the build with FMA contraction it is
@@ -588,13 +588,13 @@ __device__ __noinline__ void shade_full_call(const DevScene* sc, const DevQueues
 
 template <bool FASTMM>
 __device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b, DevQueues& q, const FrameConst& f,
-                                            int max_depth) {
+                                            int max_depth, int lanes) {
   extern __shared__ int s_stack[];
   int* stack = s_stack + threadIdx.x;
   const int npix = f.width * f.height;
   unsigned long long n_ext = 0, n_shadow = 0;
-  const int j = blockIdx.x * kPathBlock + threadIdx.x;
-  bool alive = j < npix;
+  const int j = blockIdx.x * lanes + threadIdx.x;  // lanes_for(npix) of a warp's lanes have a path
+  bool alive = (int)threadIdx.x < lanes && j < npix;
   float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f), d = o, t = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
   if (alive) primary_ray(f, tile_pixel(j, f.width, f.height), o, d);
   stored(o), stored(d);
@@ -651,14 +651,15 @@ __device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b,
     }
   }
 }
-__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth) {
-  trace_paths<true>(sc, b, q, f, max_depth);
+__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth,
+                                                     int lanes) {
+  trace_paths<true>(sc, b, q, f, max_depth, lanes);
 }
 #if CT_EXACT
 // with the reference's traversal (CT_MATH_EXACT)
 __global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
-                                                         int max_depth) {
-  trace_paths<false>(sc, b, q, f, max_depth);
+                                                         int max_depth, int lanes) {
+  trace_paths<false>(sc, b, q, f, max_depth, lanes);
 }
 #endif
 

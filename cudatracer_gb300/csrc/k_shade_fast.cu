@@ -12,9 +12,10 @@ __global__ void __launch_bounds__(128) k_raygen(DevQueues q, FrameConst f);
 __global__ void __launch_bounds__(128) k_batch_raygen(DevBatch bt, DevQueues q);
 __global__ void __launch_bounds__(128) k_batch_shade(DevBatch bt, DevQueues q, int cur, uint32_t path_length, int pass);
 __global__ void k_batch_advance(DevBatch bt, DevQueues q);
-__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth);
+__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth,
+                                                     int lanes);
 __global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
-                                                         int max_depth);
+                                                         int max_depth, int lanes);
 }  // namespace exact
 
 namespace {
@@ -95,8 +96,8 @@ cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q,
                         int exact_math, bool fast_traversal, cudaStream_t s) {
   auto kernel = !exact_math ? fast::k_path : (fast_traversal ? exact::k_path : exact::k_path_ref);
   const size_t smem = (size_t)b.stack_entries * fast::kPathBlock * sizeof(int);  // at most 256 entries: 32 KB
-  const int grid = (f.width * f.height + fast::kPathBlock - 1) / fast::kPathBlock;
-  kernel<<<grid, fast::kPathBlock, smem, s>>>(sc, b, q, f, max_depth);
+  const int npix = f.width * f.height, lanes = lanes_for((uint32_t)npix);
+  kernel<<<(npix + lanes - 1) / lanes, fast::kPathBlock, smem, s>>>(sc, b, q, f, max_depth, lanes);
   return cudaGetLastError();
 }
 

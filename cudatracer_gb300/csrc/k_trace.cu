@@ -102,9 +102,10 @@ struct ExtendIO {
 };
 
 template <bool ANY>
-__global__ void __launch_bounds__(kBlock) k_query(DevBVH b, QueryIO io, int n, int* cursor, float eps) {
+__global__ void __launch_bounds__(kBlock) k_query(DevBVH b, QueryIO io, int n, int* cursor, float eps,
+                                              int lanes) {
   extern __shared__ int s_stack[];
-  trace_persistent<ANY, false, kQueryRefill>(b, n, cursor, eps, io, s_stack + threadIdx.x, kBlock);
+  trace_persistent<ANY, false, kQueryRefill>(b, n, cursor, eps, io, s_stack + threadIdx.x, kBlock, lanes);
 }
 
 template <bool FASTMM>
@@ -161,9 +162,10 @@ cudaError_t launch_query(const DevBVH& b, const QueryIO& io, uint32_t n, int* cu
   cudaError_t e = prepare(k_query<ANY>, smem);
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(cursor, 0, sizeof(int), s)) != cudaSuccess) return e;
-  const uint32_t blocks = (n + kBlock - 1) / kBlock;
+  const int lanes = lanes_for(n);
+  const uint32_t per = (kBlock / 32) * (uint32_t)lanes, blocks = (n + per - 1) / per;
   const uint32_t grid = std::min<uint32_t>(blocks, (uint32_t)resident_grid(k_query<ANY>, smem));
-  k_query<ANY><<<grid, kBlock, smem, s>>>(b, io, (int)n, cursor, eps);
+  k_query<ANY><<<grid, kBlock, smem, s>>>(b, io, (int)n, cursor, eps, lanes);
   return cudaGetLastError();
 }
 

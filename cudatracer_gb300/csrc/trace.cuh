@@ -425,9 +425,10 @@ __device__ __forceinline__ bool traverse(const DevBVH& b, RayState& r, float eps
 //   IO::store(int i, const RayState& r, bool overflow)
 template <bool ANY, bool FASTMM, int REFILL, class IO>
 __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cursor, float eps, IO& io, int* stack,
-                                                 int stride) {
+                                                 int stride, int lanes = 32) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const unsigned own = FULL >> (32 - lanes);  // the lanes that take rays (lanes_for)
   const unsigned below = (1u << lane) - 1u;
   const int limit = b.stack_entries;
   int rid = -1;
@@ -436,14 +437,14 @@ __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cu
   r.ref = kEmptyChild;
   while (true) {
     if (!exhausted) {
-      const unsigned m = __ballot_sync(FULL, rid < 0);
-      if (m == FULL || __popc(m) >= REFILL) {
+      const unsigned m = __ballot_sync(FULL, rid < 0) & own;
+      if (m == own || __popc(m) >= REFILL) {
         const int leader = __ffs(m) - 1;
         int base = 0;
         if (lane == leader) base = atomicAdd(cursor, __popc(m));
         base = __shfl_sync(FULL, base, leader);
         if (base + __popc(m) >= n) exhausted = true;
-        if (rid < 0) {
+        if (rid < 0 && lane < lanes) {
           const int my = base + __popc(m & below);
           if (my < n) {
             float4 o, d;
