@@ -232,25 +232,42 @@ struct Cand {
 };
 
 // Lane l < 30 evaluates axis l / 10, plane l % 10 + 1; returns the winning
-// lane (first lowest cost below 1e34) or 32 when no candidate qualifies.
+// lane (first lowest cost below 1e34) or 32 when no candidate qualifies. The
+// left and right unions of an axis' ten planes are two scans over its ten lanes
+// (a lane that walks all intervals reads 77 words and decodes 66 keys); they keep
+// the walk's order, earlier intervals on the left, so that equal bounds give the
+// same bits.
 __device__ __forceinline__ int choose_split(const uint32_t* bins, int lane, Cand& c) {
+  const unsigned FULL = 0xffffffffu;
+  const int a = lane / kPlanes, k = lane % kPlanes;
+  const bool in = lane < 3 * kPlanes;
   bool valid = false;
   c.cost = 0.0f;
   c.lc = c.rc = 0;
-  if (lane < 3 * kPlanes) {
-    const int a = lane / kPlanes, i = lane % kPlanes + 1;
-    for (int k = 0; k < 3; k++) c.lmn[k] = c.rmn[k] = 1e34f, c.lmx[k] = c.rmx[k] = -1e34f;
-    for (int iv = 0; iv < kIntervals; iv++) {
-      const uint32_t* e = bins + (a * kIntervals + iv) * kBinFields;
-      const uint32_t n = e[0];
-      if (iv < i) {
-        c.lc += n;
-        for (int k = 0; k < 3; k++) c.lmn[k] = gmin(c.lmn[k], unkey(e[1 + k])), c.lmx[k] = gmax(c.lmx[k], unkey(e[4 + k]));
-      } else {
-        c.rc += n;
-        for (int k = 0; k < 3; k++) c.rmn[k] = gmin(c.rmn[k], unkey(e[1 + k])), c.rmx[k] = gmax(c.rmx[k], unkey(e[4 + k]));
-      }
+  for (int x = 0; x < 3; x++) c.lmn[x] = c.rmn[x] = 1e34f, c.lmx[x] = c.rmx[x] = -1e34f;
+  if (in) {
+    const uint32_t* e = bins + (a * kIntervals + k) * kBinFields;
+    c.lc = e[0], c.rc = e[kBinFields];
+    for (int x = 0; x < 3; x++) {
+      c.lmn[x] = gmin(c.lmn[x], unkey(e[1 + x])), c.lmx[x] = gmax(c.lmx[x], unkey(e[4 + x]));
+      c.rmn[x] = gmin(c.rmn[x], unkey(e[kBinFields + 1 + x])), c.rmx[x] = gmax(c.rmx[x], unkey(e[kBinFields + 4 + x]));
     }
+  }
+#pragma unroll
+  for (int off = 1; off < kPlanes; off <<= 1) {
+    const uint32_t ul = __shfl_up_sync(FULL, c.lc, off), dr = __shfl_down_sync(FULL, c.rc, off);
+    const bool up = k >= off, down = k + off < kPlanes;
+    if (up) c.lc += ul;
+    if (down) c.rc += dr;
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+      const float umn = __shfl_up_sync(FULL, c.lmn[x], off), umx = __shfl_up_sync(FULL, c.lmx[x], off);
+      const float dmn = __shfl_down_sync(FULL, c.rmn[x], off), dmx = __shfl_down_sync(FULL, c.rmx[x], off);
+      if (up) c.lmn[x] = gmin(umn, c.lmn[x]), c.lmx[x] = gmax(umx, c.lmx[x]);
+      if (down) c.rmn[x] = gmin(c.rmn[x], dmn), c.rmx[x] = gmax(c.rmx[x], dmx);
+    }
+  }
+  if (in) {
     c.cost = __fadd_rn(__fmul_rn(area3(c.lmn, c.lmx), __uint2float_rn(c.lc)),
                        __fmul_rn(area3(c.rmn, c.rmx), __uint2float_rn(c.rc)));
     valid = c.cost < 1e34f;

@@ -279,31 +279,6 @@ struct Cand {
   float lmn[3], lmx[3], rmn[3], rmx[3];
 };
 
-__device__ __forceinline__ void eval_cand(const uint32_t* bins, const float scale[3], int j, float s, Cand& c) {
-  c.j = kCands + 32;
-  c.cost = 0.0f;
-  const int a = j / (kBins - 1), i = j % (kBins - 1) + 1;
-  if (!(scale[a] > 0.0f)) return;
-  c.lc = c.rc = 0;
-  for (int k = 0; k < 3; k++) c.lmn[k] = c.rmn[k] = 1e34f, c.lmx[k] = c.rmx[k] = -1e34f;
-  for (int b = 0; b < kBins; b++) {
-    const uint32_t* e = bins + (a * kBins + b) * kBinFields;
-    if (b < i) {
-      c.lc += e[0];
-      for (int k = 0; k < 3; k++) c.lmn[k] = gmin(c.lmn[k], unkey(e[1 + k])), c.lmx[k] = gmax(c.lmx[k], unkey(e[4 + k]));
-    } else {
-      c.rc += e[0];
-      for (int k = 0; k < 3; k++) c.rmn[k] = gmin(c.rmn[k], unkey(e[1 + k])), c.rmx[k] = gmax(c.rmx[k], unkey(e[4 + k]));
-    }
-  }
-  if (c.lc == 0 || c.rc == 0) return;
-  const float cost = __fadd_rn(__fmul_rn(farea(c.lmn, c.lmx, s), __uint2float_rn(c.lc)),
-                               __fmul_rn(farea(c.rmn, c.rmx, s), __uint2float_rn(c.rc)));
-  if (!(cost < 3e38f)) return;  // the host's running best starts at 3e38
-  c.cost = cost;
-  c.j = j;
-}
-
 __device__ __forceinline__ void bcast_cand(Cand& c, int src) {
   c.cost = __shfl_sync(0xffffffffu, c.cost, src);
   c.j = __shfl_sync(0xffffffffu, c.j, src);
@@ -320,27 +295,69 @@ __device__ __forceinline__ void bcast_cand(Cand& c, int src) {
 // First lowest cost over the 45 bin splits in axis-major order (the host's
 // strict "cost < best" scan); the whole warp returns the winner, j >= kCands
 // when no split qualifies.
+//
+// Half a warp takes an axis: lane k of it is the split behind bin k, and the left
+// and right unions of all splits are two scans over the half. (A candidate per lane
+// that walks all bins reads 112 words and decodes 96 keys, twice: k_fsmall took 853
+// us of a 2.0 M-triangle build so, 507 with the scans, and the k_fsplit of its 21
+// levels 380 and 264.) Unions keep the walk's order, earlier bins on the left, so
+// that equal bounds give the same bits.
 __device__ __forceinline__ void choose_bin_split(const uint32_t* bins, const float scale[3], float s, int lane,
                                                  Cand& best) {
-  eval_cand(bins, scale, lane, s, best);
-  if (lane + 32 < kCands) {
-    Cand c2;
-    eval_cand(bins, scale, lane + 32, s, c2);
-    if (c2.j < kCands && (best.j >= kCands || c2.cost < best.cost)) best = c2;
+  const unsigned FULL = 0xffffffffu;
+  const int k = lane & 15;
+  best.j = kCands + 32;
+  best.cost = 0.0f;
+#pragma unroll
+  for (int pass = 0; pass < 2; pass++) {
+    const int a = 2 * pass + (lane >> 4);
+    Cand c;
+    c.j = kCands + 32;
+    c.lc = c.rc = 0;
+    for (int x = 0; x < 3; x++) c.lmn[x] = c.rmn[x] = 1e34f, c.lmx[x] = c.rmx[x] = -1e34f;
+    if (a < 3 && k < kBins - 1) {
+      const uint32_t* e = bins + (a * kBins + k) * kBinFields;
+      c.lc = e[0], c.rc = e[kBinFields];
+      for (int x = 0; x < 3; x++) {
+        c.lmn[x] = gmin(c.lmn[x], unkey(e[1 + x])), c.lmx[x] = gmax(c.lmx[x], unkey(e[4 + x]));
+        c.rmn[x] = gmin(c.rmn[x], unkey(e[kBinFields + 1 + x])), c.rmx[x] = gmax(c.rmx[x], unkey(e[kBinFields + 4 + x]));
+      }
+    }
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+      const uint32_t ul = __shfl_up_sync(FULL, c.lc, off, 16), dr = __shfl_down_sync(FULL, c.rc, off, 16);
+      const bool up = k >= off, down = k + off < 16;
+      if (up) c.lc += ul;
+      if (down) c.rc += dr;
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        const float umn = __shfl_up_sync(FULL, c.lmn[x], off, 16), umx = __shfl_up_sync(FULL, c.lmx[x], off, 16);
+        const float dmn = __shfl_down_sync(FULL, c.rmn[x], off, 16), dmx = __shfl_down_sync(FULL, c.rmx[x], off, 16);
+        if (up) c.lmn[x] = gmin(umn, c.lmn[x]), c.lmx[x] = gmax(umx, c.lmx[x]);
+        if (down) c.rmn[x] = gmin(c.rmn[x], dmn), c.rmx[x] = gmax(c.rmx[x], dmx);
+      }
+    }
+    if (a < 3 && k < kBins - 1 && scale[a] > 0.0f && c.lc != 0 && c.rc != 0) {
+      c.cost = __fadd_rn(__fmul_rn(farea(c.lmn, c.lmx, s), __uint2float_rn(c.lc)),
+                         __fmul_rn(farea(c.rmn, c.rmx, s), __uint2float_rn(c.rc)));
+      c.j = a * (kBins - 1) + k;
+      // the host's running best starts at 3e38
+      if (c.cost < 3e38f && (best.j >= kCands || c.cost < best.cost)) best = c;
+    }
   }
   float bc = best.cost;
   int bj = best.j;
 #pragma unroll
   for (int off = 16; off; off >>= 1) {
-    const float oc = __shfl_xor_sync(0xffffffffu, bc, off);
-    const int oj = __shfl_xor_sync(0xffffffffu, bj, off);
+    const float oc = __shfl_xor_sync(FULL, bc, off);
+    const int oj = __shfl_xor_sync(FULL, bj, off);
     if (oj < kCands && (bj >= kCands || oc < bc || (oc == bc && oj < bj))) bc = oc, bj = oj;
   }
   if (bj >= kCands) {
     best.j = kCands + 32;
     return;
   }
-  bcast_cand(best, bj < 32 ? bj : bj - 32);
+  bcast_cand(best, bj % (kBins - 1) + (bj / (kBins - 1) == 1 ? 16 : 0));
 }
 
 // Union of the boxes of prims[b, e) by one warp (order-free).
@@ -972,8 +989,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
 // One warp per node (sweep_split, kept for subtrees near the depth limit) spends
 // its shuffles, scans and latencies on a range of two as on one of sixteen, and
 // nine in ten nodes are in such ranges: k_fsmall took 4.33 ms of a 2.0
-// M-triangle build by itself; with the leaves here it takes 0.81 and this kernel
-// 0.51 ms.
+// M-triangle build by itself; with the leaves here it takes 0.51 and this kernel
+// 0.52 ms.
 constexpr int kLeafThreads = 64;
 constexpr int kLeafWords = 16 * 6 + 16 * 3 + 16 + 16;  // boxes, centroids (then right areas), ids, nodes
 constexpr size_t kLeafShared = sizeof(float) * kLeafWords * kLeafThreads;
