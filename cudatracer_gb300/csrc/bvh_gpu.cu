@@ -82,6 +82,19 @@ struct __align__(16) BNode {
 };
 static_assert(sizeof(BNode) == 48, "BNode");
 
+// A primitive's box: 32 bytes, one load and one sector wherever it lies (the
+// kernels read primitives in the order of the ranges they make).
+struct __align__(32) PrimBox {
+  float4 lo, hi;
+};
+__device__ __forceinline__ PrimBox prim_box(const PrimBox* b) {
+  PrimBox v;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v.lo.x), "=f"(v.lo.y), "=f"(v.lo.z), "=f"(v.lo.w), "=f"(v.hi.x), "=f"(v.hi.y), "=f"(v.hi.z), "=f"(v.hi.w)
+      : "l"(b));
+  return v;
+}
+
 struct Chunk {
   int32_t slot;
   uint32_t begin, end;
@@ -95,7 +108,7 @@ struct Split {
 
 // Carving of the scratch block for n primitives.
 struct Layout {
-  size_t lo, hi, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, chunk_loff, split, bins,
+  size_t box, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, chunk_loff, split, bins,
       counters, total;
   uint32_t chunk, cap, max_large, max_chunks, max_small;
   explicit Layout(uint32_t n) {
@@ -110,8 +123,7 @@ struct Layout {
       o += (bytes + 255) & ~(size_t)255;
       return at;
     };
-    lo = take(sizeof(float4) * (size_t)n);
-    hi = take(sizeof(float4) * (size_t)n);
+    box = take(sizeof(PrimBox) * (size_t)n);
     prims = take(4 * (size_t)n);
     tmp = take(4 * (size_t)n);
     arena = take(sizeof(BNode) * (size_t)cap);
@@ -336,7 +348,7 @@ __device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn
 }
 
 __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
-                                              float4* __restrict__ lo, float4* __restrict__ hi,
+                                              PrimBox* __restrict__ box,
                                               uint32_t* __restrict__ prims, uint32_t* counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
@@ -349,8 +361,7 @@ __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, cons
                          __fsub_rn(gmin(a.z, gmin(b.z, c.z)), plo)};
     const float mx[3] = {__fadd_rn(gmax(a.x, gmax(b.x, c.x)), phi), __fadd_rn(gmax(a.y, gmax(b.y, c.y)), phi),
                          __fadd_rn(gmax(a.z, gmax(b.z, c.z)), phi)};
-    lo[i] = make_float4(mn[0], mn[1], mn[2], 0.0f);
-    hi[i] = make_float4(mx[0], mx[1], mx[2], 0.0f);
+    box[i] = PrimBox{make_float4(mn[0], mn[1], mn[2], 0.0f), make_float4(mx[0], mx[1], mx[2], 0.0f)};
     prims[i] = i;
     for (int k = 0; k < 3; k++) kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
   }
@@ -397,7 +408,7 @@ __global__ void __launch_bounds__(256) k_chunks(const BNode* __restrict__ arena,
 
 __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
                                              const Chunk* __restrict__ chunks, const uint32_t* counters,
-                                             const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                             const PrimBox* __restrict__ box,
                                              const uint32_t* __restrict__ prims, uint32_t* gbins) {
   __shared__ float planes[3 * kPlanes];
   __shared__ uint32_t bins[kBinWords];
@@ -412,10 +423,10 @@ __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, co
   __syncthreads();
   for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
     const bool in = k0 + threadIdx.x < ch.end;
-    const uint32_t p = in ? prims[k0 + threadIdx.x] : 0u;
+    const PrimBox v = prim_box(box + (in ? prims[k0 + threadIdx.x] : 0u));
     int iv[3];
-    intervals_of(planes, lo[p], hi[p], iv);
-    bin_warp(bins, iv, lo[p], hi[p], in);
+    intervals_of(planes, v.lo, v.hi, iv);
+    bin_warp(bins, iv, v.lo, v.hi, in);
   }
   __syncthreads();
   uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
@@ -482,13 +493,14 @@ __global__ void __launch_bounds__(256) k_split(BNode* arena, const int32_t* __re
   classify((int32_t)cid + 1, c.rc, nd.depth + 1, next_large, small, counters);
 }
 
-__device__ __forceinline__ bool goes_left(const float4* lo, const float4* hi, uint32_t p, int axis, float coord) {
-  return centroid(comp(lo[p], axis), comp(hi[p], axis)) <= coord;
+__device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, int axis, float coord) {
+  const PrimBox v = prim_box(box + p);
+  return centroid(comp(v.lo, axis), comp(v.hi, axis)) <= coord;
 }
 
 __global__ void __launch_bounds__(256) k_part_count(const Chunk* __restrict__ chunks, const Split* __restrict__ split,
-                                                    const uint32_t* counters, const float4* __restrict__ lo,
-                                                    const float4* __restrict__ hi, const uint32_t* __restrict__ prims,
+                                                    const uint32_t* counters, const PrimBox* __restrict__ box,
+                                                    const uint32_t* __restrict__ prims,
                                                     uint32_t* chunk_left) {
   __shared__ uint32_t warp_sum[8];
   if (blockIdx.x >= counters[kChunkCursor]) return;
@@ -496,7 +508,7 @@ __global__ void __launch_bounds__(256) k_part_count(const Chunk* __restrict__ ch
   const Split sp = split[ch.slot];
   if (sp.axis < 0) return;
   uint32_t n = 0;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(lo, hi, prims[k], sp.axis, sp.coord);
+  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(box, prims[k], sp.axis, sp.coord);
   n = __reduce_add_sync(0xffffffffu, n);
   if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = n;
   __syncthreads();
@@ -540,7 +552,7 @@ __global__ void __launch_bounds__(256) k_part_offsets(const BNode* __restrict__ 
 __global__ void __launch_bounds__(256) k_part_scatter(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
                                                       const Chunk* __restrict__ chunks, const Split* __restrict__ split,
                                                       const uint32_t* counters, const uint32_t* __restrict__ chunk_loff,
-                                                      const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                      const PrimBox* __restrict__ box,
                                                       const uint32_t* __restrict__ prims, uint32_t* tmp) {
   __shared__ uint32_t wl[8], wr[8];
   if (blockIdx.x >= counters[kChunkCursor]) return;
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(256) k_part_scatter(const BNode* __restrict__ 
     const uint32_t k = k0 + threadIdx.x;
     const bool in = k < ch.end;
     const uint32_t p = in ? prims[k] : 0u;
-    const bool left = in && goes_left(lo, hi, p, sp.axis, sp.coord);
+    const bool left = in && goes_left(box, p, sp.axis, sp.coord);
     const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
     if (lane == 0) wl[warp] = __popc(bl), wr[warp] = __popc(br);
     __syncthreads();
@@ -586,8 +598,8 @@ __global__ void __launch_bounds__(256) k_part_copy(const Chunk* __restrict__ chu
 // tasks: ranges of 4..kLeafTask primitives for k_leaf, counted in counters[kTasks]
 // (disjoint, so at most n / 4).
 __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const int32_t* __restrict__ small,
-                                                            const uint32_t* counters_ro, const float4* __restrict__ lo,
-                                                            const float4* __restrict__ hi, uint32_t* prims,
+                                                            const uint32_t* counters_ro,
+                                                            const PrimBox* __restrict__ box, uint32_t* prims,
                                                             uint32_t* counters, uint32_t cap, uint32_t* tasks) {
   __shared__ uint32_t sbins[kSmallWarps][kBinWords];
   __shared__ float splanes[kSmallWarps][3 * kPlanes];
@@ -619,10 +631,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
       __syncwarp();
       for (uint32_t k0 = 0; k0 < count; k0 += 32) {
         const bool in = k0 + lane < count;
-        const uint32_t p = in ? prims[first + k0 + lane] : 0u;
+        const PrimBox v = prim_box(box + (in ? prims[first + k0 + lane] : 0u));
         int iv[3];
-        intervals_of(planes, lo[p], hi[p], iv);
-        bin_warp(bins, iv, lo[p], hi[p], in);
+        intervals_of(planes, v.lo, v.hi, iv);
+        bin_warp(bins, iv, v.lo, v.hi, in);
       }
       __syncwarp();
       Cand c;
@@ -642,7 +654,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
         const uint32_t k = k0 + lane;
         const bool in = k < count;
         const uint32_t p = in ? prims[first + k] : 0u;
-        const bool left = in && goes_left(lo, hi, p, a, coord);
+        const bool left = in && goes_left(box, p, a, coord);
         const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
         if (left) tmp[nl + __popc(bl & lt)] = p;
         else if (in) tmp[kWarpMax + nr + __popc(br & lt)] = p;
@@ -723,7 +735,7 @@ __device__ __forceinline__ unsigned long long part_order(unsigned long long o, u
 }
 
 __global__ void __launch_bounds__(kLeafThreads) k_leaf(BNode* arena, const uint32_t* __restrict__ tasks,
-                                                       const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                       const PrimBox* __restrict__ boxes,
                                                        uint32_t* prims, uint32_t* counters, uint32_t cap) {
   extern __shared__ float sh[];
   constexpr int T = kLeafThreads;
@@ -744,7 +756,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf(BNode* arena, const uint3
       first = (uint32_t)nd.first, count = (uint32_t)nd.count, depth0 = nd.depth;
       for (uint32_t j = 0; j < count; j++) {
         const uint32_t p = prims[first + j];
-        const float4 l = lo[p], h = hi[p];
+        const PrimBox v = prim_box(boxes + p);
+        const float4 l = v.lo, h = v.hi;
         float* b = box + 6 * j * T;
         b[0] = l.x, b[T] = l.y, b[2 * T] = l.z, b[3 * T] = h.x, b[4 * T] = h.y, b[5 * T] = h.z;
         id[j * T] = p;
@@ -1005,8 +1018,7 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   const uint32_t n = sc.tri_count;
   const Layout L(n);
   uint32_t* counters = at<uint32_t>(scratch, L.counters);
-  float4* lo = at<float4>(scratch, L.lo);
-  float4* hi = at<float4>(scratch, L.hi);
+  PrimBox* box = at<PrimBox>(scratch, L.box);
   uint32_t* prims = at<uint32_t>(scratch, L.prims);
   uint32_t* tmp = at<uint32_t>(scratch, L.tmp);
   BNode* arena = at<BNode>(scratch, L.arena);
@@ -1021,7 +1033,7 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   uint32_t* qidx = at<uint32_t>(scratch, L.qidx);
 
   k_init<<<1, 32, 0, s>>>(counters);
-  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, lo, hi, prims, counters);
+  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, prims, counters);
   k_root<<<1, 1, 0, s>>>(arena, large[0], small, n, counters);
   GB_TRY(cudaGetLastError());
   GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));
@@ -1034,13 +1046,13 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     GB_TRY(cudaMemsetAsync(counters + kLargeNext, 0, 8, s));  // kLargeNext, kChunkCursor
     k_chunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, chunks, split, bins, counters);
     const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / L.chunk + nl + 1, L.max_chunks);
-    k_bin<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, counters, lo, hi, prims, bins);
+    k_bin<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, counters, box, prims, bins);
     k_split<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, bins, split, large[cur ^ 1], small,
                                                           counters, L.cap);
-    k_part_count<<<nchunk, 256, 0, s>>>(chunks, split, counters, lo, hi, prims, chunk_left);
+    k_part_count<<<nchunk, 256, 0, s>>>(chunks, split, counters, box, prims, chunk_left);
     k_part_offsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, split, chunk_left, chunk_loff,
                                                                  counters);
-    k_part_scatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, chunk_loff, lo, hi, prims, tmp);
+    k_part_scatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, chunk_loff, box, prims, tmp);
     k_part_copy<<<nchunk, 256, 0, s>>>(chunks, split, counters, tmp, prims);
     GB_TRY(cudaGetLastError());
     GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));
@@ -1056,14 +1068,14 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sms * 8);
     GB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
     // the partition's scratch (4 bytes per primitive) is free now: it takes the tasks
-    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, small, counters, lo, hi, prims, counters, L.cap, tmp);
+    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, small, counters, box, prims, counters, L.cap, tmp);
     GB_TRY(cudaGetLastError());
     GB_TRY(cudaFuncSetAttribute(k_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
     GB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_leaf, kLeafThreads, kLeafShared));
     const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 4 + 1, kLeafThreads),
                                                      (uint64_t)sms * std::max(1, per_sm));
-    k_leaf<<<gl, kLeafThreads, kLeafShared, s>>>(arena, tmp, lo, hi, prims, counters, L.cap);
+    k_leaf<<<gl, kLeafThreads, kLeafShared, s>>>(arena, tmp, box, prims, counters, L.cap);
     GB_TRY(cudaGetLastError());
   }
   GB_TRY(cudaMemsetAsync(arrive, 0, 4 * (size_t)L.cap, s));

@@ -102,6 +102,19 @@ struct __align__(16) FCostD {
 };
 static_assert(sizeof(FCostD) == 32, "FCostD");
 
+// A primitive's box: 32 bytes, one load and one sector wherever it lies (the
+// kernels read primitives in the order of the ranges they make).
+struct __align__(32) PrimBox {
+  float4 lo, hi;
+};
+__device__ __forceinline__ PrimBox prim_box(const PrimBox* b) {
+  PrimBox v;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v.lo.x), "=f"(v.lo.y), "=f"(v.lo.z), "=f"(v.lo.w), "=f"(v.hi.x), "=f"(v.hi.y), "=f"(v.hi.z), "=f"(v.hi.w)
+      : "l"(b));
+  return v;
+}
+
 struct Chunk {
   int32_t slot;
   uint32_t begin, end;
@@ -126,7 +139,7 @@ struct QRec {
 static_assert(sizeof(QRec) == 64, "QRec");
 
 struct Layout {
-  size_t lo, hi, cent, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, chunk_loff, split,
+  size_t box, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, chunk_loff, split,
       bins, cbk, qlist, qrec, scan, sums, counters, total;
   uint32_t chunk, cap, qcap, max_large, max_chunks, max_small, max_sums;
   explicit Layout(uint32_t n, int wide = 0) {
@@ -143,9 +156,7 @@ struct Layout {
       o += (bytes + 255) & ~(size_t)255;
       return at;
     };
-    lo = take(sizeof(float4) * (size_t)n);
-    hi = take(sizeof(float4) * (size_t)n);
-    cent = take(sizeof(float4) * (size_t)n);
+    box = take(sizeof(PrimBox) * (size_t)n);
     prims = take(4 * (size_t)n);
     tmp = take(4 * (size_t)n);
     arena = take(sizeof(FNodeD) * (size_t)cap);
@@ -190,6 +201,12 @@ __device__ __forceinline__ uint32_t bin_init(int w) {
 __device__ __forceinline__ float gmin(float a, float b) { return b < a ? b : a; }
 __device__ __forceinline__ float gmax(float a, float b) { return a < b ? b : a; }
 __device__ __forceinline__ float comp(const float4& v, int a) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); }
+
+// the box's centre as k_fprep checked it
+__device__ __forceinline__ float4 centre(const PrimBox& b) {
+  return make_float4(__fmul_rn(0.5f, __fadd_rn(b.lo.x, b.hi.x)), __fmul_rn(0.5f, __fadd_rn(b.lo.y, b.hi.y)),
+                     __fmul_rn(0.5f, __fadd_rn(b.lo.z, b.hi.z)), 0.0f);
+}
 
 // farea (bvh_fast.cpp): surface area with extents scaled by s
 __device__ __forceinline__ float farea(const float mn[3], const float mx[3], float s) {
@@ -361,12 +378,12 @@ __device__ __forceinline__ void choose_bin_split(const uint32_t* bins, const flo
 }
 
 // Union of the boxes of prims[b, e) by one warp (order-free).
-__device__ __forceinline__ void warp_union(const float4* lo, const float4* hi, const uint32_t* prims, uint32_t b,
+__device__ __forceinline__ void warp_union(const PrimBox* box, const uint32_t* prims, uint32_t b,
                                            uint32_t e, int lane, float mn[3], float mx[3]) {
   uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
   for (uint32_t k = b + lane; k < e; k += 32) {
-    const uint32_t p = prims[k];
-    const float4 l = lo[p], h = hi[p];
+    const PrimBox v = prim_box(box + prims[k]);
+    const float4 l = v.lo, h = v.hi;
     kmn[0] = min(kmn[0], fkey(l.x)), kmn[1] = min(kmn[1], fkey(l.y)), kmn[2] = min(kmn[2], fkey(l.z));
     kmx[0] = max(kmx[0], fkey(h.x)), kmx[1] = max(kmx[1], fkey(h.y)), kmx[2] = max(kmx[2], fkey(h.z));
   }
@@ -452,8 +469,7 @@ __global__ void __launch_bounds__(256) k_fmag(const float4* __restrict__ v, cons
 
 // rel_pad: kPad for the traversal-speed quad tree, 0 (exact bounds) for the wide tree
 __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
-                                               float4* __restrict__ lo, float4* __restrict__ hi,
-                                               float4* __restrict__ cent, uint32_t* __restrict__ prims,
+                                               PrimBox* __restrict__ box, uint32_t* __restrict__ prims,
                                                uint32_t* counters, float rel_pad) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
@@ -474,9 +490,7 @@ __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, con
       ok &= isfinite(lo_k) && isfinite(hi_k) && isfinite(ce[k]);
     }
     if (!ok) atomicOr(&counters[kError], kErrRange);
-    lo[i] = make_float4(mn[0], mn[1], mn[2], 0.0f);
-    hi[i] = make_float4(mx[0], mx[1], mx[2], 0.0f);
-    cent[i] = make_float4(ce[0], ce[1], ce[2], 0.0f);
+    box[i] = PrimBox{make_float4(mn[0], mn[1], mn[2], 0.0f), make_float4(mx[0], mx[1], mx[2], 0.0f)};
     prims[i] = i;
     for (int k = 0; k < 3; k++) kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
   }
@@ -535,7 +549,7 @@ __device__ __forceinline__ uint32_t nchunks_used(const uint32_t* counters, uint3
 }
 
 __global__ void __launch_bounds__(256) k_fcb(const Chunk* __restrict__ chunks, const uint32_t* counters,
-                                             uint32_t max_chunks, const float4* __restrict__ cent,
+                                             uint32_t max_chunks, const PrimBox* __restrict__ box,
                                              const uint32_t* __restrict__ prims, uint32_t* cbk) {
   __shared__ uint32_t red[6];
   if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
@@ -544,7 +558,7 @@ __global__ void __launch_bounds__(256) k_fcb(const Chunk* __restrict__ chunks, c
   __syncthreads();
   uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
   for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
-    const float4 c = cent[prims[k]];
+    const float4 c = centre(prim_box(box + prims[k]));
     kmn[0] = min(kmn[0], fkey(c.x)), kmn[1] = min(kmn[1], fkey(c.y)), kmn[2] = min(kmn[2], fkey(c.z));
     kmx[0] = max(kmx[0], fkey(c.x)), kmx[1] = max(kmx[1], fkey(c.y)), kmx[2] = max(kmx[2], fkey(c.z));
   }
@@ -564,8 +578,7 @@ __global__ void __launch_bounds__(256) k_fcb(const Chunk* __restrict__ chunks, c
 
 __global__ void __launch_bounds__(256) k_fbin(const Chunk* __restrict__ chunks, const uint32_t* counters,
                                               uint32_t max_chunks, const uint32_t* __restrict__ cbk,
-                                              const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                              const float4* __restrict__ cent, const uint32_t* __restrict__ prims,
+                                              const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
                                               uint32_t* gbins) {
   __shared__ uint32_t bins[kBinWords];
   if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
@@ -576,10 +589,10 @@ __global__ void __launch_bounds__(256) k_fbin(const Chunk* __restrict__ chunks, 
   __syncthreads();
   for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
     const bool in = k0 + threadIdx.x < ch.end;
-    const uint32_t p = in ? prims[k0 + threadIdx.x] : 0u;
+    const PrimBox v = prim_box(box + (in ? prims[k0 + threadIdx.x] : 0u));
     int bin[3];
-    bins_of(blo, bscale, cent[p], bin);
-    bin_warp(bins, bin, lo[p], hi[p], in);
+    bins_of(blo, bscale, centre(v), bin);
+    bin_warp(bins, bin, v.lo, v.hi, in);
   }
   __syncthreads();
   uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
@@ -628,8 +641,7 @@ __device__ __forceinline__ void add_children(const LevelArgs& A, int32_t ni, con
 
 __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, const uint32_t* __restrict__ gbins,
                                                 const uint32_t* __restrict__ cbk, FSplit* split,
-                                                const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                const uint32_t* __restrict__ prims) {
+                                                const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= A.nl) return;  // whole warp
@@ -662,21 +674,21 @@ __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, const uint32_t* __r
   // every centroid in one bin on every axis: halve the range as it lies
   const uint32_t mid = count / 2;
   float lmn[3], lmx[3], rmn[3], rmx[3];
-  warp_union(lo, hi, prims, (uint32_t)nd.first, (uint32_t)nd.first + mid, lane, lmn, lmx);
-  warp_union(lo, hi, prims, (uint32_t)nd.first + mid, (uint32_t)nd.first + count, lane, rmn, rmx);
+  warp_union(box, prims, (uint32_t)nd.first, (uint32_t)nd.first + mid, lane, lmn, lmx);
+  warp_union(box, prims, (uint32_t)nd.first + mid, (uint32_t)nd.first + count, lane, rmn, rmx);
   if (lane == 0) {
     split[s].mode = 1;
     add_children(A, ni, nd, mid, lmn, lmx, rmn, rmx);
   }
 }
 
-__device__ __forceinline__ bool goes_left(const float4* cent, uint32_t p, const FSplit& sp) {
-  return bin_of(comp(cent[p], sp.axis), sp.lo, sp.scale) < sp.bsp;
+__device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, const FSplit& sp) {
+  return bin_of(comp(centre(prim_box(box + p)), sp.axis), sp.lo, sp.scale) < sp.bsp;
 }
 
 __global__ void __launch_bounds__(256) k_fpcount(const Chunk* __restrict__ chunks, const FSplit* __restrict__ split,
                                                  const uint32_t* counters, uint32_t max_chunks,
-                                                 const float4* __restrict__ cent, const uint32_t* __restrict__ prims,
+                                                 const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
                                                  uint32_t* chunk_left) {
   __shared__ uint32_t warp_sum[8];
   if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
@@ -684,7 +696,7 @@ __global__ void __launch_bounds__(256) k_fpcount(const Chunk* __restrict__ chunk
   const FSplit sp = split[ch.slot];
   if (sp.mode != 0) return;
   uint32_t n = 0;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(cent, prims[k], sp);
+  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(box, prims[k], sp);
   n = __reduce_add_sync(0xffffffffu, n);
   if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = n;
   __syncthreads();
@@ -728,7 +740,7 @@ __global__ void __launch_bounds__(256) k_fpscatter(const FNodeD* __restrict__ ar
                                                    const Chunk* __restrict__ chunks, const FSplit* __restrict__ split,
                                                    const uint32_t* counters, uint32_t max_chunks,
                                                    const uint32_t* __restrict__ chunk_loff,
-                                                   const float4* __restrict__ cent, const uint32_t* __restrict__ prims,
+                                                   const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
                                                    uint32_t* tmp) {
   __shared__ uint32_t wl[8], wr[8];
   if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
@@ -745,7 +757,7 @@ __global__ void __launch_bounds__(256) k_fpscatter(const FNodeD* __restrict__ ar
     const uint32_t k = k0 + threadIdx.x;
     const bool in = k < ch.end;
     const uint32_t p = in ? prims[k] : 0u;
-    const bool left = in && goes_left(cent, p, sp);
+    const bool left = in && goes_left(box, p, sp);
     const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
     if (lane == 0) wl[warp] = __popc(bl), wr[warp] = __popc(br);
     __syncthreads();
@@ -774,13 +786,13 @@ __global__ void __launch_bounds__(256) k_fpcopy(const Chunk* __restrict__ chunks
 // Exact SAH sweep of a range of 2..16 primitives (sweep_split): every split of
 // the centroid order (ties by primitive id) on each axis; reorders the range to
 // the winning axis' order. Returns the left count and the child boxes.
-__device__ __forceinline__ uint32_t sweep_split(const float4* lo, const float4* hi, const float4* cent, uint32_t* prims,
+__device__ __forceinline__ uint32_t sweep_split(const PrimBox* box, uint32_t* prims,
                                                 uint32_t first, uint32_t count, float s, int lane,
                                                 uint32_t (*ord)[kSweepMax], float lmn[3], float lmx[3],
                                                 float rmn[3], float rmx[3]) {
   const bool in = (uint32_t)lane < count;
   const uint32_t p = in ? prims[first + lane] : 0u;
-  const float4 pc = in ? cent[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float4 pc = in ? centre(prim_box(box + p)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float best = 3e38f;
   int bax = 0;
   uint32_t bmid = count / 2;
@@ -797,8 +809,8 @@ __device__ __forceinline__ uint32_t sweep_split(const float4* lo, const float4* 
     // lane r holds the box of the r-th primitive in this axis' order
     float bmn[3] = {1e34f, 1e34f, 1e34f}, bmx[3] = {-1e34f, -1e34f, -1e34f};
     if (in) {
-      const uint32_t q = ord[a][lane];
-      const float4 l = lo[q], h = hi[q];
+      const PrimBox v = prim_box(box + ord[a][lane]);
+      const float4 l = v.lo, h = v.hi;
       bmn[0] = l.x, bmn[1] = l.y, bmn[2] = l.z, bmx[0] = h.x, bmx[1] = h.y, bmx[2] = h.z;
     }
     float pmn[3], pmx[3], smn[3], smx[3];  // inclusive prefix / suffix unions
@@ -837,8 +849,8 @@ __device__ __forceinline__ uint32_t sweep_split(const float4* lo, const float4* 
   if (in) prims[first + lane] = ord[bax][lane];
   __syncwarp();
   // cut_boxes over the reordered range
-  warp_union(lo, hi, prims, first, first + bmid, lane, lmn, lmx);
-  warp_union(lo, hi, prims, first + bmid, first + count, lane, rmn, rmx);
+  warp_union(box, prims, first, first + bmid, lane, lmn, lmx);
+  warp_union(box, prims, first + bmid, first + count, lane, rmn, rmx);
   return bmid;
 }
 
@@ -852,9 +864,7 @@ __device__ __forceinline__ bool leaf_task(uint32_t count, int32_t depth) {
 // tasks: ranges for k_fleaf, counted in counters[kTasks]; at most n / 2 of them
 // (disjoint, two primitives or more each).
 __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const int32_t* __restrict__ small_ro,
-                                                             const float4* __restrict__ lo,
-                                                             const float4* __restrict__ hi,
-                                                             const float4* __restrict__ cent, uint32_t* prims,
+                                                             const PrimBox* __restrict__ box, uint32_t* prims,
                                                              uint32_t* tasks) {
   __shared__ uint32_t sbins[kSmallWarps][kBinWords];
   __shared__ int32_t sstack[kSmallWarps][kSmallStack];
@@ -883,12 +893,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
       float lmn[3], lmx[3], rmn[3], rmx[3];
       uint32_t mid;
       if (count <= kSweepMax) {
-        mid = sweep_split(lo, hi, cent, prims, first, count, A.ascale, lane, sord[warp], lmn, lmx, rmn, rmx);
+        mid = sweep_split(box, prims, first, count, A.ascale, lane, sord[warp], lmn, lmx, rmn, rmx);
       } else {
         // centroid bounds, bins, the 45 bin splits
         uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
         for (uint32_t k = lane; k < count; k += 32) {
-          const float4 c = cent[prims[first + k]];
+          const float4 c = centre(prim_box(box + prims[first + k]));
           kmn[0] = min(kmn[0], fkey(c.x)), kmn[1] = min(kmn[1], fkey(c.y)), kmn[2] = min(kmn[2], fkey(c.z));
           kmx[0] = max(kmx[0], fkey(c.x)), kmx[1] = max(kmx[1], fkey(c.y)), kmx[2] = max(kmx[2], fkey(c.z));
         }
@@ -903,10 +913,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
         __syncwarp();
         for (uint32_t k0 = 0; k0 < count; k0 += 32) {
           const bool in = k0 + lane < count;
-          const uint32_t p = in ? prims[first + k0 + lane] : 0u;
+          const PrimBox v = prim_box(box + (in ? prims[first + k0 + lane] : 0u));
           int bin[3];
-          bins_of(blo, bscale, cent[p], bin);
-          bin_warp(bins, bin, lo[p], hi[p], in);
+          bins_of(blo, bscale, centre(v), bin);
+          bin_warp(bins, bin, v.lo, v.hi, in);
         }
         __syncwarp();
         Cand c;
@@ -922,7 +932,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
             const uint32_t k = k0 + lane;
             const bool in = k < count;
             const uint32_t p = in ? prims[first + k] : 0u;
-            const bool left = in && goes_left(cent, p, sp_);
+            const bool left = in && goes_left(box, p, sp_);
             const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
             if (left) tmp[nl + __popc(bl & lt)] = p;
             else if (in) tmp[kWarpMax + nr + __popc(br & lt)] = p;
@@ -938,8 +948,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
           for (int k = 0; k < 3; k++) lmn[k] = c.lmn[k], lmx[k] = c.lmx[k], rmn[k] = c.rmn[k], rmx[k] = c.rmx[k];
         } else {
           mid = count / 2;
-          warp_union(lo, hi, prims, first, first + mid, lane, lmn, lmx);
-          warp_union(lo, hi, prims, first + mid, first + count, lane, rmn, rmx);
+          warp_union(box, prims, first, first + mid, lane, lmn, lmx);
+          warp_union(box, prims, first + mid, first + count, lane, rmn, rmx);
         }
       }
       __syncwarp();
@@ -998,8 +1008,7 @@ constexpr size_t kLeafShared = sizeof(float) * kLeafWords * kLeafThreads;
 __device__ __forceinline__ uint32_t nib(unsigned long long o, uint32_t i) { return (uint32_t)(o >> (4 * i)) & 15u; }
 
 __global__ void __launch_bounds__(kLeafThreads) k_fleaf(LevelArgs A, const uint32_t* __restrict__ tasks,
-                                                        const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                        const float4* __restrict__ cent, uint32_t* prims) {
+                                                        const PrimBox* __restrict__ boxes, uint32_t* prims) {
   extern __shared__ float sh[];
   constexpr int T = kLeafThreads;
   float* box = sh + threadIdx.x;                         // box[(6 j + c) T]: min x/y/z, max x/y/z of primitive j
@@ -1035,7 +1044,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_fleaf(LevelArgs A, const uint3
     }
     for (uint32_t j = 0; j < count; j++) {
       const uint32_t p = prims[first + j];
-      const float4 l = lo[p], h = hi[p], c = cent[p];
+      const PrimBox v = prim_box(boxes + p);
+      const float4 l = v.lo, h = v.hi, c = centre(v);
       float* b = box + 6 * j * T;
       b[0] = l.x, b[T] = l.y, b[2 * T] = l.z, b[3 * T] = h.x, b[4 * T] = h.y, b[5 * T] = h.z;
       float* e = cen + 3 * j * T;
@@ -1505,9 +1515,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   const uint32_t n = sc.tri_count;
   const Layout Lo(n, wide);
   uint32_t* counters = at<uint32_t>(scratch, Lo.counters);
-  float4* lo = at<float4>(scratch, Lo.lo);
-  float4* hi = at<float4>(scratch, Lo.hi);
-  float4* cent = at<float4>(scratch, Lo.cent);
+  PrimBox* box = at<PrimBox>(scratch, Lo.box);
   uint32_t* prims = at<uint32_t>(scratch, Lo.prims);
   uint32_t* tmp = at<uint32_t>(scratch, Lo.tmp);
   FNodeD* arena = at<FNodeD>(scratch, Lo.arena);
@@ -1529,7 +1537,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
 
   k_finit<<<1, 32, 0, s>>>(counters);
   k_fmag<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, counters);
-  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, lo, hi, cent, prims, counters, wide ? 0.0f : kPad);
+  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, prims, counters, wide ? 0.0f : kPad);
   k_froot<<<1, 1, 0, s>>>(arena, large[0], small, n, counters);
   FB_TRY(cudaGetLastError());
   FB_TRY(read_counters(hc, counters, s));
@@ -1561,13 +1569,13 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     k_fchunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, Lo.max_chunks, chunks, split, bins, cbk,
                                               counters);
     const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / Lo.chunk + nl + 1, Lo.max_chunks);
-    k_fcb<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cent, prims, cbk);
-    k_fbin<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cbk, lo, hi, cent, prims, bins);
-    k_fsplit<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(A, bins, cbk, split, lo, hi, prims);
-    k_fpcount<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, cent, prims, chunk_left);
+    k_fcb<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, box, prims, cbk);
+    k_fbin<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cbk, box, prims, bins);
+    k_fsplit<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(A, bins, cbk, split, box, prims);
+    k_fpcount<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, box, prims, chunk_left);
     k_fpoffsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, split, chunk_left, chunk_loff,
                                                               counters);
-    k_fpscatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, Lo.max_chunks, chunk_loff, cent,
+    k_fpscatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, Lo.max_chunks, chunk_loff, box,
                                        prims, tmp);
     k_fpcopy<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, tmp, prims);
     FB_TRY(cudaGetLastError());
@@ -1585,14 +1593,14 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sm_count() * 16);
     FB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
     // the partition's scratch (4 bytes per primitive) is free now: it takes the tasks
-    k_fsmall<<<g, kSmallWarps * 32, 0, s>>>(A, small, lo, hi, cent, prims, tmp);
+    k_fsmall<<<g, kSmallWarps * 32, 0, s>>>(A, small, box, prims, tmp);
     FB_TRY(cudaGetLastError());
     FB_TRY(cudaFuncSetAttribute(k_fleaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
     FB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fleaf, kLeafThreads, kLeafShared));
     const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 2 + 1, kLeafThreads),
                                                      (uint64_t)sm_count() * std::max(1, per_sm));
-    k_fleaf<<<gl, kLeafThreads, kLeafShared, s>>>(A, tmp, lo, hi, cent, prims);
+    k_fleaf<<<gl, kLeafThreads, kLeafShared, s>>>(A, tmp, box, prims);
     FB_TRY(cudaGetLastError());
   }
   FB_TRY(read_counters(hc, counters, s));
