@@ -69,14 +69,14 @@ enum : uint32_t { kErrRange = 1, kErrArena = 2, kErrStack = 4, kErrPartition = 8
 enum Counter : int {
   kArenaCount = 0,
   kSmallCount = 1,
-  kLargeNext = 2,
-  kChunkCursor = 3,
   kError = 4,
   kMaxLeaf = 5,
   kMag = 6,
   kQNext = 7,
-  kTasks = kChunkCursor,  // ranges for k_fleaf, once the levels are done
-  kRootKeys = 8,  // 6 words: min x/y/z, max x/y/z
+  kChunks = 2,       // 2 words: chunks of the even and of the odd level
+  kTasks = kChunks,  // ranges for k_fleaf, once the levels are done
+  kRootKeys = 8,     // 6 words: min x/y/z, max x/y/z
+  kLarge = 14,       // 2 words: large nodes of the even and of the odd level
   kCounterWords = 16
 };
 
@@ -121,12 +121,12 @@ struct Chunk {
 };
 struct FSplit {
   int32_t mode;  // -1 not split yet, 0 partition by bin, 1 halves in the current order, -2 no chunks
+  int32_t kid[2];  // the children's slots of the next level, -1 where they have none
   int32_t axis;
   float lo, scale;
   int32_t bsp;  // primitives with bin < bsp go left
   uint32_t lc;
   uint32_t chunk0;
-  uint32_t pad;
 };
 
 // one quad node (index = breadth-first allocation order)
@@ -139,7 +139,7 @@ struct QRec {
 static_assert(sizeof(QRec) == 64, "QRec");
 
 struct Layout {
-  size_t box, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, chunk_loff, split,
+  size_t box, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, split,
       bins, cbk, qlist, qrec, scan, sums, counters, total;
   uint32_t chunk, cap, qcap, max_large, max_chunks, max_small, max_sums;
   explicit Layout(uint32_t n, int wide = 0) {
@@ -167,10 +167,9 @@ struct Layout {
     small = take(4 * (size_t)max_small);
     chunks = take(sizeof(Chunk) * (size_t)max_chunks);
     chunk_left = take(4 * (size_t)max_chunks);
-    chunk_loff = take(4 * (size_t)max_chunks);
     split = take(sizeof(FSplit) * (size_t)max_large);
     bins = take(4 * (size_t)kBinWords * max_large);
-    cbk = take(4 * 6 * (size_t)max_large);
+    cbk = take(2 * 4 * 6 * (size_t)max_large);
     qlist = take(4 * (size_t)qcap);
     qrec = take(sizeof(QRec) * (size_t)qcap);
     scan = take(4 * (size_t)qcap);
@@ -406,24 +405,32 @@ __device__ __forceinline__ FNodeD make_node(const float mn[3], const float mx[3]
   return b;
 }
 
-// A child is split further when it holds more than one primitive above the depth limit.
-__device__ __forceinline__ void classify(int32_t id, uint32_t count, int32_t depth, int32_t* next_large,
-                                         uint32_t max_large, int32_t* small, uint32_t max_small, uint32_t* counters) {
-  if (count <= 1 || depth >= kDepthLimit) return;
+// A child is split further when it holds more than one primitive above the depth
+// limit: by the next level's kernels (returns its slot there) or by a warp (-1).
+__device__ __forceinline__ int32_t classify(int32_t id, uint32_t count, int32_t depth, int32_t* next_large,
+                                            uint32_t* next_count, uint32_t max_large, uint32_t* next_cbk,
+                                            int32_t* small, uint32_t max_small, uint32_t* counters) {
+  if (count <= 1 || depth >= kDepthLimit) return -1;
   if (count > kWarpMax) {
-    const uint32_t s = atomicAdd(&counters[kLargeNext], 1u);
-    if (s < max_large) next_large[s] = id;
-    else atomicOr(&counters[kError], kErrArena);
-  } else {
-    const uint32_t s = atomicAdd(&counters[kSmallCount], 1u);
-    if (s < max_small) small[s] = id;
-    else atomicOr(&counters[kError], kErrArena);
+    const uint32_t s = atomicAdd(next_count, 1u);
+    if (s >= max_large) {
+      atomicOr(&counters[kError], kErrArena);
+      return -1;
+    }
+    next_large[s] = id;
+    for (int k = 0; k < 6; k++) next_cbk[6 * (size_t)s + k] = k < 3 ? fkey(1e34f) : fkey(-1e34f);
+    return (int32_t)s;
   }
+  const uint32_t s = atomicAdd(&counters[kSmallCount], 1u);
+  if (s < max_small) small[s] = id;
+  else atomicOr(&counters[kError], kErrArena);
+  return -1;
 }
 
 // ---------------------------------------------------------------- prep
-__global__ void k_finit(uint32_t* counters) {
+__global__ void k_finit(uint32_t* counters, uint32_t* cbk) {
   const int w = threadIdx.x;
+  if (w < 6) cbk[w] = w < 3 ? fkey(1e34f) : fkey(-1e34f);
   if (w < kCounterWords)
     counters[w] = (w >= kRootKeys && w < kRootKeys + 3) ? fkey(1e34f)
                   : (w >= kRootKeys + 3 && w < kRootKeys + 6) ? fkey(-1e34f)
@@ -433,7 +440,7 @@ __global__ void k_finit(uint32_t* counters) {
 // Root bounds: reduced over the block before the six counters every block shares
 // are touched. With one atomic per warp the 2.0 M-triangle prep spent 290 of its
 // us on them.
-__device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn[3], uint32_t kmx[3]) {
+__device__ __forceinline__ void block_root_keys(uint32_t* root, uint32_t kmn[3], uint32_t kmx[3]) {
   __shared__ uint32_t red[6];
   if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
   __syncthreads();
@@ -444,8 +451,8 @@ __device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn
   if ((threadIdx.x & 31) == 0)
     for (int k = 0; k < 3; k++) atomicMin(&red[k], kmn[k]), atomicMax(&red[3 + k], kmx[k]);
   __syncthreads();
-  if (threadIdx.x < 3) atomicMin(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
-  else if (threadIdx.x < 6) atomicMax(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
+  if (threadIdx.x < 3) atomicMin(&root[threadIdx.x], red[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(&root[threadIdx.x], red[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(256) k_fmag(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
@@ -467,12 +474,15 @@ __global__ void __launch_bounds__(256) k_fmag(const float4* __restrict__ v, cons
   if (threadIdx.x == 0) atomicMax(&counters[kMag], red);
 }
 
+// prims: the buffer of the first level, or the final one when the root is small.
+// cbk: the root's centroid bounds.
 // rel_pad: kPad for the traversal-speed quad tree, 0 (exact bounds) for the wide tree
 __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
                                                PrimBox* __restrict__ box, uint32_t* __restrict__ prims,
-                                               uint32_t* counters, float rel_pad) {
+                                               uint32_t* counters, uint32_t* cbk, float rel_pad) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
+  uint32_t cmn[3] = {kmn[0], kmn[1], kmn[2]}, cmx[3] = {kmx[0], kmx[1], kmx[2]};
   if (i < n) {
     const float floor_mag = __fmul_rn(0.25f, __uint_as_float(counters[kMag]));
     const uint4 t = idx[i];
@@ -492,9 +502,14 @@ __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, con
     if (!ok) atomicOr(&counters[kError], kErrRange);
     box[i] = PrimBox{make_float4(mn[0], mn[1], mn[2], 0.0f), make_float4(mx[0], mx[1], mx[2], 0.0f)};
     prims[i] = i;
-    for (int k = 0; k < 3; k++) kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
+    for (int k = 0; k < 3; k++) {
+      kmn[k] = fkey(mn[k]), kmx[k] = fkey(mx[k]);
+      cmn[k] = min(cmn[k], fkey(ce[k])), cmx[k] = max(cmx[k], fkey(ce[k]));
+    }
   }
-  block_root_keys(counters, kmn, kmx);
+  block_root_keys(counters + kRootKeys, kmn, kmx);
+  __syncthreads();  // its shared words are used again
+  block_root_keys(cbk, cmn, cmx);
 }
 
 __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t n, uint32_t* counters) {
@@ -505,7 +520,7 @@ __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t 
   if (n >= 2) {
     if (n > kWarpMax) {
       large[0] = 0;
-      counters[kLargeNext] = 1;
+      counters[kLarge] = 1;
     } else {
       small[0] = 0;
       counters[kSmallCount] = 1;
@@ -514,88 +529,88 @@ __global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t 
 }
 
 // ---------------------------------------------------------------- large nodes, one level
+// The kernels of a level read how many nodes and chunks it has from the counters of
+// its parity, so that several levels can be issued without asking the device (their
+// grids are upper bounds). A large node's primitives lie in the buffer of its
+// level's parity; the partition writes those of its children to the other one when
+// they are large and to the final array otherwise, so nothing is copied back, and
+// takes the children's centroid bounds on the way. With a copy pass, a pass for the
+// bounds and one for the offsets a level of 2.0 M triangles took 128 us, now 94.
+struct LevelArgs {
+  FNodeD* arena;
+  int32_t* large[2];
+  uint32_t max_large;
+  int32_t* small;
+  uint32_t max_small;
+  uint32_t* counters;
+  uint32_t cap;
+  float ascale;
+  uint32_t chunk, max_chunks;
+  Chunk* chunks;
+  FSplit* split;
+  uint32_t* bins;
+  uint32_t* cbk[2];
+  uint32_t* chunk_left;
+  uint32_t* left;  // a bit per primitive of a chunk: goes left (chunk / 32 words each)
+  const PrimBox* box;
+  uint32_t* buf[2];
+  uint32_t* prims;
+};
+__device__ __forceinline__ uint32_t large_count(const LevelArgs& A, int par) {
+  return min(A.counters[kLarge + par], A.max_large);
+}
+__device__ __forceinline__ uint32_t chunk_count(const LevelArgs& A, int par) {
+  return min(A.counters[kChunks + par], A.max_chunks);
+}
+
 // One warp per node: its lanes write the chunks and the empty bins (one thread
 // took up to 31 us a level over the 336 bin words of its node).
-__global__ void __launch_bounds__(256) k_fchunks(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
-                                                 uint32_t nl, uint32_t chunk, uint32_t max_chunks, Chunk* chunks, FSplit* split,
-                                                 uint32_t* bins, uint32_t* cbk, uint32_t* counters) {
+__global__ void __launch_bounds__(256) k_fchunks(LevelArgs A, int par) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (s >= nl) return;  // whole warp
-  const FNodeD& nd = arena[large[s]];
-  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + chunk - 1) / chunk;
+  // the next level's counters: its last reader was the level before this one
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.counters[kLarge + (par ^ 1)] = 0, A.counters[kChunks + (par ^ 1)] = 0;
+  if (s >= large_count(A, par)) return;  // whole warp
+  const FNodeD& nd = A.arena[A.large[par][s]];
+  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + A.chunk - 1) / A.chunk;
   uint32_t base = 0;
-  if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
+  if (lane == 0) base = atomicAdd(&A.counters[kChunks + par], nc);
   base = __shfl_sync(0xffffffffu, base, 0);
-  if (base + nc > max_chunks) {
+  if (base + nc > A.max_chunks) {
     if (lane == 0) {
-      atomicOr(&counters[kError], kErrArena);
-      split[s] = FSplit{-2, 0, 0.0f, 0.0f, 0, 0u, 0u, 0u};
+      atomicOr(&A.counters[kError], kErrArena);
+      A.split[s] = FSplit{-2, {-1, -1}, 0, 0.0f, 0.0f, 0, 0u, 0u};
     }
+    for (uint32_t c = base + lane; c < A.max_chunks; c += 32) A.chunks[c] = Chunk{(int32_t)s, 0u, 0u};
     return;
   }
   for (uint32_t c = lane; c < nc; c += 32) {
-    const uint32_t b = (uint32_t)nd.first + c * chunk;
-    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * chunk)};
+    const uint32_t b = (uint32_t)nd.first + c * A.chunk;
+    A.chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * A.chunk)};
   }
-  if (lane == 0) split[s] = FSplit{-1, 0, 0.0f, 0.0f, 0, 0u, base, 0u};
-  uint32_t* b = bins + (size_t)s * kBinWords;
+  if (lane == 0) A.split[s] = FSplit{-1, {-1, -1}, 0, 0.0f, 0.0f, 0, 0u, base};
+  uint32_t* b = A.bins + (size_t)s * kBinWords;
   for (int w = lane; w < kBinWords; w += 32) b[w] = bin_init(w);
-  if (lane < 6) cbk[6 * (size_t)s + lane] = lane < 3 ? fkey(1e34f) : fkey(-1e34f);
 }
 
-__device__ __forceinline__ uint32_t nchunks_used(const uint32_t* counters, uint32_t max_chunks) {
-  return min(counters[kChunkCursor], max_chunks);
-}
-
-__global__ void __launch_bounds__(256) k_fcb(const Chunk* __restrict__ chunks, const uint32_t* counters,
-                                             uint32_t max_chunks, const PrimBox* __restrict__ box,
-                                             const uint32_t* __restrict__ prims, uint32_t* cbk) {
-  __shared__ uint32_t red[6];
-  if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
-  const Chunk ch = chunks[blockIdx.x];
-  if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? fkey(1e34f) : fkey(-1e34f);
-  __syncthreads();
-  uint32_t kmn[3] = {fkey(1e34f), fkey(1e34f), fkey(1e34f)}, kmx[3] = {fkey(-1e34f), fkey(-1e34f), fkey(-1e34f)};
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) {
-    const float4 c = centre(prim_box(box + prims[k]));
-    kmn[0] = min(kmn[0], fkey(c.x)), kmn[1] = min(kmn[1], fkey(c.y)), kmn[2] = min(kmn[2], fkey(c.z));
-    kmx[0] = max(kmx[0], fkey(c.x)), kmx[1] = max(kmx[1], fkey(c.y)), kmx[2] = max(kmx[2], fkey(c.z));
-  }
-  for (int a = 0; a < 3; a++) {
-    kmn[a] = __reduce_min_sync(0xffffffffu, kmn[a]);
-    kmx[a] = __reduce_max_sync(0xffffffffu, kmx[a]);
-  }
-  if ((threadIdx.x & 31) == 0)
-    for (int a = 0; a < 3; a++) atomicMin(&red[a], kmn[a]), atomicMax(&red[3 + a], kmx[a]);
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    uint32_t* k = cbk + 6 * (size_t)ch.slot;
-    if (threadIdx.x < 3) atomicMin(&k[threadIdx.x], red[threadIdx.x]);
-    else atomicMax(&k[threadIdx.x], red[threadIdx.x]);
-  }
-}
-
-__global__ void __launch_bounds__(256) k_fbin(const Chunk* __restrict__ chunks, const uint32_t* counters,
-                                              uint32_t max_chunks, const uint32_t* __restrict__ cbk,
-                                              const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
-                                              uint32_t* gbins) {
+__global__ void __launch_bounds__(256) k_fbin(LevelArgs A, int par) {
   __shared__ uint32_t bins[kBinWords];
-  if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
-  const Chunk ch = chunks[blockIdx.x];
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const uint32_t* prims = A.buf[par];
   float blo[3], bscale[3];
-  bin_frame(cbk + 6 * (size_t)ch.slot, blo, bscale);
+  bin_frame(A.cbk[par] + 6 * (size_t)ch.slot, blo, bscale);
   for (int w = threadIdx.x; w < kBinWords; w += blockDim.x) bins[w] = bin_init(w);
   __syncthreads();
   for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
     const bool in = k0 + threadIdx.x < ch.end;
-    const PrimBox v = prim_box(box + (in ? prims[k0 + threadIdx.x] : 0u));
+    const PrimBox v = prim_box(A.box + (in ? prims[k0 + threadIdx.x] : 0u));
     int bin[3];
     bins_of(blo, bscale, centre(v), bin);
     bin_warp(bins, bin, v.lo, v.hi, in);
   }
   __syncthreads();
-  uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
+  uint32_t* g = A.bins + (size_t)ch.slot * kBinWords;
   for (int w = threadIdx.x; w < kBinWords; w += blockDim.x) {
     const uint32_t v = bins[w];
     const int f = w % kBinFields;
@@ -609,23 +624,10 @@ __global__ void __launch_bounds__(256) k_fbin(const Chunk* __restrict__ chunks, 
   }
 }
 
-struct LevelArgs {
-  FNodeD* arena;
-  const int32_t* large;
-  uint32_t nl;
-  int32_t* next_large;
-  uint32_t max_large;
-  int32_t* small;
-  uint32_t max_small;
-  uint32_t* counters;
-  uint32_t cap;
-  float ascale;
-};
-
-// Allocate the two children of node ni and queue them.
-__device__ __forceinline__ void add_children(const LevelArgs& A, int32_t ni, const FNodeD& nd, uint32_t mid,
+// Allocate the two children of node ni and queue them; their slots go to sp.kid.
+__device__ __forceinline__ void add_children(const LevelArgs& A, int par, int32_t ni, const FNodeD& nd, uint32_t mid,
                                              const float lmn[3], const float lmx[3], const float rmn[3],
-                                             const float rmx[3]) {
+                                             const float rmx[3], FSplit& sp) {
   const uint32_t cid = atomicAdd(&A.counters[kArenaCount], 2u);
   if (cid + 2 > A.cap) {
     atomicOr(&A.counters[kError], kErrArena);
@@ -635,25 +637,26 @@ __device__ __forceinline__ void add_children(const LevelArgs& A, int32_t ni, con
   A.arena[cid] = make_node(lmn, lmx, (uint32_t)nd.first, mid, ni, nd.depth + 1);
   A.arena[cid + 1] = make_node(rmn, rmx, (uint32_t)nd.first + mid, count - mid, ni, nd.depth + 1);
   A.arena[ni].left = (int32_t)cid;
-  classify((int32_t)cid, mid, nd.depth + 1, A.next_large, A.max_large, A.small, A.max_small, A.counters);
-  classify((int32_t)cid + 1, count - mid, nd.depth + 1, A.next_large, A.max_large, A.small, A.max_small, A.counters);
+  const int nx = par ^ 1;
+  sp.kid[0] = classify((int32_t)cid, mid, nd.depth + 1, A.large[nx], &A.counters[kLarge + nx], A.max_large, A.cbk[nx],
+                       A.small, A.max_small, A.counters);
+  sp.kid[1] = classify((int32_t)cid + 1, count - mid, nd.depth + 1, A.large[nx], &A.counters[kLarge + nx], A.max_large,
+                       A.cbk[nx], A.small, A.max_small, A.counters);
 }
 
-__global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, const uint32_t* __restrict__ gbins,
-                                                const uint32_t* __restrict__ cbk, FSplit* split,
-                                                const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims) {
+__global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, int par) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (s >= A.nl) return;  // whole warp
-  if (split[s].mode == -2) return;  // no chunks (the build fails)
-  const int32_t ni = A.large[s];
+  if (s >= large_count(A, par)) return;  // whole warp
+  if (A.split[s].mode == -2) return;     // no chunks (the build fails)
+  const int32_t ni = A.large[par][s];
   const FNodeD nd = A.arena[ni];
   float blo[3], bscale[3];
-  bin_frame(cbk + 6 * (size_t)s, blo, bscale);
+  bin_frame(A.cbk[par] + 6 * (size_t)s, blo, bscale);
   // the candidates walk the bins word by word: from shared memory
   __shared__ uint32_t sbins[8][kBinWords];
   uint32_t* bins = sbins[threadIdx.x >> 5];
-  for (int w = lane; w < kBinWords; w += 32) bins[w] = gbins[(size_t)s * kBinWords + w];
+  for (int w = lane; w < kBinWords; w += 32) bins[w] = A.bins[(size_t)s * kBinWords + w];
   __syncwarp();
   Cand c;
   choose_bin_split(bins, bscale, A.ascale, lane, c);
@@ -661,128 +664,146 @@ __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, const uint32_t* __r
   if (c.j < kCands) {
     if (lane == 0) {
       const int a = c.j / (kBins - 1);
-      split[s].mode = 0;
-      split[s].axis = a;
-      split[s].lo = blo[a];
-      split[s].scale = bscale[a];
-      split[s].bsp = c.j % (kBins - 1) + 1;
-      split[s].lc = c.lc;
-      add_children(A, ni, nd, c.lc, c.lmn, c.lmx, c.rmn, c.rmx);
+      FSplit sp{0, {-1, -1}, a, blo[a], bscale[a], c.j % (kBins - 1) + 1, c.lc, A.split[s].chunk0};
+      add_children(A, par, ni, nd, c.lc, c.lmn, c.lmx, c.rmn, c.rmx, sp);
+      A.split[s] = sp;
     }
     return;
   }
   // every centroid in one bin on every axis: halve the range as it lies
   const uint32_t mid = count / 2;
   float lmn[3], lmx[3], rmn[3], rmx[3];
-  warp_union(box, prims, (uint32_t)nd.first, (uint32_t)nd.first + mid, lane, lmn, lmx);
-  warp_union(box, prims, (uint32_t)nd.first + mid, (uint32_t)nd.first + count, lane, rmn, rmx);
+  const uint32_t* prims = A.buf[par];
+  warp_union(A.box, prims, (uint32_t)nd.first, (uint32_t)nd.first + mid, lane, lmn, lmx);
+  warp_union(A.box, prims, (uint32_t)nd.first + mid, (uint32_t)nd.first + count, lane, rmn, rmx);
   if (lane == 0) {
-    split[s].mode = 1;
-    add_children(A, ni, nd, mid, lmn, lmx, rmn, rmx);
+    FSplit sp{1, {-1, -1}, 0, 0.0f, 0.0f, 0, mid, A.split[s].chunk0};
+    add_children(A, par, ni, nd, mid, lmn, lmx, rmn, rmx, sp);
+    A.split[s] = sp;
   }
 }
 
+// Which side each primitive of a chunk goes to (a bit each), how many go left, and
+// the centroid bounds of the children that are split on the next level.
+__global__ void __launch_bounds__(256) k_fpcount(LevelArgs A, int par) {
+  __shared__ uint32_t red[2][6], nleft;
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const FSplit sp = A.split[ch.slot];
+  if (sp.mode < 0) return;
+  const uint32_t* prims = A.buf[par];
+  const uint32_t half = (uint32_t)A.arena[A.large[par][ch.slot]].first + sp.lc;  // mode 1: the left half's end
+  if (threadIdx.x < 12) red[threadIdx.x / 6][threadIdx.x % 6] = threadIdx.x % 6 < 3 ? 0xffffffffu : 0u;
+  if (threadIdx.x == 0) nleft = 0;
+  __syncthreads();
+  uint32_t key[2][6];
+  for (int i = 0; i < 2; i++)
+    for (int k = 0; k < 6; k++) key[i][k] = k < 3 ? 0xffffffffu : 0u;
+  const int lane = threadIdx.x & 31;
+  uint32_t n = 0;
+  uint32_t* bits = A.left + (size_t)blockIdx.x * (A.chunk / 32);
+  for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
+    const uint32_t k = k0 + threadIdx.x;
+    const bool in = k < ch.end;
+    const float4 c = centre(prim_box(A.box + (in ? prims[k] : 0u)));
+    const bool left = in && (sp.mode == 1 ? k < half : bin_of(comp(c, sp.axis), sp.lo, sp.scale) < sp.bsp);
+    const bool right = in && !left;
+    const uint32_t b = __ballot_sync(0xffffffffu, left);
+    if (lane == 0) bits[(k0 - ch.begin + threadIdx.x) / 32] = b, n += __popc(b);
+    const uint32_t v[3] = {fkey(c.x), fkey(c.y), fkey(c.z)};
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      key[0][a] = min(key[0][a], left ? v[a] : 0xffffffffu), key[0][3 + a] = max(key[0][3 + a], left ? v[a] : 0u);
+      key[1][a] = min(key[1][a], right ? v[a] : 0xffffffffu), key[1][3 + a] = max(key[1][3 + a], right ? v[a] : 0u);
+    }
+  }
+  if (lane == 0 && n) atomicAdd(&nleft, n);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    if (sp.kid[i] < 0) continue;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const uint32_t mn = __reduce_min_sync(0xffffffffu, key[i][a]), mx = __reduce_max_sync(0xffffffffu, key[i][3 + a]);
+      if (lane == 0) atomicMin(&red[i][a], mn), atomicMax(&red[i][3 + a], mx);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) A.chunk_left[blockIdx.x] = nleft;
+  if (threadIdx.x < 12) {
+    const int i = threadIdx.x / 6, k = threadIdx.x % 6;
+    const int32_t kid = i ? sp.kid[1] : sp.kid[0];
+    if (kid >= 0) {
+      uint32_t* g = A.cbk[par ^ 1] + 6 * (size_t)kid + k;
+      if (k < 3) atomicMin(g, red[i][k]);
+      else atomicMax(g, red[i][k]);
+    }
+  }
+}
+
+// Stable partition by k_fpcount's bits; every block adds up the node's chunk counts
+// before its own. Should they not give the split's left count (they come from the
+// same bins), the range stays as it lies and the build fails.
+constexpr int kMaxWords = 2048 / 32;  // bit words of a chunk
+__global__ void __launch_bounds__(256) k_fpscatter(LevelArgs A, int par) {
+  __shared__ uint32_t word[kMaxWords], before[kMaxWords], sum[2];
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const FSplit sp = A.split[ch.slot];
+  if (sp.mode < 0) return;
+  const FNodeD& nd = A.arena[A.large[par][ch.slot]];
+  const uint32_t first = (uint32_t)nd.first, nc = ((uint32_t)nd.count + A.chunk - 1) / A.chunk;
+  const uint32_t mine = blockIdx.x - sp.chunk0, cnt = ch.end - ch.begin, words = (cnt + 31) / 32;
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t pre = 0, all = 0;
+  for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) {
+    const uint32_t v = A.chunk_left[sp.chunk0 + c];
+    all += v;
+    if (c < mine) pre += v;
+  }
+  pre = __reduce_add_sync(0xffffffffu, pre), all = __reduce_add_sync(0xffffffffu, all);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0 && all) atomicAdd(&sum[0], pre), atomicAdd(&sum[1], all);
+  if (warp == 0) {  // left counts before each word
+    uint32_t run = 0;
+    for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+      const uint32_t w = w0 + lane, b = w < words ? A.left[(size_t)blockIdx.x * (A.chunk / 32) + w] : 0u;
+      const uint32_t v = __popc(b);
+      uint32_t x = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+      }
+      if (w < words) word[w] = b, before[w] = run + x - v;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  __syncthreads();
+  const uint32_t* from = A.buf[par];
+  uint32_t* to_l = sp.kid[0] >= 0 ? A.buf[par ^ 1] : A.prims;
+  uint32_t* to_r = sp.kid[1] >= 0 ? A.buf[par ^ 1] : A.prims;
+  if (sum[1] != sp.lc) {
+    if (threadIdx.x == 0) atomicOr(&A.counters[kError], kErrPartition);
+    for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x)
+      (k < first + sp.lc ? to_l : to_r)[k] = from[k];
+    return;
+  }
+  const uint32_t dl = first + sum[0], dr = first + sp.lc + (ch.begin - first) - sum[0];
+  const uint32_t lt = (1u << lane) - 1u;
+  for (uint32_t w = warp; w < words; w += 8) {
+    if (32 * w + lane >= cnt) continue;
+    const uint32_t b = word[w], l = before[w] + __popc(b & lt), p = from[ch.begin + 32 * w + lane];
+    if ((b >> lane) & 1u) to_l[dl + l] = p;
+    else to_r[dr + 32 * w + lane - l] = p;
+  }
+}
+
+// ---------------------------------------------------------------- small subtrees, one warp each
 __device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, const FSplit& sp) {
   return bin_of(comp(centre(prim_box(box + p)), sp.axis), sp.lo, sp.scale) < sp.bsp;
 }
 
-__global__ void __launch_bounds__(256) k_fpcount(const Chunk* __restrict__ chunks, const FSplit* __restrict__ split,
-                                                 const uint32_t* counters, uint32_t max_chunks,
-                                                 const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
-                                                 uint32_t* chunk_left) {
-  __shared__ uint32_t warp_sum[8];
-  if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
-  const Chunk ch = chunks[blockIdx.x];
-  const FSplit sp = split[ch.slot];
-  if (sp.mode != 0) return;
-  uint32_t n = 0;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(box, prims[k], sp);
-  n = __reduce_add_sync(0xffffffffu, n);
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = n;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += warp_sum[w];
-    chunk_left[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_fpoffsets(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
-                                                   uint32_t nl, uint32_t chunk, FSplit* split, const uint32_t* __restrict__ chunk_left,
-                                                   uint32_t* chunk_loff, uint32_t* counters) {
-  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (s >= nl) return;
-  const FSplit sp = split[s];
-  if (sp.mode != 0) return;
-  const uint32_t nc = ((uint32_t)arena[large[s]].count + chunk - 1) / chunk;
-  uint32_t run = 0;
-  for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
-    const uint32_t c = c0 + lane;
-    const uint32_t v = c < nc ? chunk_left[sp.chunk0 + c] : 0u;
-    uint32_t x = v;  // inclusive warp scan
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-      if (lane >= off) x += y;
-    }
-    if (c < nc) chunk_loff[sp.chunk0 + c] = run + x - v;
-    run += __shfl_sync(0xffffffffu, x, 31);
-  }
-  if (lane == 0 && run != sp.lc) {
-    // the bins and the predicate disagree: keep the range (the build fails)
-    atomicOr(&counters[kError], kErrPartition);
-    split[s].mode = -1;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_fpscatter(const FNodeD* __restrict__ arena, const int32_t* __restrict__ large,
-                                                   const Chunk* __restrict__ chunks, const FSplit* __restrict__ split,
-                                                   const uint32_t* counters, uint32_t max_chunks,
-                                                   const uint32_t* __restrict__ chunk_loff,
-                                                   const PrimBox* __restrict__ box, const uint32_t* __restrict__ prims,
-                                                   uint32_t* tmp) {
-  __shared__ uint32_t wl[8], wr[8];
-  if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
-  const Chunk ch = chunks[blockIdx.x];
-  const FSplit sp = split[ch.slot];
-  if (sp.mode != 0) return;
-  const uint32_t first = (uint32_t)arena[large[ch.slot]].first;
-  const uint32_t loff = chunk_loff[blockIdx.x];
-  const uint32_t roff = (ch.begin - first) - loff;
-  uint32_t dl = first + loff, dr = first + sp.lc + roff;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
-    const uint32_t k = k0 + threadIdx.x;
-    const bool in = k < ch.end;
-    const uint32_t p = in ? prims[k] : 0u;
-    const bool left = in && goes_left(box, p, sp);
-    const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
-    if (lane == 0) wl[warp] = __popc(bl), wr[warp] = __popc(br);
-    __syncthreads();
-    uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
-    for (int w = 0; w < nw; w++) {
-      if (w < warp) pl += wl[w], pr += wr[w];
-      tl += wl[w], tr += wr[w];
-    }
-    if (left) tmp[dl + pl + __popc(bl & lt)] = p;
-    else if (in) tmp[dr + pr + __popc(br & lt)] = p;
-    dl += tl, dr += tr;
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(256) k_fpcopy(const Chunk* __restrict__ chunks, const FSplit* __restrict__ split,
-                                                const uint32_t* counters, uint32_t max_chunks,
-                                                const uint32_t* __restrict__ tmp, uint32_t* prims) {
-  if (blockIdx.x >= nchunks_used(counters, max_chunks)) return;
-  const Chunk ch = chunks[blockIdx.x];
-  if (split[ch.slot].mode != 0) return;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) prims[k] = tmp[k];
-}
-
-// ---------------------------------------------------------------- small subtrees, one warp each
 // Exact SAH sweep of a range of 2..16 primitives (sweep_split): every split of
 // the centroid order (ties by primitive id) on each axis; reorders the range to
 // the winning axis' order. Returns the left count and the child boxes.
@@ -863,9 +884,9 @@ __device__ __forceinline__ bool leaf_task(uint32_t count, int32_t depth) {
 
 // tasks: ranges for k_fleaf, counted in counters[kTasks]; at most n / 2 of them
 // (disjoint, two primitives or more each).
-__global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const int32_t* __restrict__ small_ro,
-                                                             const PrimBox* __restrict__ box, uint32_t* prims,
-                                                             uint32_t* tasks) {
+__global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, uint32_t* tasks) {
+  const PrimBox* __restrict__ box = A.box;
+  uint32_t* prims = A.prims;
   __shared__ uint32_t sbins[kSmallWarps][kBinWords];
   __shared__ int32_t sstack[kSmallWarps][kSmallStack];
   __shared__ uint32_t stmp[kSmallWarps][2 * kWarpMax];
@@ -877,7 +898,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, const 
   uint32_t* tmp = stmp[warp];
   const uint32_t nsmall = min(A.counters[kSmallCount], A.max_small);
   for (uint32_t sidx = blockIdx.x * kSmallWarps + warp; sidx < nsmall; sidx += gridDim.x * kSmallWarps) {
-    const int32_t root = small_ro[sidx];
+    const int32_t root = A.small[sidx];
     if (leaf_task((uint32_t)A.arena[root].count, A.arena[root].depth)) {
       if (lane == 0) tasks[atomicAdd(&A.counters[kTasks], 1u)] = (uint32_t)root;
       continue;
@@ -1007,8 +1028,9 @@ constexpr size_t kLeafShared = sizeof(float) * kLeafWords * kLeafThreads;
 
 __device__ __forceinline__ uint32_t nib(unsigned long long o, uint32_t i) { return (uint32_t)(o >> (4 * i)) & 15u; }
 
-__global__ void __launch_bounds__(kLeafThreads) k_fleaf(LevelArgs A, const uint32_t* __restrict__ tasks,
-                                                        const PrimBox* __restrict__ boxes, uint32_t* prims) {
+__global__ void __launch_bounds__(kLeafThreads) k_fleaf(LevelArgs A, const uint32_t* __restrict__ tasks) {
+  const PrimBox* __restrict__ boxes = A.box;
+  uint32_t* prims = A.prims;
   extern __shared__ float sh[];
   constexpr int T = kLeafThreads;
   float* box = sh + threadIdx.x;                         // box[(6 j + c) T]: min x/y/z, max x/y/z of primitive j
@@ -1521,13 +1543,6 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   FNodeD* arena = at<FNodeD>(scratch, Lo.arena);
   FCostD* cost = at<FCostD>(scratch, Lo.cost);
   uint32_t* arrive = at<uint32_t>(scratch, Lo.arrive);
-  int32_t* large[2] = {at<int32_t>(scratch, Lo.large0), at<int32_t>(scratch, Lo.large1)};
-  int32_t* small = at<int32_t>(scratch, Lo.small);
-  Chunk* chunks = at<Chunk>(scratch, Lo.chunks);
-  uint32_t* chunk_left = at<uint32_t>(scratch, Lo.chunk_left);
-  uint32_t* chunk_loff = at<uint32_t>(scratch, Lo.chunk_loff);
-  FSplit* split = at<FSplit>(scratch, Lo.split);
-  uint32_t* bins = at<uint32_t>(scratch, Lo.bins);
   uint32_t* cbk = at<uint32_t>(scratch, Lo.cbk);
   uint32_t* qlist = at<uint32_t>(scratch, Lo.qlist);
   QRec* qrec = at<QRec>(scratch, Lo.qrec);
@@ -1535,10 +1550,32 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   uint32_t* sums = at<uint32_t>(scratch, Lo.sums);
   r = GpuBvhResult{};
 
-  k_finit<<<1, 32, 0, s>>>(counters);
+  // the levels' second buffer and partition bits lie where the quad phase works later
+  LevelArgs A;
+  A.arena = arena;
+  A.large[0] = at<int32_t>(scratch, Lo.large0), A.large[1] = at<int32_t>(scratch, Lo.large1);
+  A.max_large = Lo.max_large;
+  A.small = at<int32_t>(scratch, Lo.small);
+  A.max_small = Lo.max_small;
+  A.counters = counters;
+  A.cap = Lo.cap;
+  A.ascale = 0.0f;
+  A.chunk = Lo.chunk, A.max_chunks = Lo.max_chunks;
+  A.chunks = at<Chunk>(scratch, Lo.chunks);
+  A.split = at<FSplit>(scratch, Lo.split);
+  A.bins = at<uint32_t>(scratch, Lo.bins);
+  A.cbk[0] = cbk, A.cbk[1] = cbk + 6 * (size_t)Lo.max_large;
+  A.chunk_left = at<uint32_t>(scratch, Lo.chunk_left);
+  A.left = qlist;
+  A.box = box;
+  A.buf[0] = tmp, A.buf[1] = scan;
+  A.prims = prims;
+
+  k_finit<<<1, 32, 0, s>>>(counters, cbk);
   k_fmag<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, counters);
-  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, prims, counters, wide ? 0.0f : kPad);
-  k_froot<<<1, 1, 0, s>>>(arena, large[0], small, n, counters);
+  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > kWarpMax ? A.buf[0] : prims, counters, cbk,
+                                           wide ? 0.0f : kPad);
+  k_froot<<<1, 1, 0, s>>>(arena, A.large[0], A.small, n, counters);
   FB_TRY(cudaGetLastError());
   FB_TRY(read_counters(hc, counters, s));
   if (hc[kError]) {
@@ -1554,53 +1591,46 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     std::memcpy(&rmx[k], &b, 4);
   }
   const float ascale = fast_area_scale(rmn, rmx);
-  LevelArgs A{arena, nullptr, 0, nullptr, Lo.max_large, small, Lo.max_small, counters, Lo.cap, ascale};
-  uint32_t nl = hc[kLargeNext];
-  int cur = 0;
+  A.ascale = ascale;
+  // Up to four levels are issued before the counters are read back (12 us each time),
+  // while all their nodes could be large ones: a level that turns out empty costs
+  // five launches.
+  uint64_t nl = hc[kLarge];
+  int par = 0;
   while (nl > 0) {
-    if (nl > Lo.max_large) {
-      r.error |= kErrArena;
-      return cudaSuccess;
+    int batch = 1;
+    while (batch < 4 && (nl << batch) * kWarpMax <= n) batch++;
+    for (int i = 0; i < batch; i++, par ^= 1) {
+      const uint64_t most = std::min<uint64_t>(nl << i, Lo.max_large);
+      const unsigned gn = blocks(most * 32, 256);
+      const unsigned gc = (unsigned)std::min<uint64_t>((uint64_t)n / Lo.chunk + most + 1, Lo.max_chunks);
+      k_fchunks<<<gn, 256, 0, s>>>(A, par);
+      k_fbin<<<gc, 256, 0, s>>>(A, par);
+      k_fsplit<<<gn, 256, 0, s>>>(A, par);
+      k_fpcount<<<gc, 256, 0, s>>>(A, par);
+      k_fpscatter<<<gc, 256, 0, s>>>(A, par);
     }
-    FB_TRY(cudaMemsetAsync(counters + kLargeNext, 0, 8, s));  // kLargeNext, kChunkCursor
-    A.large = large[cur];
-    A.nl = nl;
-    A.next_large = large[cur ^ 1];
-    k_fchunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, Lo.max_chunks, chunks, split, bins, cbk,
-                                              counters);
-    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / Lo.chunk + nl + 1, Lo.max_chunks);
-    k_fcb<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, box, prims, cbk);
-    k_fbin<<<nchunk, 256, 0, s>>>(chunks, counters, Lo.max_chunks, cbk, box, prims, bins);
-    k_fsplit<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(A, bins, cbk, split, box, prims);
-    k_fpcount<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, box, prims, chunk_left);
-    k_fpoffsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, Lo.chunk, split, chunk_left, chunk_loff,
-                                                              counters);
-    k_fpscatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, Lo.max_chunks, chunk_loff, box,
-                                       prims, tmp);
-    k_fpcopy<<<nchunk, 256, 0, s>>>(chunks, split, counters, Lo.max_chunks, tmp, prims);
     FB_TRY(cudaGetLastError());
     FB_TRY(read_counters(hc, counters, s));
-    nl = hc[kLargeNext];
-    cur ^= 1;
-    r.levels++;
     if (hc[kError]) {
       r.error = hc[kError];
       return cudaSuccess;
     }
+    nl = hc[kLarge + par];
   }
   const uint32_t nsmall = std::min(hc[kSmallCount], Lo.max_small);
   if (nsmall > 0) {
     const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sm_count() * 16);
     FB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
-    // the partition's scratch (4 bytes per primitive) is free now: it takes the tasks
-    k_fsmall<<<g, kSmallWarps * 32, 0, s>>>(A, small, box, prims, tmp);
+    // the levels' first buffer (4 bytes per primitive) is free now: it takes the tasks
+    k_fsmall<<<g, kSmallWarps * 32, 0, s>>>(A, tmp);
     FB_TRY(cudaGetLastError());
     FB_TRY(cudaFuncSetAttribute(k_fleaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
     FB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fleaf, kLeafThreads, kLeafShared));
     const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 2 + 1, kLeafThreads),
                                                      (uint64_t)sm_count() * std::max(1, per_sm));
-    k_fleaf<<<gl, kLeafThreads, kLeafShared, s>>>(A, tmp, box, prims);
+    k_fleaf<<<gl, kLeafThreads, kLeafShared, s>>>(A, tmp);
     FB_TRY(cudaGetLastError());
   }
   FB_TRY(read_counters(hc, counters, s));
