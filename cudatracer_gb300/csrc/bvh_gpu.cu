@@ -60,13 +60,13 @@ enum : uint32_t { kErrDegenerate = 1, kErrArena = 2, kErrStack = 4, kErrPartitio
 enum Counter : int {
   kArenaCount = 0,
   kSmallCount = 1,
-  kLargeNext = 2,
-  kChunkCursor = 3,
-  kTasks = kChunkCursor,  // ranges for k_leaf, once the levels are done
+  kChunks = 2,       // 2 words: chunks of the even and of the odd level
+  kTasks = kChunks,  // ranges for k_leaf, once the levels are done
   kError = 4,
   kMaxLeaf = 5,
   kQuadDepth = 6,
-  kRootKeys = 8,  // 6 words: min x/y/z, max x/y/z
+  kRootKeys = 8,     // 6 words: min x/y/z, max x/y/z
+  kLarge = 14,       // 2 words: large nodes of the even and of the odd level
   kCounterWords = 16
 };
 
@@ -104,11 +104,12 @@ struct Split {
   float coord;
   uint32_t lc;
   uint32_t chunk0;
+  uint32_t queued;  // bit 0, 1: the left, right child is split on the next level
 };
 
 // Carving of the scratch block for n primitives.
 struct Layout {
-  size_t box, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, chunk_loff, split, bins,
+  size_t box, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, split, bins,
       counters, total;
   uint32_t chunk, cap, max_large, max_chunks, max_small;
   explicit Layout(uint32_t n) {
@@ -134,7 +135,6 @@ struct Layout {
     small = take(4 * (size_t)max_small);
     chunks = take(sizeof(Chunk) * (size_t)max_chunks);
     chunk_left = take(4 * (size_t)max_chunks);
-    chunk_loff = take(4 * (size_t)max_chunks);
     split = take(sizeof(Split) * (size_t)max_large);
     bins = take(4 * (size_t)kBinWords * max_large);
     counters = take(4 * kCounterWords);
@@ -347,6 +347,7 @@ __device__ __forceinline__ void block_root_keys(uint32_t* counters, uint32_t kmn
   else if (threadIdx.x < 6) atomicMax(&counters[kRootKeys + threadIdx.x], red[threadIdx.x]);
 }
 
+// prims: the buffer of the first level, or the final one when the root is small
 __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, const uint4* __restrict__ idx, uint32_t n,
                                               PrimBox* __restrict__ box,
                                               uint32_t* __restrict__ prims, uint32_t* counters) {
@@ -376,7 +377,7 @@ __global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n,
   if (n >= 4) {
     if (n > kWarpMax) {
       large[0] = 0;
-      counters[kLargeNext] = 1;
+      counters[kLarge] = 1;
     } else {
       small[0] = 0;
       counters[kSmallCount] = 1;
@@ -385,36 +386,64 @@ __global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n,
 }
 
 // ---------------------------------------------------------------- large nodes, one level
+// The kernels of a level read how many nodes and chunks it has from the counters of
+// its parity, so that several levels can be issued without asking the device (their
+// grids are upper bounds). A large node's primitives lie in the buffer of its
+// level's parity; the partition writes those of its children to the other one when
+// they are large and to the final array otherwise, so nothing is copied back.
+struct LevelArgs {
+  BNode* arena;
+  int32_t* large[2];
+  uint32_t max_large;
+  int32_t* small;
+  uint32_t* counters;
+  uint32_t cap;
+  uint32_t chunk, max_chunks;
+  Chunk* chunks;
+  Split* split;
+  uint32_t* bins;
+  uint32_t* chunk_left;
+  uint32_t* left;  // a bit per primitive of a chunk: goes left (chunk / 32 words each)
+  const PrimBox* box;
+  uint32_t* buf[2];
+  uint32_t* prims;
+};
+__device__ __forceinline__ uint32_t large_count(const LevelArgs& A, int par) {
+  return min(A.counters[kLarge + par], A.max_large);
+}
+__device__ __forceinline__ uint32_t chunk_count(const LevelArgs& A, int par) {
+  return min(A.counters[kChunks + par], A.max_chunks);
+}
+
 // One warp per node: its lanes write the chunks and the empty bins.
-__global__ void __launch_bounds__(256) k_chunks(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                                uint32_t nl, uint32_t chunk, Chunk* chunks, Split* split, uint32_t* bins,
-                                                uint32_t* counters) {
+__global__ void __launch_bounds__(256) k_chunks(LevelArgs A, int par) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (s >= nl) return;  // whole warp
-  const BNode& nd = arena[large[s]];
-  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + chunk - 1) / chunk;
+  // the next level's counters: its last reader was the level before this one
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.counters[kLarge + (par ^ 1)] = 0, A.counters[kChunks + (par ^ 1)] = 0;
+  if (s >= large_count(A, par)) return;  // whole warp
+  const BNode& nd = A.arena[A.large[par][s]];
+  const uint32_t cnt = (uint32_t)nd.count, nc = (cnt + A.chunk - 1) / A.chunk;
   uint32_t base = 0;
-  if (lane == 0) base = atomicAdd(&counters[kChunkCursor], nc);
+  if (lane == 0) base = atomicAdd(&A.counters[kChunks + par], nc);
   base = __shfl_sync(0xffffffffu, base, 0);
   for (uint32_t c = lane; c < nc; c += 32) {
-    const uint32_t b = (uint32_t)nd.first + c * chunk;
-    chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * chunk)};
+    const uint32_t b = (uint32_t)nd.first + c * A.chunk;
+    if (base + c < A.max_chunks)  // always: the ranges are disjoint
+      A.chunks[base + c] = Chunk{(int32_t)s, b, (uint32_t)nd.first + min(cnt, (c + 1) * A.chunk)};
   }
-  if (lane == 0) split[s] = Split{-1, 0.0f, 0u, base};
-  uint32_t* b = bins + (size_t)s * kBinWords;
+  if (lane == 0) A.split[s] = Split{-1, 0.0f, 0u, base, 0u};
+  uint32_t* b = A.bins + (size_t)s * kBinWords;
   for (int w = lane; w < kBinWords; w += 32) b[w] = bin_init(w);
 }
 
-__global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                             const Chunk* __restrict__ chunks, const uint32_t* counters,
-                                             const PrimBox* __restrict__ box,
-                                             const uint32_t* __restrict__ prims, uint32_t* gbins) {
+__global__ void __launch_bounds__(256) k_bin(LevelArgs A, int par) {
   __shared__ float planes[3 * kPlanes];
   __shared__ uint32_t bins[kBinWords];
-  if (blockIdx.x >= counters[kChunkCursor]) return;
-  const Chunk ch = chunks[blockIdx.x];
-  const BNode& nd = arena[large[ch.slot]];
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const BNode& nd = A.arena[A.large[par][ch.slot]];
+  const uint32_t* prims = A.buf[par];
   if (threadIdx.x < 3 * kPlanes) {
     const int a = threadIdx.x / kPlanes, i = threadIdx.x % kPlanes + 1;
     planes[threadIdx.x] = plane_at(nd.mn[a], nd.mx[a], i);
@@ -423,13 +452,13 @@ __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, co
   __syncthreads();
   for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
     const bool in = k0 + threadIdx.x < ch.end;
-    const PrimBox v = prim_box(box + (in ? prims[k0 + threadIdx.x] : 0u));
+    const PrimBox v = prim_box(A.box + (in ? prims[k0 + threadIdx.x] : 0u));
     int iv[3];
     intervals_of(planes, v.lo, v.hi, iv);
     bin_warp(bins, iv, v.lo, v.hi, in);
   }
   __syncthreads();
-  uint32_t* g = gbins + (size_t)ch.slot * kBinWords;
+  uint32_t* g = A.bins + (size_t)ch.slot * kBinWords;
   for (int w = threadIdx.x; w < kBinWords; w += blockDim.x) {
     const uint32_t v = bins[w];
     const int f = w % kBinFields;
@@ -443,54 +472,52 @@ __global__ void __launch_bounds__(256) k_bin(const BNode* __restrict__ arena, co
   }
 }
 
-// Place a new child: leaf, a node for the next level, or a warp-built subtree root.
-__device__ __forceinline__ void classify(int32_t id, uint32_t count, int32_t depth, int32_t* next_large,
-                                         int32_t* small, uint32_t* counters) {
-  if (count < 4 || depth > kMaxSplitDepth) return;
-  if (count > kWarpMax)
-    next_large[atomicAdd(&counters[kLargeNext], 1u)] = id;
-  else
-    small[atomicAdd(&counters[kSmallCount], 1u)] = id;
+// Place a new child: leaf, a node for the next level (true), or a warp-built subtree root.
+__device__ __forceinline__ bool classify(const LevelArgs& A, int par, int32_t id, uint32_t count, int32_t depth) {
+  if (count < 4 || depth > kMaxSplitDepth) return false;
+  if (count > kWarpMax) {
+    const uint32_t s = atomicAdd(&A.counters[kLarge + (par ^ 1)], 1u);
+    if (s < A.max_large) A.large[par ^ 1][s] = id;
+    return s < A.max_large;
+  }
+  A.small[atomicAdd(&A.counters[kSmallCount], 1u)] = id;
+  return false;
 }
 
-__global__ void __launch_bounds__(256) k_split(BNode* arena, const int32_t* __restrict__ large, uint32_t nl,
-                                               const uint32_t* __restrict__ gbins, Split* split, int32_t* next_large,
-                                               int32_t* small, uint32_t* counters, uint32_t cap) {
+__global__ void __launch_bounds__(256) k_split(LevelArgs A, int par) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (s >= nl) return;  // whole warp
-  const int32_t ni = large[s];
-  const BNode nd = arena[ni];
+  if (s >= large_count(A, par)) return;  // whole warp
+  const int32_t ni = A.large[par][s];
+  const BNode nd = A.arena[ni];
   // the candidates walk the bins word by word: from shared memory
   __shared__ uint32_t sbins[8][kBinWords];
   uint32_t* bins = sbins[threadIdx.x >> 5];
-  for (int w = lane; w < kBinWords; w += 32) bins[w] = gbins[(size_t)s * kBinWords + w];
+  for (int w = lane; w < kBinWords; w += 32) bins[w] = A.bins[(size_t)s * kBinWords + w];
   __syncwarp();
   Cand c;
   const int best = choose_split(bins, lane, c);
   const float parent_cost = __fmul_rn(area3(nd.mn, nd.mx), __uint2float_rn((uint32_t)nd.count));
   if (best == 32) {
     // no candidate below 1e34: a leaf unless the parent's cost is not below it either
-    if (!(parent_cost < 1e34f) && lane == 0) atomicOr(&counters[kError], kErrDegenerate);
+    if (!(parent_cost < 1e34f) && lane == 0) atomicOr(&A.counters[kError], kErrDegenerate);
     return;
   }
   bcast_cand(c, best);
   if (parent_cost < c.cost) return;
   if (lane != 0) return;
   const int a = best / kPlanes, i = best % kPlanes + 1;
-  const uint32_t cid = atomicAdd(&counters[kArenaCount], 2u);
-  if (cid + 2 > cap) {
-    atomicOr(&counters[kError], kErrArena);
+  const uint32_t cid = atomicAdd(&A.counters[kArenaCount], 2u);
+  if (cid + 2 > A.cap) {
+    atomicOr(&A.counters[kError], kErrArena);
     return;
   }
-  arena[cid] = make_node(c.lmn, c.lmx, (uint32_t)nd.first, c.lc, ni, nd.depth + 1);
-  arena[cid + 1] = make_node(c.rmn, c.rmx, (uint32_t)nd.first + c.lc, c.rc, ni, nd.depth + 1);
-  arena[ni].left = (int32_t)cid;
-  split[s].axis = a;
-  split[s].coord = plane_at(nd.mn[a], nd.mx[a], i);
-  split[s].lc = c.lc;
-  classify((int32_t)cid, c.lc, nd.depth + 1, next_large, small, counters);
-  classify((int32_t)cid + 1, c.rc, nd.depth + 1, next_large, small, counters);
+  A.arena[cid] = make_node(c.lmn, c.lmx, (uint32_t)nd.first, c.lc, ni, nd.depth + 1);
+  A.arena[cid + 1] = make_node(c.rmn, c.rmx, (uint32_t)nd.first + c.lc, c.rc, ni, nd.depth + 1);
+  A.arena[ni].left = (int32_t)cid;
+  uint32_t queued = classify(A, par, (int32_t)cid, c.lc, nd.depth + 1) ? 1u : 0u;
+  queued |= classify(A, par, (int32_t)cid + 1, c.rc, nd.depth + 1) ? 2u : 0u;
+  A.split[s] = Split{a, plane_at(nd.mn[a], nd.mx[a], i), c.lc, A.split[s].chunk0, queued};
 }
 
 __device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, int axis, float coord) {
@@ -498,100 +525,89 @@ __device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, int ax
   return centroid(comp(v.lo, axis), comp(v.hi, axis)) <= coord;
 }
 
-__global__ void __launch_bounds__(256) k_part_count(const Chunk* __restrict__ chunks, const Split* __restrict__ split,
-                                                    const uint32_t* counters, const PrimBox* __restrict__ box,
-                                                    const uint32_t* __restrict__ prims,
-                                                    uint32_t* chunk_left) {
-  __shared__ uint32_t warp_sum[8];
-  if (blockIdx.x >= counters[kChunkCursor]) return;
-  const Chunk ch = chunks[blockIdx.x];
-  const Split sp = split[ch.slot];
+// Which side each primitive of a chunk goes to (a bit each), and how many go left.
+__global__ void __launch_bounds__(256) k_part_count(LevelArgs A, int par) {
+  __shared__ uint32_t nleft;
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const Split sp = A.split[ch.slot];
   if (sp.axis < 0) return;
-  uint32_t n = 0;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) n += goes_left(box, prims[k], sp.axis, sp.coord);
-  n = __reduce_add_sync(0xffffffffu, n);
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = n;
+  const uint32_t* prims = A.buf[par];
+  if (threadIdx.x == 0) nleft = 0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += warp_sum[w];
-    chunk_left[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_part_offsets(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                                      uint32_t nl, uint32_t chunk, Split* split,
-                                                      const uint32_t* __restrict__ chunk_left, uint32_t* chunk_loff,
-                                                      uint32_t* counters) {
-  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (s >= nl) return;
-  const Split sp = split[s];
-  if (sp.axis < 0) return;
-  const uint32_t nc = ((uint32_t)arena[large[s]].count + chunk - 1) / chunk;
-  uint32_t run = 0;
-  for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
-    const uint32_t c = c0 + lane;
-    const uint32_t v = c < nc ? chunk_left[sp.chunk0 + c] : 0u;
-    uint32_t x = v;  // inclusive warp scan
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-      if (lane >= off) x += y;
-    }
-    if (c < nc) chunk_loff[sp.chunk0 + c] = run + x - v;
-    run += __shfl_sync(0xffffffffu, x, 31);
-  }
-  if (lane == 0 && run != sp.lc) {
-    // the flags disagree with the bins: leave the range as it is (the build fails)
-    atomicOr(&counters[kError], kErrPartition);
-    split[s].axis = -1;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_part_scatter(const BNode* __restrict__ arena, const int32_t* __restrict__ large,
-                                                      const Chunk* __restrict__ chunks, const Split* __restrict__ split,
-                                                      const uint32_t* counters, const uint32_t* __restrict__ chunk_loff,
-                                                      const PrimBox* __restrict__ box,
-                                                      const uint32_t* __restrict__ prims, uint32_t* tmp) {
-  __shared__ uint32_t wl[8], wr[8];
-  if (blockIdx.x >= counters[kChunkCursor]) return;
-  const Chunk ch = chunks[blockIdx.x];
-  const Split sp = split[ch.slot];
-  if (sp.axis < 0) return;
-  const uint32_t first = (uint32_t)arena[large[ch.slot]].first;
-  const uint32_t loff = chunk_loff[blockIdx.x];
-  const uint32_t roff = (ch.begin - first) - loff;
-  uint32_t dl = first + loff, dr = first + sp.lc + roff;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
+  uint32_t n = 0;
+  uint32_t* bits = A.left + (size_t)blockIdx.x * (A.chunk / 32);
   for (uint32_t k0 = ch.begin; k0 < ch.end; k0 += blockDim.x) {
     const uint32_t k = k0 + threadIdx.x;
-    const bool in = k < ch.end;
-    const uint32_t p = in ? prims[k] : 0u;
-    const bool left = in && goes_left(box, p, sp.axis, sp.coord);
-    const uint32_t bl = __ballot_sync(0xffffffffu, left), br = __ballot_sync(0xffffffffu, in && !left);
-    if (lane == 0) wl[warp] = __popc(bl), wr[warp] = __popc(br);
-    __syncthreads();
-    uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
-    for (int w = 0; w < nw; w++) {
-      if (w < warp) pl += wl[w], pr += wr[w];
-      tl += wl[w], tr += wr[w];
-    }
-    if (left) tmp[dl + pl + __popc(bl & lt)] = p;
-    else if (in) tmp[dr + pr + __popc(br & lt)] = p;
-    dl += tl, dr += tr;
-    __syncthreads();
+    const uint32_t b = __ballot_sync(0xffffffffu, k < ch.end && goes_left(A.box, prims[k], sp.axis, sp.coord));
+    if ((threadIdx.x & 31) == 0) bits[(k0 - ch.begin + threadIdx.x) / 32] = b, n += __popc(b);
   }
+  if (n) atomicAdd(&nleft, n);
+  __syncthreads();
+  if (threadIdx.x == 0) A.chunk_left[blockIdx.x] = nleft;
 }
 
-__global__ void __launch_bounds__(256) k_part_copy(const Chunk* __restrict__ chunks, const Split* __restrict__ split,
-                                                   const uint32_t* counters, const uint32_t* __restrict__ tmp,
-                                                   uint32_t* prims) {
-  if (blockIdx.x >= counters[kChunkCursor]) return;
-  const Chunk ch = chunks[blockIdx.x];
-  if (split[ch.slot].axis < 0) return;
-  for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) prims[k] = tmp[k];
+// Stable partition by k_part_count's bits; every block adds up the node's chunk
+// counts before its own. A node that stays a leaf goes to the final array as it
+// lies, and so does a range whose counts don't give the split's left count (they
+// come from the same bins; the build fails).
+constexpr int kMaxWords = 2048 / 32;  // bit words of a chunk
+__global__ void __launch_bounds__(256) k_part_scatter(LevelArgs A, int par) {
+  __shared__ uint32_t word[kMaxWords], before[kMaxWords], sum[2];
+  if (blockIdx.x >= chunk_count(A, par)) return;
+  const Chunk ch = A.chunks[blockIdx.x];
+  const Split sp = A.split[ch.slot];
+  const uint32_t* from = A.buf[par];
+  if (sp.axis < 0) {
+    for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x) A.prims[k] = from[k];
+    return;
+  }
+  const BNode& nd = A.arena[A.large[par][ch.slot]];
+  const uint32_t first = (uint32_t)nd.first, nc = ((uint32_t)nd.count + A.chunk - 1) / A.chunk;
+  const uint32_t mine = blockIdx.x - sp.chunk0, cnt = ch.end - ch.begin, words = (cnt + 31) / 32;
+  if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t pre = 0, all = 0;
+  for (uint32_t c = threadIdx.x; c < nc; c += blockDim.x) {
+    const uint32_t v = A.chunk_left[sp.chunk0 + c];
+    all += v;
+    if (c < mine) pre += v;
+  }
+  pre = __reduce_add_sync(0xffffffffu, pre), all = __reduce_add_sync(0xffffffffu, all);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0 && all) atomicAdd(&sum[0], pre), atomicAdd(&sum[1], all);
+  if (warp == 0) {  // left counts before each word
+    uint32_t run = 0;
+    for (uint32_t w0 = 0; w0 < words; w0 += 32) {
+      const uint32_t w = w0 + lane, b = w < words ? A.left[(size_t)blockIdx.x * (A.chunk / 32) + w] : 0u;
+      const uint32_t v = __popc(b);
+      uint32_t x = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+      }
+      if (w < words) word[w] = b, before[w] = run + x - v;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  __syncthreads();
+  uint32_t* to_l = sp.queued & 1u ? A.buf[par ^ 1] : A.prims;
+  uint32_t* to_r = sp.queued & 2u ? A.buf[par ^ 1] : A.prims;
+  if (sum[1] != sp.lc) {
+    if (threadIdx.x == 0) atomicOr(&A.counters[kError], kErrPartition);
+    for (uint32_t k = ch.begin + threadIdx.x; k < ch.end; k += blockDim.x)
+      (k < first + sp.lc ? to_l : to_r)[k] = from[k];
+    return;
+  }
+  const uint32_t dl = first + sum[0], dr = first + sp.lc + (ch.begin - first) - sum[0];
+  const uint32_t lt = (1u << lane) - 1u;
+  for (uint32_t w = warp; w < words; w += 8) {
+    if (32 * w + lane >= cnt) continue;
+    const uint32_t b = word[w], l = before[w] + __popc(b & lt), p = from[ch.begin + 32 * w + lane];
+    if ((b >> lane) & 1u) to_l[dl + l] = p;
+    else to_r[dr + 32 * w + lane - l] = p;
+  }
 }
 
 // ---------------------------------------------------------------- small subtrees, one warp each
@@ -1022,44 +1038,56 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   uint32_t* prims = at<uint32_t>(scratch, L.prims);
   uint32_t* tmp = at<uint32_t>(scratch, L.tmp);
   BNode* arena = at<BNode>(scratch, L.arena);
-  int32_t* large[2] = {at<int32_t>(scratch, L.large0), at<int32_t>(scratch, L.large1)};
-  int32_t* small = at<int32_t>(scratch, L.small);
-  Chunk* chunks = at<Chunk>(scratch, L.chunks);
-  uint32_t* chunk_left = at<uint32_t>(scratch, L.chunk_left);
-  uint32_t* chunk_loff = at<uint32_t>(scratch, L.chunk_loff);
-  Split* split = at<Split>(scratch, L.split);
-  uint32_t* bins = at<uint32_t>(scratch, L.bins);
   uint32_t* arrive = at<uint32_t>(scratch, L.arrive);
   uint32_t* qidx = at<uint32_t>(scratch, L.qidx);
 
+  // the levels' second buffer and partition bits lie where the quad phase works later
+  LevelArgs A;
+  A.arena = arena;
+  A.large[0] = at<int32_t>(scratch, L.large0), A.large[1] = at<int32_t>(scratch, L.large1);
+  A.max_large = L.max_large;
+  A.small = at<int32_t>(scratch, L.small);
+  A.counters = counters;
+  A.cap = L.cap;
+  A.chunk = L.chunk, A.max_chunks = L.max_chunks;
+  A.chunks = at<Chunk>(scratch, L.chunks);
+  A.split = at<Split>(scratch, L.split);
+  A.bins = at<uint32_t>(scratch, L.bins);
+  A.chunk_left = at<uint32_t>(scratch, L.chunk_left);
+  A.left = arrive;
+  A.box = box;
+  A.buf[0] = tmp, A.buf[1] = qidx;
+  A.prims = prims;
+
   k_init<<<1, 32, 0, s>>>(counters);
-  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, prims, counters);
-  k_root<<<1, 1, 0, s>>>(arena, large[0], small, n, counters);
+  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > kWarpMax ? A.buf[0] : prims, counters);
+  k_root<<<1, 1, 0, s>>>(arena, A.large[0], A.small, n, counters);
   GB_TRY(cudaGetLastError());
   GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));
   GB_TRY(cudaStreamSynchronize(s));
-  uint32_t nl = host_counters[kLargeNext];
-  int cur = 0;
-  r.levels = 0;
+  uint64_t nl = host_counters[kLarge];
+  int par = 0;
+  // Up to four levels are issued before the counters are read back (12 us each time),
+  // while all their nodes could be large ones: a level that turns out empty costs
+  // five launches.
   while (nl > 0) {
     if (nl > L.max_large) return cudaErrorInvalidValue;
-    GB_TRY(cudaMemsetAsync(counters + kLargeNext, 0, 8, s));  // kLargeNext, kChunkCursor
-    k_chunks<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, chunks, split, bins, counters);
-    const unsigned nchunk = (unsigned)std::min<uint64_t>((uint64_t)n / L.chunk + nl + 1, L.max_chunks);
-    k_bin<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, counters, box, prims, bins);
-    k_split<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, bins, split, large[cur ^ 1], small,
-                                                          counters, L.cap);
-    k_part_count<<<nchunk, 256, 0, s>>>(chunks, split, counters, box, prims, chunk_left);
-    k_part_offsets<<<blocks((uint64_t)nl * 32, 256), 256, 0, s>>>(arena, large[cur], nl, L.chunk, split, chunk_left, chunk_loff,
-                                                                 counters);
-    k_part_scatter<<<nchunk, 256, 0, s>>>(arena, large[cur], chunks, split, counters, chunk_loff, box, prims, tmp);
-    k_part_copy<<<nchunk, 256, 0, s>>>(chunks, split, counters, tmp, prims);
+    int batch = 1;
+    while (batch < 4 && (nl << batch) * kWarpMax <= n) batch++;
+    for (int i = 0; i < batch; i++, par ^= 1) {
+      const uint64_t most = std::min<uint64_t>(nl << i, L.max_large);
+      const unsigned gn = blocks(most * 32, 256);
+      const unsigned gc = (unsigned)std::min<uint64_t>((uint64_t)n / L.chunk + most + 1, L.max_chunks);
+      k_chunks<<<gn, 256, 0, s>>>(A, par);
+      k_bin<<<gc, 256, 0, s>>>(A, par);
+      k_split<<<gn, 256, 0, s>>>(A, par);
+      k_part_count<<<gc, 256, 0, s>>>(A, par);
+      k_part_scatter<<<gc, 256, 0, s>>>(A, par);
+    }
     GB_TRY(cudaGetLastError());
     GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));
     GB_TRY(cudaStreamSynchronize(s));
-    nl = host_counters[kLargeNext];
-    cur ^= 1;
-    r.levels++;
+    nl = host_counters[kLarge + par];
     if (host_counters[kError]) break;
   }
   const uint32_t nsmall = host_counters[kSmallCount];
@@ -1067,8 +1095,8 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     const int sms = sm_count();
     const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sms * 8);
     GB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
-    // the partition's scratch (4 bytes per primitive) is free now: it takes the tasks
-    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, small, counters, box, prims, counters, L.cap, tmp);
+    // the levels' first buffer (4 bytes per primitive) is free now: it takes the tasks
+    k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, A.small, counters, box, prims, counters, L.cap, tmp);
     GB_TRY(cudaGetLastError());
     GB_TRY(cudaFuncSetAttribute(k_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
