@@ -730,6 +730,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(BNode* arena, const 
 // One warp per node spent its shuffles and 231 bin words on four primitives as
 // on 128: k_small took 2.69 ms of a 2.0 M-triangle build; with the leaves here it
 // takes 0.55 and this kernel 0.57 ms.
+// Few tasks are spread over all resident warps, a few lanes each: a warp is as slow
+// as its lanes' different paths added up (20,480 triangles: 158 us with 32 tasks to
+// a warp, 96 spread).
 constexpr int kLeafThreads = 64;
 // boxes, centroids or right areas, ids, nodes: a node of 4 or more splits, so 16
 // primitives make at most 13 splits and 27 nodes
@@ -761,8 +764,9 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaf(BNode* arena, const uint3
   uint32_t* node = id + 16 * T;  // node k (k-th made): b | n << 4 | left count << 9 | depth << 14
   const uint32_t ntask = counters[kTasks];
   const int lane = threadIdx.x & 31;
-  for (uint32_t t0 = blockIdx.x * T + (threadIdx.x & ~31u); t0 < ntask; t0 += gridDim.x * T) {
-    const bool in = t0 + lane < ntask;
+  const uint32_t warps = gridDim.x * (T / 32), lanes = min(32u, (ntask + warps - 1) / warps);
+  for (uint32_t t0 = (blockIdx.x * (T / 32) + (threadIdx.x >> 5)) * lanes; t0 < ntask; t0 += warps * lanes) {
+    const bool in = lane < (int)lanes && t0 + lane < ntask;
     const int32_t root = in ? (int32_t)tasks[t0 + lane] : 0;
     uint32_t first = 0, count = 0, splits = 0;
     int32_t depth0 = 0;
@@ -1101,7 +1105,7 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     GB_TRY(cudaFuncSetAttribute(k_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
     GB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_leaf, kLeafThreads, kLeafShared));
-    const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 4 + 1, kLeafThreads),
+    const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 4 + 1, kLeafThreads / 32),
                                                      (uint64_t)sms * std::max(1, per_sm));
     k_leaf<<<gl, kLeafThreads, kLeafShared, s>>>(arena, tmp, box, prims, counters, L.cap);
     GB_TRY(cudaGetLastError());

@@ -1022,6 +1022,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, uint32
 // nine in ten nodes are in such ranges: k_fsmall took 4.33 ms of a 2.0
 // M-triangle build by itself; with the leaves here it takes 0.51 and this kernel
 // 0.52 ms.
+// Few tasks are spread over all resident warps, a few lanes each: a warp is as slow
+// as its lanes' different paths added up (a 20,480-triangle build 1,034 us with 32
+// tasks to a warp, 991 spread).
 constexpr int kLeafThreads = 64;
 constexpr int kLeafWords = 16 * 6 + 16 * 3 + 16 + 16;  // boxes, centroids (then right areas), ids, nodes
 constexpr size_t kLeafShared = sizeof(float) * kLeafWords * kLeafThreads;
@@ -1039,8 +1042,9 @@ __global__ void __launch_bounds__(kLeafThreads) k_fleaf(LevelArgs A, const uint3
   uint32_t* node = id + 16 * T;                          // two nodes per word: b | count << 4 | depth << 9
   const uint32_t ntask = A.counters[kTasks];
   const int lane = threadIdx.x & 31;
-  for (uint32_t t0 = blockIdx.x * T + (threadIdx.x & ~31u); t0 < ntask; t0 += gridDim.x * T) {
-    const bool in = t0 + lane < ntask;
+  const uint32_t warps = gridDim.x * (T / 32), lanes = min(32u, (ntask + warps - 1) / warps);
+  for (uint32_t t0 = (blockIdx.x * (T / 32) + (threadIdx.x >> 5)) * lanes; t0 < ntask; t0 += warps * lanes) {
+    const bool in = lane < (int)lanes && t0 + lane < ntask;
     const int32_t root = in ? (int32_t)tasks[t0 + lane] : 0;
     uint32_t first = 0, count = 0;
     int32_t depth0 = 0;
@@ -1628,7 +1632,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     FB_TRY(cudaFuncSetAttribute(k_fleaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeafShared));
     int per_sm = 0;
     FB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fleaf, kLeafThreads, kLeafShared));
-    const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 2 + 1, kLeafThreads),
+    const unsigned gl = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 2 + 1, kLeafThreads / 32),
                                                      (uint64_t)sm_count() * std::max(1, per_sm));
     k_fleaf<<<gl, kLeafThreads, kLeafShared, s>>>(A, tmp);
     FB_TRY(cudaGetLastError());
