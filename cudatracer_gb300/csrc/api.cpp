@@ -50,7 +50,7 @@ namespace {
 // 4 M triangle tree alive, a 2 M triangle rebuild gave its scratch back at every
 // wait for its counters and took 6.23 instead of 5.47 ms.)
 constexpr uint64_t kPoolKeepBytes = (uint64_t)1 << 30;
-constexpr size_t kPinnedBytes = 64;
+constexpr size_t kPinnedBytes = 128;
 
 struct Allocs {
   std::vector<std::pair<void*, size_t>> list;

@@ -32,6 +32,7 @@
 
 #include "bvh_build.h"
 #include "ct_internal.h"
+#include "launch.cuh"
 
 namespace ct {
 namespace {
@@ -417,6 +418,7 @@ __device__ __forceinline__ uint32_t chunk_count(const LevelArgs& A, int par) {
 
 // One warp per node: its lanes write the chunks and the empty bins.
 __global__ void __launch_bounds__(256) k_chunks(LevelArgs A, int par) {
+  after_previous();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   // the next level's counters: its last reader was the level before this one
@@ -438,6 +440,7 @@ __global__ void __launch_bounds__(256) k_chunks(LevelArgs A, int par) {
 }
 
 __global__ void __launch_bounds__(256) k_bin(LevelArgs A, int par) {
+  after_previous();
   __shared__ float planes[3 * kPlanes];
   __shared__ uint32_t bins[kBinWords];
   if (blockIdx.x >= chunk_count(A, par)) return;
@@ -485,6 +488,7 @@ __device__ __forceinline__ bool classify(const LevelArgs& A, int par, int32_t id
 }
 
 __global__ void __launch_bounds__(256) k_split(LevelArgs A, int par) {
+  after_previous();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= large_count(A, par)) return;  // whole warp
@@ -527,6 +531,7 @@ __device__ __forceinline__ bool goes_left(const PrimBox* box, uint32_t p, int ax
 
 // Which side each primitive of a chunk goes to (a bit each), and how many go left.
 __global__ void __launch_bounds__(256) k_part_count(LevelArgs A, int par) {
+  after_previous();
   __shared__ uint32_t nleft;
   if (blockIdx.x >= chunk_count(A, par)) return;
   const Chunk ch = A.chunks[blockIdx.x];
@@ -553,6 +558,7 @@ __global__ void __launch_bounds__(256) k_part_count(LevelArgs A, int par) {
 // come from the same bins; the build fails).
 constexpr int kMaxWords = 2048 / 32;  // bit words of a chunk
 __global__ void __launch_bounds__(256) k_part_scatter(LevelArgs A, int par) {
+  after_previous();
   __shared__ uint32_t word[kMaxWords], before[kMaxWords], sum[2];
   if (blockIdx.x >= chunk_count(A, par)) return;
   const Chunk ch = A.chunks[blockIdx.x];
@@ -1082,11 +1088,11 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
       const uint64_t most = std::min<uint64_t>(nl << i, L.max_large);
       const unsigned gn = blocks(most * 32, 256);
       const unsigned gc = (unsigned)std::min<uint64_t>((uint64_t)n / L.chunk + most + 1, L.max_chunks);
-      k_chunks<<<gn, 256, 0, s>>>(A, par);
-      k_bin<<<gc, 256, 0, s>>>(A, par);
-      k_split<<<gn, 256, 0, s>>>(A, par);
-      k_part_count<<<gc, 256, 0, s>>>(A, par);
-      k_part_scatter<<<gc, 256, 0, s>>>(A, par);
+      GB_TRY(launch_after(k_chunks, gn, 256, 0, s, A, par));
+      GB_TRY(launch_after(k_bin, gc, 256, 0, s, A, par));
+      GB_TRY(launch_after(k_split, gn, 256, 0, s, A, par));
+      GB_TRY(launch_after(k_part_count, gc, 256, 0, s, A, par));
+      GB_TRY(launch_after(k_part_scatter, gc, 256, 0, s, A, par));
     }
     GB_TRY(cudaGetLastError());
     GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));

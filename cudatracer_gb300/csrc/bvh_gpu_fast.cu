@@ -38,6 +38,7 @@
 
 #include "bvh_build.h"
 #include "ct_internal.h"
+#include "launch.cuh"
 
 namespace ct {
 namespace {
@@ -72,12 +73,16 @@ enum Counter : int {
   kError = 4,
   kMaxLeaf = 5,
   kMag = 6,
-  kQNext = 7,
   kChunks = 2,       // 2 words: chunks of the even and of the odd level
   kTasks = kChunks,  // ranges for k_fleaf, once the levels are done
   kRootKeys = 8,     // 6 words: min x/y/z, max x/y/z
   kLarge = 14,       // 2 words: large nodes of the even and of the odd level
-  kCounterWords = 16
+  kCounterWords = 16,
+  // after these, for the quad phase: where each level's nodes begin and how many it has
+  kQuadLevels = 64,  // the binary depth limit of 60 bounds them
+  kQuadFirst = kCounterWords,
+  kQuadCount = kQuadFirst + kQuadLevels,
+  kAllWords = kQuadCount + kQuadLevels
 };
 
 struct __align__(16) FNodeD {
@@ -174,7 +179,7 @@ struct Layout {
     qrec = take(sizeof(QRec) * (size_t)qcap);
     scan = take(4 * (size_t)qcap);
     sums = take(4 * (size_t)max_sums);
-    counters = take(4 * kCounterWords);
+    counters = take(4 * kAllWords);
     total = o;
   }
 };
@@ -566,6 +571,7 @@ __device__ __forceinline__ uint32_t chunk_count(const LevelArgs& A, int par) {
 // One warp per node: its lanes write the chunks and the empty bins (one thread
 // took up to 31 us a level over the 336 bin words of its node).
 __global__ void __launch_bounds__(256) k_fchunks(LevelArgs A, int par) {
+  after_previous();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   // the next level's counters: its last reader was the level before this one
@@ -594,6 +600,7 @@ __global__ void __launch_bounds__(256) k_fchunks(LevelArgs A, int par) {
 }
 
 __global__ void __launch_bounds__(256) k_fbin(LevelArgs A, int par) {
+  after_previous();
   __shared__ uint32_t bins[kBinWords];
   if (blockIdx.x >= chunk_count(A, par)) return;
   const Chunk ch = A.chunks[blockIdx.x];
@@ -645,6 +652,7 @@ __device__ __forceinline__ void add_children(const LevelArgs& A, int par, int32_
 }
 
 __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, int par) {
+  after_previous();
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (s >= large_count(A, par)) return;  // whole warp
@@ -686,6 +694,7 @@ __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, int par) {
 // Which side each primitive of a chunk goes to (a bit each), how many go left, and
 // the centroid bounds of the children that are split on the next level.
 __global__ void __launch_bounds__(256) k_fpcount(LevelArgs A, int par) {
+  after_previous();
   __shared__ uint32_t red[2][6], nleft;
   if (blockIdx.x >= chunk_count(A, par)) return;
   const Chunk ch = A.chunks[blockIdx.x];
@@ -745,6 +754,7 @@ __global__ void __launch_bounds__(256) k_fpcount(LevelArgs A, int par) {
 // same bins), the range stays as it lies and the build fails.
 constexpr int kMaxWords = 2048 / 32;  // bit words of a chunk
 __global__ void __launch_bounds__(256) k_fpscatter(LevelArgs A, int par) {
+  after_previous();
   __shared__ uint32_t word[kMaxWords], before[kMaxWords], sum[2];
   if (blockIdx.x >= chunk_count(A, par)) return;
   const Chunk ch = A.chunks[blockIdx.x];
@@ -1299,11 +1309,16 @@ __global__ void __launch_bounds__(256) k_fcost8(const FNodeD* __restrict__ arena
 // ---------------------------------------------------------------- collapse
 __device__ __forceinline__ uint32_t split_of(uint32_t meta, int i) { return (meta >> (8 * (i - 1))) & 0xffu; }
 
-__global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* __restrict__ arena, const FCostD* __restrict__ cost,
-                                                 uint32_t* qlist, QRec* qrec, uint32_t b, uint32_t e,
-                                                 uint32_t next_base, uint32_t qcap, uint32_t* counters, float s) {
+// One level; its nodes follow the previous level's, and their number is read on the
+// device, so that several levels can be issued together.
+__global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCostD* cost, uint32_t* qlist, QRec* qrec,
+                                                 int level, uint32_t qcap, uint32_t* counters, float s) {
+  after_previous();
+  const uint32_t b = level ? counters[kQuadFirst + level] : 0u;
+  const uint32_t e = level ? b + counters[kQuadCount + level] : 1u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) counters[kQuadFirst + level + 1] = min(e, qcap);
   const uint32_t q = b + blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= e) return;
+  if (q >= min(e, qcap)) return;
   const int32_t bn = (int32_t)qlist[q];
   const FNodeD n = arena[bn];
   const int32_t L = n.left, R = L + 1;
@@ -1371,7 +1386,7 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* __restrict__ aren
       const uint32_t cnt = (uint32_t)arena[sl[j]].count;
       if (cnt > __ldcg(&counters[kMaxLeaf])) atomicMax(&counters[kMaxLeaf], cnt);  // few raise it
     } else {
-      const uint32_t at_ = next_base + atomicAdd(&counters[kQNext], 1u);
+      const uint32_t at_ = e + atomicAdd(&counters[kQuadCount + level + 1], 1u);
       if (at_ >= qcap) {
         atomicOr(&counters[kError], kErrQuad);
         continue;
@@ -1385,6 +1400,7 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* __restrict__ aren
 }
 
 __global__ void k_fqsize(QRec* qrec, uint32_t b, uint32_t e) {
+  after_previous();
   const uint32_t q = b + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= e) return;
   uint32_t sz = 1;
@@ -1394,6 +1410,7 @@ __global__ void k_fqsize(QRec* qrec, uint32_t b, uint32_t e) {
 }
 
 __global__ void k_fqrank(QRec* qrec, uint32_t b, uint32_t e) {
+  after_previous();
   const uint32_t q = b + blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= e) return;
   uint32_t r = qrec[q].rank + 1;
@@ -1608,11 +1625,11 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
       const uint64_t most = std::min<uint64_t>(nl << i, Lo.max_large);
       const unsigned gn = blocks(most * 32, 256);
       const unsigned gc = (unsigned)std::min<uint64_t>((uint64_t)n / Lo.chunk + most + 1, Lo.max_chunks);
-      k_fchunks<<<gn, 256, 0, s>>>(A, par);
-      k_fbin<<<gc, 256, 0, s>>>(A, par);
-      k_fsplit<<<gn, 256, 0, s>>>(A, par);
-      k_fpcount<<<gc, 256, 0, s>>>(A, par);
-      k_fpscatter<<<gc, 256, 0, s>>>(A, par);
+      FB_TRY(launch_after(k_fchunks, gn, 256, 0, s, A, par));
+      FB_TRY(launch_after(k_fbin, gc, 256, 0, s, A, par));
+      FB_TRY(launch_after(k_fsplit, gn, 256, 0, s, A, par));
+      FB_TRY(launch_after(k_fpcount, gc, 256, 0, s, A, par));
+      FB_TRY(launch_after(k_fpscatter, gc, 256, 0, s, A, par));
     }
     FB_TRY(cudaGetLastError());
     FB_TRY(read_counters(hc, counters, s));
@@ -1662,25 +1679,37 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   k_fcost<<<blocks(nb, 256), 256, 0, s>>>(arena, cost, arrive, counters, Lo.cap, ascale);
   // quad levels from the root (binary node 0)
   FB_TRY(cudaMemsetAsync(qlist, 0, 4, s));
+  FB_TRY(cudaMemsetAsync(counters + kCounterWords, 0, 4 * (kAllWords - kCounterWords), s));
   std::vector<uint32_t> off{0u, 1u};
+  // four levels per readback: their grids are bounds, a level has at most four times
+  // the nodes of the one before
   while (off.back() > off[off.size() - 2]) {
-    const uint32_t b = off[off.size() - 2], e = off.back();
-    FB_TRY(cudaMemsetAsync(counters + kQNext, 0, 4, s));
-    k_fqlevel<<<blocks(e - b, 256), 256, 0, s>>>(arena, cost, qlist, qrec, b, e, e, Lo.qcap, counters, ascale);
-    FB_TRY(cudaGetLastError());
+    const int l0 = (int)off.size() - 2, batch = std::min(4, kQuadLevels - 1 - l0);
+    if (batch <= 0) {
+      r.error = kErrQuad;
+      return cudaSuccess;
+    }
+    for (int i = 0; i < batch; i++) {
+      const uint64_t most = std::min<uint64_t>((uint64_t)(off[l0 + 1] - off[l0]) << (2 * i), n);
+      FB_TRY(launch_after(k_fqlevel, blocks(most, 256), 256, 0, s, arena, cost, qlist, qrec, l0 + i, Lo.qcap, counters,
+                          ascale));
+    }
+    FB_TRY(cudaMemcpyAsync(hc + kCounterWords, counters + kQuadCount + l0 + 1, 4 * (size_t)batch, cudaMemcpyDeviceToHost,
+                           s));
     FB_TRY(read_counters(hc, counters, s));
     if (hc[kError]) {
       r.error = hc[kError];
       return cudaSuccess;
     }
-    off.push_back(e + hc[kQNext]);
+    for (int i = 0; i < batch && off.back() > off[off.size() - 2]; i++)
+      off.push_back(off.back() + hc[kCounterWords + i]);
   }
   const uint32_t nq = off.back();
   const size_t nlev = off.size() - 2;  // levels with nodes
   for (size_t l = nlev; l-- > 0;)
-    k_fqsize<<<blocks(off[l + 1] - off[l], 256), 256, 0, s>>>(qrec, off[l], off[l + 1]);
+    FB_TRY(launch_after(k_fqsize, blocks(off[l + 1] - off[l], 256), 256, 0, s, qrec, off[l], off[l + 1]));
   for (size_t l = 0; l < nlev; l++)
-    k_fqrank<<<blocks(off[l + 1] - off[l], 256), 256, 0, s>>>(qrec, off[l], off[l + 1]);
+    FB_TRY(launch_after(k_fqrank, blocks(off[l + 1] - off[l], 256), 256, 0, s, qrec, off[l], off[l + 1]));
   k_fqscatter<<<blocks(nq, 256), 256, 0, s>>>(qrec, nq, scan);
   const uint32_t nsb = blocks(nq, kScanBlock);
   k_scan_blocks<<<nsb, kScanBlock, 0, s>>>(scan, nq, sums);
