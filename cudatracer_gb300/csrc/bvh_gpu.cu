@@ -1173,12 +1173,15 @@ cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& 
 // ================================================================ 8-wide quantised collapse
 namespace {
 
-enum WCounter : int { kWideCount = 0, kWidePrims = 1, kWideNext = 2, kWideError = 3, kWideCounterWords = 8 };
-enum : uint32_t { kWErrSlots = 1, kWErrCapacity = 2, kWErrQuant = 4 };
-
-struct WEntry {
-  uint32_t wide, bin;
+enum WCounter : int {
+  kWidePrims = 0,
+  kWideError = 1,
+  kWideLevel = 2,                         // the nodes of each level (from the second on)
+  kWideLevels = 64,
+  kWideFirst = kWideLevel + kWideLevels,  // and the first one's index
+  kWideCounterWords = kWideFirst + kWideLevels
 };
+enum : uint32_t { kWErrSlots = 1, kWErrCapacity = 2, kWErrQuant = 4 };
 
 struct WLayout {
   size_t nodes, list0, list1, counters, total;
@@ -1192,8 +1195,8 @@ struct WLayout {
       return a;
     };
     nodes = take(sizeof(WNode8) * (size_t)cap);
-    list0 = take(sizeof(WEntry) * (size_t)cap);
-    list1 = take(sizeof(WEntry) * (size_t)cap);
+    list0 = take(sizeof(uint32_t) * (size_t)cap);
+    list1 = take(sizeof(uint32_t) * (size_t)cap);
     counters = take(4 * kWideCounterWords);
     total = o;
   }
@@ -1227,26 +1230,14 @@ __device__ __forceinline__ bool quantise(float p, float s, float lo, float hi, u
 
 __device__ __forceinline__ uint32_t wsplit(const WideCost& c, int i) { return (c.split >> (3 * (i - 2))) & 7u; }
 
-__global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ arena, const uint32_t* __restrict__ bprims,
-                                                   const WideCost* __restrict__ cost, const float4* __restrict__ v,
-                                                   const uint4* __restrict__ idx, const WEntry* __restrict__ in,
-                                                   uint32_t n_in, WEntry* out, uint32_t* counters, WNode8* wn,
-                                                   float4* wtris, uint32_t cap, uint32_t n_prims) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_in) return;
-  const WEntry en = in[i];
-  const BNode b = arena[en.bin];
-  // frontier of binary nodes under this wide node, in left-to-right order;
-  // leafy[k]: entry k becomes leaf slots (its primitive range, three per slot)
-  int32_t F[8];
-  bool leafy[8];
+// The binary nodes that become the entries of wide node b (at most eight), left to
+// right; leafy[k]: entry k becomes leaf slots (its primitive range, three per slot).
+// Returns their number, -1 when they don't fit.
+__device__ __forceinline__ int wide_entries(const BNode* arena, const WideCost* cost, uint32_t bin, const BNode& b,
+                                            int32_t F[8], bool leafy[8]) {
   int nf = 0;
-  auto usage = [&](int32_t x, bool lf) {
-    const BNode& c = arena[x];
-    return lf ? leaf_slots(c.count) : 1u;
-  };
   if (b.left < 0) {
-    F[nf] = (int32_t)en.bin, leafy[nf++] = true;
+    F[nf] = (int32_t)bin, leafy[nf++] = true;
   } else {
     // the slots of least cost (the optimal n-wide collapse of Ylitie, Karras and
     // Laine, HPG 2017): k of 8 to the left child, then each side as its table says
@@ -1268,38 +1259,56 @@ __global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ are
       const BNode& c = arena[x];
       while (ix > 1 && (c.left < 0 || wsplit(cost[x], ix) == 0)) ix--;
       if (ix == 1) {
-        if (nf >= 8) {
-          atomicOr(&counters[kWideError], kWErrSlots);
-          return;
-        }
+        if (nf >= 8) return -1;
         F[nf] = x, leafy[nf++] = c.left < 0 || cost[x].leaf1 != 0;
         continue;
       }
       const int k = (int)wsplit(cost[x], ix);
-      if (sp + 2 > 16) {
-        atomicOr(&counters[kWideError], kWErrSlots);
-        return;
-      }
+      if (sp + 2 > 16) return -1;
       stn[sp] = c.left + 1, sti[sp++] = ix - k;
       stn[sp] = c.left, sti[sp++] = k;
     }
   }
   uint32_t used = 0;
-  for (int k = 0; k < nf; k++) used += usage(F[k], leafy[k]);
-  if (used > 8) {
-    atomicOr(&counters[kWideError], kWErrSlots);
-    return;
-  }
+  for (int k = 0; k < nf; k++) used += leafy[k] ? leaf_slots(arena[F[k]].count) : 1u;
+  return used > 8 ? -1 : nf;
+}
+
+// One level: its nodes follow the previous level's. Children and triangles are
+// placed for a warp's nodes at once (three atomics a node on shared counters: 536
+// against 500 us for the levels of a 1 M-triangle tree).
+__global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ arena, const uint32_t* __restrict__ bprims,
+                                                   const WideCost* __restrict__ cost, const float4* __restrict__ v,
+                                                   const uint4* __restrict__ idx, const uint32_t* in, int level,
+                                                   uint32_t* out, uint32_t* counters, WNode8* wn, float4* wtris,
+                                                   uint32_t cap, uint32_t n_prims) {
+  after_previous();
+  if (counters[kWideError]) return;  // an earlier level failed: its list has gaps
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t first = level ? counters[kWideFirst + level] : 0u, n_in = level ? counters[kWideLevel + level] : 1u;
+  if (i == 0) counters[kWideFirst + level + 1] = first + n_in;
+  if ((i & ~31u) >= n_in) return;  // whole warp
+  const bool live = i < n_in;
+  int32_t F[8];
+  bool leafy[8];
+  int nf = 0;
   uint32_t n_int = 0, n_tri = 0;
-  for (int k = 0; k < nf; k++) {
-    const BNode& c = arena[F[k]];
-    if (!leafy[k]) n_int++;
-    else n_tri += (uint32_t)c.count;
+  BNode b;
+  if (live) {
+    const uint32_t bin = level ? in[i] : 0u;
+    b = arena[bin];
+    nf = wide_entries(arena, cost, bin, b, F, leafy);
+    if (nf < 0) atomicOr(&counters[kWideError], kWErrSlots);
+    for (int k = 0; k < nf; k++) {
+      if (!leafy[k]) n_int++;
+      else n_tri += (uint32_t)arena[F[k]].count;
+    }
   }
-  const uint32_t child_base = n_int ? atomicAdd(&counters[kWideCount], n_int) : 0u;
-  const uint32_t prim_base = n_tri ? atomicAdd(&counters[kWidePrims], n_tri) : 0u;
-  const uint32_t out_base = n_int ? atomicAdd(&counters[kWideNext], n_int) : 0u;
-  if (child_base + n_int > cap || prim_base + n_tri > n_prims || out_base + n_int > cap) {
+  const uint32_t out_base = warp_alloc(&counters[kWideLevel + level + 1], n_int);
+  const uint32_t prim_base = warp_alloc(&counters[kWidePrims], n_tri);
+  const uint32_t child_base = first + n_in + out_base;
+  if (!live || nf < 0) return;
+  if (child_base + n_int > cap || prim_base + n_tri > n_prims) {
     atomicOr(&counters[kWideError], kWErrCapacity);
     return;
   }
@@ -1313,8 +1322,8 @@ __global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ are
     sc[a] = pow2(e);
   }
   w.px = p[0], w.py = p[1], w.pz = p[2];
-  w.child_base = child_base;
-  w.prim_base = prim_base;
+  w.child_base = n_int ? child_base : 0u;
+  w.prim_base = n_tri ? prim_base : 0u;
   bool ok = true;
   int slot = 0;
   uint32_t rank = 0, off = 0;
@@ -1324,7 +1333,7 @@ __global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ are
       for (int a = 0; a < 3; a++) ok &= quantise(p[a], sc[a], c.mn[a], c.mx[a], w.qlo[a][slot], w.qhi[a][slot]);
       w.meta[slot] = (uint8_t)(0x80u | rank);
       w.imask |= (uint8_t)(1u << slot);
-      out[out_base + rank] = WEntry{child_base + rank, (uint32_t)F[k]};
+      out[out_base + rank] = (uint32_t)F[k];
       rank++, slot++;
       continue;
     }
@@ -1350,7 +1359,7 @@ __global__ void __launch_bounds__(128) k_wcollapse(const BNode* __restrict__ are
     }
   }
   if (!ok) atomicOr(&counters[kWideError], kWErrQuant);
-  wn[en.wide] = w;
+  wn[first + i] = w;
 }
 
 }  // namespace
@@ -1365,27 +1374,31 @@ cudaError_t gpu_wbvh_collapse(const DevScene& sc, const void* arena_v, const uin
   // both binary builders write this 48-byte node layout (BNode here, FNodeD in bvh_gpu_fast.cu)
   const BNode* arena = static_cast<const BNode*>(arena_v);
   WNode8* wn = at<WNode8>(scratch2, W.nodes);
-  WEntry* lists[2] = {at<WEntry>(scratch2, W.list0), at<WEntry>(scratch2, W.list1)};
+  uint32_t* lists[2] = {at<uint32_t>(scratch2, W.list0), at<uint32_t>(scratch2, W.list1)};
   uint32_t* counters = at<uint32_t>(scratch2, W.counters);
-  const uint32_t init[kWideCounterWords] = {1, 0, 0, 0, 0, 0, 0, 0};
-  const WEntry root{0, 0};
-  GB_TRY(cudaMemcpyAsync(counters, init, sizeof(init), cudaMemcpyHostToDevice, s));
-  GB_TRY(cudaMemcpyAsync(lists[0], &root, sizeof(root), cudaMemcpyHostToDevice, s));
-  uint32_t n_in = 1, levels = 0;
-  int cur = 0;
+  GB_TRY(cudaMemsetAsync(counters, 0, 4 * kWideCounterWords, s));
+  // four levels per readback, as the quad tree's (a node has at most eight children)
+  uint32_t n_in = 1, levels = 0, nodes = 0;
   while (n_in > 0) {
-    GB_TRY(cudaMemsetAsync(counters + kWideNext, 0, 4, s));
-    k_wcollapse<<<blocks(n_in, 128), 128, 0, s>>>(arena, bprims, cost, sc.verts, sc.idx, lists[cur], n_in,
-                                                  lists[cur ^ 1], counters, wn, tris, W.cap, n);
-    GB_TRY(cudaGetLastError());
-    GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kWideCounterWords, cudaMemcpyDeviceToHost, s));
+    const int batch = std::min(4, kWideLevels - 1 - (int)levels);
+    if (batch <= 0) {
+      *error = kWErrCapacity;
+      return cudaSuccess;
+    }
+    for (int i = 0; i < batch; i++) {
+      const int l = (int)levels + i;
+      const uint64_t most = std::min<uint64_t>((uint64_t)n_in << (3 * i), W.cap);
+      GB_TRY(launch_after(k_wcollapse, blocks(most, 128), 128, 0, s, arena, bprims, cost, sc.verts, sc.idx, lists[l & 1], l,
+                          lists[(l + 1) & 1], counters, wn, tris, W.cap, n));
+    }
+    GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kWideLevel, cudaMemcpyDeviceToHost, s));
+    GB_TRY(cudaMemcpyAsync(host_counters + kWideLevel, counters + kWideLevel + levels + 1, 4 * (size_t)batch,
+                           cudaMemcpyDeviceToHost, s));
     GB_TRY(cudaStreamSynchronize(s));
-    levels++;
+    for (int i = 0; i < batch && n_in > 0; i++) nodes += n_in, n_in = host_counters[kWideLevel + i], levels++;
     if (host_counters[kWideError]) break;
-    n_in = host_counters[kWideNext];
-    cur ^= 1;
   }
-  *wide_nodes = host_counters[kWideCount];
+  *wide_nodes = nodes;
   *depth = levels;
   *error = host_counters[kWideError] | (host_counters[kWidePrims] != n ? kWErrCapacity : 0u);
   return cudaSuccess;

@@ -1309,32 +1309,18 @@ __global__ void __launch_bounds__(256) k_fcost8(const FNodeD* __restrict__ arena
 // ---------------------------------------------------------------- collapse
 __device__ __forceinline__ uint32_t split_of(uint32_t meta, int i) { return (meta >> (8 * (i - 1))) & 0xffu; }
 
-// One level; its nodes follow the previous level's, and their number is read on the
-// device, so that several levels can be issued together.
-__global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCostD* cost, uint32_t* qlist, QRec* qrec,
-                                                 int level, uint32_t qcap, uint32_t* counters, float s) {
-  after_previous();
-  const uint32_t b = level ? counters[kQuadFirst + level] : 0u;
-  const uint32_t e = level ? b + counters[kQuadCount + level] : 1u;
-  if (blockIdx.x == 0 && threadIdx.x == 0) counters[kQuadFirst + level + 1] = min(e, qcap);
-  const uint32_t q = b + blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= min(e, qcap)) return;
-  const int32_t bn = (int32_t)qlist[q];
-  const FNodeD n = arena[bn];
+// emit (bvh_fast.cpp): the slots of quad node n, depth first, then largest box first
+// (stable). Returns their number, -1 when the table is not consistent.
+__device__ __forceinline__ int quad_slots(const FNodeD* arena, const FCostD* cost, const FNodeD& n, float s,
+                                          int32_t sl[4], bool lf[4]) {
   const int32_t L = n.left, R = L + 1;
-  if (L < 0) {  // a quad node is an inner binary node (cannot happen for a consistent table)
-    atomicOr(&counters[kError], kErrQuad);
-    return;
-  }
+  if (L < 0) return -1;  // a quad node is an inner binary node
   float best = 3e38f;
   int bk = 1;
   for (int k = 1; k < 4; k++) {
     const float v = __fadd_rn(cost[L].c[k - 1], cost[R].c[4 - k - 1]);
     if (v < best) best = v, bk = k;
   }
-  // emit (bvh_fast.cpp): the slots of a subtree given i of them, depth first
-  int32_t sl[4];
-  bool lf[4];
   int ns = 0;
   int32_t stn[8];
   int sti[8];
@@ -1352,14 +1338,10 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCos
     }
     const int k = (int)split_of(meta, i);
     const int32_t xl = arena[x].left;
-    if (sp + 2 > 8 || xl < 0) {  // cannot happen for a consistent table
-      atomicOr(&counters[kError], kErrQuad);
-      return;
-    }
+    if (sp + 2 > 8 || xl < 0) return -1;
     stn[sp] = xl + 1, sti[sp++] = i - k;
     stn[sp] = xl, sti[sp++] = k;
   }
-  // largest box first, stable
   float ar[4];
   for (int j = 0; j < ns; j++) ar[j] = farea(arena[sl[j]].mn, arena[sl[j]].mx, s);
   for (int j = 1; j < ns; j++) {
@@ -1370,6 +1352,30 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCos
     while (k > 0 && ar[k - 1] < a) ar[k] = ar[k - 1], sl[k] = sl[k - 1], lf[k] = lf[k - 1], k--;
     ar[k] = a, sl[k] = x, lf[k] = f;
   }
+  return ns;
+}
+
+// One level; its nodes follow the previous level's, and their number is read on the
+// device, so that several levels can be issued together.
+__global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCostD* cost, uint32_t* qlist, QRec* qrec,
+                                                 int level, uint32_t qcap, uint32_t* counters, float s) {
+  after_previous();
+  const uint32_t b = level ? counters[kQuadFirst + level] : 0u;
+  const uint32_t e = level ? b + counters[kQuadCount + level] : 1u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) counters[kQuadFirst + level + 1] = min(e, qcap);
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, n = min(e, qcap) - b;
+  if ((i & ~31u) >= n) return;  // whole warp
+  int32_t sl[4];
+  bool lf[4];
+  int ns = 0;
+  uint32_t inner = 0;
+  if (i < n) {
+    ns = quad_slots(arena, cost, arena[qlist[b + i]], s, sl, lf);
+    if (ns < 0) atomicOr(&counters[kError], kErrQuad);
+    for (int j = 0; j < ns; j++) inner += !lf[j];
+  }
+  uint32_t at_ = e + warp_alloc(&counters[kQuadCount + level + 1], inner);
+  if (i >= n || ns < 0) return;
   QRec r;
   r.leafmask = 0;
   r.nk = 0;
@@ -1385,18 +1391,15 @@ __global__ void __launch_bounds__(256) k_fqlevel(const FNodeD* arena, const FCos
       r.leafmask |= 1u << j;
       const uint32_t cnt = (uint32_t)arena[sl[j]].count;
       if (cnt > __ldcg(&counters[kMaxLeaf])) atomicMax(&counters[kMaxLeaf], cnt);  // few raise it
+    } else if (at_ >= qcap) {
+      atomicOr(&counters[kError], kErrQuad);
     } else {
-      const uint32_t at_ = e + atomicAdd(&counters[kQuadCount + level + 1], 1u);
-      if (at_ >= qcap) {
-        atomicOr(&counters[kError], kErrQuad);
-        continue;
-      }
       qlist[at_] = (uint32_t)sl[j];
-      r.kid[j] = (int32_t)at_;
+      r.kid[j] = (int32_t)at_++;
       r.nk++;
     }
   }
-  qrec[q] = r;
+  qrec[b + i] = r;
 }
 
 __global__ void k_fqsize(QRec* qrec, uint32_t b, uint32_t e) {

@@ -1,4 +1,5 @@
-// Launches whose set-up overlaps the kernel before them on the stream.
+// Launches whose set-up overlaps the kernel before them on the stream, and warps
+// that take places from a counter together.
 //
 // A tree build is a chain of small kernels: for 20,480 triangles five kernels of 4
 // to 9 us a level, and as much again of their time between them. A kernel launched
@@ -33,6 +34,21 @@ inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned bl
   c.attrs = a;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+// Places for a warp's threads that want `want` units each from a counter, with one
+// atomic for the warp.
+__device__ __forceinline__ uint32_t warp_alloc(uint32_t* counter, uint32_t want) {
+  const int lane = threadIdx.x & 31;
+  uint32_t inc = want;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += y;
+  }
+  uint32_t base = 0;
+  if (lane == 31 && inc) base = atomicAdd(counter, inc);
+  return __shfl_sync(0xffffffffu, base, 31) + inc - want;
 }
 
 }  // namespace ct
