@@ -15,6 +15,7 @@
 #pragma once
 
 #include "bsdf_full.cuh"
+#include "launch.cuh"
 #include "ct_internal.h"
 #include "portable_math.h"
 #include "trace.cuh"
@@ -477,6 +478,7 @@ __device__ __forceinline__ int warp_append(bool want, int* counter) {
 
 __global__ void __launch_bounds__(kBlock) k_shade(DevScene sc, DevQueues q, FrameConst f, int cur,
                                                    uint32_t path_length) {
+  wait_previous();
   const int n = q.counts[cur];
   const int nxt = cur ^ 1;
   if (blockIdx.x == 0 && threadIdx.x == 0) q.counts[4] = 0;  // fetch cursor of the next extend
@@ -549,6 +551,7 @@ __device__ __forceinline__ void primary_ray(const FrameConst& f, int i, float4& 
 }
 
 __global__ void __launch_bounds__(kBlock) k_raygen(DevQueues q, FrameConst f) {
+  wait_previous();
   const int npix = f.width * f.height;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     q.counts[0] = npix;
@@ -667,6 +670,7 @@ __global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, 
 
 // Primary rays of the jobs that still take samples, appended to queue 0.
 __global__ void __launch_bounds__(kBlock) k_batch_raygen(DevBatch bt, DevQueues q) {
+  wait_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) q.counts[4] = 0;
   for (int base = blockIdx.x * kBlock + (threadIdx.x & ~31); base < bt.total_pix; base += gridDim.x * kBlock) {
     const int g = base + (threadIdx.x & 31);
@@ -694,6 +698,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_raygen(DevBatch bt, DevQueues 
 // job's paths stop after its own max_depth passes.
 __global__ void __launch_bounds__(kBlock) k_batch_shade(DevBatch bt, DevQueues q, int cur, uint32_t path_length,
                                                         int pass) {
+  wait_previous();
   const int n = q.counts[cur];
   const int nxt = cur ^ 1;
   if (blockIdx.x == 0 && threadIdx.x == 0) q.counts[4] = 0;
@@ -733,6 +738,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_shade(DevBatch bt, DevQueues q
 // seed by 2 (launchKernels' samples += 2) and counts the sample; queue 0 is
 // emptied for the next raygen.
 __global__ void k_batch_advance(DevBatch bt, DevQueues q) {
+  wait_previous();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j == 0) {
     q.counts[0] = 0;

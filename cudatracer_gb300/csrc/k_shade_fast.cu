@@ -84,12 +84,8 @@ cudaError_t launch_fold(float4* accum, float4* frame, int n, cudaStream_t s) {
 
 cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact_math, cudaStream_t s) {
   const int npix = f.width * f.height;
-  if (exact_math) {
-    exact::k_raygen<<<fill_grid(exact::k_raygen, npix), kBlock, 0, s>>>(q, f);
-  } else {
-    fast::k_raygen<<<fill_grid(fast::k_raygen, npix), kBlock, 0, s>>>(q, f);
-  }
-  return cudaGetLastError();
+  auto kernel = exact_math ? exact::k_raygen : fast::k_raygen;
+  return launch_after(kernel, fill_grid(kernel, npix), kBlock, 0, s, q, f);
 }
 
 cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
@@ -103,12 +99,8 @@ cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q,
 
 cudaError_t launch_shade(const DevScene& sc, const DevQueues& q, const FrameConst& f, int queue, int path_length,
                          int exact_math, cudaStream_t s) {
-  if (exact_math) {
-    exact::k_shade<<<fill_grid(exact::k_shade, q.capacity), kBlock, 0, s>>>(sc, q, f, queue, (uint32_t)path_length);
-  } else {
-    fast::k_shade<<<fill_grid(fast::k_shade, q.capacity), kBlock, 0, s>>>(sc, q, f, queue, (uint32_t)path_length);
-  }
-  return cudaGetLastError();
+  auto kernel = exact_math ? exact::k_shade : fast::k_shade;
+  return launch_after(kernel, fill_grid(kernel, q.capacity), kBlock, 0, s, sc, q, f, queue, (uint32_t)path_length);
 }
 
 cudaError_t launch_present(const float4* accum, float4* out, int n, float samples, cudaStream_t s) {
@@ -120,11 +112,8 @@ cudaError_t launch_present(const float4* accum, float4* out, int n, float sample
 
 
 cudaError_t launch_batch_raygen(const DevBatch& b, const DevQueues& q, int exact, cudaStream_t s) {
-  if (exact)
-    exact::k_batch_raygen<<<fill_grid(exact::k_batch_raygen, b.total_pix), kBlock, 0, s>>>(b, q);
-  else
-    fast::k_batch_raygen<<<fill_grid(fast::k_batch_raygen, b.total_pix), kBlock, 0, s>>>(b, q);
-  return cudaGetLastError();
+  auto kernel = exact ? exact::k_batch_raygen : fast::k_batch_raygen;
+  return launch_after(kernel, fill_grid(kernel, b.total_pix), kBlock, 0, s, b, q);
 }
 
 cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue, uint32_t path_length, int pass,
@@ -135,12 +124,10 @@ cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue,
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBlock, 0);
   const int cap_blocks = (q.capacity + kBlock - 1) / kBlock;
   const int grid = std::max(1, std::min(cap_blocks, std::max(1, per_sm) * sm_count() * std::max(1, grid_mult)));
-  k<<<grid, kBlock, 0, s>>>(b, q, queue, path_length, pass);
-  return cudaGetLastError();
+  return launch_after(k, grid, kBlock, 0, s, b, q, queue, path_length, pass);
 }
 
 cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s) {
-  fast::k_batch_advance<<<(b.n_jobs + 127) / 128, 128, 0, s>>>(b, q);
-  return cudaGetLastError();
+  return launch_after(fast::k_batch_advance, (b.n_jobs + 127) / 128, 128, 0, s, b, q);
 }
 }  // namespace ct

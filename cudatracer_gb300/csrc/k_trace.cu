@@ -9,6 +9,7 @@
 // Queue-driven stages read their active count on the device: no host round
 // trip between stages. The traversal stack lives in dynamic shared memory laid
 // out [entry][thread], so a warp's pushes and pops hit 32 distinct banks.
+#include "launch.cuh"
 #include "trace.cuh"
 
 namespace ct {
@@ -85,13 +86,13 @@ struct ExtendIO {
   uint32_t* err;
   const int32_t* __restrict__ perm;
   __device__ void load(int i, float4& o, float4& d, float& t0) {
-    if (perm) i = __ldg(perm + i);
-    o = __ldg(org + i);
-    d = __ldg(dir + i);
+    if (perm) i = perm[i];
+    o = org[i];
+    d = dir[i];
     t0 = kMaxDistance;
   }
   __device__ void store(int i, const RayState& r, bool overflow) {
-    if (perm) i = __ldg(perm + i);
+    if (perm) i = perm[i];
     if (overflow) {
       atomicOr(err, kErrStackOverflow);
       hit[i] = make_int2(-1, __float_as_int(kMaxDistance));
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(kBlock) k_query(DevBVH b, QueryIO io, int n, i
 
 template <bool FASTMM>
 __global__ void __launch_bounds__(kBlock) k_extend(DevBVH b, DevQueues q, int qi, float eps) {
+  wait_previous();
   extern __shared__ int s_stack[];
   const int n = q.counts[qi];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -126,12 +128,13 @@ __global__ void __launch_bounds__(kBlock) k_extend(DevBVH b, DevQueues q, int qi
 // contribution to their pixel (one shadow ray per pixel per pass: no race)
 template <bool FASTMM>
 __global__ void __launch_bounds__(kBlock) k_connect(DevBVH b, DevQueues q, float eps) {
+  wait_previous();
   extern __shared__ int s_stack[];
   int* stack = s_stack + threadIdx.x;
   const int n = q.counts[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&q.stats[1], (unsigned long long)n);
   for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-    const float4 o = __ldg(q.sorg + i), d = __ldg(q.sdir + i);
+    const float4 o = q.sorg[i], d = q.sdir[i];
     RayState r;
     ray_begin(b, r, o, d, d.w);
     if (!traverse<true, FASTMM>(b, r, eps, stack, kBlock)) {
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(kBlock) k_connect(DevBVH b, DevQueues q, float
       continue;
     }
     if (r.hit < 0) {
-      const float4 c = __ldg(q.scol + i);
+      const float4 c = q.scol[i];
       const int pix = __float_as_int(o.w);
       if (q.log) {  // an exact frame in a slot: this launch's log entry (DevQueues::log)
         q.log[(size_t)q.log_entry * q.capacity + pix] = make_float4(c.x, c.y, c.z, __uint_as_float(q.log_tag));
@@ -188,8 +191,7 @@ cudaError_t launch_extend(const DevBVH& b, const DevQueues& q, int queue, float 
   if (e != cudaSuccess) return e;
   const int cap_blocks = (q.capacity + kBlock - 1) / kBlock;
   const int grid = std::max(1, std::min(cap_blocks, resident_grid(kernel, smem)));
-  kernel<<<grid, kBlock, smem, s>>>(b, q, queue, eps);
-  return cudaGetLastError();
+  return launch_after(kernel, grid, kBlock, smem, s, b, q, queue, eps);
 }
 
 cudaError_t launch_connect(const DevBVH& b, const DevQueues& q, float eps, bool fast, cudaStream_t s) {
@@ -199,8 +201,7 @@ cudaError_t launch_connect(const DevBVH& b, const DevQueues& q, float eps, bool 
   if (e != cudaSuccess) return e;
   const int cap_blocks = (q.capacity + kBlock - 1) / kBlock;
   const int grid = std::max(1, std::min(cap_blocks, resident_grid(kernel, smem)));
-  kernel<<<grid, kBlock, smem, s>>>(b, q, eps);
-  return cudaGetLastError();
+  return launch_after(kernel, grid, kBlock, smem, s, b, q, eps);
 }
 
 
@@ -315,16 +316,16 @@ struct BatchExtendIO {
   int n_jobs;
   const int32_t* __restrict__ perm;
   __device__ void load(int i, float4& o, float4& d, float& t0, DevBVH& b, float& eps) {
-    if (perm) i = __ldg(perm + i);
-    o = __ldg(org + i);
-    d = __ldg(dir + i);
+    if (perm) i = perm[i];
+    o = org[i];
+    d = dir[i];
     t0 = kMaxDistance;
     const BatchJob& J = jobs[batch_job_of(bases, n_jobs, __float_as_int(o.w))];
     b = J.bvh;
     eps = J.f.tri_eps;
   }
   __device__ void store(int i, const RayState& r, bool overflow) {
-    if (perm) i = __ldg(perm + i);
+    if (perm) i = perm[i];
     if (overflow) {
       atomicOr(err, kErrStackOverflow);
       hit[i] = make_int2(-1, __float_as_int(kMaxDistance));
@@ -336,6 +337,7 @@ struct BatchExtendIO {
 
 template <bool FASTMM, int BLOCK, int REFILL>
 __global__ void __launch_bounds__(BLOCK) k_batch_extend(DevBatch bt, DevQueues q, int qi) {
+  wait_previous();
   extern __shared__ int s_stack[];
   const int n = q.counts[qi];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -349,12 +351,13 @@ __global__ void __launch_bounds__(BLOCK) k_batch_extend(DevBatch bt, DevQueues q
 
 template <bool FASTMM, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_batch_connect(DevBatch bt, DevQueues q) {
+  wait_previous();
   extern __shared__ int s_stack[];
   int* stack = s_stack + threadIdx.x;
   const int n = q.counts[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&q.stats[1], (unsigned long long)n);
   for (int i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
-    const float4 o = __ldg(q.sorg + i), d = __ldg(q.sdir + i);
+    const float4 o = q.sorg[i], d = q.sdir[i];
     const int pix = __float_as_int(o.w);
     const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, pix)];
     const DevBVH b = J.bvh;
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(BLOCK) k_batch_connect(DevBatch bt, DevQueues 
       continue;
     }
     if (r.hit < 0) {
-      const float4 c = __ldg(q.scol + i);
+      const float4 c = q.scol[i];
       float4* acc = J.accum + (pix - J.pix_base);
       float4 a = *acc;
       a.x = __fadd_rn(a.x, c.x);
@@ -389,8 +392,7 @@ cudaError_t batch_extend(const DevBatch& b, const DevQueues& q, int queue, cudaS
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem);
   const int cap_blocks = (q.capacity + BLOCK - 1) / BLOCK;
   const int grid = std::max(1, std::min(cap_blocks, std::max(1, per_sm) * sm_count()));
-  kernel<<<grid, BLOCK, smem, s>>>(b, q, queue);
-  return cudaGetLastError();
+  return launch_after(kernel, grid, BLOCK, smem, s, b, q, queue);
 }
 
 template <bool FASTMM, int BLOCK>
@@ -405,8 +407,7 @@ cudaError_t batch_connect(const DevBatch& b, const DevQueues& q, cudaStream_t s)
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem);
   const int cap_blocks = (q.capacity + BLOCK - 1) / BLOCK;
   const int grid = std::max(1, std::min(cap_blocks, std::max(1, per_sm) * sm_count()));
-  kernel<<<grid, BLOCK, smem, s>>>(b, q);
-  return cudaGetLastError();
+  return launch_after(kernel, grid, BLOCK, smem, s, b, q);
 }
 
 }  // namespace

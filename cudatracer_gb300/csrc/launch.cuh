@@ -1,22 +1,29 @@
 // Launches whose set-up overlaps the kernel before them on the stream, and warps
 // that take places from a counter together.
 //
-// A tree build is a chain of small kernels: for 20,480 triangles five kernels of 4
-// to 9 us a level, and as much again of their time between them. A kernel launched
-// with launch_after may be set up, and its blocks placed, while the kernel before it
-// still runs; it begins with after_previous(), which waits until that kernel has
-// completed and its writes are visible, and then lets the next one be set up.
-// Every block of such a kernel calls it first, before any return, and the kernel
-// reads nothing through the non-coherent path (const __restrict__) that an earlier
-// kernel of the chain writes. With plain launches a 20,480-triangle reference-rule
-// build (9 levels) took 642 us, so 542.
+// A tree build is a chain of small kernels, 4 to 9 us each, and as much again of
+// their time lies between them; a frame's stages are such a chain too. A kernel
+// launched with launch_after may be set up while the kernel before it still runs; it
+// begins with wait_previous(), which returns when that kernel has completed and its
+// writes are visible. Every block of such a kernel calls it first, before any return,
+// and the kernel reads nothing through the non-coherent path (__ldg, const
+// __restrict__) that an earlier kernel of the chain writes.
+//
+// after_previous() also lets the blocks of the next kernel be placed right away, to
+// wait there: for the builds' kernels, which don't fill the chip (a 20,480-triangle
+// reference-rule build of 9 levels 642 -> 542 us). The stages fill it, and blocks
+// that wait would hold the places of the other frames in flight: four frames of
+// 641x360 948 us with plain launches, 826 with wait_previous(), 1,072 with
+// after_previous().
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace ct {
 
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_previous();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
