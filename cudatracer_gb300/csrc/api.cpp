@@ -1323,11 +1323,11 @@ static ct_status ensure_logs(ct_ctx* ctx, ct_render* r, int max_depth, bool* ok)
 }
 
 // Frames of at most this many pixels run as one kernel (launch_path) unless their
-// stages are profiled. Sixteen frames in a row on a 571,000-triangle terrain, depth
-// 8, one kernel against the stages: 256x192 0.79 and 2.31 ms (on 256,000
-// triangles), 362x362 2.79 and 3.44 ms, 400x400 3.37 and 3.27 ms, 512x384 3.97 and
-// 3.73 ms: beyond about 160,000 pixels the stages' compaction and refills pay (a
-// frame waited for alone is faster in one kernel up to 640x360).
+// stages are profiled. Sixteen frames in a row on a 256,000-triangle terrain, depth 8,
+// one kernel against the stages: 256x192 0.80 and 1.46 ms, 320x240 1.21 and 1.64,
+// 362x362 2.07 and 2.00, 512x384 2.93 and 2.49: beyond about 130,000 pixels the
+// stages' compaction and refills pay (a frame waited for alone is faster in one
+// kernel up to 640x480: 0.48 against 0.93 ms).
 constexpr int kPathPixels = 131072;
 
 // Issue one frame's stages on stream st into queues q.
