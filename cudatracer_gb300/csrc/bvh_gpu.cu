@@ -42,6 +42,9 @@ constexpr int kIntervals = kPlanes + 1;
 constexpr int kBinFields = 7;  // count, min key x/y/z, max key x/y/z
 constexpr int kBinWords = 3 * kIntervals * kBinFields;
 constexpr uint32_t kWarpMax = 128;  // nodes up to this size are built by one warp
+// Nodes up to this size are split by one block down to those (64 KB of shared memory
+// leave three blocks of 2,048 on an SM and six of 1,024).
+inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
 constexpr uint32_t kLeafTask = 16;  // subtrees up to this size are built by one thread
 // Primitives per block of the level kernels: the fewest, as a power of two from
 // 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
@@ -66,6 +69,7 @@ enum Counter : int {
   kError = 4,
   kMaxLeaf = 5,
   kQuadDepth = 6,
+  kMid = 7,          // nodes for k_mid
   kRootKeys = 8,     // 6 words: min x/y/z, max x/y/z
   kLarge = 14,       // 2 words: large nodes of the even and of the odd level
   kCounterWords = 16
@@ -110,12 +114,14 @@ struct Split {
 
 // Carving of the scratch block for n primitives.
 struct Layout {
-  size_t box, prims, tmp, arena, arrive, qidx, large0, large1, small, chunks, chunk_left, split, bins,
+  size_t box, prims, tmp, arena, arrive, qidx, large0, large1, mid, small, chunks, chunk_left, split, bins,
       counters, total;
-  uint32_t chunk, cap, max_large, max_chunks, max_small;
+  uint32_t chunk, cap, mid_most, max_large, max_mid, max_chunks, max_small;
   explicit Layout(uint32_t n) {
     cap = 2 * n + 2;
-    max_large = n / (kWarpMax + 1) + 2;
+    mid_most = mid_size(n);
+    max_large = n / (mid_most + 1) + 2;
+    max_mid = n / (kWarpMax + 1) + 2;
     chunk = chunk_size(n);
     max_chunks = n / chunk + max_large + 2;
     max_small = n / 4 + 2;
@@ -133,6 +139,7 @@ struct Layout {
     qidx = take(4 * (size_t)cap);
     large0 = take(4 * (size_t)max_large);
     large1 = take(4 * (size_t)max_large);
+    mid = take(4 * (size_t)max_mid);
     small = take(4 * (size_t)max_small);
     chunks = take(sizeof(Chunk) * (size_t)max_chunks);
     chunk_left = take(4 * (size_t)max_chunks);
@@ -370,15 +377,19 @@ __global__ void __launch_bounds__(256) k_prep(const float4* __restrict__ v, cons
   block_root_keys(counters, kmn, kmx);
 }
 
-__global__ void k_root(BNode* arena, int32_t* large, int32_t* small, uint32_t n, uint32_t* counters) {
+__global__ void k_root(BNode* arena, int32_t* large, int32_t* mid, int32_t* small, uint32_t n, uint32_t mid_most,
+                       uint32_t* counters) {
   float mn[3], mx[3];
   for (int k = 0; k < 3; k++) mn[k] = unkey(counters[kRootKeys + k]), mx[k] = unkey(counters[kRootKeys + 3 + k]);
   arena[0] = make_node(mn, mx, 0, n, -1, 0);
   counters[kArenaCount] = 1;
   if (n >= 4) {
-    if (n > kWarpMax) {
+    if (n > mid_most) {
       large[0] = 0;
       counters[kLarge] = 1;
+    } else if (n > kWarpMax) {
+      mid[0] = 0;
+      counters[kMid] = 1;
     } else {
       small[0] = 0;
       counters[kSmallCount] = 1;
@@ -396,6 +407,8 @@ struct LevelArgs {
   BNode* arena;
   int32_t* large[2];
   uint32_t max_large;
+  int32_t* mid;
+  uint32_t max_mid, mid_most;
   int32_t* small;
   uint32_t* counters;
   uint32_t cap;
@@ -475,16 +488,26 @@ __global__ void __launch_bounds__(256) k_bin(LevelArgs A, int par) {
   }
 }
 
-// Place a new child: leaf, a node for the next level (true), or a warp-built subtree root.
-__device__ __forceinline__ bool classify(const LevelArgs& A, int par, int32_t id, uint32_t count, int32_t depth) {
-  if (count < 4 || depth > kMaxSplitDepth) return false;
+// Queue of a child that a block or a warp splits further.
+__device__ __forceinline__ void queue_child(const LevelArgs& A, int32_t id, uint32_t count, int32_t depth) {
+  if (count < 4 || depth > kMaxSplitDepth) return;  // a leaf
   if (count > kWarpMax) {
-    const uint32_t s = atomicAdd(&A.counters[kLarge + (par ^ 1)], 1u);
-    if (s < A.max_large) A.large[par ^ 1][s] = id;
-    return s < A.max_large;
+    const uint32_t s = atomicAdd(&A.counters[kMid], 1u);
+    if (s < A.max_mid) A.mid[s] = id;  // always: the ranges are disjoint
+    return;
   }
   A.small[atomicAdd(&A.counters[kSmallCount], 1u)] = id;
-  return false;
+}
+
+// Place a new child: on the next level (true), or with queue_child.
+__device__ __forceinline__ bool classify(const LevelArgs& A, int par, int32_t id, uint32_t count, int32_t depth) {
+  if (count <= A.mid_most || depth > kMaxSplitDepth) {
+    queue_child(A, id, count, depth);
+    return false;
+  }
+  const uint32_t s = atomicAdd(&A.counters[kLarge + (par ^ 1)], 1u);
+  if (s < A.max_large) A.large[par ^ 1][s] = id;
+  return s < A.max_large;
 }
 
 __global__ void __launch_bounds__(256) k_split(LevelArgs A, int par) {
@@ -613,6 +636,179 @@ __global__ void __launch_bounds__(256) k_part_scatter(LevelArgs A, int par) {
     const uint32_t b = word[w], l = before[w] + __popc(b & lt), p = from[ch.begin + 32 * w + lane];
     if ((b >> lane) & 1u) to_l[dl + l] = p;
     else to_r[dr + 32 * w + lane - l] = p;
+  }
+}
+
+// ---------------------------------------------------------------- nodes of at most mid_size(n), one block each
+// A block splits such a node, and its children of more than kWarpMax primitives, with
+// everything in shared memory: boxes and ids by the slot they arrived in, and the
+// slots in their present order, in two arrays that a partition goes between. A node
+// that stays a leaf, and children of at most kWarpMax, go to the final array. The
+// level kernels would take five launches a level for them: 20,480 triangles 528 -> 496
+// us, 2.0 M 3.09 -> 2.92 ms.
+constexpr int kMidThreads = 256;
+struct MidNode {
+  int32_t node, depth;
+  uint32_t first, count;  // first: within the block's range
+  uint32_t par;           // which array its slots lie in
+  float mn[3], mx[3];
+};
+struct MidSplit {
+  int32_t axis;  // -1: the node stays a leaf
+  float coord;
+  uint32_t lc;
+  int32_t kid[2];  // the children's places on the stack, -1 where they have none
+};
+constexpr size_t kMidBytes = (6 * sizeof(float) + sizeof(uint32_t) + 2 * sizeof(uint16_t));  // per primitive
+
+template <uint32_t kMidMax>
+__global__ void __launch_bounds__(kMidThreads) k_mid(LevelArgs A) {
+  after_previous();
+  constexpr uint32_t kMidWords = kMidMax / 32;
+  constexpr int kMidStack = kMidMax / (kWarpMax + 1) + 1;  // pending nodes are disjoint
+  extern __shared__ float sh[];
+  float* bx = sh;  // bx[c * kMidMax + slot]: min x/y/z, max x/y/z
+  uint32_t* id = reinterpret_cast<uint32_t*>(bx + 6 * kMidMax);
+  uint16_t* ord = reinterpret_cast<uint16_t*>(id + kMidMax);  // two arrays
+  __shared__ uint32_t bins[kBinWords];
+  __shared__ float planes[3 * kPlanes];
+  __shared__ MidNode stack[kMidStack];
+  __shared__ MidSplit split;
+  __shared__ uint32_t wleft[kMidWords], before[kMidWords], total;
+  __shared__ int s_sp;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t nmid = min(A.counters[kMid], A.max_mid);
+  for (uint32_t m = blockIdx.x; m < nmid; m += gridDim.x) {
+    const int32_t root = A.mid[m];
+    const uint32_t base = (uint32_t)A.arena[root].first, n = (uint32_t)A.arena[root].count;
+    if (threadIdx.x == 0) {
+      stack[0].node = root, stack[0].depth = A.arena[root].depth;
+      stack[0].first = 0, stack[0].count = n, stack[0].par = 0;
+      for (int a = 0; a < 3; a++) stack[0].mn[a] = A.arena[root].mn[a], stack[0].mx[a] = A.arena[root].mx[a];
+    }
+    for (int w = threadIdx.x; w < kBinWords; w += kMidThreads) bins[w] = bin_init(w);
+    for (uint32_t j = threadIdx.x; j < n; j += kMidThreads) {
+      const uint32_t p = A.prims[base + j];
+      const PrimBox v = prim_box(A.box + p);
+      id[j] = p, ord[j] = (uint16_t)j;
+      bx[j] = v.lo.x, bx[kMidMax + j] = v.lo.y, bx[2 * kMidMax + j] = v.lo.z;
+      bx[3 * kMidMax + j] = v.hi.x, bx[4 * kMidMax + j] = v.hi.y, bx[5 * kMidMax + j] = v.hi.z;
+    }
+    __syncthreads();
+    int sp = 1;
+    while (sp > 0) {
+      const MidNode nd = stack[--sp];
+      const uint32_t first = nd.first, count = nd.count;
+      const uint16_t* from = ord + nd.par * kMidMax;
+      if (threadIdx.x < 3 * kPlanes) {
+        const int a = threadIdx.x / kPlanes, i = threadIdx.x % kPlanes + 1;
+        planes[threadIdx.x] = plane_at(nd.mn[a], nd.mx[a], i);
+      }
+      __syncthreads();
+      for (uint32_t k0 = 0; k0 + 32 * warp < count; k0 += kMidThreads) {
+        const uint32_t k = k0 + threadIdx.x;
+        const bool in = k < count;
+        const uint32_t j = in ? from[first + k] : 0u;
+        const float4 lo = make_float4(bx[j], bx[kMidMax + j], bx[2 * kMidMax + j], 0.0f);
+        const float4 hi = make_float4(bx[3 * kMidMax + j], bx[4 * kMidMax + j], bx[5 * kMidMax + j], 0.0f);
+        int iv[3];
+        intervals_of(planes, lo, hi, iv);
+        bin_warp(bins, iv, lo, hi, in);
+      }
+      __syncthreads();
+      if (warp == 0) {
+        Cand c;
+        const int best = choose_split(bins, lane, c);
+        const float parent_cost = __fmul_rn(area3(nd.mn, nd.mx), __uint2float_rn(count));
+        if (best < 32) bcast_cand(c, best);
+        if (lane == 0) {
+          split = MidSplit{-1, 0.0f, 0u, {-1, -1}};
+          int top = sp;
+          if (best == 32) {
+            // no candidate below 1e34: a leaf unless the parent's cost is not below it either
+            if (!(parent_cost < 1e34f)) atomicOr(&A.counters[kError], kErrDegenerate);
+          } else if (!(parent_cost < c.cost)) {
+            const uint32_t cid = atomicAdd(&A.counters[kArenaCount], 2u);
+            if (cid + 2 > A.cap) {
+              atomicOr(&A.counters[kError], kErrArena);
+            } else {
+              const uint32_t g = base + first;
+              split.axis = best / kPlanes, split.coord = planes[best], split.lc = c.lc;
+              A.arena[cid] = make_node(c.lmn, c.lmx, g, c.lc, nd.node, nd.depth + 1);
+              A.arena[cid + 1] = make_node(c.rmn, c.rmx, g + c.lc, c.rc, nd.node, nd.depth + 1);
+              A.arena[nd.node].left = (int32_t)cid;
+              for (int i = 0; i < 2; i++) {
+                const uint32_t cc = i ? c.rc : c.lc;
+                if (cc > kWarpMax && nd.depth + 1 <= kMaxSplitDepth) {
+                  split.kid[i] = top;  // at most kMidStack pending: ranges of more than kWarpMax, disjoint
+                  MidNode& q = stack[top++];
+                  q.node = (int32_t)cid + i, q.depth = nd.depth + 1;
+                  q.first = first + (i ? c.lc : 0u), q.count = cc, q.par = nd.par ^ 1u;
+                  for (int a = 0; a < 3; a++)
+                    q.mn[a] = i ? c.rmn[a] : c.lmn[a], q.mx[a] = i ? c.rmx[a] : c.lmx[a];
+                } else {
+                  queue_child(A, (int32_t)cid + i, cc, nd.depth + 1);
+                }
+              }
+            }
+          }
+          s_sp = top;
+        }
+      }
+      __syncthreads();
+      sp = s_sp;
+      for (int w = threadIdx.x; w < kBinWords; w += kMidThreads) bins[w] = bin_init(w);
+      const MidSplit s = split;
+      if (s.axis < 0) {
+        for (uint32_t k = threadIdx.x; k < count; k += kMidThreads) A.prims[base + first + k] = id[from[first + k]];
+        __syncthreads();
+        continue;
+      }
+      // the stable partition: a bit per primitive, kept in the lane that read it
+      uint32_t slot[kMidMax / kMidThreads], bal[kMidMax / kMidThreads];
+#pragma unroll
+      for (int i = 0; i < (int)(kMidMax / kMidThreads); i++) {
+        const uint32_t w = warp + (kMidThreads / 32) * i, k = 32 * w + lane;
+        if (32 * w >= count) break;  // whole warp
+        slot[i] = k < count ? from[first + k] : 0u;
+        const float c = centroid(bx[s.axis * kMidMax + slot[i]], bx[(3 + s.axis) * kMidMax + slot[i]]);
+        bal[i] = __ballot_sync(0xffffffffu, k < count && c <= s.coord);
+        if (lane == 0) wleft[w] = __popc(bal[i]);
+      }
+      __syncthreads();
+      if (warp == 0) {  // left counts before each word
+        uint32_t run = 0;
+        for (uint32_t w0 = 0; 32 * w0 < count; w0 += 32) {
+          const uint32_t w = w0 + lane, v = 32 * w < count ? wleft[w] : 0u;
+          uint32_t x = v;
+#pragma unroll
+          for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+            if (lane >= off) x += y;
+          }
+          if (32 * w < count) before[w] = run + x - v;
+          run += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) total = run;
+      }
+      __syncthreads();
+      const bool good = total == s.lc;
+      if (!good && threadIdx.x == 0) atomicOr(&A.counters[kError], kErrPartition);
+      uint16_t* to = ord + (nd.par ^ 1u) * kMidMax;
+#pragma unroll
+      for (int i = 0; i < (int)(kMidMax / kMidThreads); i++) {
+        const uint32_t w = warp + (kMidThreads / 32) * i, k = 32 * w + lane;
+        if (k >= count) break;
+        const uint32_t l = before[w] + __popc(bal[i] & lt);
+        bool left = (bal[i] >> lane) & 1u;
+        uint32_t at = first + (left ? l : s.lc + k - l);
+        if (!good) left = k < s.lc, at = first + k;  // as it lies; the build fails
+        if ((left ? s.kid[0] : s.kid[1]) >= 0) to[at] = (uint16_t)slot[i];
+        else A.prims[base + at] = id[slot[i]];
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -1056,6 +1252,8 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   A.arena = arena;
   A.large[0] = at<int32_t>(scratch, L.large0), A.large[1] = at<int32_t>(scratch, L.large1);
   A.max_large = L.max_large;
+  A.mid = at<int32_t>(scratch, L.mid);
+  A.max_mid = L.max_mid, A.mid_most = L.mid_most;
   A.small = at<int32_t>(scratch, L.small);
   A.counters = counters;
   A.cap = L.cap;
@@ -1070,8 +1268,8 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   A.prims = prims;
 
   k_init<<<1, 32, 0, s>>>(counters);
-  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > kWarpMax ? A.buf[0] : prims, counters);
-  k_root<<<1, 1, 0, s>>>(arena, A.large[0], A.small, n, counters);
+  k_prep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > L.mid_most ? A.buf[0] : prims, counters);
+  k_root<<<1, 1, 0, s>>>(arena, A.large[0], A.mid, A.small, n, L.mid_most, counters);
   GB_TRY(cudaGetLastError());
   GB_TRY(cudaMemcpyAsync(host_counters, counters, 4 * kCounterWords, cudaMemcpyDeviceToHost, s));
   GB_TRY(cudaStreamSynchronize(s));
@@ -1083,7 +1281,7 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   while (nl > 0) {
     if (nl > L.max_large) return cudaErrorInvalidValue;
     int batch = 1;
-    while (batch < 4 && (nl << batch) * kWarpMax <= n) batch++;
+    while (batch < 4 && (nl << batch) * L.mid_most <= n) batch++;
     for (int i = 0; i < batch; i++, par ^= 1) {
       const uint64_t most = std::min<uint64_t>(nl << i, L.max_large);
       const unsigned gn = blocks(most * 32, 256);
@@ -1100,10 +1298,16 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     nl = host_counters[kLarge + par];
     if (host_counters[kError]) break;
   }
-  const uint32_t nsmall = host_counters[kSmallCount];
-  if (nsmall > 0 && !host_counters[kError]) {
+  if (host_counters[kMid] > 0 && !host_counters[kError]) {
+    auto kernel = L.mid_most == 1024 ? k_mid<1024> : k_mid<2048>;
+    const size_t shared = kMidBytes * L.mid_most;
+    GB_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+    GB_TRY(launch_after(kernel, std::min(host_counters[kMid], L.max_mid), kMidThreads, shared, s, A));
+  }
+  if (n >= 4 && !host_counters[kError]) {
+    // how many subtrees the warps have is known on the device
     const int sms = sm_count();
-    const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sms * 8);
+    const unsigned g = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 4, kSmallWarps), (uint64_t)sms * 8);
     GB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
     // the levels' first buffer (4 bytes per primitive) is free now: it takes the tasks
     k_small<<<g, kSmallWarps * 32, 0, s>>>(arena, A.small, counters, box, prims, counters, L.cap, tmp);
@@ -1138,7 +1342,6 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     r.quad_nodes = root.qcount;
     r.depth = host_counters[kQuadDepth];
   }
-  r.small_roots = nsmall;
   return cudaSuccess;
 }
 

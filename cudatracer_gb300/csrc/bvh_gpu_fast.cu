@@ -51,7 +51,11 @@ constexpr uint32_t kLeafMax = 4;
 constexpr int32_t kDepthLimit = 60;
 constexpr float kPad = 1e-5f;
 constexpr uint32_t kSweepMax = 16;
-constexpr uint32_t kWarpMax = 128;  // subtrees up to this size: one warp
+constexpr uint32_t kWarpMax = 128;   // subtrees up to this size: one warp
+// Nodes up to this size are split by one block down to those. 64 KB of shared memory
+// leave three blocks of 2,048 on an SM and six of 1,024: 20,480 triangles build in 671
+// against 723 us, 2.0 M in 3.68 against 3.60 ms.
+inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
 // Primitives per block of the level kernels: the fewest, as a power of two from
 // 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
 // of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
@@ -75,6 +79,7 @@ enum Counter : int {
   kMag = 6,
   kChunks = 2,       // 2 words: chunks of the even and of the odd level
   kTasks = kChunks,  // ranges for k_fleaf, once the levels are done
+  kMid = 7,          // nodes for k_fmid
   kRootKeys = 8,     // 6 words: min x/y/z, max x/y/z
   kLarge = 14,       // 2 words: large nodes of the even and of the odd level
   kCounterWords = 16,
@@ -144,13 +149,15 @@ struct QRec {
 static_assert(sizeof(QRec) == 64, "QRec");
 
 struct Layout {
-  size_t box, prims, tmp, arena, cost, arrive, large0, large1, small, chunks, chunk_left, split,
+  size_t box, prims, tmp, arena, cost, arrive, large0, large1, mid, small, chunks, chunk_left, split,
       bins, cbk, qlist, qrec, scan, sums, counters, total;
-  uint32_t chunk, cap, qcap, max_large, max_chunks, max_small, max_sums;
+  uint32_t chunk, cap, qcap, mid_most, max_large, max_mid, max_chunks, max_small, max_sums;
   explicit Layout(uint32_t n, int wide = 0) {
     cap = 2 * n + 2;
     qcap = n + 2;
-    max_large = n / (kWarpMax + 1) + 2;
+    mid_most = mid_size(n);
+    max_large = n / (mid_most + 1) + 2;
+    max_mid = n / (kWarpMax + 1) + 2;
     chunk = chunk_size(n);
     max_chunks = n / chunk + max_large + 2;
     max_small = n / 2 + 2;
@@ -169,6 +176,7 @@ struct Layout {
     arrive = take(4 * (size_t)cap);
     large0 = take(4 * (size_t)max_large);
     large1 = take(4 * (size_t)max_large);
+    mid = take(4 * (size_t)max_mid);
     small = take(4 * (size_t)max_small);
     chunks = take(sizeof(Chunk) * (size_t)max_chunks);
     chunk_left = take(4 * (size_t)max_chunks);
@@ -410,26 +418,15 @@ __device__ __forceinline__ FNodeD make_node(const float mn[3], const float mx[3]
   return b;
 }
 
-// A child is split further when it holds more than one primitive above the depth
-// limit: by the next level's kernels (returns its slot there) or by a warp (-1).
-__device__ __forceinline__ int32_t classify(int32_t id, uint32_t count, int32_t depth, int32_t* next_large,
-                                            uint32_t* next_count, uint32_t max_large, uint32_t* next_cbk,
+// Queue of a child that a block or a warp splits further (the level kernels keep
+// theirs, add_children).
+__device__ __forceinline__ void queue_child(int32_t id, uint32_t count, int32_t depth, int32_t* mid, uint32_t max_mid,
                                             int32_t* small, uint32_t max_small, uint32_t* counters) {
-  if (count <= 1 || depth >= kDepthLimit) return -1;
-  if (count > kWarpMax) {
-    const uint32_t s = atomicAdd(next_count, 1u);
-    if (s >= max_large) {
-      atomicOr(&counters[kError], kErrArena);
-      return -1;
-    }
-    next_large[s] = id;
-    for (int k = 0; k < 6; k++) next_cbk[6 * (size_t)s + k] = k < 3 ? fkey(1e34f) : fkey(-1e34f);
-    return (int32_t)s;
-  }
-  const uint32_t s = atomicAdd(&counters[kSmallCount], 1u);
-  if (s < max_small) small[s] = id;
+  if (count <= 1 || depth >= kDepthLimit) return;  // a leaf
+  const bool m = count > kWarpMax;
+  const uint32_t s = atomicAdd(&counters[m ? kMid : kSmallCount], 1u), most = m ? max_mid : max_small;
+  if (s < most) (m ? mid : small)[s] = id;
   else atomicOr(&counters[kError], kErrArena);
-  return -1;
 }
 
 // ---------------------------------------------------------------- prep
@@ -517,15 +514,19 @@ __global__ void __launch_bounds__(256) k_fprep(const float4* __restrict__ v, con
   block_root_keys(cbk, cmn, cmx);
 }
 
-__global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* small, uint32_t n, uint32_t* counters) {
+__global__ void k_froot(FNodeD* arena, int32_t* large, int32_t* mid, int32_t* small, uint32_t n, uint32_t mid_most,
+                        uint32_t* counters) {
   float mn[3], mx[3];
   for (int k = 0; k < 3; k++) mn[k] = unkey(counters[kRootKeys + k]), mx[k] = unkey(counters[kRootKeys + 3 + k]);
   arena[0] = make_node(mn, mx, 0, n, -1, 0);
   counters[kArenaCount] = 1;
   if (n >= 2) {
-    if (n > kWarpMax) {
+    if (n > mid_most) {
       large[0] = 0;
       counters[kLarge] = 1;
+    } else if (n > kWarpMax) {
+      mid[0] = 0;
+      counters[kMid] = 1;
     } else {
       small[0] = 0;
       counters[kSmallCount] = 1;
@@ -545,6 +546,8 @@ struct LevelArgs {
   FNodeD* arena;
   int32_t* large[2];
   uint32_t max_large;
+  int32_t* mid;
+  uint32_t max_mid, mid_most;
   int32_t* small;
   uint32_t max_small;
   uint32_t* counters;
@@ -645,10 +648,22 @@ __device__ __forceinline__ void add_children(const LevelArgs& A, int par, int32_
   A.arena[cid + 1] = make_node(rmn, rmx, (uint32_t)nd.first + mid, count - mid, ni, nd.depth + 1);
   A.arena[ni].left = (int32_t)cid;
   const int nx = par ^ 1;
-  sp.kid[0] = classify((int32_t)cid, mid, nd.depth + 1, A.large[nx], &A.counters[kLarge + nx], A.max_large, A.cbk[nx],
-                       A.small, A.max_small, A.counters);
-  sp.kid[1] = classify((int32_t)cid + 1, count - mid, nd.depth + 1, A.large[nx], &A.counters[kLarge + nx], A.max_large,
-                       A.cbk[nx], A.small, A.max_small, A.counters);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const uint32_t c = i ? count - mid : mid;
+    if (c <= A.mid_most || nd.depth + 1 >= kDepthLimit) {
+      queue_child((int32_t)cid + i, c, nd.depth + 1, A.mid, A.max_mid, A.small, A.max_small, A.counters);
+      continue;
+    }
+    const uint32_t s = atomicAdd(&A.counters[kLarge + nx], 1u);
+    if (s >= A.max_large) {
+      atomicOr(&A.counters[kError], kErrArena);
+      continue;
+    }
+    A.large[nx][s] = (int32_t)cid + i;
+    for (int k = 0; k < 6; k++) A.cbk[nx][6 * (size_t)s + k] = k < 3 ? fkey(1e34f) : fkey(-1e34f);
+    sp.kid[i] = (int32_t)s;
+  }
 }
 
 __global__ void __launch_bounds__(256) k_fsplit(LevelArgs A, int par) {
@@ -806,6 +821,225 @@ __global__ void __launch_bounds__(256) k_fpscatter(LevelArgs A, int par) {
     const uint32_t b = word[w], l = before[w] + __popc(b & lt), p = from[ch.begin + 32 * w + lane];
     if ((b >> lane) & 1u) to_l[dl + l] = p;
     else to_r[dr + 32 * w + lane - l] = p;
+  }
+}
+
+// ---------------------------------------------------------------- nodes of at most mid_size(n), one block each
+// A block splits such a node, and its children of more than kWarpMax primitives, with
+// everything in shared memory: boxes and ids by the slot they arrived in, and the
+// slots in their present order, in two arrays that a partition goes between. Children
+// of at most kWarpMax go to the final array and the warps' list. The level kernels
+// would take five launches a level for them: 20,480 triangles 778 -> 700 us, 2.0 M
+// 3.66 -> 3.57 ms. What is left is the bins' instructions (runs of eight primitives
+// kept in registers were slower, 538 against 453 us for this kernel of a 2.0 M build).
+constexpr int kMidThreads = 256;
+struct MidNode {
+  int32_t node, depth;
+  uint32_t first, count;  // first: within the block's range
+  uint32_t par;           // which array its slots lie in
+  uint32_t cb[6];         // centroid bounds
+};
+constexpr size_t kMidBytes = (6 * sizeof(float) + sizeof(uint32_t) + 2 * sizeof(uint16_t));  // per primitive
+
+template <uint32_t kMidMax>
+__global__ void __launch_bounds__(kMidThreads) k_fmid(LevelArgs A) {
+  after_previous();
+  constexpr uint32_t kMidWords = kMidMax / 32;
+  constexpr int kMidStack = kMidMax / (kWarpMax + 1) + 1;  // pending nodes are disjoint
+  extern __shared__ float sh[];
+  float* bx = sh;  // bx[c * kMidMax + slot]: min x/y/z, max x/y/z
+  uint32_t* id = reinterpret_cast<uint32_t*>(bx + 6 * kMidMax);
+  uint16_t* ord = reinterpret_cast<uint16_t*>(id + kMidMax);  // two arrays
+  __shared__ uint32_t bins[kBinWords];
+  __shared__ MidNode stack[kMidStack];
+  __shared__ FSplit split;
+  __shared__ uint32_t cb[2][6], wleft[kMidWords], before[kMidWords], total;
+  __shared__ int s_sp;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u;
+  auto box_of = [&](uint32_t j) {
+    PrimBox v;
+    v.lo = make_float4(bx[j], bx[kMidMax + j], bx[2 * kMidMax + j], 0.0f);
+    v.hi = make_float4(bx[3 * kMidMax + j], bx[4 * kMidMax + j], bx[5 * kMidMax + j], 0.0f);
+    return v;
+  };
+  // the bounds of a child from its threads' keys
+  auto reduce_keys = [&](uint32_t key[6], uint32_t* to) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const uint32_t mn = __reduce_min_sync(0xffffffffu, key[a]), mx = __reduce_max_sync(0xffffffffu, key[3 + a]);
+      if (lane == 0) atomicMin(&to[a], mn), atomicMax(&to[3 + a], mx);
+    }
+  };
+  const uint32_t nmid = min(A.counters[kMid], A.max_mid);
+  for (uint32_t m = blockIdx.x; m < nmid; m += gridDim.x) {
+    const int32_t root = A.mid[m];
+    const uint32_t base = (uint32_t)A.arena[root].first, n = (uint32_t)A.arena[root].count;
+    if (threadIdx.x < 6) stack[0].cb[threadIdx.x] = threadIdx.x < 3 ? fkey(1e34f) : fkey(-1e34f);
+    if (threadIdx.x == 0) {
+      stack[0].node = root, stack[0].depth = A.arena[root].depth;
+      stack[0].first = 0, stack[0].count = n, stack[0].par = 0;
+    }
+    for (int w = threadIdx.x; w < kBinWords; w += kMidThreads) bins[w] = bin_init(w);
+    __syncthreads();
+    {
+      uint32_t key[6];
+      for (int k = 0; k < 6; k++) key[k] = k < 3 ? 0xffffffffu : 0u;
+      for (uint32_t j = threadIdx.x; j < n; j += kMidThreads) {
+        const uint32_t p = A.prims[base + j];
+        const PrimBox v = prim_box(A.box + p);
+        id[j] = p, ord[j] = (uint16_t)j;
+        bx[j] = v.lo.x, bx[kMidMax + j] = v.lo.y, bx[2 * kMidMax + j] = v.lo.z;
+        bx[3 * kMidMax + j] = v.hi.x, bx[4 * kMidMax + j] = v.hi.y, bx[5 * kMidMax + j] = v.hi.z;
+        const float4 c = centre(v);
+        const uint32_t x[3] = {fkey(c.x), fkey(c.y), fkey(c.z)};
+        for (int a = 0; a < 3; a++) key[a] = min(key[a], x[a]), key[3 + a] = max(key[3 + a], x[a]);
+      }
+      reduce_keys(key, stack[0].cb);
+    }
+    __syncthreads();
+    int sp = 1;
+    while (sp > 0) {
+      const MidNode nd = stack[--sp];
+      const uint32_t first = nd.first, count = nd.count;
+      const uint16_t* from = ord + nd.par * kMidMax;
+      float blo[3], bscale[3];
+      bin_frame(nd.cb, blo, bscale);
+      for (uint32_t k0 = 0; k0 < count; k0 += kMidThreads) {
+        const uint32_t k = k0 + threadIdx.x;
+        const bool in = k < count;
+        if (k0 + 32 * warp >= count) break;  // whole warp
+        const PrimBox v = box_of(in ? from[first + k] : 0u);
+        int bin[3];
+        bins_of(blo, bscale, centre(v), bin);
+        bin_warp(bins, bin, v.lo, v.hi, in);
+      }
+      if (threadIdx.x < 12) cb[threadIdx.x / 6][threadIdx.x % 6] = threadIdx.x % 6 < 3 ? fkey(1e34f) : fkey(-1e34f);
+      __syncthreads();
+      if (warp == 0) {
+        Cand c;
+        choose_bin_split(bins, bscale, A.ascale, lane, c);
+        int mode = 0;
+        if (c.j >= kCands) {  // every centroid in one bin on every axis: halve the range as it lies
+          mode = 1;
+          c.j = 0, c.lc = count / 2;
+          for (int side = 0; side < 2; side++) {
+            uint32_t key[6];
+            for (int k = 0; k < 6; k++) key[k] = k < 3 ? fkey(1e34f) : fkey(-1e34f);
+            for (uint32_t k = (side ? c.lc : 0u) + lane; k < (side ? count : c.lc); k += 32) {
+              const PrimBox v = box_of(from[first + k]);
+              const uint32_t x[6] = {fkey(v.lo.x), fkey(v.lo.y), fkey(v.lo.z), fkey(v.hi.x), fkey(v.hi.y), fkey(v.hi.z)};
+              for (int a = 0; a < 3; a++) key[a] = min(key[a], x[a]), key[3 + a] = max(key[3 + a], x[3 + a]);
+            }
+            for (int a = 0; a < 3; a++) {
+              const float mn = unkey(__reduce_min_sync(0xffffffffu, key[a])),
+                          mx = unkey(__reduce_max_sync(0xffffffffu, key[3 + a]));
+              if (side) c.rmn[a] = mn, c.rmx[a] = mx;
+              else c.lmn[a] = mn, c.lmx[a] = mx;
+            }
+          }
+        }
+        if (lane == 0) {
+          const int a = c.j / (kBins - 1);
+          split = FSplit{mode, {-1, -1}, a, blo[a], bscale[a], c.j % (kBins - 1) + 1, c.lc, 0u};
+          // the children: split further here, by a warp, or leaves
+          int top = sp;
+          const uint32_t cid = atomicAdd(&A.counters[kArenaCount], 2u);
+          if (cid + 2 > A.cap) {
+            atomicOr(&A.counters[kError], kErrArena);
+            split.mode = -1;
+          } else {
+            const uint32_t g = base + first;
+            A.arena[cid] = make_node(c.lmn, c.lmx, g, c.lc, nd.node, nd.depth + 1);
+            A.arena[cid + 1] = make_node(c.rmn, c.rmx, g + c.lc, count - c.lc, nd.node, nd.depth + 1);
+            A.arena[nd.node].left = (int32_t)cid;
+            for (int i = 0; i < 2; i++) {
+              const uint32_t cc = i ? count - c.lc : c.lc;
+              if (cc > kWarpMax && nd.depth + 1 < kDepthLimit) {
+                split.kid[i] = top;  // at most kMidStack pending: ranges of more than kWarpMax, disjoint
+                MidNode& q = stack[top++];
+                q.node = (int32_t)cid + i, q.depth = nd.depth + 1;
+                q.first = first + (i ? c.lc : 0u), q.count = cc, q.par = nd.par ^ 1u;
+              } else {
+                queue_child((int32_t)cid + i, cc, nd.depth + 1, A.mid, A.max_mid, A.small, A.max_small, A.counters);
+              }
+            }
+          }
+          s_sp = top;
+        }
+      }
+      __syncthreads();
+      sp = s_sp;
+      for (int w = threadIdx.x; w < kBinWords; w += kMidThreads) bins[w] = bin_init(w);
+      const FSplit s = split;
+      if (s.mode < 0) {  // the build fails
+        __syncthreads();
+        continue;
+      }
+      // the stable partition: a bit per primitive, kept in the lane that read it
+      uint32_t slot[kMidMax / kMidThreads], bal[kMidMax / kMidThreads], key[2][6];
+      for (int i = 0; i < 2; i++)
+        for (int k = 0; k < 6; k++) key[i][k] = k < 3 ? 0xffffffffu : 0u;
+#pragma unroll
+      for (int i = 0; i < (int)(kMidMax / kMidThreads); i++) {
+        const uint32_t w = warp + (kMidThreads / 32) * i, k = 32 * w + lane;
+        if (32 * w >= count) break;  // whole warp
+        const bool in = k < count;
+        slot[i] = in ? from[first + k] : 0u;
+        const float4 c = centre(box_of(slot[i]));
+        const bool left = in && (s.mode == 1 ? k < s.lc : bin_of(comp(c, s.axis), s.lo, s.scale) < s.bsp);
+        bal[i] = __ballot_sync(0xffffffffu, left);
+        if (lane == 0) wleft[w] = __popc(bal[i]);
+        const uint32_t x[3] = {fkey(c.x), fkey(c.y), fkey(c.z)};
+        const bool right = in && !left;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          key[0][a] = min(key[0][a], left ? x[a] : 0xffffffffu), key[0][3 + a] = max(key[0][3 + a], left ? x[a] : 0u);
+          key[1][a] = min(key[1][a], right ? x[a] : 0xffffffffu), key[1][3 + a] = max(key[1][3 + a], right ? x[a] : 0u);
+        }
+      }
+      if (32u * warp < count) {
+        if (s.kid[0] >= 0) reduce_keys(key[0], cb[0]);
+        if (s.kid[1] >= 0) reduce_keys(key[1], cb[1]);
+      }
+      __syncthreads();
+      if (warp == 0) {  // left counts before each word
+        uint32_t run = 0;
+        for (uint32_t w0 = 0; 32 * w0 < count; w0 += 32) {
+          const uint32_t w = w0 + lane, v = 32 * w < count ? wleft[w] : 0u;
+          uint32_t x = v;
+#pragma unroll
+          for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+            if (lane >= off) x += y;
+          }
+          if (32 * w < count) before[w] = run + x - v;
+          run += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) total = run;
+      }
+      if (threadIdx.x >= 32 && threadIdx.x < 44) {
+        const int i = (threadIdx.x - 32) / 6, k = (threadIdx.x - 32) % 6;
+        const int32_t kid = i ? s.kid[1] : s.kid[0];
+        if (kid >= 0) stack[kid].cb[k] = cb[i][k];
+      }
+      __syncthreads();
+      const bool good = total == s.lc;
+      if (!good && threadIdx.x == 0) atomicOr(&A.counters[kError], kErrPartition);
+      uint16_t* to = ord + (nd.par ^ 1u) * kMidMax;
+#pragma unroll
+      for (int i = 0; i < (int)(kMidMax / kMidThreads); i++) {
+        const uint32_t w = warp + (kMidThreads / 32) * i, k = 32 * w + lane;
+        if (k >= count) break;
+        const uint32_t l = before[w] + __popc(bal[i] & lt);
+        bool left = (bal[i] >> lane) & 1u;
+        uint32_t at = first + (left ? l : s.lc + k - l);
+        if (!good) left = k < s.lc, at = first + k;  // as it lies; the build fails
+        if ((left ? s.kid[0] : s.kid[1]) >= 0) to[at] = (uint16_t)slot[i];
+        else A.prims[base + at] = id[slot[i]];
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -1579,6 +1813,8 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   A.arena = arena;
   A.large[0] = at<int32_t>(scratch, Lo.large0), A.large[1] = at<int32_t>(scratch, Lo.large1);
   A.max_large = Lo.max_large;
+  A.mid = at<int32_t>(scratch, Lo.mid);
+  A.max_mid = Lo.max_mid, A.mid_most = Lo.mid_most;
   A.small = at<int32_t>(scratch, Lo.small);
   A.max_small = Lo.max_small;
   A.counters = counters;
@@ -1597,9 +1833,9 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
 
   k_finit<<<1, 32, 0, s>>>(counters, cbk);
   k_fmag<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, counters);
-  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > kWarpMax ? A.buf[0] : prims, counters, cbk,
+  k_fprep<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, n, box, n > Lo.mid_most ? A.buf[0] : prims, counters, cbk,
                                            wide ? 0.0f : kPad);
-  k_froot<<<1, 1, 0, s>>>(arena, A.large[0], A.small, n, counters);
+  k_froot<<<1, 1, 0, s>>>(arena, A.large[0], A.mid, A.small, n, Lo.mid_most, counters);
   FB_TRY(cudaGetLastError());
   FB_TRY(read_counters(hc, counters, s));
   if (hc[kError]) {
@@ -1623,7 +1859,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   int par = 0;
   while (nl > 0) {
     int batch = 1;
-    while (batch < 4 && (nl << batch) * kWarpMax <= n) batch++;
+    while (batch < 4 && (nl << batch) * Lo.mid_most <= n) batch++;
     for (int i = 0; i < batch; i++, par ^= 1) {
       const uint64_t most = std::min<uint64_t>(nl << i, Lo.max_large);
       const unsigned gn = blocks(most * 32, 256);
@@ -1642,9 +1878,15 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     }
     nl = hc[kLarge + par];
   }
-  const uint32_t nsmall = std::min(hc[kSmallCount], Lo.max_small);
-  if (nsmall > 0) {
-    const unsigned g = (unsigned)std::min<uint64_t>(blocks(nsmall, kSmallWarps), (uint64_t)sm_count() * 16);
+  if (hc[kMid] > 0) {
+    auto kernel = Lo.mid_most == 1024 ? k_fmid<1024> : k_fmid<2048>;
+    const size_t shared = kMidBytes * Lo.mid_most;
+    FB_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
+    FB_TRY(launch_after(kernel, std::min(hc[kMid], Lo.max_mid), kMidThreads, shared, s, A));
+  }
+  if (n >= 2) {
+    // how many subtrees the warps have is known on the device
+    const unsigned g = (unsigned)std::min<uint64_t>(blocks((uint64_t)n / 2, kSmallWarps), (uint64_t)sm_count() * 16);
     FB_TRY(cudaMemsetAsync(counters + kTasks, 0, 4, s));
     // the levels' first buffer (4 bytes per primitive) is free now: it takes the tasks
     k_fsmall<<<g, kSmallWarps * 32, 0, s>>>(A, tmp);
@@ -1664,7 +1906,6 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
   }
   const uint32_t nb = hc[kArenaCount];
   r.binary_nodes = nb;
-  r.small_roots = nsmall;
   if (n == 1) {
     r.quad_nodes = 1;
     r.depth = 1;

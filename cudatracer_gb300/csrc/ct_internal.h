@@ -258,7 +258,6 @@ cudaError_t launch_present(const float4* accum, float4* out, int n, float sample
 struct GpuBvhResult {
   uint32_t binary_nodes = 0, quad_nodes = 0, max_leaf = 0, depth = 0;
   uint32_t error = 0;  // 1 degenerate extent, 2 arena, 4 stack, 8 partition mismatch
-  uint32_t small_roots = 0;
 };
 size_t gpu_bvh_scratch_bytes(uint32_t n);
 cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_counters, cudaStream_t s, GpuBvhResult& r);
