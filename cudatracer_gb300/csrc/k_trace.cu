@@ -306,6 +306,14 @@ cudaError_t launch_ray_sort(const DevQueues& q, int queue, int key, cudaStream_t
 // ---------------------------------------------------------------- batches
 namespace {
 
+// How many lanes of a warp take rays in a batch stage of n: as lanes_for, spread over
+// up to 1,024 warps. A batch's later passes are small, few lanes' iterations are in
+// flight, and a pass lasts as long as its longest ray: 24 jobs of 64 to 512 pixels a
+// side 8.29 -> 7.63 ms, 12 bit-exact jobs 14.2 -> 11.6, 24 jobs of up to 128 pixels
+// 1.52 -> 1.22 (768 or 1,536 warps within 1 %). Frames, ten in flight, keep full warps:
+// 960x540 4.14 ms, spread 4.34.
+__device__ __forceinline__ int batch_lanes(int n) { return min(32, max(0, n - 1) / 1024 + 1); }
+
 struct BatchExtendIO {
   const float4* __restrict__ org;
   const float4* __restrict__ dir;
@@ -346,7 +354,7 @@ __global__ void __launch_bounds__(BLOCK) k_batch_extend(DevBatch bt, DevQueues q
     atomicAdd(&q.stats[0], (unsigned long long)n);
   }
   BatchExtendIO io{q.org_q(qi), q.dir_q(qi), q.hit, q.error, bt.jobs, bt.bases, bt.n_jobs, q.perm};
-  trace_persistent_batch<false, FASTMM, REFILL>(n, q.counts + 4, io, s_stack + threadIdx.x, BLOCK);
+  trace_persistent_batch<false, FASTMM, REFILL>(n, q.counts + 4, io, s_stack + threadIdx.x, BLOCK, batch_lanes(n));
 }
 
 template <bool FASTMM, int BLOCK>
@@ -356,7 +364,10 @@ __global__ void __launch_bounds__(BLOCK) k_batch_connect(DevBatch bt, DevQueues 
   int* stack = s_stack + threadIdx.x;
   const int n = q.counts[2];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&q.stats[1], (unsigned long long)n);
-  for (int i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
+  const int lanes = batch_lanes(n), lane = threadIdx.x & 31;
+  if (lane >= lanes) return;
+  for (int i = (blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5)) * lanes + lane; i < n;
+       i += gridDim.x * (BLOCK / 32) * lanes) {
     const float4 o = q.sorg[i], d = q.sdir[i];
     const int pix = __float_as_int(o.w);
     const BatchJob& J = bt.jobs[batch_job_of(bt.bases, bt.n_jobs, pix)];

@@ -469,10 +469,11 @@ __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cu
 // trace_persistent with a BVH and epsilon per lane: io.load(i, o, d, t0, b, eps)
 // supplies the ray and the tree it is traced against (batches of jobs).
 template <bool ANY, bool FASTMM, int REFILL, class IO>
-__device__ __forceinline__ void trace_persistent_batch(int n, int* cursor, IO& io, int* stack, int stride) {
+__device__ __forceinline__ void trace_persistent_batch(int n, int* cursor, IO& io, int* stack, int stride, int lanes) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
+  const unsigned own = FULL >> (32 - lanes);  // the lanes that take rays (batch_lanes)
   int rid = -1;
   bool exhausted = false;
   RayState r;
@@ -481,14 +482,14 @@ __device__ __forceinline__ void trace_persistent_batch(int n, int* cursor, IO& i
   float eps = 0.0f;
   while (true) {
     if (!exhausted) {
-      const unsigned m = __ballot_sync(FULL, rid < 0);
-      if (m == FULL || __popc(m) >= REFILL) {
+      const unsigned m = __ballot_sync(FULL, rid < 0) & own;
+      if (m == own || __popc(m) >= REFILL) {
         const int leader = __ffs(m) - 1;
         int base = 0;
         if (lane == leader) base = atomicAdd(cursor, __popc(m));
         base = __shfl_sync(FULL, base, leader);
         if (base + __popc(m) >= n) exhausted = true;
-        if (rid < 0) {
+        if (rid < 0 && lane < lanes) {
           const int my = base + __popc(m & below);
           if (my < n) {
             float4 o, d;
