@@ -1538,6 +1538,16 @@ ct_status ct_render_profile_read(ct_ctx* ctx, ct_render* r, ct_stage_times* out,
 // batch (172 bytes per pixel).
 constexpr int kBatchLanes = 4;
 
+// A second stream of a batch's capture, so that a pass's connect and the next pass's
+// extend are branches of the graph: neither needs the other (connect adds to the
+// accumulation, extend reads the other ray queue and writes hits), and a batch's
+// later passes are as long as their longest ray. The next shade waits for both. 24
+// jobs of 64 to 512 pixels a side 7.61 -> 6.99 ms, 12 bit-exact jobs 11.6 -> 9.3.
+struct BatchFork {
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
 struct ct_batch {
   int32_t n = 0;
   int32_t exact = 0;
@@ -1560,6 +1570,7 @@ struct ct_batch {
   std::vector<int32_t> bases;
   ct_batch_tuning tune{128, 128, 1, 1, CT_SORT_NONE, 24};
   cudaStream_t cap = nullptr;  // capture stream
+  BatchFork fork;
   cudaGraphExec_t exec[kBatchLanes] = {};
   ct_batch_tuning exec_tune{0, 0, 0, 0, 0, 0};
   cudaStream_t side[kBatchLanes] = {};  // lane streams
@@ -1570,6 +1581,9 @@ struct ct_batch {
     for (auto& x : exec)
       if (x) cudaGraphExecDestroy(x);
     if (cap) cudaStreamDestroy(cap);
+    if (fork.side) cudaStreamDestroy(fork.side);
+    if (fork.fork) cudaEventDestroy(fork.fork);
+    if (fork.join) cudaEventDestroy(fork.join);
     for (auto& x : side)
       if (x) cudaStreamDestroy(x);
     if (fork_ev) cudaEventDestroy(fork_ev);
@@ -1582,13 +1596,16 @@ namespace {
 
 
 // One iteration: every job that still takes samples traces one more.
-cudaError_t batch_iteration(ct_batch* b, int lane, const ct_batch_tuning& t, cudaStream_t st) {
+cudaError_t batch_iteration(ct_batch* b, int lane, const ct_batch_tuning& t, cudaStream_t st,
+                            const BatchFork* fork = nullptr) {
   const DevBatch& dev = b->lane_dev(lane);
-  const DevQueues& q = b->lane_q(lane);
+  DevQueues q = b->lane_q(lane);
+  if (dev.wide) fork = nullptr;  // its extend and connect share a cursor
   cudaError_t e = launch_batch_raygen(dev, q, math_exact_shading(b->exact), st);
   for (int pass = 0; pass < b->max_depth && e == cudaSuccess; pass++) {
     const int cur = pass & 1;
     const uint32_t path_length = pass == 0 ? 0u : (uint32_t)pass + 1u;  // Kernel.cu:306, 330
+    if (fork) q.shadow = 2 + cur;
     DevQueues qx = q;
     if (pass > 0 && t.sort_key != CT_SORT_NONE) {
       e = launch_ray_sort(q, cur, t.sort_key, st);
@@ -1597,12 +1614,23 @@ cudaError_t batch_iteration(ct_batch* b, int lane, const ct_batch_tuning& t, cud
     if (e == cudaSuccess)
       e = dev.wide ? launch_batch_extend_wide(dev, qx, cur, st)
                    : launch_batch_extend(dev, qx, cur, math_fast_traversal(b->exact), t.extend_block, t.refill, st);
-    if (e == cudaSuccess) e = launch_batch_shade(dev, q, cur, path_length, pass, math_exact_shading(b->exact), t.shade_waves, st);
+    const bool joins = fork && pass > 0;  // the previous pass's connect
+    if (joins && e == cudaSuccess) e = cudaStreamWaitEvent(st, fork->join, 0);
     if (e == cudaSuccess)
+      e = launch_batch_shade(dev, q, cur, path_length, pass, math_exact_shading(b->exact), t.shade_waves, st, !joins);
+    if (fork) {
+      if (e == cudaSuccess) e = cudaEventRecord(fork->fork, st);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(fork->side, fork->fork, 0);
+      if (e == cudaSuccess)
+        e = launch_batch_connect(dev, q, math_fast_traversal(b->exact), t.connect_block, fork->side, false);
+      if (e == cudaSuccess) e = cudaEventRecord(fork->join, fork->side);
+    } else if (e == cudaSuccess) {
       e = dev.wide ? launch_batch_connect_wide(dev, q, st)
                    : launch_batch_connect(dev, q, math_fast_traversal(b->exact), t.connect_block, st);
+    }
   }
-  if (e == cudaSuccess) e = launch_batch_advance(dev, q, st);
+  if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(st, fork->join, 0);
+  if (e == cudaSuccess) e = launch_batch_advance(dev, q, st, !fork);
   return e;
 }
 
@@ -1612,10 +1640,13 @@ cudaError_t batch_graph(ct_batch* b) {
     if (x) cudaGraphExecDestroy(x), x = nullptr;
   cudaError_t e = cudaSuccess;
   if (!b->cap) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !b->fork.side) e = cudaStreamCreateWithFlags(&b->fork.side, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !b->fork.fork) e = cudaEventCreateWithFlags(&b->fork.fork, cudaEventDisableTiming);
+  if (e == cudaSuccess && !b->fork.join) e = cudaEventCreateWithFlags(&b->fork.join, cudaEventDisableTiming);
   for (int lane = 0; lane < b->lanes && e == cudaSuccess; lane++) {
     e = cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return e;
-    const cudaError_t le = batch_iteration(b, lane, b->tune, b->cap);
+    const cudaError_t le = batch_iteration(b, lane, b->tune, b->cap, &b->fork);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(b->cap, &g);
     if (le != cudaSuccess) e = le;

@@ -132,7 +132,9 @@ struct DevQueues {
   float4* scol;      // shadow contribution xyz, w unused
   float4* accum;     // FP32 RGBA accumulation, one per pixel
   // device counters
-  int32_t* counts;   // [0],[1] ray queue sizes, [2] shadow queue size, [4] extend fetch cursor
+  int32_t* counts;   // [0],[1] ray queue sizes, [2],[3] shadow queue size, [4] extend fetch cursor
+  int32_t shadow = 2;  // which of them this stage's shadow queue counts in ([3] in turn where a
+                       // batch's connect runs beside the next extend)
   unsigned long long* stats;  // [0] extension rays, [1] shadow rays, [2] samples, [3] frames
   uint32_t* error;   // error bits (1 = stack overflow)
   int32_t* perm;     // order in which extend takes the queue's rays (nullptr = queue order); a
@@ -340,9 +342,10 @@ cudaError_t launch_batch_raygen(const DevBatch& b, const DevQueues& q, int exact
 cudaError_t launch_batch_extend(const DevBatch& b, const DevQueues& q, int queue, bool fast, int block, int refill,
                                 cudaStream_t s);
 cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue, uint32_t path_length, int pass,
-                               int exact, int grid_mult, cudaStream_t s);
-cudaError_t launch_batch_connect(const DevBatch& b, const DevQueues& q, bool fast, int block, cudaStream_t s);
-cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s);
+                               int exact, int grid_mult, cudaStream_t s, bool chained = true);
+cudaError_t launch_batch_connect(const DevBatch& b, const DevQueues& q, bool fast, int block, cudaStream_t s,
+                                 bool chained = true);
+cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s, bool chained = true);
 
 // Frame stages on a wide (quantised) BVH: the reference's Moller-Trumbore test
 // and epsilon over conservative 8-bit boxes (k_trace_wide.cu).

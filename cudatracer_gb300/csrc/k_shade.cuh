@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(kBlock) k_batch_shade(DevBatch bt, DevQueues q
         shade_compat(J.sc, q, J.f, o, d, t, h, path_length, e, J.pix_base, J.accum);
       if (pass + 1 >= J.max_depth) e.cont = false;
     }
-    const int si = warp_append(e.shadow, &q.counts[2]);
+    const int si = warp_append(e.shadow, &q.counts[q.shadow]);
     if (si >= 0) {
       q.sorg[si] = e.so;
       q.sdir[si] = e.sd;

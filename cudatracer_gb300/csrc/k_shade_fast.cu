@@ -117,17 +117,17 @@ cudaError_t launch_batch_raygen(const DevBatch& b, const DevQueues& q, int exact
 }
 
 cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue, uint32_t path_length, int pass,
-                               int exact, int grid_mult, cudaStream_t s) {
+                               int exact, int grid_mult, cudaStream_t s, bool chained) {
   // the live count is on the device: size the grid for the capacity, up to grid_mult waves
   auto k = exact ? exact::k_batch_shade : fast::k_batch_shade;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBlock, 0);
   const int cap_blocks = (q.capacity + kBlock - 1) / kBlock;
   const int grid = std::max(1, std::min(cap_blocks, std::max(1, per_sm) * sm_count() * std::max(1, grid_mult)));
-  return launch_after(k, grid, kBlock, 0, s, b, q, queue, path_length, pass);
+  return launch_after_if(chained, k, grid, kBlock, 0, s, b, q, queue, path_length, pass);
 }
 
-cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s) {
-  return launch_after(fast::k_batch_advance, (b.n_jobs + 127) / 128, 128, 0, s, b, q);
+cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s, bool chained) {
+  return launch_after_if(chained, fast::k_batch_advance, (b.n_jobs + 127) / 128, 128, 0, s, b, q);
 }
 }  // namespace ct

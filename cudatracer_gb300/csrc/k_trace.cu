@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(BLOCK) k_batch_extend(DevBatch bt, DevQueues q
   const int n = q.counts[qi];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     q.counts[qi ^ 1] = 0;
-    q.counts[2] = 0;
+    q.counts[q.shadow] = 0;
     atomicAdd(&q.stats[0], (unsigned long long)n);
   }
   BatchExtendIO io{q.org_q(qi), q.dir_q(qi), q.hit, q.error, bt.jobs, bt.bases, bt.n_jobs, q.perm};
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(BLOCK) k_batch_connect(DevBatch bt, DevQueues 
   wait_previous();
   extern __shared__ int s_stack[];
   int* stack = s_stack + threadIdx.x;
-  const int n = q.counts[2];
+  const int n = q.counts[q.shadow];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&q.stats[1], (unsigned long long)n);
   const int lanes = batch_lanes(n), lane = threadIdx.x & 31;
   if (lane >= lanes) return;
@@ -407,7 +407,7 @@ cudaError_t batch_extend(const DevBatch& b, const DevQueues& q, int queue, cudaS
 }
 
 template <bool FASTMM, int BLOCK>
-cudaError_t batch_connect(const DevBatch& b, const DevQueues& q, cudaStream_t s) {
+cudaError_t batch_connect(const DevBatch& b, const DevQueues& q, cudaStream_t s, bool chained) {
   const size_t smem = (size_t)b.max_stack * BLOCK * sizeof(int);
   auto kernel = k_batch_connect<FASTMM, BLOCK>;
   if (smem > 48 * 1024) {
@@ -418,7 +418,7 @@ cudaError_t batch_connect(const DevBatch& b, const DevQueues& q, cudaStream_t s)
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem);
   const int cap_blocks = (q.capacity + BLOCK - 1) / BLOCK;
   const int grid = std::max(1, std::min(cap_blocks, std::max(1, per_sm) * sm_count()));
-  return launch_after(kernel, grid, BLOCK, smem, s, b, q);
+  return launch_after_if(chained, kernel, grid, BLOCK, smem, s, b, q);
 }
 
 }  // namespace
@@ -444,10 +444,11 @@ cudaError_t launch_batch_extend(const DevBatch& b, const DevQueues& q, int queue
   return batch_extend_refill<128>(b, q, queue, fast, refill, s);
 }
 
-cudaError_t launch_batch_connect(const DevBatch& b, const DevQueues& q, bool fast, int block, cudaStream_t s) {
-  if (block == 64) return fast ? batch_connect<true, 64>(b, q, s) : batch_connect<false, 64>(b, q, s);
-  if (block == 256) return fast ? batch_connect<true, 256>(b, q, s) : batch_connect<false, 256>(b, q, s);
-  return fast ? batch_connect<true, 128>(b, q, s) : batch_connect<false, 128>(b, q, s);
+cudaError_t launch_batch_connect(const DevBatch& b, const DevQueues& q, bool fast, int block, cudaStream_t s,
+                                 bool chained) {
+  if (block == 64) return fast ? batch_connect<true, 64>(b, q, s, chained) : batch_connect<false, 64>(b, q, s, chained);
+  if (block == 256) return fast ? batch_connect<true, 256>(b, q, s, chained) : batch_connect<false, 256>(b, q, s, chained);
+  return fast ? batch_connect<true, 128>(b, q, s, chained) : batch_connect<false, 128>(b, q, s, chained);
 }
 
 }  // namespace ct

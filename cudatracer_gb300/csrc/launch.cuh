@@ -27,9 +27,10 @@ __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// chained false: an ordinary launch (a kernel that also waits for another stream).
 template <class... P, class... A>
-inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                                A... args) {
+inline cudaError_t launch_after_if(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                                   cudaStream_t s, A... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(block);
@@ -39,8 +40,13 @@ inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned bl
   a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   a[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = a;
-  c.numAttrs = 1;
+  c.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                                A... args) {
+  return launch_after_if(true, kernel, grid, block, smem, s, args...);
 }
 
 // Places for a warp's threads that want `want` units each from a counter, with one
