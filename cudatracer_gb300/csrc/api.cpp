@@ -1614,11 +1614,11 @@ cudaError_t batch_iteration(ct_batch* b, int lane, const ct_batch_tuning& t, cud
     if (e == cudaSuccess)
       e = dev.wide ? launch_batch_extend_wide(dev, qx, cur, st)
                    : launch_batch_extend(dev, qx, cur, math_fast_traversal(b->exact), t.extend_block, t.refill, st);
-    const bool joins = fork && pass > 0;  // the previous pass's connect
+    const bool joins = fork && pass > 0;  // with the previous pass's connect
     if (joins && e == cudaSuccess) e = cudaStreamWaitEvent(st, fork->join, 0);
     if (e == cudaSuccess)
       e = launch_batch_shade(dev, q, cur, path_length, pass, math_exact_shading(b->exact), t.shade_waves, st, !joins);
-    if (fork) {
+    if (fork && pass + 1 < b->max_depth) {  // nothing runs beside the last one
       if (e == cudaSuccess) e = cudaEventRecord(fork->fork, st);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(fork->side, fork->fork, 0);
       if (e == cudaSuccess)
@@ -1629,8 +1629,7 @@ cudaError_t batch_iteration(ct_batch* b, int lane, const ct_batch_tuning& t, cud
                    : launch_batch_connect(dev, q, math_fast_traversal(b->exact), t.connect_block, st);
     }
   }
-  if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(st, fork->join, 0);
-  if (e == cudaSuccess) e = launch_batch_advance(dev, q, st, !fork);
+  if (e == cudaSuccess) e = launch_batch_advance(dev, q, st);
   return e;
 }
 

@@ -345,7 +345,7 @@ cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue,
                                int exact, int grid_mult, cudaStream_t s, bool chained = true);
 cudaError_t launch_batch_connect(const DevBatch& b, const DevQueues& q, bool fast, int block, cudaStream_t s,
                                  bool chained = true);
-cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s, bool chained = true);
+cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s);
 
 // Frame stages on a wide (quantised) BVH: the reference's Moller-Trumbore test
 // and epsilon over conservative 8-bit boxes (k_trace_wide.cu).

@@ -127,7 +127,7 @@ cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue,
   return launch_after_if(chained, k, grid, kBlock, 0, s, b, q, queue, path_length, pass);
 }
 
-cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s, bool chained) {
-  return launch_after_if(chained, fast::k_batch_advance, (b.n_jobs + 127) / 128, 128, 0, s, b, q);
+cudaError_t launch_batch_advance(const DevBatch& b, const DevQueues& q, cudaStream_t s) {
+  return launch_after(fast::k_batch_advance, (b.n_jobs + 127) / 128, 128, 0, s, b, q);
 }
 }  // namespace ct
