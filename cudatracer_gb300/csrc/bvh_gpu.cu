@@ -45,6 +45,10 @@ constexpr uint32_t kWarpMax = 128;  // nodes up to this size are built by one wa
 // Nodes up to this size are split by one block down to those (64 KB of shared memory
 // leave three blocks of 2,048 on an SM and six of 1,024).
 inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
+// Builds of at most this many triangles leave an SM at most one such block, which has
+// 512 threads then instead of 256: 20,480 triangles 511 -> 487 us, 2.0 M with 512
+// 2.93 -> 3.32 ms.
+constexpr uint32_t kFewMid = 100000;
 constexpr uint32_t kLeafTask = 16;  // subtrees up to this size are built by one thread
 // Primitives per block of the level kernels: the fewest, as a power of two from
 // 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
@@ -646,7 +650,6 @@ __global__ void __launch_bounds__(256) k_part_scatter(LevelArgs A, int par) {
 // that stays a leaf, and children of at most kWarpMax, go to the final array. The
 // level kernels would take five launches a level for them: 20,480 triangles 528 -> 496
 // us, 2.0 M 3.09 -> 2.92 ms.
-constexpr int kMidThreads = 256;
 struct MidNode {
   int32_t node, depth;
   uint32_t first, count;  // first: within the block's range
@@ -661,7 +664,7 @@ struct MidSplit {
 };
 constexpr size_t kMidBytes = (6 * sizeof(float) + sizeof(uint32_t) + 2 * sizeof(uint16_t));  // per primitive
 
-template <uint32_t kMidMax>
+template <uint32_t kMidMax, int kMidThreads>
 __global__ void __launch_bounds__(kMidThreads) k_mid(LevelArgs A) {
   after_previous();
   constexpr uint32_t kMidWords = kMidMax / 32;
@@ -1299,10 +1302,11 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
     if (host_counters[kError]) break;
   }
   if (host_counters[kMid] > 0 && !host_counters[kError]) {
-    auto kernel = L.mid_most == 1024 ? k_mid<1024> : k_mid<2048>;
+    const unsigned threads = n > kFewMid ? 256 : 512;
+    auto kernel = L.mid_most == 1024 ? k_mid<1024, 256> : n > kFewMid ? k_mid<2048, 256> : k_mid<2048, 512>;
     const size_t shared = kMidBytes * L.mid_most;
     GB_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
-    GB_TRY(launch_after(kernel, std::min(host_counters[kMid], L.max_mid), kMidThreads, shared, s, A));
+    GB_TRY(launch_after(kernel, std::min(host_counters[kMid], L.max_mid), threads, shared, s, A));
   }
   if (n >= 4 && !host_counters[kError]) {
     // how many subtrees the warps have is known on the device

@@ -56,6 +56,10 @@ constexpr uint32_t kWarpMax = 128;   // subtrees up to this size: one warp
 // leave three blocks of 2,048 on an SM and six of 1,024: 20,480 triangles build in 671
 // against 723 us, 2.0 M in 3.68 against 3.60 ms.
 inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
+// Builds of at most this many triangles leave an SM at most one such block, which has
+// 512 threads then instead of 256: 20,480 triangles 730 -> 700 us, 2.0 M with 512
+// 3.58 -> 3.74 ms.
+constexpr uint32_t kFewMid = 100000;
 // Primitives per block of the level kernels: the fewest, as a power of two from
 // 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
 // of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
@@ -832,7 +836,6 @@ __global__ void __launch_bounds__(256) k_fpscatter(LevelArgs A, int par) {
 // would take five launches a level for them: 20,480 triangles 778 -> 700 us, 2.0 M
 // 3.66 -> 3.57 ms. What is left is the bins' instructions (runs of eight primitives
 // kept in registers were slower, 538 against 453 us for this kernel of a 2.0 M build).
-constexpr int kMidThreads = 256;
 struct MidNode {
   int32_t node, depth;
   uint32_t first, count;  // first: within the block's range
@@ -841,7 +844,7 @@ struct MidNode {
 };
 constexpr size_t kMidBytes = (6 * sizeof(float) + sizeof(uint32_t) + 2 * sizeof(uint16_t));  // per primitive
 
-template <uint32_t kMidMax>
+template <uint32_t kMidMax, int kMidThreads>
 __global__ void __launch_bounds__(kMidThreads) k_fmid(LevelArgs A) {
   after_previous();
   constexpr uint32_t kMidWords = kMidMax / 32;
@@ -1879,10 +1882,11 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
     nl = hc[kLarge + par];
   }
   if (hc[kMid] > 0) {
-    auto kernel = Lo.mid_most == 1024 ? k_fmid<1024> : k_fmid<2048>;
+    const unsigned threads = n > kFewMid ? 256 : 512;
+    auto kernel = Lo.mid_most == 1024 ? k_fmid<1024, 256> : n > kFewMid ? k_fmid<2048, 256> : k_fmid<2048, 512>;
     const size_t shared = kMidBytes * Lo.mid_most;
     FB_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared));
-    FB_TRY(launch_after(kernel, std::min(hc[kMid], Lo.max_mid), kMidThreads, shared, s, A));
+    FB_TRY(launch_after(kernel, std::min(hc[kMid], Lo.max_mid), threads, shared, s, A));
   }
   if (n >= 2) {
     // how many subtrees the warps have is known on the device
