@@ -14,10 +14,12 @@
 //
 // Phases:
 //   prep      per-primitive padded bounds (triangle::getBounds) and the root box
-//   levels    nodes with more than kWarpMax primitives, one level per round:
-//             chunks of primitives bin into shared memory and flush to
-//             the node's global bins; one warp per node picks the split; a
-//             chunk-ordered scan gives a stable partition through a scratch copy
+//   levels    nodes with more than mid_size(n) primitives, level by level: chunks of
+//             primitives bin into shared memory and flush to the node's global
+//             bins; one warp per node picks the split; a bit per primitive and
+//             chunk counts give a stable partition into the other level's buffer
+//   mid       one block splits each node down to ranges of <= kWarpMax in shared
+//             memory
 //   small     one warp splits the subtree of each node of <= kWarpMax primitives
 //             down to ranges of <= kLeafTask, bins and partition in shared memory
 //   leaf      one thread builds the whole subtree of each such range

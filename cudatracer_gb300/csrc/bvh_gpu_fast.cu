@@ -13,11 +13,13 @@
 // Phases:
 //   prep      the largest coordinate magnitude M, padded boxes and centroids,
 //             the root box
-//   levels    nodes of more than kWarpMax primitives, one level per round:
-//             per chunk of primitives the centroid bounds, then the bins
-//             (shared memory, flushed into the node's global bins); one warp per
-//             node evaluates the 45 bin splits; a chunk-ordered scan gives the
-//             stable partition through a scratch copy
+//   levels    nodes of more than mid_size(n) primitives, level by level: per chunk
+//             of primitives the bins (shared memory, flushed into the node's global
+//             bins); one warp per node evaluates the 45 bin splits; a bit per
+//             primitive and chunk counts give the stable partition into the other
+//             level's buffer, and the children's centroid bounds with it
+//   mid       one block splits each node down to ranges of at most kWarpMax in
+//             shared memory
 //   small     one warp splits each subtree of at most kWarpMax primitives by bins
 //             down to ranges of at most 16
 //   leaf      one thread builds the whole subtree of each such range (the exact

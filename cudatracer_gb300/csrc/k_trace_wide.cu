@@ -1,4 +1,4 @@
-// Ray queries on the 8-wide quantised BVH (WNode8).
+// Ray queries on the 8-wide quantised BVH (WNodeDev, the device form of WNode8).
 //
 // Boxes: the builder rounds child bounds outward so that fl(p + 2^e q)
 // contains the child; the slab test evaluates each plane as one fused

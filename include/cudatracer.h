@@ -250,7 +250,7 @@ ct_status ct_bvh_build_fast(ct_ctx* ctx, const ct_scene* scene, int32_t nthreads
  * order, byte for byte, built on the GPU (no reference counterpart; for
  * batches and served renders, whose scenes would otherwise wait on the host
  * build). Runs on `stream` (a cudaStream_t, NULL = legacy) and returns when
- * the tree is ready; reads one counter back per tree level. Fails with
+ * the tree is ready; reads counters back once per few tree levels. Fails with
  * CT_ERR_UNSUPPORTED when a padded triangle box is not finite (coordinates
  * within about 1e-5 of the float range). Exports the QUAD layout only. */
 ct_status ct_bvh_build_fast_device(ct_ctx* ctx, const ct_scene* scene, void* stream, ct_bvh** out);
@@ -268,7 +268,8 @@ ct_status ct_bvh_build_fast_device(ct_ctx* ctx, const ct_scene* scene, void* str
  * (ct_render_accumulate, ct_batch) may trace it too: there the triangle test
  * is the reference's Moller-Trumbore with tri_eps, so the hits are the quad
  * tree's up to the winner of an exact t tie. Export with CT_BVH_WIDE8_Q8
- * (80-byte nodes; prim_indices in leaf order). info.quad_node_count and
+ * (80-byte nodes; prim_indices in leaf order; the device holds 96 bytes a node,
+ * the slot codes resolved). info.quad_node_count and
  * info.quad_depth describe the wide tree. Queries on it write a 32-byte
  * settlement record per ray whose FP32 result needs FP64 re-tests; the
  * context keeps a buffer of 32 bytes per ray of its largest wide query,

@@ -37,3 +37,11 @@ def test_level_kernels_equal_the_host(gpu_ctx, ntri, kind):
         c[:, 1:] = 0.0
     v, ix = _scene(c, rng, size)
     _compare(gpu_ctx, v, ix)
+
+
+@pytest.mark.parametrize("ntri", [100001, 1000001])
+def test_mid_size_rules_equal_the_host(gpu_ctx, ntri):
+    """Past the sizes at which the blocks for mid-size nodes change (256 threads, 1,024 primitives)."""
+    rng = np.random.default_rng(ntri)
+    v, ix = _scene(rng.uniform(-1, 1, size=(ntri, 3)), rng, 0.004)
+    _compare(gpu_ctx, v, ix)
