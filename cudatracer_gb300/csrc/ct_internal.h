@@ -366,7 +366,7 @@ cudaError_t launch_fold(float4* accum, float4* frame, int n, cudaStream_t s);
 cudaError_t launch_fold_log(float4* accum, const float4* log, int entries, int stride, int n, uint32_t tag,
                             cudaStream_t s);
 
-// allocation-free frame (noalloc.cu): queues in a static device array
+// allocation-free frame (noalloc.cu): the one kernel of small frames
 uint32_t noalloc_max_pixels();
 cudaError_t noalloc_render(int device, const DevScene& sc, const DevBVH& bvh, const FrameConst& f, int max_depth,
                            int exact_math, float4* accum, uint32_t* err, cudaStream_t s);

@@ -505,15 +505,13 @@ ct_status ct_render_profile_read(ct_ctx* ctx, ct_render* r, ct_stage_times* out,
  * BVH are made once beforehand; per frame the caller passes the camera,
  * the parameters and its own accumulation buffer (DEVICE float4 per pixel,
  * 16-byte aligned, added to exactly as ct_render_accumulate adds to a
- * ct_render's buffer). The ray and shadow queues live in one static device
- * array inside the library (about 9.5 MiB, held by every GPU that loads the
- * library until the process exits), so:
+ * ct_render's buffer). A path stays in its thread's registers, so there are no
+ * queues; the library counts rays in a few static words nobody reads:
  *   - width * height must not exceed CT_NOALLOC_MAX_PIXELS, or the call fails
  *     with CT_ERR_INVALID_ARGUMENT;
- *   - every call shares that array: calls whose work overlaps on the GPU
- *     (other streams, threads or contexts on the same device) race and must
- *     be serialised by the caller;
- *   - the first call on each device looks up the array's device address
+ *   - calls whose work overlaps on the GPU must use different accumulation
+ *     buffers (each pixel is a read, an addition and a write);
+ *   - the first call on each device looks up those words' device address
  *     (cudaGetSymbolAddress); make that first call before any stream capture;
  *   - that address is kept for the life of the process. A cudaDeviceReset
  *     destroys the context it belongs to, so after a reset of a device the
