@@ -525,11 +525,16 @@ std::string to_device_layout(const HostBVH& h, const float* verts, const uint32_
     const float* p0 = verts + 3 * (size_t)idx[3 * (size_t)p];
     const float* p1 = verts + 3 * (size_t)idx[3 * (size_t)p + 1];
     const float* p2 = verts + 3 * (size_t)idx[3 * (size_t)p + 2];
+    float t[10] = {p0[0],         p0[1],         p0[2],         0.0f,          p1[0] - p0[0],
+                   p1[1] - p0[1], p1[2] - p0[2], p2[0] - p0[0], p2[1] - p0[1], p2[2] - p0[2]};
+    std::memcpy(&t[3], &p, 4);
     float* o = out.tris.data() + 4 * kTriFloat4 * (size_t)j;
-    o[0] = p0[0], o[1] = p0[1], o[2] = p0[2];
-    std::memcpy(&o[3], &p, 4);
-    o[4] = p1[0] - p0[0], o[5] = p1[1] - p0[1], o[6] = p1[2] - p0[2], o[7] = 0.0f;
-    o[8] = p2[0] - p0[0], o[9] = p2[1] - p0[1], o[10] = p2[2] - p0[2], o[11] = 0.0f;
+    std::memcpy(o, t, 24);
+    std::memcpy(o + 8, t + 6, 16);
+    if (j == 0) continue;
+    o -= 4 * kTriFloat4;  // the part of this triangle that the one before it carries
+    std::memcpy(o + 6, t + 4, 8);
+    std::memcpy(o + 12, t, 16);
   }
   return "";
 }

@@ -1222,10 +1222,16 @@ __global__ void k_tris(const float4* __restrict__ v, const uint4* __restrict__ i
   const uint32_t p = prims[j];
   const uint4 t = idx[p];
   const float4 a = v[t.x], b = v[t.y], c = v[t.z];
+  const float4 q0 = make_float4(a.x, a.y, a.z, __uint_as_float(p));
+  const float2 q1 = make_float2(__fsub_rn(b.x, a.x), __fsub_rn(b.y, a.y));
   float4* o = tris + kTriFloat4 * (size_t)j;
-  o[0] = make_float4(a.x, a.y, a.z, __uint_as_float(p));
-  o[1] = make_float4(__fsub_rn(b.x, a.x), __fsub_rn(b.y, a.y), __fsub_rn(b.z, a.z), 0.0f);
-  o[2] = make_float4(__fsub_rn(c.x, a.x), __fsub_rn(c.y, a.y), __fsub_rn(c.z, a.z), 0.0f);
+  o[0] = q0;
+  *reinterpret_cast<float2*>(o + 1) = q1;
+  o[2] = make_float4(__fsub_rn(b.z, a.z), __fsub_rn(c.x, a.x), __fsub_rn(c.y, a.y), __fsub_rn(c.z, a.z));
+  if (j == 0) return;
+  o -= kTriFloat4;  // the part of this triangle that the one before it carries
+  reinterpret_cast<float2*>(o + 1)[1] = q1;
+  o[3] = q0;
 }
 
 unsigned blocks(uint64_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }

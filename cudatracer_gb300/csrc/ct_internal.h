@@ -28,12 +28,14 @@ struct __align__(128) QNodeDev {
 static_assert(sizeof(QNodeDev) == 128, "QNodeDev is 128 bytes");
 constexpr int32_t kEmptyChild = -1;
 
-// Triangle in leaf order, 64 bytes: {p0.xyz, prim id}, {p1-p0, 0}, {p2-p0, 0},
-// unused. The edges are the exact float differences the reference forms per test
-// (src/Core/Triangle.cuh:15-16), precomputed once. 64 bytes rather than 48 keep
-// every record on a 32-byte boundary and two records within 128 bytes, so a leaf
-// step reads two with the loads of a node step (trace.cuh); the array holds one
-// record more than there are primitives, which such a step may read and ignores.
+// Triangle in leaf order: t[10] = p0.xyz, prim id, e1 = p1 - p0, e2 = p2 - p0. The
+// edges are the exact float differences the reference forms per test
+// (src/Core/Triangle.cuh:15-16), precomputed once. 64 bytes, two 32-byte sectors:
+//   {t[0..5], next[4..5]}  {t[6..9], next[0..3]}
+// where next is the triangle after it, whose t[6..9] its own record has: a leaf step
+// reads two triangles from three sectors with the loads of a node step (trace.cuh).
+// The array holds one record more than there are primitives, which such a step may
+// read and ignores.
 constexpr size_t kTriFloat4 = 4;
 inline size_t tri_array_bytes(size_t prims) { return (prims + 1) * kTriFloat4 * sizeof(float4); }
 
@@ -268,7 +270,7 @@ cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& 
 
 struct QuadNode;  // bvh_build.h
 // QuadNode -> traversal node conversion, and the leaf-ordered triangle records
-// (kTriFloat4 float4 per primitive: v0 + id, e1, e2, unused), for trees built on the device.
+// (kTriFloat4 float4 per primitive), for trees built on the device.
 cudaError_t launch_quad_to_dev(const QuadNode* quad, uint32_t nq, uint32_t leaf_shift, QNodeDev* nodes, cudaStream_t s);
 cudaError_t launch_leaf_tris(const DevScene& sc, const uint32_t* prims, uint32_t n, float4* tris, cudaStream_t s);
 

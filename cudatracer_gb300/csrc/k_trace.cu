@@ -110,7 +110,9 @@ __global__ void __launch_bounds__(kBlock) k_query(DevBVH b, QueryIO io, int n, i
 }
 
 template <bool FASTMM>
-__global__ void __launch_bounds__(kBlock) k_extend(DevBVH b, DevQueues q, int qi, float eps) {
+// 16 blocks of 64 threads: 64 registers; without the bound it takes 68 and sixteen
+// 1920x1080 frames 27.2 ms instead of 26.4
+__global__ void __launch_bounds__(kBlock, 16) k_extend(DevBVH b, DevQueues q, int qi, float eps) {
   wait_previous();
   extern __shared__ int s_stack[];
   const int n = q.counts[qi];
