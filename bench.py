@@ -408,7 +408,7 @@ def precision_soup(ctx, ntri: int = 10_000_000, nray: int = 16_000_000, sample_e
         "plain_quad_fp32": {"mrays_per_s": nray / q_trace / 1e3, "build_ms": q_ms, **against(hq, tq)},
         "plain_quad_fp32_fast_tree": {"mrays_per_s": nray / f_trace / 1e3, "build_ms": f_ms, **against(hf, tf)},
         "wide8_q8": {"mrays_per_s": nray / w_trace / 1e3, "build_ms": w_ms, "nodes": wb.info()["quad_node_count"],
-                     "node_bytes": 80, "fp64_retest_frac": st["fp64_retests"] / max(1, st["rays"]),
+                     "node_bytes": 96, "fp64_retest_frac": st["fp64_retests"] / max(1, st["rays"]),
                      "fp64_full_traversals": st["fp64_full"], **against(hw, tw)},
         "oracle_sample": f"FP64 watertight closest hit on every {sample_every}th ray ({ho.shape[0]:,} rays, "
                          f"{int((ho >= 0).sum()):,} hits)",
@@ -972,7 +972,7 @@ def run_ours(args, world, rank, local):
         "config": {"workload": WORKLOAD, "width": W, "height": H, "max_depth": DEPTH, "triangles": int(ts.ntri),
                    "frames_per_step": FRAMES_PER_STEP, "spp_per_frame": 1, "shading": "compat (reference shade)",
                    "math": args.math,
-                   "l2": "inputs larger than L2: 85-94 MB nodes + 150 MB triangles + 150 MB scene arrays + 300 MB queues",
+                   "l2": "inputs larger than L2: 85-94 MB nodes + 200 MB triangles + 150 MB scene arrays + 300 MB queues",
                    "parallelism": f"replicas x{world}"},
         "mrays_per_s": mrays, "rays_per_step": (st["extension_rays"] + st["shadow_rays"]) / args.steps,
         "stage_ms": {k: v["ms"] for k, v in prof.items()}, "stage_frames": prof_frames,
