@@ -1269,8 +1269,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_fsmall(LevelArgs A, uint32
 // One warp per node (sweep_split, kept for subtrees near the depth limit) spends
 // its shuffles, scans and latencies on a range of two as on one of sixteen, and
 // nine in ten nodes are in such ranges: k_fsmall took 4.33 ms of a 2.0
-// M-triangle build by itself; with the leaves here it takes 0.51 and this kernel
-// 0.52 ms.
+// M-triangle build by itself; with the leaves here it takes 0.49 and this kernel
+// 0.47 ms.
 // Few tasks are spread over all resident warps, a few lanes each: a warp is as slow
 // as its lanes' different paths added up (a 20,480-triangle build 1,034 us with 32
 // tasks to a warp, 991 spread).
