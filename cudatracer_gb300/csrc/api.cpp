@@ -9,6 +9,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -1004,12 +1005,17 @@ ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, ui
     if (layout != CT_BVH_WIDE8_Q8) return nodes ? CT_ERR_UNSUPPORTED : CT_OK;
     if (cudaSetDevice(bvh->device) != cudaSuccess) return CT_ERR_CUDA;
     if (nodes) {
-      std::vector<WNodeDev> dev(bvh->wdev.node_count);
-      if (cudaMemcpy(dev.data(), bvh->wdev.nodes, dev.size() * sizeof(WNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return CT_ERR_CUDA;
-      for (size_t i = 0; i < dev.size(); i++) {
-        const WNode8 w = wide_node8(dev[i]);
-        std::memcpy((char*)nodes + i * sizeof(w), &w, sizeof(w));
+      const size_t n = bvh->wdev.node_count, piece = std::min<size_t>(n, 65536);
+      std::unique_ptr<WNodeDev[]> dev(new (std::nothrow) WNodeDev[piece]);
+      if (!dev) return CT_ERR_OUT_OF_MEMORY;
+      for (size_t i0 = 0; i0 < n; i0 += piece) {
+        const size_t c = std::min(piece, n - i0);
+        if (cudaMemcpy(dev.get(), bvh->wdev.nodes + i0, c * sizeof(WNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
+          return CT_ERR_CUDA;
+        for (size_t i = 0; i < c; i++) {
+          const WNode8 w = wide_node8(dev[i]);
+          std::memcpy((char*)nodes + (i0 + i) * sizeof(w), &w, sizeof(w));
+        }
       }
     }
     if (prim_indices) {

@@ -80,11 +80,11 @@ struct QueryIO {
 
 // extend (src/CUDA/Kernel.cu:236-245): t restarts at MAX_DISTANCE every pass
 struct ExtendIO {
-  const float4* __restrict__ org;
-  const float4* __restrict__ dir;
+  const float4* org;
+  const float4* dir;
   int2* hit;
   uint32_t* err;
-  const int32_t* __restrict__ perm;
+  const int32_t* perm;
   __device__ void load(int i, float4& o, float4& d, float& t0) {
     if (perm) i = perm[i];
     o = org[i];
@@ -317,14 +317,14 @@ namespace {
 __device__ __forceinline__ int batch_lanes(int n) { return min(32, max(0, n - 1) / 1024 + 1); }
 
 struct BatchExtendIO {
-  const float4* __restrict__ org;
-  const float4* __restrict__ dir;
+  const float4* org;
+  const float4* dir;
   int2* hit;
   uint32_t* err;
   const BatchJob* jobs;
   const int32_t* bases;
   int n_jobs;
-  const int32_t* __restrict__ perm;
+  const int32_t* perm;
   __device__ void load(int i, float4& o, float4& d, float& t0, DevBVH& b, float& eps) {
     if (perm) i = perm[i];
     o = org[i];

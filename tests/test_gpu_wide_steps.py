@@ -93,3 +93,16 @@ def test_wide_steps_equal_fp64(gpu_ctx, orc, kind, ntri, n, axis, scale):
     got = wb.trace_any(O, torch.from_numpy(d3).cuda())
     gpu_ctx.check()
     assert np.array_equal(got.cpu().numpy().astype(bool), occ >= 0)
+
+
+def test_export_of_several_pieces(gpu_ctx):
+    """More than 65,536 nodes: the device's form goes back to the 80-byte one in pieces."""
+    from cudatracer_gb300 import _lib, scenes
+    from tests.test_gpu_wide import _check_structure
+    from tests.test_gpu_wide import _scene as scene_of
+
+    s = scenes.soup_scene(300000, seed=77)
+    b = scene_of(gpu_ctx, s.vertices, s.indices).build_bvh_wide()
+    nodes, prims = b.export(_lib.CT_BVH_WIDE8_Q8)
+    assert nodes.shape[0] > 65536
+    _check_structure(s.vertices, s.indices, nodes, prims)
