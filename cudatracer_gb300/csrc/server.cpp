@@ -51,9 +51,10 @@ constexpr uint32_t kIterPixels = 1u << 22;  // default pixel-samples a job may t
 // queue sets).
 constexpr int kStreams = 2;
 // Iterations of at least this many pixel-samples run a pass's connect beside the next
-// pass's extend: 640,000 (4 requests) 1.26 -> 1.09 ms; 160,000 (2 requests), whose
-// launches count, 0.63 without and 0.64 with it.
-constexpr int32_t kBesidePixels = 1 << 18;
+// pass's extend: 4 requests (renders of up to 200 pixels a side, 4 samples) 1.24 ms
+// without and 1.13 with it; smaller iterations are launch-bound and gain nothing (6 of
+// up to 128 pixels 1.53 and 1.55).
+constexpr int32_t kBesidePixels = 1 << 16;
 
 enum Kind { kRender = 0, kClosest = 1, kAny = 2 };
 enum State { kPending, kActive, kFinishing, kDone };
