@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const fl
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const unsigned own = FULL >> (32 - lanes);  // the lanes that take rays (lanes_for)
-  unsigned long long n_rays = 0;
+  uint32_t n_rays = 0;
   int rid = -1;
   bool exhausted = false;
   WRay r;
@@ -523,7 +523,13 @@ __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const fl
       }
     }
   }
-  if (stats) atomicAdd(stats + 0, n_rays);
+  // One addition per warp that had rays. With one per thread every thread of the grid
+  // went through this one address, the lanes that take no rays in a small call too:
+  // 4,096 closest-hit rays that miss the scene took 26.8 us, now 15.6; 155,648 127 and 35.
+  if (stats) {
+    n_rays = __reduce_add_sync(FULL, n_rays);
+    if (lane == 0 && n_rays) atomicAdd(stats + 0, (unsigned long long)n_rays);
+  }
 }
 
 // FP64 settlement of the records: the best FP32 hit and the candidates are
