@@ -51,8 +51,8 @@ def _cost(trees, n, any_hit):
     return tuple(_best_us(lambda: x.trace_closest(o, d, hit, t)) for x in (wide, quad))
 
 
-# 4,096: rays spread over 768 warps
-@pytest.mark.parametrize("n", [64, 4096])
+# 4,096: rays spread over 768 warps; 155,648: every lane of the chip has one
+@pytest.mark.parametrize("n", [64, 4096, 155648])
 @pytest.mark.parametrize("any_hit", [False, True])
 def test_rays_that_miss_cost_the_launches(trees, n, any_hit):
     wide, quad = _cost(trees, n, any_hit)
