@@ -1329,19 +1329,31 @@ static ct_status ensure_logs(ct_ctx* ctx, ct_render* r, int max_depth, bool* ok)
 }
 
 // Frames of at most this many pixels run as one kernel (launch_path) unless their
-// stages are profiled. Sixteen frames in a row on a 256,000-triangle terrain, depth 8,
-// one kernel against the stages: 256x192 0.80 and 1.46 ms, 320x240 1.21 and 1.64,
-// 362x362 2.07 and 2.00, 512x384 2.93 and 2.49: beyond about 130,000 pixels the
-// stages' compaction and refills pay (a frame waited for alone is faster in one
-// kernel up to 640x480: 0.48 against 0.93 ms).
-constexpr int kPathPixels = 131072;
+// stages are profiled. The stages' compaction and refills pay with the pixels, the
+// launches they need weigh the more the fewer there are, and a scene in which most paths
+// live on (a material zoo) crosses sooner than one whose paths leave early (a terrain).
+// Eight frames in a row, us, one kernel / stages:
+//                            256x256      290x290      320x320      362x362
+//   terrain, depth 8          701 / 1011   889 / 1106  1067 / 1176  1348 / 1302
+//   terrain, depth 3          318 / 311    398 / 362    475 / 433    598 / 542
+//   zoo, depth 8             1111 / 1462  1413 / 1511  1700 / 1625  2143 / 1827
+//   zoo, depth 4              664 / 500    839 / 619   1009 / 739   1274 / 926
+//   terrain, full, depth 8    576 / 961    722 / 1054   860 / 1123  1090 / 1298
+//   zoo, full, depth 5        891 / 615   1116 / 731   1347 / 866   1695 / 1067
+// One frame a pass crosses between 300x300 and 362x362, a frame that is waited for is
+// twice as fast in one kernel at all of these. The line is where they balance. Frames
+// with the reference's traversal cross later: terrain 1274 / 1502 at 362x362, zoo 976 /
+// 1041 at 256x256, 1864 / 1391 at 362x362; full shading with it, which runs one frame
+// after another, 2000 / 4748 and 1733 / 2634 for four frames at 362x362.
+constexpr int kPathPixels = 81920, kPathPixelsExact = 131072;
 
 // Issue one frame's stages on stream st into queues q.
 static ct_status emit_frame(ct_ctx* ctx, ct_render* r, const DevQueues& q, const ct_scene* scene, const ct_bvh* bvh,
                             const FrameConst& f, const ct_render_params* p, cudaStream_t st) {
   const bool fast = math_fast_traversal(p->exact_math);
   const int exact_shade = math_exact_shading(p->exact_math);
-  if (!r->profile && !bvh->wide && r->w * r->h <= kPathPixels) {
+  const int most = p->exact_math == CT_MATH_EXACT ? kPathPixelsExact : kPathPixels;
+  if (!r->profile && !bvh->wide && r->w * r->h <= most) {
     CT_CUDA(ctx, launch_path(scene->dev, bvh->dev, q, f, p->max_depth, exact_shade, fast, st));
     return CT_OK;
   }

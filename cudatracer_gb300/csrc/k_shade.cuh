@@ -38,6 +38,7 @@ constexpr float kOneOverPi = 0.318309886183790671537767526745028724f;
 constexpr float kTwoPi = 6.28318530717958647692528676655900576f;
 constexpr int kBlock = 128;
 constexpr int kPathBlock = 32;  // k_path: a block's threads share nothing, and few pixels spread over all SMs
+constexpr int kPathBlocks = 24;  // of them resident on an SM
 
 #if CT_EXACT
 // reproducible binary32 functions (portable_math.h): the oracle evaluates the
@@ -572,6 +573,13 @@ __global__ void __launch_bounds__(kBlock) k_raygen(DevQueues q, FrameConst f) {
 // fused across this point, so both ways round alike in every build.
 __device__ __forceinline__ void stored(float4& v) { asm volatile("" : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)); }
 
+// shade_full as a function of its own, so that in the build with FMA contraction it is
+// contracted as k_shade's copy is (inlined beside the traversal it was not).
+__device__ __noinline__ void shade_full_call(const DevScene* sc, const DevQueues* q, const FrameConst* f, float4 o4,
+                                             float4 d4, float4 t4, int2 h, uint32_t path_length, Emit* e) {
+  shade_full(*sc, *q, *f, o4, d4, t4, h, path_length, *e);
+}
+
 // A whole frame in one kernel, one path per thread: ray generation, then up to
 // max_depth x (closest hit, shade, shadow any hit). For frames of few pixels,
 // whose wavefront stages (1 + 3 max_depth launches) are a few warps each: what
@@ -581,15 +589,7 @@ __device__ __forceinline__ void stored(float4& v) { asm volatile("" : "+f"(v.x),
 // contributions are the same bits, added to q.accum (or logged) per pixel in
 // the same order. A 64x48, depth-5 frame takes 99 us when waited for and 50 us
 // among others (the host calls), with the stages 343 and 98 us.
-// shade_full as a function of its own: k_path then holds 93 registers instead of
-// 124 (362x362 frames 191 -> 174 us), and in the build with FMA contraction it is
-// contracted as k_shade's copy is (inlined beside the traversal it was not).
-__device__ __noinline__ void shade_full_call(const DevScene* sc, const DevQueues* q, const FrameConst* f, float4 o4,
-                                             float4 d4, float4 t4, int2 h, uint32_t path_length, Emit* e) {
-  shade_full(*sc, *q, *f, o4, d4, t4, h, path_length, *e);
-}
-
-template <bool FASTMM>
+template <bool FASTMM, bool FULL>
 __device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b, DevQueues& q, const FrameConst& f,
                                             int max_depth, int lanes) {
   extern __shared__ int s_stack[];
@@ -619,7 +619,7 @@ __device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b,
       }
       q.log_entry = 2u * (uint32_t)pass;
       const uint32_t path_length = pass == 0 ? 0u : (uint32_t)pass + 1u;  // Kernel.cu:306, 330
-      if (f.shading_mode == CT_MODE_FULL)
+      if (FULL)
         shade_full_call(&sc, &q, &f, o, d, t, h, path_length, &e);
       else
         shade_compat(sc, q, f, o, d, t, h, path_length, e);
@@ -654,15 +654,32 @@ __device__ __forceinline__ void trace_paths(const DevScene& sc, const DevBVH& b,
     }
   }
 }
-__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth,
-                                                     int lanes) {
-  trace_paths<true>(sc, b, q, f, max_depth, lanes);
+// One kernel per shading mode: a kernel that could call either held 121 registers and
+// 384 bytes of stack for compat frames too. kPathBlocks blocks on an SM (80 registers,
+// some spills) instead of the 16 that 115 registers allow: eight 362x362 frames 1.59 ->
+// 1.35 ms on a 522,000-triangle terrain, 1.48 -> 1.27 on a material zoo; 20 blocks 1.42
+// and 1.33, 32 blocks 1.33 and 1.29.
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+           const __grid_constant__ FrameConst f, int max_depth, int lanes) {
+  trace_paths<true, false>(sc, b, q, f, max_depth, lanes);
+}
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_full(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+                const __grid_constant__ FrameConst f, int max_depth, int lanes) {
+  trace_paths<true, true>(sc, b, q, f, max_depth, lanes);
 }
 #if CT_EXACT
 // with the reference's traversal (CT_MATH_EXACT)
-__global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
-                                                         int max_depth, int lanes) {
-  trace_paths<false>(sc, b, q, f, max_depth, lanes);
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_ref(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+               const __grid_constant__ FrameConst f, int max_depth, int lanes) {
+  trace_paths<false, false>(sc, b, q, f, max_depth, lanes);
+}
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_ref_full(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+                    const __grid_constant__ FrameConst f, int max_depth, int lanes) {
+  trace_paths<false, true>(sc, b, q, f, max_depth, lanes);
 }
 #endif
 

@@ -6,16 +6,24 @@
 
 namespace ct {
 namespace exact {
-constexpr int kPathBlock = fast::kPathBlock;
+constexpr int kPathBlock = fast::kPathBlock, kPathBlocks = fast::kPathBlocks;
 __global__ void __launch_bounds__(128) k_shade(DevScene sc, DevQueues q, FrameConst f, int cur, uint32_t path_length);
 __global__ void __launch_bounds__(128) k_raygen(DevQueues q, FrameConst f);
 __global__ void __launch_bounds__(128) k_batch_raygen(DevBatch bt, DevQueues q);
 __global__ void __launch_bounds__(128) k_batch_shade(DevBatch bt, DevQueues q, int cur, uint32_t path_length, int pass);
 __global__ void k_batch_advance(DevBatch bt, DevQueues q);
-__global__ void __launch_bounds__(kPathBlock) k_path(DevScene sc, DevBVH b, DevQueues q, FrameConst f, int max_depth,
-                                                     int lanes);
-__global__ void __launch_bounds__(kPathBlock) k_path_ref(DevScene sc, DevBVH b, DevQueues q, FrameConst f,
-                                                         int max_depth, int lanes);
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+           const __grid_constant__ FrameConst f, int max_depth, int lanes);
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_full(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+                const __grid_constant__ FrameConst f, int max_depth, int lanes);
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_ref(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+               const __grid_constant__ FrameConst f, int max_depth, int lanes);
+__global__ void __launch_bounds__(kPathBlock, kPathBlocks)
+    k_path_ref_full(const __grid_constant__ DevScene sc, const __grid_constant__ DevBVH b, DevQueues q,
+                    const __grid_constant__ FrameConst f, int max_depth, int lanes);
 }  // namespace exact
 
 namespace {
@@ -91,6 +99,8 @@ cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact_mat
 cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
                         int exact_math, bool fast_traversal, cudaStream_t s) {
   auto kernel = !exact_math ? fast::k_path : (fast_traversal ? exact::k_path : exact::k_path_ref);
+  if (f.shading_mode == CT_MODE_FULL)
+    kernel = !exact_math ? fast::k_path_full : (fast_traversal ? exact::k_path_full : exact::k_path_ref_full);
   const size_t smem = (size_t)b.stack_entries * fast::kPathBlock * sizeof(int);  // at most 256 entries: 32 KB
   const int npix = f.width * f.height, lanes = lanes_for((uint32_t)npix);
   kernel<<<(npix + lanes - 1) / lanes, fast::kPathBlock, smem, s>>>(sc, b, q, f, max_depth, lanes);
