@@ -552,7 +552,6 @@ __device__ __forceinline__ void primary_ray(const FrameConst& f, int i, float4& 
 }
 
 __global__ void __launch_bounds__(kBlock) k_raygen(DevQueues q, FrameConst f) {
-  wait_previous();
   const int npix = f.width * f.height;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     q.counts[0] = npix;
@@ -687,7 +686,6 @@ __global__ void __launch_bounds__(kPathBlock, kPathBlocks)
 
 // Primary rays of the jobs that still take samples, appended to queue 0.
 __global__ void __launch_bounds__(kBlock) k_batch_raygen(DevBatch bt, DevQueues q) {
-  wait_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) q.counts[4] = 0;
   for (int base = blockIdx.x * kBlock + (threadIdx.x & ~31); base < bt.total_pix; base += gridDim.x * kBlock) {
     const int g = base + (threadIdx.x & 31);

@@ -93,7 +93,8 @@ cudaError_t launch_fold(float4* accum, float4* frame, int n, cudaStream_t s) {
 cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact_math, cudaStream_t s) {
   const int npix = f.width * f.height;
   auto kernel = exact_math ? exact::k_raygen : fast::k_raygen;
-  return launch_after(kernel, fill_grid(kernel, npix), kBlock, 0, s, q, f);
+  // ordinary: a slot's first stage comes after a wait for another stream
+  return launch_after_if(false, kernel, fill_grid(kernel, npix), kBlock, 0, s, q, f);
 }
 
 cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
@@ -123,7 +124,8 @@ cudaError_t launch_present(const float4* accum, float4* out, int n, float sample
 
 cudaError_t launch_batch_raygen(const DevBatch& b, const DevQueues& q, int exact, cudaStream_t s) {
   auto kernel = exact ? exact::k_batch_raygen : fast::k_batch_raygen;
-  return launch_after(kernel, fill_grid(kernel, b.total_pix), kBlock, 0, s, b, q);
+  // ordinary: it comes after the job table's copy and waits for other streams
+  return launch_after_if(false, kernel, fill_grid(kernel, b.total_pix), kBlock, 0, s, b, q);
 }
 
 cudaError_t launch_batch_shade(const DevBatch& b, const DevQueues& q, int queue, uint32_t path_length, int pass,

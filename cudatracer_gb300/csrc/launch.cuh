@@ -27,7 +27,8 @@ __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// chained false: an ordinary launch (a kernel that also waits for another stream).
+// chained false: an ordinary launch. A kernel whose stream waits for an event of another
+// stream right before it is launched so (ray generation, a shade that joins a connect).
 template <class... P, class... A>
 inline cudaError_t launch_after_if(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                                    cudaStream_t s, A... args) {
