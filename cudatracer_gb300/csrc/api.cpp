@@ -21,6 +21,21 @@
 
 using namespace ct;
 
+// Memory of device builds: their scratch and the trees themselves come from a pool
+// of the context, kept between builds (the pool orders its reuse by stream). A build
+// allocates once or twice whatever its size: with cudaMalloc, cudaMallocHost and their
+// frees (55 to 250 us each) a 20,480-triangle build spent 770 of its 1,330 us there.
+// A tree holds its pool: it gives its memory back there whichever context it is
+// destroyed through, and a pool lives as long as its last tree.
+struct BuildPool {
+  cudaMemPool_t pool = nullptr;
+  std::mutex mu;
+  uint64_t live = 0;  // bytes of it in use (guarded by mu)
+  ~BuildPool() {
+    if (pool) cudaMemPoolDestroy(pool);
+  }
+};
+
 struct ct_ctx {
   int device = 0;
   mutable std::mutex mu;
@@ -32,14 +47,8 @@ struct ct_ctx {
   // settlement records of wide-tree queries (kWideRecordBytes per ray), grown on demand
   void* d_recs = nullptr;
   size_t recs_bytes = 0;
-  // Memory of device builds: their scratch and the trees themselves come from a
-  // pool of this context, and each build reads its counters back through a
-  // pinned block, both kept between builds (guarded by mu; the pool orders its
-  // reuse by stream). A build allocates once or twice whatever its size: with
-  // cudaMalloc, cudaMallocHost and their frees (55 to 250 us each) a 20,480-
-  // triangle build spent 770 of its 1,330 us there.
-  cudaMemPool_t pool = nullptr;
-  uint64_t pool_live = 0;  // bytes of it in use
+  std::shared_ptr<BuildPool> pool;  // made by the first device build (guarded by mu)
+  // each build reads its counters back through a pinned block (guarded by mu)
   std::vector<uint32_t*> pinned;  // free blocks of kPinnedBytes
 };
 
@@ -79,7 +88,7 @@ ct_status cuda_fail(ct_ctx* ctx, cudaError_t e, const char* what) {
 // Gives the idle part of the build pool back to the device.
 void trim_pool(ct_ctx* ctx) {
   std::lock_guard<std::mutex> g(ctx->mu);
-  if (ctx->pool) cudaMemPoolTrimTo(ctx->pool, 0);
+  if (ctx->pool) cudaMemPoolTrimTo(ctx->pool->pool, 0);
 }
 
 ct_status over_budget(ct_ctx* ctx, size_t bytes) {
@@ -117,35 +126,37 @@ void free_all(ct_ctx* ctx, Allocs& a) {
   a.list.clear();
 }
 
-// Memory of a device build from the context's pool, ordered on the build's stream.
-ct_status pool_alloc(ct_ctx* ctx, Allocs& a, void** p, size_t bytes, cudaStream_t st) {
+// The context's build pool, made on first use.
+ct_status build_pool(ct_ctx* ctx, std::shared_ptr<BuildPool>& out) {
+  std::lock_guard<std::mutex> g(ctx->mu);
+  if (!ctx->pool) {
+    auto p = std::make_shared<BuildPool>();
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaError_t e = cudaMemPoolCreate(&p->pool, &props);
+    uint64_t keep = kPoolKeepBytes;  // pool_free keeps it at the live bytes more than this
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      ctx->err = std::string("build pool: ") + cudaGetErrorString(e);
+      return e == cudaErrorMemoryAllocation ? CT_ERR_OUT_OF_MEMORY : CT_ERR_CUDA;
+    }
+    ctx->pool = std::move(p);
+  }
+  out = ctx->pool;
+  return CT_OK;
+}
+
+// Memory of a device build, ordered on the build's stream.
+ct_status pool_alloc(ct_ctx* ctx, BuildPool& pool, Allocs& a, void** p, size_t bytes, cudaStream_t st) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
   bytes = (bytes + 255) & ~(size_t)255;
   if (ctx->budget && ctx->bytes.load() + bytes > ctx->budget) return over_budget(ctx, bytes);
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> g(ctx->mu);
-    if (!ctx->pool) {
-      cudaMemPoolProps props;
-      std::memset(&props, 0, sizeof(props));
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = ctx->device;
-      cudaError_t e = cudaMemPoolCreate(&ctx->pool, &props);
-      uint64_t keep = kPoolKeepBytes;  // pool_free keeps it at the live bytes more than this
-      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
-        ctx->pool = nullptr;
-        ctx->err = std::string("build pool: ") + cudaGetErrorString(e);
-        return e == cudaErrorMemoryAllocation ? CT_ERR_OUT_OF_MEMORY : CT_ERR_CUDA;
-      }
-    }
-    pool = ctx->pool;
-  }
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool.pool, st);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -153,15 +164,15 @@ ct_status pool_alloc(ct_ctx* ctx, Allocs& a, void** p, size_t bytes, cudaStream_
   }
   ctx->bytes += bytes;
   {
-    std::lock_guard<std::mutex> g(ctx->mu);
-    ctx->pool_live += bytes;
+    std::lock_guard<std::mutex> g(pool.mu);
+    pool.live += bytes;
   }
   a.list.push_back({*p, bytes});
   return CT_OK;
 }
 
 // Frees pool memory in stream order: whoever used it has finished or used it on `st`.
-void pool_free(ct_ctx* ctx, Allocs& a, cudaStream_t st) {
+void pool_free(ct_ctx* ctx, BuildPool& pool, Allocs& a, cudaStream_t st) {
   if (a.list.empty()) return;
   uint64_t freed = 0;
   for (auto& p : a.list) {
@@ -171,14 +182,14 @@ void pool_free(ct_ctx* ctx, Allocs& a, cudaStream_t st) {
   }
   a.list.clear();
   {
-    std::lock_guard<std::mutex> g(ctx->mu);
-    ctx->pool_live -= std::min(freed, ctx->pool_live);
-    uint64_t keep = ctx->pool_live + kPoolKeepBytes;
-    if (ctx->pool) cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    std::lock_guard<std::mutex> g(pool.mu);
+    pool.live -= freed;
+    uint64_t keep = pool.live + kPoolKeepBytes;
+    cudaMemPoolSetAttribute(pool.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   if (ctx->budget) {
     cudaStreamSynchronize(st);
-    trim_pool(ctx);
+    cudaMemPoolTrimTo(pool.pool, 0);
   }
 }
 
@@ -254,6 +265,7 @@ struct ct_bvh {
   // device-built trees keep the reference-layout quad nodes and the primitive
   // order on the device only (exported on request)
   bool device_built = false;
+  std::shared_ptr<BuildPool> pool;  // what allocs came from
   int device = 0;
   void* d_quad = nullptr;
   uint32_t* d_prims = nullptr;
@@ -488,7 +500,6 @@ ct_status ct_ctx_destroy(ct_ctx* ctx) {
   cudaFree(ctx->d_error);
   if (ctx->d_recs) cudaFree(ctx->d_recs);
   for (uint32_t* h : ctx->pinned) cudaFreeHost(h);
-  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);  // a tree that outlives its context keeps its memory
   delete ctx;
   return CT_OK;
 }
@@ -735,20 +746,23 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   Allocs scratch_allocs;
   void* scratch = nullptr;
   uint32_t* hc = nullptr;
+  std::shared_ptr<BuildPool> pool;
+  if ((s = build_pool(ctx, pool)) != CT_OK) return s;
   auto* b = new ct_bvh();
+  b->pool = std::move(pool);
   auto cleanup = [&](ct_status r) {
     if (st) cudaStreamSynchronize(st);
     else cudaDeviceSynchronize();
-    pool_free(ctx, scratch_allocs, st);
+    pool_free(ctx, *b->pool, scratch_allocs, st);
     give_pinned(ctx, hc);
     if (r != CT_OK) {
-      pool_free(ctx, b->allocs, st);
+      pool_free(ctx, *b->pool, b->allocs, st);
       delete b;
     }
     return r;
   };
   const size_t scratch_bytes = fast ? gpu_fbvh_scratch_bytes(n) : gpu_bvh_scratch_bytes(n);
-  if ((s = pool_alloc(ctx, scratch_allocs, &scratch, scratch_bytes, st)) != CT_OK) return cleanup(s);
+  if ((s = pool_alloc(ctx, *b->pool, scratch_allocs, &scratch, scratch_bytes, st)) != CT_OK) return cleanup(s);
   cudaError_t e = cudaSuccess;
   if (!(hc = take_pinned(ctx, e))) return cleanup(cuda_fail(ctx, e, "cudaMallocHost"));
   GpuBvhResult r;
@@ -773,7 +787,7 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   const size_t quad_bytes = al((size_t)r.quad_nodes * sizeof(QuadNode));
   const size_t node_bytes = al((size_t)r.quad_nodes * sizeof(QNodeDev)), tri_bytes = al(tri_array_bytes(n));
   void* quad = nullptr;
-  if ((s = pool_alloc(ctx, b->allocs, &quad, quad_bytes + node_bytes + tri_bytes + al((size_t)n * 4), st)) != CT_OK)
+  if ((s = pool_alloc(ctx, *b->pool, b->allocs, &quad, quad_bytes + node_bytes + tri_bytes + al((size_t)n * 4), st)) != CT_OK)
     return cleanup(s);
   void* nodes = (char*)quad + quad_bytes;
   void* tris = (char*)nodes + node_bytes;
@@ -845,21 +859,25 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   void* scratch = nullptr;
   void* scratch2 = nullptr;
   uint32_t* hc = nullptr;
+  std::shared_ptr<BuildPool> pool;
+  if ((s = build_pool(ctx, pool)) != CT_OK) return s;
   auto* b = new ct_bvh();
+  b->pool = std::move(pool);
   auto cleanup = [&](ct_status r) {
     if (st) cudaStreamSynchronize(st);
     else cudaDeviceSynchronize();
-    pool_free(ctx, scratch_allocs, st);
+    pool_free(ctx, *b->pool, scratch_allocs, st);
     give_pinned(ctx, hc);
     if (r != CT_OK) {
-      pool_free(ctx, b->allocs, st);
+      pool_free(ctx, *b->pool, b->allocs, st);
       delete b;
     }
     return r;
   };
   // the binary tree of ct_bvh_build_fast's rules over exact triangle bounds, and
   // the cost table of the 8-wide collapse
-  if ((s = pool_alloc(ctx, scratch_allocs, &scratch, gpu_fbvh_scratch_bytes(n, 1), st)) != CT_OK) return cleanup(s);
+  if ((s = pool_alloc(ctx, *b->pool, scratch_allocs, &scratch, gpu_fbvh_scratch_bytes(n, 1), st)) != CT_OK)
+    return cleanup(s);
   cudaError_t e = cudaSuccess;
   if (!(hc = take_pinned(ctx, e))) return cleanup(cuda_fail(ctx, e, "cudaMallocHost"));
   GpuBvhResult r;
@@ -878,11 +896,11 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   void* tris = nullptr;
   void* stats = nullptr;
   const size_t tri_bytes = ((size_t)n * 3 * sizeof(float4) + 255) & ~(size_t)255;
-  if ((s = pool_alloc(ctx, b->allocs, &tris, tri_bytes + 256, st)) != CT_OK) return cleanup(s);
+  if ((s = pool_alloc(ctx, *b->pool, b->allocs, &tris, tri_bytes + 256, st)) != CT_OK) return cleanup(s);
   stats = (char*)tris + tri_bytes;
   e = cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "cudaMemsetAsync"));
-  if ((s = pool_alloc(ctx, scratch_allocs, &scratch2, gpu_wbvh_scratch_bytes(r.binary_nodes), st)) != CT_OK)
+  if ((s = pool_alloc(ctx, *b->pool, scratch_allocs, &scratch2, gpu_wbvh_scratch_bytes(r.binary_nodes), st)) != CT_OK)
     return cleanup(s);
   uint32_t nw = 0, depth = 0, werr = 0;
   e = gpu_wbvh_collapse(scene->dev, barena, bprims, wcost, scratch2, r.binary_nodes, (float4*)tris, hc, st, &nw, &depth,
@@ -891,7 +909,7 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   if (werr) return cleanup(fail(ctx, CT_ERR_UNSUPPORTED, "wide BVH collapse failed (code " + std::to_string(werr) +
                                                               "): a leaf needs more than 8 slots or a box did not quantise"));
   void* nodes = nullptr;
-  if ((s = pool_alloc(ctx, b->allocs, &nodes, (size_t)nw * sizeof(WNodeDev), st)) != CT_OK) return cleanup(s);
+  if ((s = pool_alloc(ctx, *b->pool, b->allocs, &nodes, (size_t)nw * sizeof(WNodeDev), st)) != CT_OK) return cleanup(s);
   e = gpu_wbvh_copy_nodes(scratch2, r.binary_nodes, (WNodeDev*)nodes, nw, st);
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "wide BVH copy"));
   e = st ? cudaStreamSynchronize(st) : cudaDeviceSynchronize();
@@ -1057,7 +1075,7 @@ ct_status ct_bvh_destroy(ct_ctx* ctx, ct_bvh* bvh) {
   if (bvh->device_built) {
     // pool memory, used on any stream until now: what cudaFree's own wait did
     cudaDeviceSynchronize();
-    pool_free(ctx, bvh->allocs, 0);
+    pool_free(ctx, *bvh->pool, bvh->allocs, 0);
   } else {
     free_all(ctx, bvh->allocs);
   }
