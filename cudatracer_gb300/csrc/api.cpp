@@ -29,10 +29,12 @@ using namespace ct;
 // destroyed through, and a pool lives as long as its last tree.
 struct BuildPool {
   cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;  // destroyed trees' memory is freed on it
   std::mutex mu;
   uint64_t live = 0;  // bytes of it in use (guarded by mu)
   ~BuildPool() {
     if (pool) cudaMemPoolDestroy(pool);
+    if (st) cudaStreamDestroy(st);
   }
 };
 
@@ -139,6 +141,7 @@ ct_status build_pool(ct_ctx* ctx, std::shared_ptr<BuildPool>& out) {
     cudaError_t e = cudaMemPoolCreate(&p->pool, &props);
     uint64_t keep = kPoolKeepBytes;  // pool_free keeps it at the live bytes more than this
     if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
       cudaGetLastError();
       ctx->err = std::string("build pool: ") + cudaGetErrorString(e);
@@ -191,6 +194,26 @@ void pool_free(ct_ctx* ctx, BuildPool& pool, Allocs& a, cudaStream_t st) {
     cudaStreamSynchronize(st);
     cudaMemPoolTrimTo(pool.pool, 0);
   }
+}
+
+// Gives a device-built tree's memory back. The tree may have been used on any stream
+// until now, so the device is waited for first: by cudaFree of a small block of the
+// tree's own, which waits for the whole device, takes 2 us on an idle one and, other
+// than cudaDeviceSynchronize and work on the legacy stream, may be called while some
+// stream captures a graph (relaxed, or in another thread). Where cudaFree is refused
+// all the same (a capture in global mode) nothing has waited, and the memory is not
+// given to others while the context lives.
+void free_tree(ct_ctx* ctx, BuildPool& pool, Allocs& fence, Allocs& a) {
+  bool waited = true;
+  for (auto& p : fence.list) {
+    waited = cudaFree(p.first) == cudaSuccess && waited;
+    ctx->bytes -= p.second;
+  }
+  fence.list.clear();
+  if (waited) return pool_free(ctx, pool, a, pool.st);
+  cudaGetLastError();
+  for (auto& p : a.list) ctx->bytes -= p.second;
+  a.list.clear();
 }
 
 // A pinned block of kPinnedBytes for one build's counters (nullptr: none to be had).
@@ -266,6 +289,7 @@ struct ct_bvh {
   // order on the device only (exported on request)
   bool device_built = false;
   std::shared_ptr<BuildPool> pool;  // what allocs came from
+  Allocs fence;                     // see free_tree
   int device = 0;
   void* d_quad = nullptr;
   uint32_t* d_prims = nullptr;
@@ -756,13 +780,15 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
     pool_free(ctx, *b->pool, scratch_allocs, st);
     give_pinned(ctx, hc);
     if (r != CT_OK) {
-      pool_free(ctx, *b->pool, b->allocs, st);
+      free_tree(ctx, *b->pool, b->fence, b->allocs);
       delete b;
     }
     return r;
   };
   const size_t scratch_bytes = fast ? gpu_fbvh_scratch_bytes(n) : gpu_bvh_scratch_bytes(n);
   if ((s = pool_alloc(ctx, *b->pool, scratch_allocs, &scratch, scratch_bytes, st)) != CT_OK) return cleanup(s);
+  void* fence = nullptr;
+  if ((s = dev_alloc(ctx, b->fence, &fence, 256)) != CT_OK) return cleanup(s);
   cudaError_t e = cudaSuccess;
   if (!(hc = take_pinned(ctx, e))) return cleanup(cuda_fail(ctx, e, "cudaMallocHost"));
   GpuBvhResult r;
@@ -826,7 +852,7 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   i.build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   i.collapse_ms = std::chrono::duration<double, std::milli>(t2 - t1).count();
   i.upload_ms = 0.0;
-  uint64_t bytes = 0;
+  uint64_t bytes = 256;  // the fence block
   for (auto& p : b->allocs.list) bytes += p.second;
   i.device_bytes = bytes;
   *out = b;
@@ -869,7 +895,7 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
     pool_free(ctx, *b->pool, scratch_allocs, st);
     give_pinned(ctx, hc);
     if (r != CT_OK) {
-      pool_free(ctx, *b->pool, b->allocs, st);
+      free_tree(ctx, *b->pool, b->fence, b->allocs);
       delete b;
     }
     return r;
@@ -878,6 +904,8 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   // the cost table of the 8-wide collapse
   if ((s = pool_alloc(ctx, *b->pool, scratch_allocs, &scratch, gpu_fbvh_scratch_bytes(n, 1), st)) != CT_OK)
     return cleanup(s);
+  void* fence = nullptr;
+  if ((s = dev_alloc(ctx, b->fence, &fence, 256)) != CT_OK) return cleanup(s);
   cudaError_t e = cudaSuccess;
   if (!(hc = take_pinned(ctx, e))) return cleanup(cuda_fail(ctx, e, "cudaMallocHost"));
   GpuBvhResult r;
@@ -936,7 +964,7 @@ ct_status ct_bvh_build_wide(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   i.build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
   i.collapse_ms = std::chrono::duration<double, std::milli>(t2 - t1).count();
   i.upload_ms = 0.0;
-  uint64_t bytes = 0;
+  uint64_t bytes = 256;  // the fence block
   for (auto& p : b->allocs.list) bytes += p.second;
   i.device_bytes = bytes;
   *out = b;
@@ -1073,9 +1101,7 @@ ct_status ct_bvh_destroy(ct_ctx* ctx, ct_bvh* bvh) {
   if (!ctx || !bvh) return CT_ERR_INVALID_ARGUMENT;
   set_device(ctx);
   if (bvh->device_built) {
-    // pool memory, used on any stream until now: what cudaFree's own wait did
-    cudaDeviceSynchronize();
-    pool_free(ctx, *bvh->pool, bvh->allocs, 0);
+    free_tree(ctx, *bvh->pool, bvh->fence, bvh->allocs);
   } else {
     free_all(ctx, bvh->allocs);
   }

@@ -43,3 +43,86 @@ def test_trees_destroyed_through_another_context_leave_the_bound(lib):
     sc.close()
     b.close()
     a.close()
+
+
+KINDS = ("build_bvh_device", "build_bvh_fast_device", "build_bvh_wide")
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("mode", ["relaxed", "thread_local"])
+def test_destroy_while_a_graph_is_captured(gpu_ctx, kind, mode):
+    """As for any cudaFree: in relaxed capture, or in another thread than a thread-local one."""
+    import threading
+
+    import torch
+
+    sc = _scene(gpu_ctx, 3000)
+    used = gpu_ctx.device_bytes
+    tree = getattr(sc, kind)()
+    x = torch.zeros(8, device="cuda")
+    st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        g.capture_begin(capture_error_mode=mode)
+        x.add_(1)
+        if mode == "relaxed":
+            tree.close()
+        else:
+            t = threading.Thread(target=tree.close)
+            t.start()
+            t.join()
+        x.add_(1)
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8 and gpu_ctx.device_bytes == used
+    sc.close()
+
+
+@pytest.mark.parametrize("kind", ["build_bvh_device", "build_bvh_fast_device"])
+def test_trees_closed_right_behind_their_queries(gpu_ctx, kind):
+    """Queries in flight on a non-blocking stream when their tree is destroyed, while other
+    threads build and destroy trees in the memory that it gives back."""
+    import threading
+
+    import torch
+
+    from cudatracer_gb300 import scenes
+
+    o, d = (torch.from_numpy(x).cuda() for x in scenes.incoherent_rays(400000, seed=3))
+    mine, other = _scene(gpu_ctx, 60000), _scene(gpu_ctx, 50000, 2)
+    tree = getattr(mine, kind)()
+    want = [x.cpu().numpy() for x in tree.trace_closest(o, d, tri_eps=1e-12)]
+    tree.close()
+    stop, bad = threading.Event(), []
+
+    def work():
+        s = torch.cuda.Stream()
+        try:
+            while not stop.is_set():
+                other.build_bvh_fast_device(s).close()
+                other.build_bvh_device(s).close()
+        except Exception as e:  # noqa: BLE001
+            bad.append(repr(e))
+
+    ts = [threading.Thread(target=work) for _ in range(3)]
+    for t in ts:
+        t.start()
+    st = torch.cuda.Stream()
+    outs = [(torch.empty(len(o), dtype=torch.int32, device="cuda"), torch.empty(len(o), device="cuda"))
+            for _ in range(8)]
+    torch.cuda.synchronize()
+    for hit, t in outs:
+        tree = getattr(mine, kind)(st)
+        tree.trace_closest(o, d, hit, t, tri_eps=1e-12, stream=st)
+        tree.close()
+    stop.set()
+    for t in ts:
+        t.join()
+    torch.cuda.synchronize()
+    gpu_ctx.check()
+    assert not bad
+    for hit, t in outs:
+        assert np.array_equal(hit.cpu().numpy(), want[0]) and np.array_equal(t.cpu().numpy(), want[1])
+    mine.close()
+    other.close()
