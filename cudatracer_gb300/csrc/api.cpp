@@ -87,10 +87,14 @@ ct_status cuda_fail(ct_ctx* ctx, cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
   } while (0)
 
-// Gives the idle part of the build pool back to the device.
+// Gives the idle part of the build pool back to the device, destroyed trees' memory
+// included. (An allocation of the process that finds no room has it without this: the
+// driver releases idle pool memory before it fails.)
 void trim_pool(ct_ctx* ctx) {
   std::lock_guard<std::mutex> g(ctx->mu);
-  if (ctx->pool) cudaMemPoolTrimTo(ctx->pool->pool, 0);
+  if (!ctx->pool) return;
+  cudaStreamSynchronize(ctx->pool->st);
+  cudaMemPoolTrimTo(ctx->pool->pool, 0);
 }
 
 ct_status over_budget(ct_ctx* ctx, size_t bytes) {
@@ -105,11 +109,6 @@ ct_status dev_alloc(ct_ctx* ctx, Allocs& a, void** p, size_t bytes) {
   bytes = (bytes + 255) & ~(size_t)255;
   if (ctx->budget && ctx->bytes.load() + bytes > ctx->budget) return over_budget(ctx, bytes);
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation) {  // again without what the build pool keeps
-    cudaGetLastError();
-    trim_pool(ctx);
-    e = cudaMalloc(p, bytes);
-  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -539,7 +538,7 @@ const char* ct_last_error(const ct_ctx* ctx) {
 ct_status ct_ctx_set_memory_budget(ct_ctx* ctx, uint64_t bytes) {
   if (!ctx) return CT_ERR_INVALID_ARGUMENT;
   ctx->budget = bytes;
-  if (bytes) trim_pool(ctx);  // a budgeted context keeps no idle memory
+  trim_pool(ctx);
   return CT_OK;
 }
 
@@ -1206,11 +1205,6 @@ static ct_status ensure_wide_records(ct_ctx* ctx, uint32_t n) {
     ctx->d_recs = nullptr, ctx->recs_bytes = 0;
   }
   cudaError_t e = cudaMalloc(&ctx->d_recs, need);
-  if (e == cudaErrorMemoryAllocation) {  // again without what the build pool keeps
-    cudaGetLastError();
-    trim_pool(ctx);
-    e = cudaMalloc(&ctx->d_recs, need);
-  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     ctx->d_recs = nullptr;

@@ -191,8 +191,14 @@ void ct_render_params_default(ct_render_params* p);
 ct_status ct_ctx_create(int32_t device, ct_ctx** out);
 ct_status ct_ctx_destroy(ct_ctx* ctx);
 const char* ct_last_error(const ct_ctx* ctx);
-/* Cap on device bytes this context may hold (0 = unlimited); creations beyond it fail with CT_ERR_OUT_OF_MEMORY. */
+/* Cap on device bytes this context may hold (0 = unlimited); creations beyond it fail with CT_ERR_OUT_OF_MEMORY.
+ * Device builds (ct_bvh_build_device, _fast_device, _wide) take their scratch and their
+ * trees from a pool of the context, which keeps up to 1 GiB of freed memory beyond what
+ * live trees hold, for the next build (an allocation of the process that finds no room
+ * gets it from the driver; other processes see it as used). A context with a budget
+ * keeps nothing, and this call gives back what is kept, with bytes 0 too. */
 ct_status ct_ctx_set_memory_budget(ct_ctx* ctx, uint64_t bytes);
+/* Device bytes in use, without what the build pool keeps. */
 uint64_t ct_ctx_device_bytes(const ct_ctx* ctx);
 /* Synchronises `stream` and reports device-side errors raised since the last
  * call (stack overflow, bounded-wait timeouts), then clears them. */

@@ -126,3 +126,14 @@ def test_trees_closed_right_behind_their_queries(gpu_ctx, kind):
         assert np.array_equal(hit.cpu().numpy(), want[0]) and np.array_equal(t.cpu().numpy(), want[1])
     mine.close()
     other.close()
+
+
+def test_a_budget_of_zero_gives_back_what_is_kept(gpu_ctx):
+    sc = _scene(gpu_ctx, 1000000)
+    gpu_ctx.set_memory_budget(0)
+    before = _free()
+    sc.build_bvh_device().close()
+    assert before - _free() > 128 << 20
+    gpu_ctx.set_memory_budget(0)
+    assert before - _free() < 64 << 20
+    sc.close()
