@@ -319,6 +319,7 @@ cudaError_t ct_server::render_iteration(std::vector<Request*>& finished) {
     if (e == cudaSuccess) e = launch_batch_connect(b, q, fast, 128, fs[slot], false);
     if (e == cudaSuccess) e = cudaEventRecord(fork_join[slot], fs[slot]);
   }
+  if (e != cudaSuccess && beside) cudaStreamSynchronize(fs[slot]);  // st may not have joined it: it reads this slot's table
   if (e == cudaSuccess) e = cudaEventRecord(table_ev[slot], st);
   slot = (slot + 1) % kStreams;
   std::vector<Request*> keep;
