@@ -106,7 +106,7 @@ template <bool ANY>
 __global__ void __launch_bounds__(kBlock) k_query(DevBVH b, QueryIO io, int n, int* cursor, float eps,
                                               int lanes) {
   extern __shared__ int s_stack[];
-  trace_persistent<ANY, false, kQueryRefill>(b, n, cursor, eps, io, s_stack + threadIdx.x, kBlock, lanes);
+  trace_persistent<ANY, false, kQueryRefill, true>(b, n, cursor, eps, io, s_stack + threadIdx.x, kBlock, lanes);
 }
 
 template <bool FASTMM>
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kBlock, 16) k_extend(DevBVH b, DevQueues q, in
     atomicAdd(&q.stats[0], (unsigned long long)n);
   }
   ExtendIO io{q.org_q(qi), q.dir_q(qi), q.hit, q.error, q.perm};
-  trace_persistent<false, FASTMM, kExtendRefill>(b, n, q.counts + 4, eps, io, s_stack + threadIdx.x, kBlock);
+  trace_persistent<false, FASTMM, kExtendRefill, false>(b, n, q.counts + 4, eps, io, s_stack + threadIdx.x, kBlock);
 }
 
 // connect (src/CUDA/Kernel.cu:247-256): unoccluded shadow rays add their

@@ -104,11 +104,11 @@ __device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
                : "l"(p));
 }
 
-// 32 bytes as ldg256, by the lanes whose ref is an inner node's.
-__device__ __forceinline__ void ldg256_inner(int ref, const float4* p, float4& a, float4& b) {
-  asm volatile("{ .reg .pred q; setp.ge.s32 q, %9, 0; @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8]; }"
+// 32 bytes as ldg256, by the lanes whose ref is at least `least`.
+__device__ __forceinline__ void ldg256_from(int ref, int least, const float4* p, float4& a, float4& b) {
+  asm volatile("{ .reg .pred q; setp.ge.s32 q, %9, %10; @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8]; }"
                : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-               : "l"(p), "r"(ref));
+               : "l"(p), "r"(ref), "r"(least));
 }
 
 // What one ray step reads. Inner node: x planes (min, max of the four children), y
@@ -118,17 +118,24 @@ __device__ __forceinline__ void ldg256_inner(int ref, const float4* p, float4& a
 // last). With both whole records, 128 bytes, trees whose triangles don't stay in L2
 // waited for memory: 1 M rays, 4 M-triangle soup on the reference's tree, closest hit
 // 7.98 -> 7.07 ms, any hit 6.81 -> 4.42.
+// LONE: a leaf with one triangle left reads that one only. A leaf reference is negative
+// with its count above the first triangle's index, so one comparison tells. Where trees
+// lie in DRAM the second sector costs: 4 M rays, 10 M-triangle soup on the reference's
+// tree 43.6 -> 39.2 ms, any hit 35.4 -> 32.4 (with records of 48 bytes 42.8 and 33.9).
+// Frames, whose trees stay in L2, lose by the predicate (960x540 4.27 -> 4.34 ms).
 struct Fetch {
   float4 v0, v1, v2, v3, v4, v5, v6;
 };
+template <bool LONE>
 __device__ __forceinline__ void fetch(const DevBVH& b, int ref, Fetch& f) {
   const float4* p = ref >= 0 ? reinterpret_cast<const float4*>(b.nodes + ref)
                              : b.tris + kTriFloat4 * (size_t)((uint32_t)ref & b.first_mask);
   float4 unused;
   ldg256(p, f.v0, f.v1);
   ldg256(p + 2, f.v2, f.v3);
-  ldg256_inner(ref, p + 4, f.v4, f.v5);
-  ldg256(p + 6, f.v6, unused);
+  ldg256_from(ref, 0, p + 4, f.v4, f.v5);
+  if (LONE) ldg256_from(ref, (int)(0x80000000u + (2u << b.leaf_shift)), p + 6, f.v6, unused);
+  else ldg256(p + 6, f.v6, unused);
 }
 
 // Moller-Trumbore with the reference's absolute epsilon. Returns the new t
@@ -398,11 +405,11 @@ __device__ __forceinline__ StepResult leaf_step(const DevBVH& b, const Fetch& f,
 }
 
 // One step of a ray: an inner node or up to two triangles of a leaf.
-template <bool ANY, bool FASTMM>
+template <bool ANY, bool FASTMM, bool LONE = false>
 __device__ __forceinline__ StepResult ray_step(const DevBVH& b, RayState& r, float eps, int* stack, int stride,
                                                int limit) {
   Fetch f;
-  fetch(b, r.ref, f);
+  fetch<LONE>(b, r.ref, f);
   if (r.ref < 0) return leaf_step<ANY>(b, f, r, eps, stack, stride);
   if (ANY) return inner_step_any<FASTMM>(b, f, r, stack, stride, limit);
   return FASTMM ? inner_step_sorted(f, r, stack, stride, limit) : inner_step(b, f, r, stack, stride, limit);
@@ -435,7 +442,7 @@ __device__ __forceinline__ bool traverse(const DevBVH& b, RayState& r, float eps
 // only the interleaving across lanes changes.
 //   IO::load(int i, float4& org, float4& dir, float& t0)
 //   IO::store(int i, const RayState& r, bool overflow)
-template <bool ANY, bool FASTMM, int REFILL, class IO>
+template <bool ANY, bool FASTMM, int REFILL, bool LONE, class IO>
 __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cursor, float eps, IO& io, int* stack,
                                                  int stride, int lanes = 32) {
   const unsigned FULL = 0xffffffffu;
@@ -470,7 +477,7 @@ __device__ __forceinline__ void trace_persistent(const DevBVH& b, int n, int* cu
     }
     if (__ballot_sync(FULL, rid >= 0) == 0) break;
     if (rid < 0) continue;
-    const StepResult s = ray_step<ANY, FASTMM>(b, r, eps, stack, stride, limit);
+    const StepResult s = ray_step<ANY, FASTMM, LONE>(b, r, eps, stack, stride, limit);
     if (s != kContinue) {
       io.store(rid, r, s == kOverflow);
       rid = -1;
