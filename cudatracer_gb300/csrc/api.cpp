@@ -284,13 +284,12 @@ struct ct_bvh {
   ct_bvh_info info{};
   uint32_t nt = 0;
   Allocs allocs;
-  // device-built trees keep the reference-layout quad nodes and the primitive
-  // order on the device only (exported on request)
+  // device-built trees are on the device only: their nodes and the primitive order are
+  // read back when they are exported
   bool device_built = false;
   std::shared_ptr<BuildPool> pool;  // what allocs came from
   Allocs fence;                     // see free_tree
   int device = 0;
-  void* d_quad = nullptr;
   uint32_t* d_prims = nullptr;
   // 8-wide quantised tree (ct_bvh_build_wide): queries only
   bool wide = false;
@@ -809,16 +808,14 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   if (!enc.empty()) return cleanup(fail(ctx, CT_ERR_UNSUPPORTED, enc));
   // the tree's arrays, each 256-byte aligned, in one piece
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t quad_bytes = al((size_t)r.quad_nodes * sizeof(QuadNode));
   const size_t node_bytes = al((size_t)r.quad_nodes * sizeof(QNodeDev)), tri_bytes = al(tri_array_bytes(n));
-  void* quad = nullptr;
-  if ((s = pool_alloc(ctx, *b->pool, b->allocs, &quad, quad_bytes + node_bytes + tri_bytes + al((size_t)n * 4), st)) != CT_OK)
+  void* nodes = nullptr;
+  if ((s = pool_alloc(ctx, *b->pool, b->allocs, &nodes, node_bytes + tri_bytes + al((size_t)n * 4), st)) != CT_OK)
     return cleanup(s);
-  void* nodes = (char*)quad + quad_bytes;
   void* tris = (char*)nodes + node_bytes;
   void* prims = (char*)tris + tri_bytes;
-  e = fast ? gpu_fbvh_emit(scene->dev, scratch, r, shift, quad, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st)
-           : gpu_bvh_emit(scene->dev, scratch, r, shift, quad, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st);
+  e = fast ? gpu_fbvh_emit(scene->dev, scratch, r, shift, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st)
+           : gpu_bvh_emit(scene->dev, scratch, r, shift, (QNodeDev*)nodes, (float4*)tris, (uint32_t*)prims, st);
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "device BVH emit"));
   e = st ? cudaStreamSynchronize(st) : cudaDeviceSynchronize();
   if (e != cudaSuccess) return cleanup(cuda_fail(ctx, e, "device BVH build"));
@@ -830,7 +827,6 @@ ct_status build_device_quad(ct_ctx* ctx, const ct_scene* scene, void* stream, ct
   const auto t2 = std::chrono::high_resolution_clock::now();
   b->device_built = true;
   b->device = ctx->device;
-  b->d_quad = quad;
   b->d_prims = (uint32_t*)prims;
   b->dev.nodes = (const QNodeDev*)nodes;
   b->dev.tris = (const float4*)tris;
@@ -1044,6 +1040,24 @@ ct_status ct_bvh_info_get(const ct_bvh* bvh, ct_bvh_info* info) {
   return CT_OK;
 }
 
+// The QuadNode that a QNodeDev was made from, where it lies (at any alignment): the
+// planes are the same, childs and counts take the place of the references.
+static void quad_node(char* node, const DevBVH& b) {
+  static_assert(sizeof(QuadNode) == sizeof(QNodeDev) && offsetof(QuadNode, childs) == offsetof(QNodeDev, child) &&
+                    offsetof(QuadNode, bmaxz) == offsetof(QNodeDev, bmaxz),
+                "same planes");
+  int32_t ref[4], count[4];
+  std::memcpy(ref, node + offsetof(QNodeDev, child), sizeof(ref));
+  for (int c = 0; c < 4; c++) {
+    const uint32_t u = (uint32_t)ref[c];
+    if (ref[c] == kEmptyChild) count[c] = 0;  // childs -1 as well
+    else if (ref[c] >= 0) count[c] = -1;
+    else count[c] = (int32_t)((u >> b.leaf_shift) & b.count_mask), ref[c] = (int32_t)(u & b.first_mask);
+  }
+  std::memcpy(node + offsetof(QuadNode, childs), ref, sizeof(ref));
+  std::memcpy(node + offsetof(QuadNode, counts), count, sizeof(count));
+}
+
 ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, uint32_t* prim_indices) {
   if (!bvh) return CT_ERR_INVALID_ARGUMENT;
   if (bvh->wide) {
@@ -1076,9 +1090,12 @@ ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, ui
     if (layout == CT_BVH_BINARY) return nodes ? CT_ERR_UNSUPPORTED : CT_OK;
     if (layout != CT_BVH_QUAD) return CT_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(bvh->device) != cudaSuccess) return CT_ERR_CUDA;
-    if (nodes && cudaMemcpy(nodes, bvh->d_quad, (size_t)bvh->info.quad_node_count * sizeof(QuadNode),
-                            cudaMemcpyDeviceToHost) != cudaSuccess)
-      return CT_ERR_CUDA;
+    if (nodes) {
+      const size_t n = bvh->info.quad_node_count;
+      if (cudaMemcpy(nodes, bvh->dev.nodes, n * sizeof(QNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return CT_ERR_CUDA;
+      for (size_t i = 0; i < n; i++) quad_node((char*)nodes + i * sizeof(QNodeDev), bvh->dev);
+    }
     if (prim_indices &&
         cudaMemcpy(prim_indices, bvh->d_prims, (size_t)bvh->nt * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
       return CT_ERR_CUDA;

@@ -1194,25 +1194,18 @@ __global__ void k_qwrite(const BNode* __restrict__ arena, const uint32_t* counte
   if (at_idx < nq) quad[at_idx] = q;
 }
 
-__global__ void k_qdev(const QuadNode* __restrict__ quad, uint32_t nq, uint32_t shift, QNodeDev* out) {
+// Turns quad nodes into traversal nodes where they lie: the planes are the same, the
+// references take the place of childs and counts.
+__global__ void k_qdev(QNodeDev* nodes, uint32_t nq, uint32_t shift) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nq) return;
-  const QuadNode& s = quad[i];
-  QNodeDev d;
-  d.bminx = make_float4(s.bminx[0], s.bminx[1], s.bminx[2], s.bminx[3]);
-  d.bmaxx = make_float4(s.bmaxx[0], s.bmaxx[1], s.bmaxx[2], s.bmaxx[3]);
-  d.bminy = make_float4(s.bminy[0], s.bminy[1], s.bminy[2], s.bminy[3]);
-  d.bmaxy = make_float4(s.bmaxy[0], s.bmaxy[1], s.bmaxy[2], s.bmaxy[3]);
-  d.bminz = make_float4(s.bminz[0], s.bminz[1], s.bminz[2], s.bminz[3]);
-  d.bmaxz = make_float4(s.bmaxz[0], s.bmaxz[1], s.bmaxz[2], s.bmaxz[3]);
-  int32_t ref[4];
-  for (int c = 0; c < 4; c++) {
-    const int32_t cnt = s.counts[c], ch = s.childs[c];
-    ref[c] = cnt == -1 ? ch : (cnt > 0 ? (int32_t)(0x80000000u | ((uint32_t)cnt << shift) | (uint32_t)ch) : kEmptyChild);
-  }
-  d.child = make_int4(ref[0], ref[1], ref[2], ref[3]);
-  d.meta = make_int4(0, 0, 0, 0);
-  out[i] = d;
+  const int4 ch = nodes[i].child, cnt = nodes[i].meta;  // QuadNode: childs, counts
+  auto ref = [&](int32_t count, int32_t child) {
+    return count == -1 ? child
+                       : (count > 0 ? (int32_t)(0x80000000u | ((uint32_t)count << shift) | (uint32_t)child) : kEmptyChild);
+  };
+  nodes[i].child = make_int4(ref(cnt.x, ch.x), ref(cnt.y, ch.y), ref(cnt.z, ch.z), ref(cnt.w, ch.w));
+  nodes[i].meta = make_int4(0, 0, 0, 0);
 }
 
 __global__ void k_tris(const float4* __restrict__ v, const uint4* __restrict__ idx, const uint32_t* __restrict__ prims,
@@ -1357,8 +1350,8 @@ cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_coun
   return cudaSuccess;
 }
 
-cudaError_t launch_quad_to_dev(const QuadNode* quad, uint32_t nq, uint32_t leaf_shift, QNodeDev* nodes, cudaStream_t s) {
-  if (nq) k_qdev<<<blocks(nq, 256), 256, 0, s>>>(quad, nq, leaf_shift, nodes);
+cudaError_t launch_quad_to_dev(QNodeDev* nodes, uint32_t nq, uint32_t leaf_shift, cudaStream_t s) {
+  if (nq) k_qdev<<<blocks(nq, 256), 256, 0, s>>>(nodes, nq, leaf_shift);
   return cudaGetLastError();
 }
 
@@ -1367,17 +1360,17 @@ cudaError_t launch_leaf_tris(const DevScene& sc, const uint32_t* prims, uint32_t
   return cudaGetLastError();
 }
 
-cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift, void* quad_out,
-                         QNodeDev* nodes, float4* tris, uint32_t* prims_out, cudaStream_t s) {
+cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift, QNodeDev* nodes,
+                         float4* tris, uint32_t* prims_out, cudaStream_t s) {
   const uint32_t n = sc.tri_count;
   const Layout L(n);
   const uint32_t* counters = at<uint32_t>(scratch, L.counters);
   const BNode* arena = at<BNode>(scratch, L.arena);
   const uint32_t* qidx = at<uint32_t>(scratch, L.qidx);
   const uint32_t* prims = at<uint32_t>(scratch, L.prims);
-  QuadNode* quad = static_cast<QuadNode*>(quad_out);
-  k_qwrite<<<blocks(r.binary_nodes, 256), 256, 0, s>>>(arena, counters, qidx, r.quad_nodes, quad);
-  k_qdev<<<blocks(r.quad_nodes, 256), 256, 0, s>>>(quad, r.quad_nodes, leaf_shift, nodes);
+  k_qwrite<<<blocks(r.binary_nodes, 256), 256, 0, s>>>(arena, counters, qidx, r.quad_nodes,
+                                                       reinterpret_cast<QuadNode*>(nodes));
+  k_qdev<<<blocks(r.quad_nodes, 256), 256, 0, s>>>(nodes, r.quad_nodes, leaf_shift);
   k_tris<<<blocks(n, 256), 256, 0, s>>>(sc.verts, sc.idx, prims, n, tris);
   GB_TRY(cudaGetLastError());
   GB_TRY(cudaMemcpyAsync(prims_out, prims, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));

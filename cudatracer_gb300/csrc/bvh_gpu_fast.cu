@@ -1976,18 +1976,18 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* hc, cuda
 }
 
 cudaError_t gpu_fbvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift,
-                          void* quad_out, QNodeDev* nodes, float4* tris, uint32_t* prims_out, cudaStream_t s) {
+                          QNodeDev* nodes, float4* tris, uint32_t* prims_out, cudaStream_t s) {
   const uint32_t n = sc.tri_count;
   const Layout Lo(n);
   uint32_t* counters = at<uint32_t>(scratch, Lo.counters);
   const FNodeD* arena = at<FNodeD>(scratch, Lo.arena);
   const QRec* qrec = at<QRec>(scratch, Lo.qrec);
   const uint32_t* prims = at<uint32_t>(scratch, Lo.prims);
-  QuadNode* quad = static_cast<QuadNode*>(quad_out);
+  QuadNode* quad = reinterpret_cast<QuadNode*>(nodes);  // until launch_quad_to_dev
   if (n == 1) k_fqsingle<<<1, 1, 0, s>>>(arena, quad, counters);
   else k_fqwrite<<<blocks(r.quad_nodes, 256), 256, 0, s>>>(arena, qrec, r.quad_nodes, quad, counters);
   FB_TRY(cudaGetLastError());
-  FB_TRY(launch_quad_to_dev(quad, r.quad_nodes, leaf_shift, nodes, s));
+  FB_TRY(launch_quad_to_dev(nodes, r.quad_nodes, leaf_shift, s));
   FB_TRY(launch_leaf_tris(sc, prims, n, tris, s));
   return cudaMemcpyAsync(prims_out, prims, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
 }

@@ -254,24 +254,23 @@ cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q,
 cudaError_t launch_present(const float4* accum, float4* out, int n, float samples, cudaStream_t s);
 // Device SAH build (bvh_gpu.cu). gpu_bvh_build runs the binary build and the
 // collapse bookkeeping in `scratch` (gpu_bvh_scratch_bytes) and returns the
-// sizes; gpu_bvh_emit then writes the reference-layout quad nodes (QuadNode,
-// pre-order), the traversal nodes, the leaf-ordered triangles and the
-// primitive order into buffers of those sizes. host_counters: 16 words of
-// pinned host memory. Both return after their work is queued on `s`; build
-// synchronises with `s` once per level to read the level's node count.
+// sizes; gpu_bvh_emit then writes the traversal nodes (in the reference's pre-order),
+// the leaf-ordered triangles and the primitive order into buffers of those sizes.
+// host_counters: 32 words of pinned host memory. Both return after their work is
+// queued on `s`; build synchronises with `s` once per few levels to read counters.
 struct GpuBvhResult {
   uint32_t binary_nodes = 0, quad_nodes = 0, max_leaf = 0, depth = 0;
   uint32_t error = 0;  // 1 degenerate extent, 2 arena, 4 stack, 8 partition mismatch
 };
 size_t gpu_bvh_scratch_bytes(uint32_t n);
 cudaError_t gpu_bvh_build(const DevScene& sc, void* scratch, uint32_t* host_counters, cudaStream_t s, GpuBvhResult& r);
-cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift, void* quad,
-                         QNodeDev* nodes, float4* tris, uint32_t* prims, cudaStream_t s);
+cudaError_t gpu_bvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift, QNodeDev* nodes,
+                         float4* tris, uint32_t* prims, cudaStream_t s);
 
-struct QuadNode;  // bvh_build.h
-// QuadNode -> traversal node conversion, and the leaf-ordered triangle records
-// (kTriFloat4 float4 per primitive), for trees built on the device.
-cudaError_t launch_quad_to_dev(const QuadNode* quad, uint32_t nq, uint32_t leaf_shift, QNodeDev* nodes, cudaStream_t s);
+// For trees built on the device: QuadNode records (bvh_build.h) made traversal nodes in
+// place (the two have the same planes; quad_node, api.cpp, is the way back), and the
+// leaf-ordered triangle records (kTriFloat4 float4 per primitive).
+cudaError_t launch_quad_to_dev(QNodeDev* nodes, uint32_t nq, uint32_t leaf_shift, cudaStream_t s);
 cudaError_t launch_leaf_tris(const DevScene& sc, const uint32_t* prims, uint32_t n, float4* tris, cudaStream_t s);
 
 // Cost table of the 8-wide collapse (gpu_fbvh_build with wide = 1): C(n, i),
@@ -291,8 +290,8 @@ static_assert(sizeof(WideCost) == 48, "WideCost");
 // host build: gpu_fbvh_build fills `scratch` (gpu_fbvh_scratch_bytes) and
 // returns the sizes (r.error: 1 a padded box is not finite, 2 capacity, 4
 // stack, 8 partition mismatch, 16 collapse); gpu_fbvh_emit writes the quad
-// nodes, traversal nodes, triangles and primitive order. host_counters: 16
-// words of pinned host memory; the build synchronises with `s` once per level.
+// nodes as traversal nodes, triangles and primitive order. host_counters: 32
+// words of pinned host memory; the build synchronises with `s` once per few levels.
 // wide = 1: the binary tree of the same rules over exact triangle bounds, then
 // the 8-wide cost table instead of the quad collapse (for gpu_wbvh_collapse;
 // gpu_fbvh_binary gives the arena, primitive order and table).
@@ -301,7 +300,7 @@ cudaError_t gpu_fbvh_build(const DevScene& sc, void* scratch, uint32_t* host_cou
                            int wide = 0);
 void gpu_fbvh_binary(void* scratch, uint32_t n, int wide, const void** arena, const uint32_t** prims,
                      const WideCost** cost);
-cudaError_t gpu_fbvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift, void* quad,
+cudaError_t gpu_fbvh_emit(const DevScene& sc, void* scratch, const GpuBvhResult& r, uint32_t leaf_shift,
                           QNodeDev* nodes, float4* tris, uint32_t* prims, cudaStream_t s);
 // error word of the last emit (reads the counters back; synchronises with `s`)
 uint32_t gpu_fbvh_error(void* scratch, uint32_t n, uint32_t* host_counters, cudaStream_t s);

@@ -33,7 +33,7 @@ def test_trees_destroyed_through_another_context_leave_the_bound(lib):
     a, b = api.Context(0), api.Context(0)
     sc = _scene(a, 1000000)
     before = _free()
-    trees = [sc.build_bvh_fast_device() for _ in range(10)]
+    trees = [sc.build_bvh_fast_device() for _ in range(16)]
     held = sum(t.info()["device_bytes"] for t in trees)
     assert held > 3 * GIB // 2
     for t in trees:
@@ -136,4 +136,30 @@ def test_a_budget_of_zero_gives_back_what_is_kept(gpu_ctx):
     assert before - _free() > 128 << 20
     gpu_ctx.set_memory_budget(0)
     assert before - _free() < 64 << 20
+    sc.close()
+
+
+# Scratch of a build of 20,000 triangles when the nodes were held twice and a triangle
+# record was 48 bytes: what a budget admitted then it still admits.
+SCRATCH = {"build_bvh_device": 3214336, "build_bvh_fast_device": 6187520}
+
+
+@pytest.mark.parametrize("kind", SCRATCH)
+@pytest.mark.parametrize("scene", ["soup", "terrain"])
+def test_a_budget_admits_what_it_did(gpu_ctx, kind, scene):
+    from cudatracer_gb300 import api, scenes
+
+    n = 20000
+    s = scenes.soup_scene(n) if scene == "soup" else scenes.terrain_scene(grid=101, spheres=0)[0]
+    sc = gpu_ctx.scene({"vertices": s.vertices, "normals": s.normals, "indices": s.indices[:n]}, [api.Material()])
+    tree = getattr(sc, kind)()
+    nodes, held = tree.info()["quad_node_count"], tree.info()["device_bytes"]
+    tree.close()
+    was = 2 * 128 * nodes + 48 * n + 4 * n
+    assert held <= was
+    gpu_ctx.set_memory_budget(gpu_ctx.device_bytes + SCRATCH[kind] + was)
+    try:
+        getattr(sc, kind)().close()
+    finally:
+        gpu_ctx.set_memory_budget(0)
     sc.close()
