@@ -45,21 +45,23 @@ constexpr int kBinFields = 7;  // count, min key x/y/z, max key x/y/z
 constexpr int kBinWords = 3 * kIntervals * kBinFields;
 constexpr uint32_t kWarpMax = 128;  // nodes up to this size are built by one warp
 // Nodes up to this size are split by one block down to those (64 KB of shared memory
-// leave three blocks of 2,048 on an SM and six of 1,024).
-inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
-// Builds of at most this many triangles leave an SM at most one such block, which has
-// 512 threads then instead of 256: 20,480 triangles 511 -> 487 us, 2.0 M with 512
-// 2.93 -> 3.32 ms.
-constexpr uint32_t kFewMid = 100000;
+// leave three blocks of 2,048 on an SM and six of 1,024). Terrains with 2,048 and with
+// 1,024, ms: 486,000 triangles 1.22 and 1.22, 864,000 1.74 and 1.69, 1.5 M 2.53 and 2.48.
+inline uint32_t mid_size(uint32_t n) { return n > 400000 ? 1024 : 2048; }
+// Builds of at most this many triangles leave an SM about one such block, which has 512
+// threads then instead of 256. Terrains with 256 and with 512 threads, us: 122,000
+// triangles 836 and 820, 231,000 977 and 960, 302,000 1,029 and 1,046, 602,000 1,406 and
+// 1,508.
+constexpr uint32_t kFewMid = 250000;
 constexpr uint32_t kLeafTask = 16;  // subtrees up to this size are built by one thread
 // Primitives per block of the level kernels: the fewest, as a power of two from
-// 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
-// of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
+// 256, that leave no more blocks than about one wave holds (8 blocks of 256 threads
+// on each SM). A 20,480-triangle build has 80 blocks of one pass over
 // their threads rather than 10 of eight (k_bin 18 -> 8 us a level); above 1.2 M
 // triangles the 2,048 of one wave stay (fewer bin flushes).
 inline uint32_t chunk_size(uint32_t n) {
   uint32_t c = 256;
-  while (c < 2048 && n / c > 152 * 8) c *= 2;
+  while (c < 2048 && n / c > (uint32_t)sm_count() * 8) c *= 2;
   return c;
 }
 constexpr int32_t kMaxSplitDepth = 61;

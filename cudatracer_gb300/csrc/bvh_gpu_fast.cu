@@ -54,22 +54,24 @@ constexpr int32_t kDepthLimit = 60;
 constexpr float kPad = 1e-5f;
 constexpr uint32_t kSweepMax = 16;
 constexpr uint32_t kWarpMax = 128;   // subtrees up to this size: one warp
-// Nodes up to this size are split by one block down to those. 64 KB of shared memory
-// leave three blocks of 2,048 on an SM and six of 1,024: 20,480 triangles build in 671
-// against 723 us, 2.0 M in 3.68 against 3.60 ms.
-inline uint32_t mid_size(uint32_t n) { return n > 1000000 ? 1024 : 2048; }
-// Builds of at most this many triangles leave an SM at most one such block, which has
-// 512 threads then instead of 256: 20,480 triangles 730 -> 700 us, 2.0 M with 512
-// 3.58 -> 3.74 ms.
-constexpr uint32_t kFewMid = 100000;
+// Nodes up to this size are split by one block down to those (64 KB of shared memory
+// leave three blocks of 2,048 on an SM and six of 1,024). Soups with 2,048 and with 1,024,
+// ms: 300,000 triangles 1.32 and 1.29, 1.1 M 2.54 and 2.50, 2.0 M 3.87 and 3.79; a terrain
+// of 486,000 1.66 and 1.65.
+inline uint32_t mid_size(uint32_t n) { return n > 400000 ? 1024 : 2048; }
+// Builds of at most this many triangles leave an SM about one such block, which has 512
+// threads then instead of 256. Terrains with 256 and with 512 threads, us: 122,000
+// triangles 1,216 and 1,202, 231,000 1,354 and 1,335, 421,000 1,598 and 1,583, 602,000
+// 1,918 and 1,972.
+constexpr uint32_t kFewMid = 250000;
 // Primitives per block of the level kernels: the fewest, as a power of two from
-// 256, that leave no more blocks than about one wave on 152 SMs holds (8 blocks
-// of 256 threads each). A 20,480-triangle build has 80 blocks of one pass over
+// 256, that leave no more blocks than about one wave holds (8 blocks of 256 threads
+// on each SM). A 20,480-triangle build has 80 blocks of one pass over
 // their threads rather than 10 of eight (k_fbin 18 -> 8 us a level); above 1.2 M
 // triangles the 2,048 of one wave stay (fewer bin flushes).
 inline uint32_t chunk_size(uint32_t n) {
   uint32_t c = 256;
-  while (c < 2048 && n / c > 152 * 8) c *= 2;
+  while (c < 2048 && n / c > (uint32_t)sm_count() * 8) c *= 2;
   return c;
 }
 constexpr int kSmallWarps = 4;
