@@ -237,8 +237,6 @@ cudaError_t launch_connect(const DevBVH& b, const DevQueues& q, float eps, bool 
 cudaError_t launch_raygen(const DevQueues& q, const FrameConst& f, int exact, cudaStream_t s);
 cudaError_t launch_shade(const DevScene& sc, const DevQueues& q, const FrameConst& f, int queue, int path_length,
                          int exact, cudaStream_t s);
-// A whole frame in one kernel on a quad tree (frames of few pixels): as raygen and
-// max_depth x (extend, shade, connect if f.shadow) into the same q.accum or q.log.
 // How many lanes of a warp take rays (or paths) when a call has n of them: a
 // small call is as long as its longest ray, and a warp's round is shorter the
 // fewer rays share it (fewer lines to fetch, seldom a node and a leaf in one round),
@@ -249,6 +247,8 @@ cudaError_t launch_shade(const DevScene& sc, const DevQueues& q, const FrameCons
 // with 32, 99 with 4; a 16x16 frame 161 with 32, 100 with 1.
 inline int lanes_for(uint32_t n) { return (int)std::min<uint32_t>(32, (n - 1) / 768 + 1); }
 
+// A whole frame in one kernel on a quad tree (frames of few pixels): as raygen and
+// max_depth x (extend, shade, connect if f.shadow) into the same q.accum or q.log.
 cudaError_t launch_path(const DevScene& sc, const DevBVH& b, const DevQueues& q, const FrameConst& f, int max_depth,
                         int exact_math, bool fast_traversal, cudaStream_t s);
 cudaError_t launch_present(const float4* accum, float4* out, int n, float samples, cudaStream_t s);

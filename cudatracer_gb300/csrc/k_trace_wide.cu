@@ -370,8 +370,8 @@ struct WStack {
 // triangles: 1.04 -> 0.80 ms. Lanes that wait until eight are at a leaf gain 3 %
 // there and lose 10 % on small calls; they don't wait.
 //   counters[0]  ray fetch cursor;  counters[1]  records written
-template <bool ANY>
 // 8 resident blocks of 128 threads per SM (64 registers): measured ahead of 6 (80 registers)
+template <bool ANY>
 __global__ void __launch_bounds__(128, 8) k_trace_wide(const DevWBVH b, const float4* __restrict__ org,
                                                     const float4* __restrict__ dir, int32_t* __restrict__ hit_out,
                                                     float* __restrict__ t_out, uint8_t* __restrict__ occ_out,

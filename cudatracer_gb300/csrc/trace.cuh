@@ -177,7 +177,9 @@ struct RayState {
 };
 
 // A slab term is NaN only as 0 * inf, inf - inf or from a NaN input: never for a
-// finite origin and finite reciprocals on finite planes.
+// finite origin and finite reciprocals on finite planes. (An infinite direction component
+// has the reciprocal 0, which a plane distance that overflows could meet; such a ray hits
+// no triangle whatever the boxes say.)
 __device__ __forceinline__ void ray_begin(const DevBVH& b, RayState& r, float4 o, float4 d, float t0) {
   r.ox = o.x, r.oy = o.y, r.oz = o.z, r.dx = d.x, r.dy = d.y, r.dz = d.z;
   r.ix = __frcp_rn(d.x), r.iy = __frcp_rn(d.y), r.iz = __frcp_rn(d.z);

@@ -175,7 +175,8 @@ typedef struct ct_render_params {
   float dist_eps;        /* SceneData::distEpsilon */
   float tri_eps;         /* SceneData::triangleEpsilon */
   int32_t texture_filter; /* CT_TEX_NEAREST (reference) or CT_TEX_BILINEAR */
-  int32_t ray_sort;      /* CT_SORT_*: order of bounce rays before closest-hit traversal (no result changes) */
+  int32_t ray_sort;      /* CT_SORT_*: order of bounce rays before closest-hit traversal (no result changes; frames
+                            of few pixels on a quad tree run as one kernel, which has no queue to sort) */
 } ct_render_params;
 
 typedef struct ct_frame_stats {
@@ -491,9 +492,11 @@ ct_status ct_render_stats(ct_ctx* ctx, ct_render* r, ct_frame_stats* stats, int3
  * build times only, src/BVH/BVHTree.cpp:53): when enabled, every stage launch
  * of ct_render_accumulate is bracketed by CUDA events on its stream, and
  * fast-math frames run one after another on the caller's stream (no frames in
- * flight), so each interval is one kernel running alone. Reading synchronises
- * on the recorded events. Stage index: 0 raygen, 1 extend (closest hit),
- * 2 shade, 3 connect (shadow any hit). */
+ * flight), so each interval is one kernel running alone. Frames of up to 81,920
+ * pixels on a quad tree (131,072 with CT_MATH_EXACT), which otherwise run as one
+ * kernel, run their stages when enabled: the same contributions, other kernels. Reading
+ * synchronises on the recorded events. Stage index: 0 raygen, 1 extend (closest
+ * hit), 2 shade, 3 connect (shadow any hit). */
 typedef struct ct_stage_times {
   double ms[4];
   uint32_t launches[4];
