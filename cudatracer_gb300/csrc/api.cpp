@@ -32,6 +32,7 @@ struct BuildPool {
   cudaStream_t st = nullptr;  // destroyed trees' memory is freed on it
   std::mutex mu;
   uint64_t live = 0;  // bytes of it in use (guarded by mu)
+  std::atomic<bool> keep{true};  // false: its context has a budget, idle memory is given back at once
   ~BuildPool() {
     if (pool) cudaMemPoolDestroy(pool);
     if (st) cudaStreamDestroy(st);
@@ -146,6 +147,7 @@ ct_status build_pool(ct_ctx* ctx, std::shared_ptr<BuildPool>& out) {
       ctx->err = std::string("build pool: ") + cudaGetErrorString(e);
       return e == cudaErrorMemoryAllocation ? CT_ERR_OUT_OF_MEMORY : CT_ERR_CUDA;
     }
+    p->keep = ctx->budget == 0;
     ctx->pool = std::move(p);
   }
   out = ctx->pool;
@@ -189,7 +191,7 @@ void pool_free(ct_ctx* ctx, BuildPool& pool, Allocs& a, cudaStream_t st) {
     uint64_t keep = pool.live + kPoolKeepBytes;
     cudaMemPoolSetAttribute(pool.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
-  if (ctx->budget) {
+  if (!pool.keep) {
     cudaStreamSynchronize(st);
     cudaMemPoolTrimTo(pool.pool, 0);
   }
@@ -213,6 +215,23 @@ void free_tree(ct_ctx* ctx, BuildPool& pool, Allocs& fence, Allocs& a) {
   cudaGetLastError();
   for (auto& p : a.list) ctx->bytes -= p.second;
   a.list.clear();
+}
+
+// run(tmp, stream) with `bytes` of the pool in tmp, or with nullptr where they are not to
+// be had. On the pool's own stream: also while another stream is being captured.
+template <class Run>
+cudaError_t export_pooled(BuildPool& pool, size_t bytes, Run&& run) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  void* tmp = nullptr;
+  if (cudaMallocFromPoolAsync(&tmp, bytes, pool.pool, pool.st) != cudaSuccess) cudaGetLastError(), tmp = nullptr;
+  const cudaError_t e = run(tmp, pool.st);
+  if (tmp) {
+    cudaFreeAsync(tmp, pool.st);
+    if (!pool.keep) cudaStreamSynchronize(pool.st), cudaMemPoolTrimTo(pool.pool, 0);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e;
 }
 
 // A pinned block of kPinnedBytes for one build's counters (nullptr: none to be had).
@@ -537,6 +556,10 @@ const char* ct_last_error(const ct_ctx* ctx) {
 ct_status ct_ctx_set_memory_budget(ct_ctx* ctx, uint64_t bytes) {
   if (!ctx) return CT_ERR_INVALID_ARGUMENT;
   ctx->budget = bytes;
+  {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    if (ctx->pool) ctx->pool->keep = bytes == 0;
+  }
   trim_pool(ctx);
   return CT_OK;
 }
@@ -1040,43 +1063,15 @@ ct_status ct_bvh_info_get(const ct_bvh* bvh, ct_bvh_info* info) {
   return CT_OK;
 }
 
-// The QuadNode that a QNodeDev was made from, where it lies (at any alignment): the
-// planes are the same, childs and counts take the place of the references.
-static void quad_node(char* node, const DevBVH& b) {
-  static_assert(sizeof(QuadNode) == sizeof(QNodeDev) && offsetof(QuadNode, childs) == offsetof(QNodeDev, child) &&
-                    offsetof(QuadNode, bmaxz) == offsetof(QNodeDev, bmaxz),
-                "same planes");
-  int32_t ref[4], count[4];
-  std::memcpy(ref, node + offsetof(QNodeDev, child), sizeof(ref));
-  for (int c = 0; c < 4; c++) {
-    const uint32_t u = (uint32_t)ref[c];
-    if (ref[c] == kEmptyChild) count[c] = 0;  // childs -1 as well
-    else if (ref[c] >= 0) count[c] = -1;
-    else count[c] = (int32_t)((u >> b.leaf_shift) & b.count_mask), ref[c] = (int32_t)(u & b.first_mask);
-  }
-  std::memcpy(node + offsetof(QuadNode, childs), ref, sizeof(ref));
-  std::memcpy(node + offsetof(QuadNode, counts), count, sizeof(count));
-}
-
 ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, uint32_t* prim_indices) {
   if (!bvh) return CT_ERR_INVALID_ARGUMENT;
   if (bvh->wide) {
     if (layout != CT_BVH_WIDE8_Q8) return nodes ? CT_ERR_UNSUPPORTED : CT_OK;
     if (cudaSetDevice(bvh->device) != cudaSuccess) return CT_ERR_CUDA;
-    if (nodes) {
-      const size_t n = bvh->wdev.node_count, piece = std::min<size_t>(n, 65536);
-      std::unique_ptr<WNodeDev[]> dev(new (std::nothrow) WNodeDev[piece]);
-      if (!dev) return CT_ERR_OUT_OF_MEMORY;
-      for (size_t i0 = 0; i0 < n; i0 += piece) {
-        const size_t c = std::min(piece, n - i0);
-        if (cudaMemcpy(dev.get(), bvh->wdev.nodes + i0, c * sizeof(WNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
-          return CT_ERR_CUDA;
-        for (size_t i = 0; i < c; i++) {
-          const WNode8 w = wide_node8(dev[i]);
-          std::memcpy((char*)nodes + (i0 + i) * sizeof(w), &w, sizeof(w));
-        }
-      }
-    }
+    if (nodes && export_pooled(*bvh->pool, std::min(bvh->wdev.node_count, kExportPiece) * sizeof(WNode8),
+                               [&](void* tmp, cudaStream_t on) { return export_wides(bvh->wdev, nodes, tmp, on); }) !=
+                     cudaSuccess)
+      return CT_ERR_CUDA;
     if (prim_indices) {
       std::vector<float4> tri((size_t)bvh->nt * 3);
       if (cudaMemcpy(tri.data(), bvh->wdev.tris, tri.size() * sizeof(float4), cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -1090,12 +1085,10 @@ ct_status ct_bvh_export(const ct_bvh* bvh, ct_bvh_layout layout, void* nodes, ui
     if (layout == CT_BVH_BINARY) return nodes ? CT_ERR_UNSUPPORTED : CT_OK;
     if (layout != CT_BVH_QUAD) return CT_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(bvh->device) != cudaSuccess) return CT_ERR_CUDA;
-    if (nodes) {
-      const size_t n = bvh->info.quad_node_count;
-      if (cudaMemcpy(nodes, bvh->dev.nodes, n * sizeof(QNodeDev), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return CT_ERR_CUDA;
-      for (size_t i = 0; i < n; i++) quad_node((char*)nodes + i * sizeof(QNodeDev), bvh->dev);
-    }
+    if (nodes && export_pooled(*bvh->pool, std::min(bvh->dev.node_count, kExportPiece) * sizeof(QuadNode),
+                               [&](void* tmp, cudaStream_t on) { return export_quads(bvh->dev, nodes, tmp, on); }) !=
+                     cudaSuccess)
+      return CT_ERR_CUDA;
     if (prim_indices &&
         cudaMemcpy(prim_indices, bvh->d_prims, (size_t)bvh->nt * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
       return CT_ERR_CUDA;

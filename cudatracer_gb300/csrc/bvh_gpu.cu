@@ -30,7 +30,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
+#include <memory>
+#include <new>
 
 #include "bvh_build.h"
 #include "ct_internal.h"
@@ -1642,29 +1645,98 @@ cudaError_t gpu_wbvh_copy_nodes(void* scratch2, uint32_t binary_nodes, WNodeDev*
   return cudaGetLastError();
 }
 
-WNode8 wide_node8(const WNodeDev& d) {
-  WNode8 w;
-  std::memset(&w, 0, sizeof(w));
-  w.px = d.p[0], w.py = d.p[1], w.pz = d.p[2];
-  w.imask = d.imask;
-  for (int a = 0; a < 3; a++) {
-    w.e[a] = d.e[a];
-    for (int k = 0; k < 8; k++) w.qlo[a][k] = d.q[a][0][k], w.qhi[a][k] = d.q[a][1][k];
+namespace {
+// The QuadNode a QNodeDev was made from: the planes are the same, childs and counts
+// take the place of the references.
+struct QuadOut {
+  using In = QNodeDev;
+  using Out = QuadNode;
+  uint32_t shift, first_mask, count_mask;
+  __host__ __device__ QuadNode operator()(const QNodeDev& d) const {
+    static_assert(sizeof(QuadNode) == sizeof(QNodeDev) && offsetof(QuadNode, childs) == offsetof(QNodeDev, child) &&
+                      offsetof(QuadNode, bmaxz) == offsetof(QNodeDev, bmaxz),
+                  "same planes");
+    QuadNode q;
+    memcpy(&q, &d, sizeof(q));
+    for (int c = 0; c < 4; c++) {
+      const int32_t ref = q.childs[c];
+      if (ref == kEmptyChild) q.counts[c] = 0;  // childs -1 as well
+      else if (ref >= 0) q.counts[c] = -1;
+      else q.counts[c] = (int32_t)(((uint32_t)ref >> shift) & count_mask), q.childs[c] = ref & (int32_t)first_mask;
+    }
+    return q;
   }
-  // children and triangles are numbered in slot order from the node's first ones
-  bool child = false, prim = false;
-  for (int k = 0; k < 8; k++) {
-    const uint32_t ent = d.ent[k];
-    if (ent == 0) continue;
-    if (ent & 0x80000000u) {
-      const uint32_t first = ent & 0x1fffffffu;
-      if (!prim) w.prim_base = first, prim = true;
-      w.meta[k] = (uint8_t)((((ent >> 29) & 3u) << 5) | (first - w.prim_base));
-    } else {
-      if (!child) w.child_base = ent, child = true;
-      w.meta[k] = (uint8_t)(0x80u | (ent - w.child_base));
+};
+
+// The 80-byte node a WNodeDev was made from.
+struct WideOut {
+  using In = WNodeDev;
+  using Out = WNode8;
+  __host__ __device__ WNode8 operator()(const WNodeDev& d) const {
+    WNode8 w;
+    memset(&w, 0, sizeof(w));
+    w.px = d.p[0], w.py = d.p[1], w.pz = d.p[2];
+    w.imask = d.imask;
+    for (int a = 0; a < 3; a++) {
+      w.e[a] = d.e[a];
+      for (int k = 0; k < 8; k++) w.qlo[a][k] = d.q[a][0][k], w.qhi[a][k] = d.q[a][1][k];
+    }
+    // children and triangles are numbered in slot order from the node's first ones
+    bool child = false, prim = false;
+    for (int k = 0; k < 8; k++) {
+      const uint32_t ent = d.ent[k];
+      if (ent == 0) continue;
+      if (ent & 0x80000000u) {
+        const uint32_t first = ent & 0x1fffffffu;
+        if (!prim) w.prim_base = first, prim = true;
+        w.meta[k] = (uint8_t)((((ent >> 29) & 3u) << 5) | (first - w.prim_base));
+      } else {
+        if (!child) w.child_base = ent, child = true;
+        w.meta[k] = (uint8_t)(0x80u | (ent - w.child_base));
+      }
+    }
+    return w;
+  }
+};
+
+template <class F>
+__global__ void __launch_bounds__(256) k_export(F f, const typename F::In* __restrict__ in, uint32_t n,
+                                                typename F::Out* out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = f(in[i]);
+}
+
+template <class F>
+cudaError_t export_nodes(F f, const typename F::In* nodes, uint32_t n, void* to, void* tmp, cudaStream_t s) {
+  using In = typename F::In;
+  using Out = typename F::Out;
+  std::unique_ptr<In[]> host(tmp ? nullptr : new (std::nothrow) In[std::min(n, kExportPiece)]);
+  if (!tmp && !host) return cudaErrorMemoryAllocation;
+  for (uint32_t i = 0; i < n; i += kExportPiece) {
+    const uint32_t c = std::min(n - i, kExportPiece);
+    char* dst = (char*)to + (size_t)i * sizeof(Out);
+    if (tmp) {
+      k_export<F><<<blocks(c, 256), 256, 0, s>>>(f, nodes + i, c, (Out*)tmp);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    cudaError_t e = tmp ? cudaMemcpyAsync(dst, tmp, c * sizeof(Out), cudaMemcpyDeviceToHost, s)
+                        : cudaMemcpyAsync(host.get(), nodes + i, c * sizeof(In), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && !tmp) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    for (uint32_t j = 0; !tmp && j < c; j++) {
+      const Out o = f(host[j]);
+      std::memcpy(dst + j * sizeof(Out), &o, sizeof(Out));  // at any alignment
     }
   }
-  return w;
+  return cudaStreamSynchronize(s);
+}
+}  // namespace
+
+cudaError_t export_quads(const DevBVH& b, void* to, void* tmp, cudaStream_t s) {
+  return export_nodes(QuadOut{b.leaf_shift, b.first_mask, b.count_mask}, b.nodes, b.node_count, to, tmp, s);
+}
+cudaError_t export_wides(const DevWBVH& b, void* to, void* tmp, cudaStream_t s) {
+  return export_nodes(WideOut{}, b.nodes, b.node_count, to, tmp, s);
 }
 }  // namespace ct
